@@ -409,46 +409,61 @@ __global__ void __launch_bounds__(128) k_nl_query(const float2* __restrict__ qpo
   if (!kFill) counts[b] = cnt;
 }
 
-// One thread per original particle i: its row of the (i, j)-ordered COO list, plus the
+// One warp per original particle i: its row of the (i, j)-ordered COO list, plus the
 // reference's fluidDistances / fluidRadialDistances (src/modules/neighborSearch.py:218-223).
-__global__ void k_nl_to_coo(const float2* __restrict__ xy, int64_t n, const uint32_t* __restrict__ order,
-                            const uint32_t* __restrict__ rank, const int32_t* __restrict__ offsets,
-                            const int32_t* __restrict__ cols, const int64_t* __restrict__ orig_offsets,
-                            float thr, float support, int64_t* __restrict__ pairs, int64_t P,
-                            float* __restrict__ dist, float* __restrict__ radial) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// A lane holds one pair; its place in the row is the number of the row's columns below its
+// own (they are distinct), counted over the warp's registers 32 columns at a time, so rows of
+// any length sort without scratch.  The lanes' columns are loaded, and the row's four outputs
+// stored, as contiguous pieces, where one thread per row moved every column through global
+// memory once per inversion: 558 -> 103 us for 260,017 particles, 7.2 M pairs (201 MB of
+// pairs and distances stored).  Bound by instruction issue (81 % of the slots): the count,
+// and the correctly rounded root and divisions.  Tiles in shared memory instead of shuffles
+// gave the same time.
+__global__ void __launch_bounds__(256) k_nl_to_coo(const float2* __restrict__ xy, int64_t n,
+                                                   const uint32_t* __restrict__ order,
+                                                   const uint32_t* __restrict__ rank,
+                                                   const int32_t* __restrict__ offsets,
+                                                   const int32_t* __restrict__ cols,
+                                                   const int64_t* __restrict__ orig_offsets, float thr, float support,
+                                                   int64_t* __restrict__ pairs, int64_t P, float* __restrict__ dist,
+                                                   float* __restrict__ radial) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   if (i >= n) return;
   const uint32_t s = rank[i];
-  const int32_t b = offsets[s], e = offsets[s + 1];
+  const int32_t b = offsets[s], m = offsets[s + 1] - b;
   const int64_t o = orig_offsets[i];
   int64_t* prow = pairs;
   int64_t* pcol = pairs + P;
-  for (int k = b; k < e; ++k) {  // insertion sort by original column index
-    int64_t jo = (int64_t)order[cols[k]];
-    int64_t t = o + (k - b);
-    while (t > o && pcol[t - 1] > jo) {
-      pcol[t] = pcol[t - 1];
-      --t;
-    }
-    pcol[t] = jo;
-  }
   const float2 pi = xy[s];
-  for (int k = 0; k < e - b; ++k) {
-    prow[o + k] = i;
+  for (int t0 = 0; t0 < m; t0 += 32) {
+    const int t = t0 + lane;
+    const int32_t c = t < m ? __ldg(cols + b + t) : 0;
+    const uint32_t jo = t < m ? __ldg(order + c) : 0xffffffffu;
+    int r = 0;
+    for (int u0 = 0; u0 < m; u0 += 32) {
+      const int u = u0 + lane;
+      const uint32_t ju = u0 == t0 ? jo : (u < m ? __ldg(order + __ldg(cols + b + u)) : 0xffffffffu);
+      const int len = min(m - u0, 32);
+      for (int k = 0; k < len; ++k) r += __shfl_sync(0xffffffffu, ju, k) < jo;
+    }
+    if (t >= m) continue;
+    prow[o + r] = i;
+    pcol[o + r] = (int64_t)jo;
     if (dist || radial) {
-      float2 pj = xy[rank[pcol[o + k]]];
-      float dx = pi.x - pj.x, dy = pi.y - pj.y;
-      float rr = sqrtf(dx * dx + dy * dy);
+      const float2 pj = __ldg(xy + c);
+      const float dx = pi.x - pj.x, dy = pi.y - pj.y;
+      const float rr = sqrtf(dx * dx + dy * dy);
       if (dist) {
-        if (rr < thr) {
-          dist[2 * (o + k)] = 0.f;
-          dist[2 * (o + k) + 1] = 0.f;
+        const float2 e = rr < thr ? make_float2(0.f, 0.f) : make_float2(dx / rr, dy / rr);
+        if ((reinterpret_cast<uintptr_t>(dist) & 7) == 0) {
+          reinterpret_cast<float2*>(dist)[o + r] = e;
         } else {
-          dist[2 * (o + k)] = dx / rr;
-          dist[2 * (o + k) + 1] = dy / rr;
+          dist[2 * (o + r)] = e.x;
+          dist[2 * (o + r) + 1] = e.y;
         }
       }
-      if (radial) radial[o + k] = rr / support;
+      if (radial) radial[o + r] = rr / support;
     }
   }
 }
@@ -637,7 +652,7 @@ sph_status_t sph_nl_to_coo(const float* xy, int64_t n, const uint32_t* order, co
                            float* radial, void* stream) {
   SPH_REQUIRE(n >= 0 && xy && order && rank && offsets && cols && orig_offsets && pairs, "nl_to_coo: bad arguments");
   if (n == 0) return SPH_OK;
-  k_nl_to_coo<<<grid_for(n, 128), 128, 0, as_stream(stream)>>>(reinterpret_cast<const float2*>(xy), n, order, rank,
+  k_nl_to_coo<<<grid_for(n, 8), 256, 0, as_stream(stream)>>>(reinterpret_cast<const float2*>(xy), n, order, rank,
                                                                 offsets, cols, orig_offsets, grad_threshold,
                                                                 kernel_support, pairs, num_pairs, dist, radial);
   SPH_CHECK_LAUNCH("nl_to_coo");
