@@ -748,8 +748,18 @@ typedef struct sph_dfsph_buffers {
   double* partials;         /* [sph_dfsph_partials_count()] */
   float* errors;            /* [max iterations + 1] error of every iteration */
   int32_t* iters;           /* [1] iterations run */
-  float* records;           /* [9 n], 16-byte aligned: per-particle pair records of the Jacobi sweeps */
+  float* records;           /* [sph_dfsph_records_count()], 16-byte aligned: per-particle pair records of the Jacobi
+                               sweeps and, with pairs from the cell rows, neighbor lists */
 } sph_dfsph_buffers;
+
+/* The DFSPH calls below take their pairs from the CSR list of the fluid view, or, when the view
+ * has neither offsets nor cols, from the cell rows: sph_dfsph_densities then keeps each
+ * particle's neighbor list in bufs->records for the calls of the same step, and sums rho_fluid
+ * itself where that is NULL. */
+
+/* Floats of sph_dfsph_buffers.records: 9 n with a CSR list; more with pairs from the cell
+ * rows, for the neighbor lists. */
+size_t sph_dfsph_records_count(int64_t n, int64_t nb, int32_t cell_rows);
 
 size_t sph_dfsph_partials_count(void);
 /* Static wall-wall density term sum_b' W(|x_b - x_b'| / h) A_b' (solidBoundary.py:180-200). */

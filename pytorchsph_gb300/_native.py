@@ -120,6 +120,7 @@ SIGNATURES.update({  # simulation kernels
     "sph_permute": (_I32, [_P, _I64, _I32] + [_P] * 3),
     "sph_permute_arrays": (_I32, [_P, _I64, _I32, _P, _P, _P, _P]),
     "sph_dfsph_partials_count": (_SZ, []),
+    "sph_dfsph_records_count": (_SZ, [_I64, _I64, _I32]),
     "sph_dfsph_wall_wall_term": (_I32, [_P] * 5),
     "sph_dfsph_densities": (_I32, [_P] * 7),
     "sph_dfsph_solve": (_I32, [_P] * 7 + [_I32] + [_P] * 2),

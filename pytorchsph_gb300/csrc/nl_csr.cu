@@ -17,42 +17,6 @@ namespace sph {
 // up to 8 x 32 candidates each, ~9x the density of a jittered lattice at support 3 dx.
 constexpr int kSearchSegments = 24;
 
-// segment_mask with the density terms of the accepted candidates added to acc in index
-// order, in the same unrolled pass: the terms of a candidate pair are formed together on
-// the paired float32 instructions and only the accepted ones are added (the caller scales
-// the sum by c_w).  Distance r = v * rsqrt(max(v, 1e-30)): 0 for the particle itself,
-// within a few ulp of sqrt(v) otherwise.  W(q) / c_w = (1-q)^4 (1+4q), src/kernels.py:20-24.
-__device__ __forceinline__ uint32_t segment_mask_density(const float2* __restrict__ x, const float* __restrict__ sa,
-                                                         int c, int e, float xi, float yi, float thr,
-                                                         float inv_support, float& acc) {
-  const int len = min(e - c, 32);
-  uint32_t m = 0;
-  const float2 qx = make_float2(xi, xi), qy = make_float2(yi, yi), is2 = make_float2(inv_support, inv_support);
-#pragma unroll
-  for (int t = 0; t < 32; t += 2) {
-    if (t < len) {
-      const bool two = t + 1 < len;
-      const float2 a = __ldg(x + c + t), b = two ? __ldg(x + c + t + 1) : a;
-      const float2 dx = __fadd2_rn(qx, make_float2(-a.x, -b.x));
-      const float2 dy = __fadd2_rn(qy, make_float2(-a.y, -b.y));
-      const float2 v = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
-      const bool in0 = v.x <= thr, in1 = two && v.y <= thr;
-      if (in0) m |= 1u << t;
-      if (in1) m |= 2u << t;
-      if (in0 || in1) {
-        const float2 rs = __fmul2_rn(make_float2(rsqrt_normal(fmaxf(v.x, 1e-30f)), rsqrt_normal(fmaxf(v.y, 1e-30f))), is2);
-        const float2 q = __fmul2_rn(v, rs);
-        const float2 am = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-q.x, -q.y));
-        const float2 a2 = __fmul2_rn(am, am);
-        const float2 w = __fmul2_rn(__fmul2_rn(a2, a2), __ffma2_rn(make_float2(4.f, 4.f), q, make_float2(1.f, 1.f)));
-        if (in0) acc = fmaf(w.x, __ldg(sa + c + t), acc);
-        if (in1) acc = fmaf(w.y, __ldg(sa + c + t + 1), acc);
-      }
-    }
-  }
-  return m;
-}
-
 template <typename F>
 __device__ __forceinline__ void scan_candidates(const float2* __restrict__ xy, const int32_t* __restrict__ cell_start,
                                                 const sph_grid& g, int r, int cx, int cy, float xi, float yi,

@@ -142,127 +142,6 @@ __device__ __forceinline__ PairG pair_g(float xi, float yi, float xj, float yj, 
   return g;
 }
 
-// ---------------------------------------------------------------------------- cell-row pairs
-// The pairs of particle i straight from the cell table, without a CSR list: its candidates
-// are the contiguous sorted ranges of its 2r+1 cell rows (cells cx-r..cx+r of each row).
-// A range is tested in segments of 32 candidates into a bit mask, and the accepted
-// candidates are visited in increasing index: the CSR fill's order, so every sum is the
-// same.  Visiting set bits keeps a warp's lanes together the way a CSR row does (a lane
-// runs the pair body only for its own neighbors).
-//
-// The records pass stores each particle's non-empty segments in order, at most
-// kMaxSegments: start seg_start[k * n + i] and mask seg_mask[k * n + i] for k < nseg[i]
-// (nseg[i] = -1 when there are more; the force passes then test its cell rows
-// themselves).  A force pass holds one segment and the next one, loaded ahead, so moving
-// on to the next segment costs a lane a register move.
-// Every row of the window, tested here (any r); with kTpp lanes per particle, lane `sub`
-// takes rows y0 + sub, y0 + sub + kTpp, ...
-// kPaired: the candidate tests two at a time (segment_mask) or one at a time; the sums are
-// the same either way (which one a pass uses is a measured code-generation choice).
-template <int kTpp = 1, bool kPaired = false, typename Fn>
-__device__ __forceinline__ void cell_pairs(const FluidView& F, const sph_grid& g, int r, int coff, int cx, int cy,
-                                           float xi, float yi, float thr, Fn&& fn, int sub = 0) {
-  const int x0 = max(cx - r, 0), x1 = min(cx + r, g.cells_x - 1);
-  if (x0 > x1) return;
-  const int y0 = max(cy - r, 0), y1 = min(cy + r, g.cells_y - 1);
-  const int32_t* cs = F.cell_start + coff;
-  for (int yy = y0 + sub; yy <= y1; yy += kTpp) {
-    const int row = yy * g.cells_x;
-    const int b = __ldg(cs + row + x0), e = __ldg(cs + row + x1 + 1);
-    for (int c = b; c < e; c += 32) {
-      uint32_t w = kPaired ? segment_mask(F.x, c, e, xi, yi, thr) : segment_mask_scalar(F.x, c, e, xi, yi, thr);
-      while (w) {
-        const int j = c - 1 + __ffs(w);
-        w &= w - 1;
-        fn(j);
-      }
-    }
-  }
-}
-
-// The segment list of particle i.
-__device__ __forceinline__ void segments_body(int i, const FluidView& F, const sph_grid& g, int coff, int r,
-                                              float thr, int32_t* __restrict__ nseg, int32_t* __restrict__ seg_start,
-                                              uint32_t* __restrict__ seg_mask) {
-  int cx, cy;
-  cell_of(F.keys[i] - (uint32_t)coff, g, &cx, &cy);
-  const float2 xi = F.x[i];
-  const size_t n = (size_t)F.n;
-  int k = 0;
-  const int x0 = max(cx - r, 0), x1 = min(cx + r, g.cells_x - 1);
-  const int y0 = max(cy - r, 0), y1 = min(cy + r, g.cells_y - 1);
-  const int32_t* cs = F.cell_start + coff;
-  if (x0 <= x1) {
-    for (int yy = y0; yy <= y1; ++yy) {
-      const int row = yy * g.cells_x;
-      const int b = __ldg(cs + row + x0), e = __ldg(cs + row + x1 + 1);
-      for (int c = b; c < e; c += 32) {
-        const uint32_t w = c + 32 <= F.n ? segment_mask_full(F.x, c, e, xi.x, xi.y, thr)
-                                         : segment_mask(F.x, c, e, xi.x, xi.y, thr);
-        if (w == 0) continue;
-        if (k < kMaxSegments) {
-          seg_start[k * n + i] = c;
-          seg_mask[k * n + i] = w;
-        }
-        ++k;
-      }
-    }
-  }
-  nseg[i] = k <= kMaxSegments ? k : -1;
-}
-
-// The pairs of particle i from its segment list (its cell rows when the list overflowed).
-// With kTpp lanes per particle, lane `sub` takes segments sub, sub + kTpp, ... (rows, on the
-// overflow path); each lane holds its current segment and its next one, loaded ahead.
-template <int kTpp = 1, bool kPaired = false, typename Fn>
-__device__ __forceinline__ void stored_pairs(int i, const FluidView& F, const sph_grid& g, int coff, int r,
-                                             const int32_t* __restrict__ nseg, const int32_t* __restrict__ seg_start,
-                                             const uint32_t* __restrict__ seg_mask, float xi, float yi, float thr,
-                                             Fn&& fn, int sub = 0) {
-  const int ns = nseg[i];
-  if (ns < 0 || ns > kMaxSegments) {
-    int cx, cy;
-    cell_of(F.keys[i] - (uint32_t)coff, g, &cx, &cy);
-    cell_pairs<kTpp, kPaired>(F, g, r, coff, cx, cy, xi, yi, thr, fn, sub);
-    return;
-  }
-  if (ns <= sub) return;
-  const size_t n = (size_t)F.n;
-  int k = sub;
-  int b = seg_start[k * n + i];
-  uint32_t w = clip_segment(seg_mask[k * n + i], b, F.n);
-  int bn = 0;
-  uint32_t wn = 0;
-  if (k + kTpp < ns) {
-    bn = seg_start[(k + kTpp) * n + i];
-    wn = seg_mask[(k + kTpp) * n + i];
-  }
-  for (;;) {
-    while (w == 0) {
-      k += kTpp;
-      if (k >= ns) return;
-      b = bn;
-      w = clip_segment(wn, bn, F.n);
-      if (k + kTpp < ns) {
-        bn = seg_start[(k + kTpp) * n + i];
-        wn = seg_mask[(k + kTpp) * n + i];
-      }
-    }
-    const int j = b - 1 + __ffs(w);
-    w &= w - 1;
-    fn(j);
-  }
-}
-
-// Sum of v over the kTpp consecutive lanes of one particle (every lane gets the sum; the
-// whole warp must take part).
-template <int kTpp>
-__device__ __forceinline__ float lane_sum(float v) {
-#pragma unroll
-  for (int o = 1; o < kTpp; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 // ---------------------------------------------------------------------------- pass 1
 // dpdt (continuity + MOG), acceleration (gravity, pressure, artificial and laminar
 // viscosity) and, for the deltaSPH scheme, the renormalization matrix L_i and the density
@@ -278,13 +157,6 @@ struct Pass1 {
   float4 L;        // renormalization matrix, fluid + walls
   float2 grad_rho;
   float ddiff;     // deltaSPH: the pass-1 part of D_i
-};
-
-// Pairs from the segment lists S (kCells) instead of the CSR row.
-struct Segments {
-  const int32_t* nseg;
-  const int32_t* start;
-  const uint32_t* mask;
 };
 
 // kTpp lanes per particle (kCells only): lane `sub` sums its share of the pairs, the lanes

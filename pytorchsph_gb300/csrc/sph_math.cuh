@@ -275,6 +275,34 @@ __device__ __forceinline__ void for_each_wall(const WallView& W, const sph_grid&
   }
 }
 
+// for_each_wall shared by kLanes consecutive lanes (one particle's): lane `sub` takes every
+// kLanes-th wall of each cell row.
+template <int kLanes, typename F>
+__device__ __forceinline__ void for_each_wall_lanes(const WallView& W, const sph_grid& g, int r, int cx, int cy,
+                                                    float xf, float yf, float thr_b, int sub, F&& f, int coff = 0) {
+  const int x0 = max(cx - r, 0), x1 = min(cx + r, g.cells_x - 1);
+  if (x0 > x1) return;
+  const int y0 = max(cy - r, 0), y1 = min(cy + r, g.cells_y - 1);
+  const int32_t* cs = W.cell_start + coff;
+  for (int yy = y0; yy <= y1; ++yy) {
+    const int row = yy * g.cells_x;
+    const int b0 = __ldg(cs + row + x0), b1 = __ldg(cs + row + x1 + 1);
+    for (int b = b0 + sub; b < b1; b += kLanes) {
+      const float2 xb = __ldg(W.x + b);
+      if (dist2_ref(xb.x, xb.y, xf, yf) <= thr_b) f(b, xb);
+    }
+  }
+}
+
+// Sum of v over the kLanes consecutive lanes of one particle (every lane gets the sum; the
+// whole warp must take part).
+template <int kLanes>
+__device__ __forceinline__ float lane_sum(float v) {
+#pragma unroll
+  for (int o = 1; o < kLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // ---------------------------------------------------------------- candidate segments
 // The candidates of a particle in one cell row are a contiguous sorted range; it is tested
 // in segments of 32 candidates into bit masks (bit t: candidate c + t passes the pair test),
@@ -341,6 +369,42 @@ __device__ __forceinline__ uint32_t segment_mask_full(const float2* __restrict__
   return len >= 32 ? m : m & ((1u << len) - 1u);
 }
 
+// segment_mask with the density terms of the accepted candidates added to acc in index
+// order, in the same unrolled pass: the terms of a candidate pair are formed together on
+// the paired float32 instructions and only the accepted ones are added (the caller scales
+// the sum by c_w).  Distance r = v * rsqrt(max(v, 1e-30)): 0 for the particle itself,
+// within a few ulp of sqrt(v) otherwise.  W(q) / c_w = (1-q)^4 (1+4q), src/kernels.py:20-24.
+__device__ __forceinline__ uint32_t segment_mask_density(const float2* __restrict__ x, const float* __restrict__ sa,
+                                                         int c, int e, float xi, float yi, float thr,
+                                                         float inv_support, float& acc) {
+  const int len = min(e - c, 32);
+  uint32_t m = 0;
+  const float2 qx = make_float2(xi, xi), qy = make_float2(yi, yi), is2 = make_float2(inv_support, inv_support);
+#pragma unroll
+  for (int t = 0; t < 32; t += 2) {
+    if (t < len) {
+      const bool two = t + 1 < len;
+      const float2 a = __ldg(x + c + t), b = two ? __ldg(x + c + t + 1) : a;
+      const float2 dx = __fadd2_rn(qx, make_float2(-a.x, -b.x));
+      const float2 dy = __fadd2_rn(qy, make_float2(-a.y, -b.y));
+      const float2 v = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
+      const bool in0 = v.x <= thr, in1 = two && v.y <= thr;
+      if (in0) m |= 1u << t;
+      if (in1) m |= 2u << t;
+      if (in0 || in1) {
+        const float2 rs = __fmul2_rn(make_float2(rsqrt_normal(fmaxf(v.x, 1e-30f)), rsqrt_normal(fmaxf(v.y, 1e-30f))), is2);
+        const float2 q = __fmul2_rn(v, rs);
+        const float2 am = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-q.x, -q.y));
+        const float2 a2 = __fmul2_rn(am, am);
+        const float2 w = __fmul2_rn(__fmul2_rn(a2, a2), __ffma2_rn(make_float2(4.f, 4.f), q, make_float2(1.f, 1.f)));
+        if (in0) acc = fmaf(w.x, __ldg(sa + c + t), acc);
+        if (in1) acc = fmaf(w.y, __ldg(sa + c + t + 1), acc);
+      }
+    }
+  }
+  return m;
+}
+
 // The bits of a stored segment that name a particle: none for a start outside [0, n),
 // none at index n or past it.
 __device__ __forceinline__ uint32_t clip_segment(uint32_t w, int b, int n) {
@@ -379,6 +443,134 @@ __device__ __forceinline__ void cell_of(uint32_t key, const sph_grid& g, int* cx
   *cx = (int)(key % (uint32_t)g.cells_x);
   *cy = (int)(key / (uint32_t)g.cells_x);
 }
+
+// ---------------------------------------------------------------------------- cell-row pairs
+// The pairs of particle i straight from the cell table, without a CSR list: its candidates
+// are the contiguous sorted ranges of its 2r+1 cell rows (cells cx-r..cx+r of each row).
+// A range is tested in segments of 32 candidates into a bit mask, and the accepted
+// candidates are visited in increasing index: the CSR fill's order, so every sum is the
+// same.  Visiting set bits keeps a warp's lanes together the way a CSR row does (a lane
+// runs the pair body only for its own neighbors).
+//
+// The records pass stores each particle's non-empty segments in order, at most
+// kMaxSegments: start seg_start[k * n + i] and mask seg_mask[k * n + i] for k < nseg[i]
+// (nseg[i] = -1 when there are more; the force passes then test its cell rows
+// themselves).  A force pass holds one segment and the next one, loaded ahead, so moving
+// on to the next segment costs a lane a register move.
+// Every row of the window, tested here (any r); with kTpp lanes per particle, lane `sub`
+// takes rows y0 + sub, y0 + sub + kTpp, ...
+// kPaired: the candidate tests two at a time (segment_mask) or one at a time; the sums are
+// the same either way (which one a pass uses is a measured code-generation choice).
+template <int kTpp = 1, bool kPaired = false, typename Fn>
+__device__ __forceinline__ void cell_pairs(const FluidView& F, const sph_grid& g, int r, int coff, int cx, int cy,
+                                           float xi, float yi, float thr, Fn&& fn, int sub = 0) {
+  const int x0 = max(cx - r, 0), x1 = min(cx + r, g.cells_x - 1);
+  if (x0 > x1) return;
+  const int y0 = max(cy - r, 0), y1 = min(cy + r, g.cells_y - 1);
+  const int32_t* cs = F.cell_start + coff;
+  for (int yy = y0 + sub; yy <= y1; yy += kTpp) {
+    const int row = yy * g.cells_x;
+    const int b = __ldg(cs + row + x0), e = __ldg(cs + row + x1 + 1);
+    for (int c = b; c < e; c += 32) {
+      uint32_t w = kPaired ? segment_mask(F.x, c, e, xi, yi, thr) : segment_mask_scalar(F.x, c, e, xi, yi, thr);
+      while (w) {
+        const int j = c - 1 + __ffs(w);
+        w &= w - 1;
+        fn(j);
+      }
+    }
+  }
+}
+
+// The segment list of particle i.
+__device__ __forceinline__ void segments_body(int i, const FluidView& F, const sph_grid& g, int coff, int r,
+                                              float thr, int32_t* __restrict__ nseg, int32_t* __restrict__ seg_start,
+                                              uint32_t* __restrict__ seg_mask) {
+  int cx, cy;
+  cell_of(F.keys[i] - (uint32_t)coff, g, &cx, &cy);
+  const float2 xi = F.x[i];
+  const size_t n = (size_t)F.n;
+  int k = 0;
+  const int x0 = max(cx - r, 0), x1 = min(cx + r, g.cells_x - 1);
+  const int y0 = max(cy - r, 0), y1 = min(cy + r, g.cells_y - 1);
+  const int32_t* cs = F.cell_start + coff;
+  if (x0 <= x1) {
+    for (int yy = y0; yy <= y1; ++yy) {
+      const int row = yy * g.cells_x;
+      const int b = __ldg(cs + row + x0), e = __ldg(cs + row + x1 + 1);
+      for (int c = b; c < e; c += 32) {
+        const uint32_t w = c + 32 <= F.n ? segment_mask_full(F.x, c, e, xi.x, xi.y, thr)
+                                         : segment_mask(F.x, c, e, xi.x, xi.y, thr);
+        if (w == 0) continue;
+        if (k < kMaxSegments) {
+          seg_start[k * n + i] = c;
+          seg_mask[k * n + i] = w;
+        }
+        ++k;
+      }
+    }
+  }
+  nseg[i] = k <= kMaxSegments ? k : -1;
+}
+
+// Lane `sub`'s candidates of a segment shared by kTpp lanes: every kTpp-th bit.
+template <int kTpp>
+__device__ __forceinline__ uint32_t lane_bits(uint32_t w, int sub) {
+  static_assert(kTpp == 1 || kTpp == 2 || kTpp == 4 || kTpp == 8, "lanes per particle");
+  constexpr uint32_t every = kTpp == 1 ? 0xffffffffu : kTpp == 2 ? 0x55555555u : kTpp == 4 ? 0x11111111u : 0x01010101u;
+  return w & (every << sub);
+}
+
+// The pairs of particle i from its segment list (its cell rows when the list overflowed).
+// With kTpp lanes per particle every lane walks all segments and takes its lane_bits of each
+// (about 28 / kTpp pairs, however the accepted candidates fall into segments; rows are dealt
+// on the overflow path); each lane holds its current segment and the next one, loaded ahead.
+template <int kTpp = 1, bool kPaired = false, typename Fn>
+__device__ __forceinline__ void stored_pairs(int i, const FluidView& F, const sph_grid& g, int coff, int r,
+                                             const int32_t* __restrict__ nseg, const int32_t* __restrict__ seg_start,
+                                             const uint32_t* __restrict__ seg_mask, float xi, float yi, float thr,
+                                             Fn&& fn, int sub = 0) {
+  const int ns = nseg[i];
+  if (ns < 0 || ns > kMaxSegments) {
+    int cx, cy;
+    cell_of(F.keys[i] - (uint32_t)coff, g, &cx, &cy);
+    cell_pairs<kTpp, kPaired>(F, g, r, coff, cx, cy, xi, yi, thr, fn, sub);
+    return;
+  }
+  if (ns == 0) return;
+  const size_t n = (size_t)F.n;
+  int k = 0;
+  int b = seg_start[i];
+  uint32_t w = lane_bits<kTpp>(clip_segment(seg_mask[i], b, F.n), sub);
+  int bn = 0;
+  uint32_t wn = 0;
+  if (1 < ns) {
+    bn = seg_start[n + i];
+    wn = seg_mask[n + i];
+  }
+  for (;;) {
+    while (w == 0) {
+      ++k;
+      if (k >= ns) return;
+      b = bn;
+      w = lane_bits<kTpp>(clip_segment(wn, bn, F.n), sub);
+      if (k + 1 < ns) {
+        bn = seg_start[(k + 1) * n + i];
+        wn = seg_mask[(k + 1) * n + i];
+      }
+    }
+    const int j = b - 1 + __ffs(w);
+    w &= w - 1;
+    fn(j);
+  }
+}
+
+// Pairs from the segment lists S (kCells) instead of the CSR row.
+struct Segments {
+  const int32_t* nseg;
+  const int32_t* start;
+  const uint32_t* mask;
+};
 
 }  // namespace sph
 

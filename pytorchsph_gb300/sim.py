@@ -103,10 +103,17 @@ DIFFUSION = {"none": 0, "MOG": 1, "deltaSPH": 2}
 
 class Simulation:
     """One scene on the GPU.  `scene` holds numpy arrays (pos, vel, rho, area, support,
-    wall_pos, ghost_pos, wall_area, vmin, vmax), e.g. from pytorchsph_gb300.workloads."""
+    wall_pos, ghost_pos, wall_area, vmin, vmax), e.g. from pytorchsph_gb300.workloads.
 
-    def __init__(self, scene: dict, cfg: SimConfig, device=None):
+    pairs = "cells": the summations take each particle's pairs from its cell rows, tested once a
+    step into segment bit masks.  pairs = "csr": a CSR neighbor list is counted and filled every
+    step first.  Both visit the same pairs."""
+
+    def __init__(self, scene: dict, cfg: SimConfig, device=None, pairs: str = "cells"):
+        if pairs not in ("cells", "csr"):
+            raise ValueError("pairs must be 'cells' or 'csr'")
         self.lib = N.load()
+        self.pairs = pairs
         self.cfg = cfg
         self.device = torch.device(device or torch.device("cuda", torch.cuda.current_device()))
         dev = self.device
@@ -139,7 +146,8 @@ class Simulation:
         self.nb = len(scene.get("wall_pos", ()))
         self._setup_walls(scene)
         self.pair_cap = 0
-        self.cols = None
+        self.offsets = self.cols = None
+        self.stepped = False     # a right-hand side has run: every buffer has its size
         self.extra = {}
         self.last = {}
         self.graph = None
@@ -243,7 +251,7 @@ class Simulation:
 
     # ------------------------------------------------------------------ one right-hand side
     def _search(self, sync):
-        """Re-sort every particle array by cell key and build the CSR neighbor list."""
+        """Re-sort every particle array by cell key and (pairs = "csr") build the neighbor list."""
         st = N.stream_ptr()
         n = self.n
         order, skeys, cs = self._sort_keys(self.arr["x"], n, "f_", tie=self.arr["uid"])
@@ -252,6 +260,12 @@ class Simulation:
         for k in list(self.extra):
             self.extra[k] = self._permute(order, self.extra[k])
         self.skeys, self.cell_start = skeys, cs
+        self.stepped = True
+        if self._cell_pairs():
+            self.rho_fluid = None
+            self.fluid_view = FluidViewC(N.ptr(self.arr["x"]), N.ptr(self.arr["v"]), N.ptr(self.arr["rho"]),
+                                         N.ptr(self.arr["area"]), N.ptr(skeys), None, None, N.ptr(cs), n, 0)
+            return
         counts = self.ws.get("counts", n)
         rho_fluid = self.ws.get("rho_fluid", n, torch.float32)
         dens = self.cfg.solver == "dfsph"
@@ -273,6 +287,9 @@ class Simulation:
         self.fluid_view = FluidViewC(N.ptr(self.arr["x"]), N.ptr(self.arr["v"]), N.ptr(self.arr["rho"]),
                                      N.ptr(self.arr["area"]), N.ptr(skeys), N.ptr(offsets), N.ptr(self.cols), N.ptr(cs), n,
                                      self.pair_cap)
+
+    def _cell_pairs(self):
+        return self.pairs == "cells" and self.cfg.solver == "dfsph"
 
     def rhs(self, sync=True):
         """Evaluate one timestep() at the current state; returns (acc, vel, dpdt or None)."""
@@ -303,7 +320,7 @@ class Simulation:
              "wall_alpha": g("walpha", nb), "wall_source": g("wsrc", nb), "wall_pressure": g("wp", nb),
              "wall_residual": g("wres", nb), "wall_density_term": self.wall_term,
              "partials": g("partials", int(self.lib.sph_dfsph_partials_count()), torch.float64),
-             "errors": g("errors", maxit), "iters": g("iters", 1, torch.int32), "records": g("records", 9 * n)}
+             "errors": g("errors", maxit), "iters": g("iters", 1, torch.int32), "records": g("records", self.lib.sph_dfsph_records_count(n, self.nb, int(self._cell_pairs())))}
         self.dfsph_arrays = b
         return DfsphBuffersC(*[N.ptr(b[k]) for k, _ in DfsphBuffersC._fields_])
 
@@ -339,8 +356,9 @@ class Simulation:
         """Record one step() in a CUDA graph; every later step() replays it (one launch of
         the whole step instead of ~20 host calls).  The state arrays become fixed device
         buffers: the recorded step ends by copying its new state into them.  Needs one eager
-        step first (it sizes the neighbor buffer; a step that overflows it raises at check())."""
-        if self.cols is None:
+        step first (it sizes the buffers; with pairs = "csr" a step whose pairs overflow the
+        neighbor buffer raises at check())."""
+        if not self.stepped:
             raise N.SPHError("capture: run one step first")
         torch.cuda.synchronize(self.device)
         inputs = dict(self.arr)
