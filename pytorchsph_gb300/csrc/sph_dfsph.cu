@@ -149,18 +149,10 @@ __device__ __forceinline__ void wall_candidates(const FluidView& F, const sph_gr
   const float fcx = ceilf(__fdiv_rn(__fsub_rn(xb.x, g.qmin[0]), g.hmax));
   const float fcy = ceilf(__fdiv_rn(__fsub_rn(xb.y, g.qmin[1]), g.hmax));
   if (!(grid_ok(g, P.cell_capacity) && fcx > -1e9f && fcx < 1e9f && fcy > -1e9f && fcy < 1e9f)) return;
-  const int qx = (int)fcx, qy = (int)fcy, r = P.search_radius;
-  const int x0 = max(qx - r, 0), x1 = min(qx + r, g.cells_x - 1);
-  const int y0 = max(qy - r, 0), y1 = min(qy + r, g.cells_y - 1);
-  if (x0 > x1) return;
-  for (int yy = y0; yy <= y1; ++yy) {
-    const int row = yy * g.cells_x;
-    const int j1 = __ldg(F.cell_start + row + x1 + 1);
-    for (int j = __ldg(F.cell_start + row + x0) + sub; j < j1; j += kWallLanes) {
-      const float2 xj = __ldg(F.x + j);
-      if (dist2_ref(xb.x, xb.y, xj.x, xj.y) <= P.thr) use(j);
-    }
-  }
+  for_each_member<kWallLanes>(F.cell_start, g, P.search_radius, (int)fcx, (int)fcy, sub, [&](int j) {
+    const float2 xj = __ldg(F.x + j);
+    if (dist2_ref(xb.x, xb.y, xj.x, xj.y) <= P.thr) use(j);
+  });
 }
 
 template <bool kCells, typename Use>

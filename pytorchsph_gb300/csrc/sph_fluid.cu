@@ -28,76 +28,123 @@
 namespace sph {
 
 // ---------------------------------------------------------------------------- mDBC
-// Shepard and first-order MLS sums over the fluid particles within h of wall b's ghost
-// (accumulated in double), the 3x3 pseudo-inverse solve, then wall density, volume and
-// Tait pressure.
-__device__ __forceinline__ void mdbc_body(int b, const FluidView& F, const WallView& W, const sph_grid& g,
-                                          const SphParams& P, int coff) {
-  const float2 xg = W.xg[b];
+// Shepard and first-order MLS sums over the fluid particles within h of wall b's ghost, shared by
+// kLanes lanes, then the 3x3 pseudo-inverse solve, wall density, volume and Tait pressure.
+// Latency-bound: one scene has few walls, each a chain of ~80 candidate loads and a solve on the
+// FP64 pipe.  1,380 walls 20 -> 7.3 us a launch (8 / 32 lanes: 7.8 / 6.8), 5,976 walls 35 ->
+// 7.8 us (8.0 / 7.7); the 210,000 walls of 50 served tanks fill the GPU with one lane each and
+// take 78 -> 36 us with the shorter solve (119 with 8 lanes and the long one).
+constexpr int kMdbcSums = 12;
+constexpr int kMdbcSplitWalls = 32768;   // up to here kMdbcLanes lanes per wall
+constexpr int kMdbcLanes = 16, kMdbcThreads = 256, kMdbcWalls = kMdbcThreads / kMdbcLanes;
+
+// float sums (GB300's FP64 rate is low); the 3x3 solve runs in double
+template <int kLanes>
+__device__ __forceinline__ void mdbc_sums(float2 xg, int sub, const FluidView& F, const sph_grid& g,
+                                          const SphParams& P, int coff, float (&s)[kMdbcSums], int& cnt) {
   const float thr = P.thr;
-  // float sums (GB300's FP64 rate is low); the 3x3 solve below runs in double
-  float nom = 0, den = 0, gx = 0, gy = 0, vgx = 0, vgy = 0, px = 0, py = 0;
-  float m00 = 0, m01 = 0, m10 = 0, m11 = 0;
-  int cnt = 0;
   const int32_t* cs = F.cell_start + coff;
-  if (grid_ok(g, P.cell_capacity)) {
-    float fcx = ceilf(__fdiv_rn(__fsub_rn(xg.x, g.qmin[0]), g.hmax));
-    float fcy = ceilf(__fdiv_rn(__fsub_rn(xg.y, g.qmin[1]), g.hmax));
-    if (fcx > -1e9f && fcx < 1e9f && fcy > -1e9f && fcy < 1e9f) {
-      const int cx = (int)fcx, cy = (int)fcy, r = P.search_radius;
-      const int x0 = max(cx - r, 0), x1 = min(cx + r, g.cells_x - 1);
-      const int y0 = max(cy - r, 0), y1 = min(cy + r, g.cells_y - 1);
-      if (x0 <= x1) {
-        for (int yy = y0; yy <= y1; ++yy) {
-          const int row = yy * g.cells_x;
-          const int j0 = cs[row + x0], j1 = cs[row + x1 + 1];
-          for (int j = j0; j < j1; ++j) {
-            const float2 xj = F.x[j];
-            if (!(dist2_ref(xg.x, xg.y, xj.x, xj.y) <= thr)) continue;
-            // e = (x_g - x_j) / r from one rsqrt (zero below r = 1e-7, as the reference's e_ij)
-            const float dx = xg.x - xj.x, dy = xg.y - xj.y;
-            const float r2 = dx * dx + dy * dy;
-            const float ir = r2 >= 1e-14f ? rsqrt_normal(r2) : 0.f;
-            const float q = r2 * ir * P.inv_h;
-            const float k = kW(q, P.c_w);
-            const float gwr = kGW(q, P.c_g) * ir;
-            const float ggx = gwr * dx, ggy = gwr * dy;
-            const float Aj = F.area[j];
-            const float mass = Aj * P.rho0;
-            const float Vj = Aj * rcp_normal(F.rho[j]);
-            const float xx = xj.x - xg.x, xy = xj.y - xg.y;
-            nom += mass * k;
-            den += Vj * k;
-            gx += mass * ggx;
-            gy += mass * ggy;
-            vgx += Vj * ggx;
-            vgy += Vj * ggy;
-            px += Vj * k * xx;
-            py += Vj * k * xy;
-            m00 += Vj * xx * ggx;
-            m01 += Vj * xx * ggy;
-            m10 += Vj * xy * ggx;
-            m11 += Vj * xy * ggy;
-            ++cnt;
-          }
-        }
-      }
-    }
-  }
+  if (!grid_ok(g, P.cell_capacity)) return;
+  const float fcx = ceilf(__fdiv_rn(__fsub_rn(xg.x, g.qmin[0]), g.hmax));
+  const float fcy = ceilf(__fdiv_rn(__fsub_rn(xg.y, g.qmin[1]), g.hmax));
+  if (!(fcx > -1e9f && fcx < 1e9f && fcy > -1e9f && fcy < 1e9f)) return;
+  for_each_member<kLanes>(cs, g, P.search_radius, (int)fcx, (int)fcy, sub, [&](int j) {
+    const float2 xj = F.x[j];
+    const float Aj = F.area[j], rj = F.rho[j];   // loaded beside the position: one latency per member
+    if (!(dist2_ref(xg.x, xg.y, xj.x, xj.y) <= thr)) return;
+    // e = (x_g - x_j) / r from one rsqrt (zero below r = 1e-7, as the reference's e_ij)
+    const float dx = xg.x - xj.x, dy = xg.y - xj.y;
+    const float r2 = dx * dx + dy * dy;
+    const float ir = r2 >= 1e-14f ? rsqrt_normal(r2) : 0.f;
+    const float q = r2 * ir * P.inv_h;
+    const float k = kW(q, P.c_w);
+    const float gwr = kGW(q, P.c_g) * ir;
+    const float ggx = gwr * dx, ggy = gwr * dy;
+    const float mass = Aj * P.rho0;
+    const float Vj = Aj * rcp_normal(rj);
+    const float xx = xj.x - xg.x, xy = xj.y - xg.y;
+    s[0] += mass * k;        // Shepard numerator and denominator
+    s[1] += Vj * k;
+    s[2] += mass * ggx;      // first-order MLS: gradient sums and moments
+    s[3] += mass * ggy;
+    s[4] += Vj * ggx;
+    s[5] += Vj * ggy;
+    s[6] += Vj * k * xx;
+    s[7] += Vj * k * xy;
+    s[8] += Vj * xx * ggx;
+    s[9] += Vj * xx * ggy;
+    s[10] += Vj * xy * ggx;
+    s[11] += Vj * xy * ggy;
+    ++cnt;
+  });
+}
+
+__device__ __forceinline__ void mdbc_finish(int b, const float* s, int stride, int cnt, const WallView& W,
+                                            const SphParams& P) {
+  const auto v = [&](int k) { return s[k * stride]; };
   double rho_b = 1.0;
-  if (cnt > 0) rho_b = ((double)nom / (double)den) / P.rho0;
   if (cnt > 10) {
-    const double A[3][3] = {{den, px, py}, {vgx, m00, m01}, {vgy, m10, m11}};
-    const double bb[3] = {nom, gx, gy};
+    const float A[3][3] = {{v(1), v(6), v(7)}, {v(4), v(8), v(9)}, {v(5), v(10), v(11)}};
+    const float bb[3] = {v(0), v(2), v(3)};
     double res[3];
     pinv3_solve(A, bb, res);
-    const float2 xb = W.x[b];
+    const float2 xb = W.x[b], xg = W.xg[b];
     rho_b = (res[0] + ((double)xb.x - xg.x) * res[1] + ((double)xb.y - xg.y) * res[2]) / P.rho0;
+  } else if (cnt > 0) {
+    rho_b = ((double)v(0) / (double)v(1)) / P.rho0;
   }
-  float rb = (float)fmax(rho_b, 1.0);
+  const float rb = (float)fmax(rho_b, 1.0);
   W.rho[b] = rb;
   W.vol[b] = W.area[b] / rb;
   W.p[b] = tait(rb, P);
+}
+
+// One wall per thread.
+// `scene(b)`: grid, parameters and cell offset of wall b, or null for a wall of no scene.
+struct MdbcScene {
+  const sph_grid* g;
+  const SphParams* P;
+  int coff;
+};
+template <typename Scene>
+__device__ __forceinline__ void mdbc_wall(const FluidView& F, const WallView& W, Scene&& scene) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= W.n) return;
+  const MdbcScene S = scene(b);
+  if (!S.g) return;
+  float s[kMdbcSums] = {};
+  int cnt = 0;
+  mdbc_sums<1>(W.xg[b], 0, F, *S.g, *S.P, S.coff, s, cnt);
+  mdbc_finish(b, s, 1, cnt, W, *S.P);
+}
+
+// The walls of one block: kMdbcLanes lanes sum each wall, then one lane per wall (a single warp) runs the
+// double-precision solves: a warp's FP64 instruction costs the same for 1 lane as for 32.
+template <typename Scene>
+__device__ __forceinline__ void mdbc_block(const FluidView& F, const WallView& W, Scene&& scene) {
+  __shared__ float sums[kMdbcSums][kMdbcWalls];
+  __shared__ int found[kMdbcWalls];
+  const int slot = threadIdx.x / kMdbcLanes, sub = threadIdx.x % kMdbcLanes;
+  const int b = blockIdx.x * kMdbcWalls + slot;
+  float s[kMdbcSums] = {};
+  int cnt = 0;
+  if (b < W.n) {
+    const MdbcScene S = scene(b);
+    if (S.g) mdbc_sums<kMdbcLanes>(W.xg[b], sub, F, *S.g, *S.P, S.coff, s, cnt);
+  }
+#pragma unroll
+  for (int o = 1; o < kMdbcLanes; o <<= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+  if (sub == 0) found[slot] = cnt;
+#pragma unroll
+  for (int k = 0; k < kMdbcSums; ++k) {
+    s[k] = lane_sum<kMdbcLanes>(s[k]);
+    if (sub == 0) sums[k][slot] = s[k];
+  }
+  __syncthreads();
+  const int wall = blockIdx.x * kMdbcWalls + threadIdx.x;
+  if (threadIdx.x >= kMdbcWalls || wall >= W.n) return;
+  const MdbcScene S = scene(wall);
+  if (S.g) mdbc_finish(wall, &sums[0][threadIdx.x], kMdbcWalls, found[threadIdx.x], W, *S.P);
 }
 
 // ---------------------------------------------------------------------------- neighbor records
@@ -368,10 +415,9 @@ __device__ __forceinline__ void sie_apply(int i, float2 xi, float2 vi, float rti
 }
 
 // ---------------------------------------------------------------------------- one scene
-__global__ void __launch_bounds__(128) k_mdbc(FluidView F, WallView W, const sph_grid* __restrict__ gp, SphParams P) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= W.n) return;
-  mdbc_body(b, F, W, *gp, P, 0);
+__global__ void __launch_bounds__(kMdbcThreads) k_mdbc(FluidView F, WallView W, const sph_grid* __restrict__ gp,
+                                                       SphParams P) {
+  mdbc_block(F, W, [&](int) { return MdbcScene{gp, &P, 0}; });
 }
 
 __global__ void __launch_bounds__(256) k_prep(FluidView F, SphParams P, Rec* __restrict__ rec) {
@@ -411,12 +457,22 @@ __global__ void k_sie(int n, const float2* __restrict__ x, const float2* __restr
 
 // ---------------------------------------------------------------------------- batch of scenes
 // scenes[sid[i]] gives particle i's grid, parameters, cell-table offset and time step.
+struct BatchScene {
+  const SceneDev* scenes;
+  const int32_t* wsid;
+  __device__ __forceinline__ MdbcScene operator()(int b) const {
+    const int s = wsid[b];   // negative: wall of no scene (free slot of a pooled batch)
+    return s < 0 ? MdbcScene{nullptr, nullptr, 0} : MdbcScene{&scenes[s].g, &scenes[s].P, scenes[s].coff};
+  }
+};
+__global__ void __launch_bounds__(kMdbcThreads) k_batch_mdbc_lanes(FluidView F, WallView W,
+                                                                   const SceneDev* __restrict__ scenes,
+                                                                   const int32_t* __restrict__ wsid) {
+  mdbc_block(F, W, BatchScene{scenes, wsid});
+}
 __global__ void __launch_bounds__(128, 8) k_batch_mdbc(FluidView F, WallView W, const SceneDev* __restrict__ scenes,
-                                                    const int32_t* __restrict__ wsid) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= W.n || wsid[b] < 0) return;   // wall of no scene (free slot of a pooled batch)
-  const SceneDev& S = scenes[wsid[b]];
-  mdbc_body(b, F, W, S.g, S.P, S.coff);
+                                                       const int32_t* __restrict__ wsid) {
+  mdbc_wall(F, W, BatchScene{scenes, wsid});
 }
 
 // Neighbor records and, with pairs from the cell rows (nseg != NULL), the segment lists.
@@ -586,8 +642,8 @@ sph_status_t sph_mdbc_wall_density(const sph_fluid_view* fluid, const sph_wall_v
   SPH_VIEW_CHECK(walls);
   SPH_REQUIRE(grid && params && params->support > 0.f, "mdbc: bad arguments");
   if (walls->n == 0) return SPH_OK;
-  k_mdbc<<<grid_for(walls->n, 128), 128, 0, as_stream(stream)>>>(to_fluid(fluid), to_walls(walls), grid,
-                                                                 to_params(params));
+  k_mdbc<<<grid_for(walls->n, kMdbcWalls), kMdbcThreads, 0, as_stream(stream)>>>(to_fluid(fluid), to_walls(walls),
+                                                                                  grid, to_params(params));
   SPH_CHECK_LAUNCH("mdbc_wall_density");
   return SPH_OK;
 }
@@ -711,7 +767,12 @@ sph_status_t sph_batch_deltasph_step(const sph_fluid_view* fluid, const sph_wall
   const FluidView F = to_fluid(fluid);
   const WallView W = to_walls(walls);
   const SceneDev* S = static_cast<const SceneDev*>(scenes);
-  if (W.n > 0 && (phases & SPH_PHASE_WALLS)) k_batch_mdbc<<<grid_for(W.n, 128), 128, 0, st>>>(F, W, S, wall_sid);
+  if (W.n > 0 && (phases & SPH_PHASE_WALLS))  {
+    if (W.n <= kMdbcSplitWalls)
+      k_batch_mdbc_lanes<<<grid_for(W.n, kMdbcWalls), kMdbcThreads, 0, st>>>(F, W, S, wall_sid);
+    else
+      k_batch_mdbc<<<grid_for(W.n, 128), 128, 0, st>>>(F, W, S, wall_sid);
+  }
   if (phases & SPH_PHASE_RECORDS)
     k_batch_prep<<<grid_for(n, 256), 256, 0, st>>>(F, S, sid, rec, const_cast<int32_t*>(seg.nseg),
                                                    const_cast<int32_t*>(seg.start), const_cast<uint32_t*>(seg.mask));

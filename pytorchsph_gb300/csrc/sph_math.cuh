@@ -191,6 +191,7 @@ static __device__ __noinline__ void pinv3_solve_jacobi(const double A[3][3], con
           V[k][p] = c * vkp - s * vkq;
           V[k][q] = s * vkp + c * vkq;
         }
+        S[p][q] = S[q][p] = 0.0;   // what the rotation is for; its rounding would keep the sweeps going
       }
   }
   double lmax = fmax(fmax(S[0][0], S[1][1]), S[2][2]);
@@ -207,51 +208,62 @@ static __device__ __noinline__ void pinv3_solve_jacobi(const double A[3][3], con
   }
 }
 
-__device__ inline void pinv3_solve(const double A[3][3], const double b[3], double x[3]) {
-  // Well-conditioned A (Frobenius condition bound ||A|| ||A^-1|| below 1e5, far under the
-  // 1/(3 FLT_EPSILON) at which a singular value would be dropped): pinv(A) = A^-1, applied
-  // through the adjugate.  This is the common case and costs ~50 double operations instead
-  // of the Jacobi sweeps (GB300's FP64 rate is low).
-  {
-    // cofactors a*b - c*d as fma(a, b, -(c*d)): two double operations each
-    const auto cof = [](double a, double b, double c, double d) { return fma(a, b, -(c * d)); };
-    const double c00 = cof(A[1][1], A[2][2], A[1][2], A[2][1]), c01 = cof(A[1][2], A[2][0], A[1][0], A[2][2]),
-                 c02 = cof(A[1][0], A[2][1], A[1][1], A[2][0]);
-    const double c10 = cof(A[0][2], A[2][1], A[0][1], A[2][2]), c11 = cof(A[0][0], A[2][2], A[0][2], A[2][0]),
-                 c12 = cof(A[0][1], A[2][0], A[0][0], A[2][1]);
-    const double c20 = cof(A[0][1], A[1][2], A[0][2], A[1][1]), c21 = cof(A[0][2], A[1][0], A[0][0], A[1][2]),
-                 c22 = cof(A[0][0], A[1][1], A[0][1], A[1][0]);
-    const double det = fma(A[0][0], c00, fma(A[0][1], c01, A[0][2] * c02));
-    // The bound only decides between two exact-enough paths: its norms run in float, on A
-    // scaled by its largest entry (cofactors by its square, det by its cube), so that the
-    // squares neither underflow nor overflow whatever the matrix's scale (MLS moment
-    // matrices with volumes A / rho0 have entries near 1e-12).
-    double amax = 0.0;
-    for (int r = 0; r < 3; ++r)
-      for (int c = 0; c < 3; ++c) amax = fmax(amax, fabs(A[r][c]));
-    const double is = amax > 0.0 ? 1.0 / amax : 0.0, is2 = is * is;
-    float na = 0.f;
+// x = pinv(A) b of float32 sums, solved in double.  While the Frobenius condition bound
+// ||A|| ||A^-1|| stays below 2.5e6, under the 1/(3 FLT_EPSILON) = 2.8e6 at which a singular value
+// would be dropped, pinv(A) = A^-1, applied through the adjugate; |det| > 1e-10 ||A||^3 keeps the
+// determinant's rounding below 1e-5, far under what the float32 sums contribute at such
+// conditions (the Jacobi sweeps work on A^T A and lose more).  GB300 does two double
+// operations a clock and SM, and a launch waits for its slowest wall: so A is scaled by a power
+// of two (exact) and the bounds run in float, about 60 double operations in all, and only
+// systems that may lose a singular value go to the sweeps (some 5,000 operations; with a bound
+// of 1e5 the corner walls of a tank did).
+__device__ inline void pinv3_solve(const float A[3][3], const float b[3], double x[3]) {
+  float amax = 0.f;
+  for (int r = 0; r < 3; ++r)
+    for (int c = 0; c < 3; ++c) amax = fmaxf(amax, fabsf(A[r][c]));
+  const int ex = (__float_as_int(amax) >> 23) & 255;
+  if (ex >= 2 && ex <= 252) {
+    const float sc = __int_as_float((254 - ex) << 23);   // amax * sc in [1, 2)
+    float f[3][3], na = 0.f;
+    double d[3][3];
     for (int r = 0; r < 3; ++r)
       for (int c = 0; c < 3; ++c) {
-        const float v = (float)(A[r][c] * is);
-        na += v * v;
+        f[r][c] = A[r][c] * sc;
+        na = fmaf(f[r][c], f[r][c], na);
+        d[r][c] = f[r][c];
       }
-    const float f00 = (float)(c00 * is2), f01 = (float)(c01 * is2), f02 = (float)(c02 * is2),
-                f10 = (float)(c10 * is2), f11 = (float)(c11 * is2), f12 = (float)(c12 * is2),
-                f20 = (float)(c20 * is2), f21 = (float)(c21 * is2), f22 = (float)(c22 * is2);
-    const float nc = f00 * f00 + f01 * f01 + f02 * f02 + f10 * f10 + f11 * f11 + f12 * f12 + f20 * f20 +
-                     f21 * f21 + f22 * f22;
-    const double ds = det * is2 * is;
-    // ||A^-1||_F = ||adj A||_F / |det|, all three scaled alike
-    if (det != 0.0 && amax > 0.0 && (double)na * (double)nc < 1e10 * ds * ds) {
-      const double id = 1.0 / det;  // A^-1 = adj(A) / det, adj(A)[r][c] = cofactor c_cr
-      x[0] = fma(c00, b[0], fma(c10, b[1], c20 * b[2])) * id;
-      x[1] = fma(c01, b[0], fma(c11, b[1], c21 * b[2])) * id;
-      x[2] = fma(c02, b[0], fma(c12, b[1], c22 * b[2])) * id;
+    // cofactor (r, c) = a b - c d as fma(a, b, -(c d)); in float only for the norm
+    const auto cof = [](double p, double q, double u, double v) { return fma(p, q, -(u * v)); };
+    const auto sqr = [](float p, float q, float u, float v) {
+      const float c = fmaf(p, q, -(u * v));
+      return c * c;
+    };
+    const double c00 = cof(d[1][1], d[2][2], d[1][2], d[2][1]), c01 = cof(d[1][2], d[2][0], d[1][0], d[2][2]),
+                 c02 = cof(d[1][0], d[2][1], d[1][1], d[2][0]);
+    const double det = fma(d[0][0], c00, fma(d[0][1], c01, d[0][2] * c02));
+    const float nc = sqr(f[1][1], f[2][2], f[1][2], f[2][1]) + sqr(f[1][2], f[2][0], f[1][0], f[2][2]) +
+                     sqr(f[1][0], f[2][1], f[1][1], f[2][0]) + sqr(f[0][2], f[2][1], f[0][1], f[2][2]) +
+                     sqr(f[0][0], f[2][2], f[0][2], f[2][0]) + sqr(f[0][1], f[2][0], f[0][0], f[2][1]) +
+                     sqr(f[0][1], f[1][2], f[0][2], f[1][1]) + sqr(f[0][2], f[1][0], f[0][0], f[1][2]) +
+                     sqr(f[0][0], f[1][1], f[0][1], f[1][0]);
+    const float ds = (float)det, ds2 = ds * ds;
+    // ||A^-1||_F = ||adj A||_F / |det|
+    if (na * nc < 6.25e12f * ds2 && ds2 > 1e-20f * (na * na * na)) {
+      const double c10 = cof(d[0][2], d[2][1], d[0][1], d[2][2]), c11 = cof(d[0][0], d[2][2], d[0][2], d[2][0]),
+                   c12 = cof(d[0][1], d[2][0], d[0][0], d[2][1]);
+      const double c20 = cof(d[0][1], d[1][2], d[0][2], d[1][1]), c21 = cof(d[0][2], d[1][0], d[0][0], d[1][2]),
+                   c22 = cof(d[0][0], d[1][1], d[0][1], d[1][0]);
+      const double id = (double)sc / det;  // A^-1 = sc adj(sc A) / det(sc A), adj(A)[r][c] = cofactor c_cr
+      const double b0 = b[0], b1 = b[1], b2 = b[2];
+      x[0] = fma(c00, b0, fma(c10, b1, c20 * b2)) * id;
+      x[1] = fma(c01, b0, fma(c11, b1, c21 * b2)) * id;
+      x[2] = fma(c02, b0, fma(c12, b1, c22 * b2)) * id;
       return;
     }
   }
-  pinv3_solve_jacobi(A, b, x);
+  const double Ad[3][3] = {{A[0][0], A[0][1], A[0][2]}, {A[1][0], A[1][1], A[1][2]}, {A[2][0], A[2][1], A[2][2]}};
+  const double bd[3] = {b[0], b[1], b[2]};
+  pinv3_solve_jacobi(Ad, bd, x);
 }
 
 // Iterate the wall particles whose cell is within +-r of fluid cell (cx, cy) and that pass
@@ -275,23 +287,37 @@ __device__ __forceinline__ void for_each_wall(const WallView& W, const sph_grid&
   }
 }
 
+// The members of the cells within r of (cx, cy) that a cell table lists, dealt to kLanes
+// consecutive lanes: f(j) for every kLanes-th member j.  Three rows of cells at a time: their six
+// bounds are loaded together and the rows are walked as one range, so that a lane's chain is
+// the bounds and then members that do not wait for each other.
+template <int kLanes, typename Fn>
+__device__ __forceinline__ void for_each_member(const int32_t* __restrict__ cs, const sph_grid& g, int r, int cx,
+                                                int cy, int sub, Fn&& f) {
+  const int x0 = max(cx - r, 0), x1 = min(cx + r, g.cells_x - 1);
+  if (x0 > x1) return;
+  const int y1 = min(cy + r, g.cells_y - 1);
+  for (int yy = max(cy - r, 0); yy <= y1; yy += 3) {
+    const int32_t* row = cs + (int64_t)yy * g.cells_x;
+    const int two = yy + 1 <= y1 ? g.cells_x : 0, three = yy + 2 <= y1 ? 2 * g.cells_x : 0;
+    const int b0 = __ldg(row + x0), b1 = __ldg(row + two + x0), b2 = __ldg(row + three + x0);
+    const int n0 = __ldg(row + x1 + 1) - b0;
+    const int e1 = __ldg(row + two + x1 + 1), e2 = __ldg(row + three + x1 + 1);
+    const int n1 = two ? n0 + e1 - b1 : n0, n2 = three ? n1 + e2 - b2 : n1;   // members up to each row's end
+#pragma unroll 2
+    for (int t = sub; t < n2; t += kLanes) f(t < n0 ? b0 + t : t < n1 ? b1 + t - n0 : b2 + t - n1);
+  }
+}
+
 // for_each_wall shared by kLanes consecutive lanes (one particle's): lane `sub` takes every
-// kLanes-th wall of each cell row.
+// kLanes-th wall of the cells.
 template <int kLanes, typename F>
 __device__ __forceinline__ void for_each_wall_lanes(const WallView& W, const sph_grid& g, int r, int cx, int cy,
                                                     float xf, float yf, float thr_b, int sub, F&& f, int coff = 0) {
-  const int x0 = max(cx - r, 0), x1 = min(cx + r, g.cells_x - 1);
-  if (x0 > x1) return;
-  const int y0 = max(cy - r, 0), y1 = min(cy + r, g.cells_y - 1);
-  const int32_t* cs = W.cell_start + coff;
-  for (int yy = y0; yy <= y1; ++yy) {
-    const int row = yy * g.cells_x;
-    const int b0 = __ldg(cs + row + x0), b1 = __ldg(cs + row + x1 + 1);
-    for (int b = b0 + sub; b < b1; b += kLanes) {
-      const float2 xb = __ldg(W.x + b);
-      if (dist2_ref(xb.x, xb.y, xf, yf) <= thr_b) f(b, xb);
-    }
-  }
+  for_each_member<kLanes>(W.cell_start + coff, g, r, cx, cy, sub, [&](int b) {
+    const float2 xb = __ldg(W.x + b);
+    if (dist2_ref(xb.x, xb.y, xf, yf) <= thr_b) f(b, xb);
+  });
 }
 
 // Sum of v over the kLanes consecutive lanes of one particle (every lane gets the sum; the

@@ -193,8 +193,8 @@ __global__ void __launch_bounds__(128) k_wall_side_term(WallTermIn in, SphParams
     double rho_b = 1.0;
     if (cnt > 0) rho_b = ((double)nom / (double)den) / P.rho0;
     if (cnt > 10) {
-      const double A[3][3] = {{den, px, py}, {vgx, m00, m01}, {vgy, m10, m11}};
-      const double bb[3] = {nom, gx, gy};
+      const float A[3][3] = {{den, px, py}, {vgx, m00, m01}, {vgy, m10, m11}};
+      const float bb[3] = {nom, gx, gy};
       double res[3];
       pinv3_solve(A, bb, res);
       const float2 xb = in.wpos[b];
@@ -339,8 +339,8 @@ __global__ void __launch_bounds__(128) k_wall_mls_pressure(WallTermIn in, SphPar
     m12 += 2.0f * (dx * dy) * t;
     m22 += 2.0f * (dy * dy) * t;
   }
-  const double A[3][3] = {{m00, m01, m02}, {m01, m11, m12}, {m02, m12, m22}};
-  const double e1[3] = {1.0, 0.0, 0.0};
+  const float A[3][3] = {{m00, m01, m02}, {m01, m11, m12}, {m02, m12, m22}};
+  const float e1[3] = {1.f, 0.f, 0.f};
   double c[3];
   pinv3_solve(A, e1, c);
   float s = 0.f;
