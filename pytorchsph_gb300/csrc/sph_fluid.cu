@@ -28,41 +28,39 @@
 namespace sph {
 
 // ---------------------------------------------------------------------------- mDBC
-// Shepard and first-order MLS sums over the fluid particles within h of wall b's ghost, shared by
-// kLanes lanes, then the 3x3 pseudo-inverse solve, wall density, volume and Tait pressure.
-// Latency-bound: one scene has few walls, each a chain of ~80 candidate loads and a solve on the
-// FP64 pipe.  1,380 walls 20 -> 7.3 us a launch (8 / 32 lanes: 7.8 / 6.8), 5,976 walls 35 ->
-// 7.8 us (8.0 / 7.7); the 210,000 walls of 50 served tanks fill the GPU with one lane each and
-// take 78 -> 36 us with the shorter solve (119 with 8 lanes and the long one).
-constexpr int kMdbcSums = 12;
-constexpr int kMdbcSplitWalls = 32768;   // up to here kMdbcLanes lanes per wall
-constexpr int kMdbcLanes = 16, kMdbcThreads = 256, kMdbcWalls = kMdbcThreads / kMdbcLanes;
+// Shepard and first-order MLS sums over the fluid particles within h of wall b's ghost, then the
+// 3x3 pseudo-inverse solve, wall density, volume and Tait pressure.  One scene has few walls,
+// so its launch is one wall's chain: a cell row's candidates are tested 32 at a time (all loads
+// in flight), the accepted ones summed with four records in flight, and kLanes = 4 lanes take a
+// row each.  Every row is summed by itself and the rows are added in order, so a wall's sums
+// are the same with 1 lane, which a batch's hundreds of thousands of walls fill the GPU with.
+// 1,380 walls 20 -> 10.2 us a launch, 5,976 walls 35 -> 9.3 us, the 210,000 walls of 50 served
+// tanks 78 -> 34 us, most of it by the shorter solve (pinv3_solve).
+struct MdbcRec {
+  float2 x;
+  float area, rho;
+};
 
-// float sums (GB300's FP64 rate is low); the 3x3 solve runs in double
-template <int kLanes>
-__device__ __forceinline__ void mdbc_sums(float2 xg, int sub, const FluidView& F, const sph_grid& g,
-                                          const SphParams& P, int coff, float (&s)[kMdbcSums], int& cnt) {
-  const float thr = P.thr;
-  const int32_t* cs = F.cell_start + coff;
-  if (!grid_ok(g, P.cell_capacity)) return;
-  const float fcx = ceilf(__fdiv_rn(__fsub_rn(xg.x, g.qmin[0]), g.hmax));
-  const float fcy = ceilf(__fdiv_rn(__fsub_rn(xg.y, g.qmin[1]), g.hmax));
-  if (!(fcx > -1e9f && fcx < 1e9f && fcy > -1e9f && fcy < 1e9f)) return;
-  for_each_member<kLanes>(cs, g, P.search_radius, (int)fcx, (int)fcy, sub, [&](int j) {
-    const float2 xj = F.x[j];
-    const float Aj = F.area[j], rj = F.rho[j];   // loaded beside the position: one latency per member
-    if (!(dist2_ref(xg.x, xg.y, xj.x, xj.y) <= thr)) return;
+constexpr int kMdbcSums = 12;
+constexpr int kMdbcSplitWalls = 32768;   // walls up to which a launch takes 4 lanes per wall
+
+// s += the sums of the candidates [j0, j1) of one cell row; float sums (GB300's FP64 rate is
+// low), the 3x3 solve runs in double.
+__device__ __forceinline__ int mdbc_row(float2 xg, int j0, int j1, const FluidView& F, const SphParams& P,
+                                        float (&s)[kMdbcSums]) {
+  int cnt = 0;
+  const auto use = [&](const MdbcRec& f) {
     // e = (x_g - x_j) / r from one rsqrt (zero below r = 1e-7, as the reference's e_ij)
-    const float dx = xg.x - xj.x, dy = xg.y - xj.y;
+    const float dx = xg.x - f.x.x, dy = xg.y - f.x.y;
     const float r2 = dx * dx + dy * dy;
     const float ir = r2 >= 1e-14f ? rsqrt_normal(r2) : 0.f;
     const float q = r2 * ir * P.inv_h;
     const float k = kW(q, P.c_w);
     const float gwr = kGW(q, P.c_g) * ir;
     const float ggx = gwr * dx, ggy = gwr * dy;
-    const float mass = Aj * P.rho0;
-    const float Vj = Aj * rcp_normal(rj);
-    const float xx = xj.x - xg.x, xy = xj.y - xg.y;
+    const float mass = f.area * P.rho0;
+    const float Vj = f.area * rcp_normal(f.rho);
+    const float xx = f.x.x - xg.x, xy = f.x.y - xg.y;
     s[0] += mass * k;        // Shepard numerator and denominator
     s[1] += Vj * k;
     s[2] += mass * ggx;      // first-order MLS: gradient sums and moments
@@ -75,76 +73,96 @@ __device__ __forceinline__ void mdbc_sums(float2 xg, int sub, const FluidView& F
     s[9] += Vj * xx * ggy;
     s[10] += Vj * xy * ggx;
     s[11] += Vj * xy * ggy;
-    ++cnt;
-  });
+  };
+  const auto load = [&](int j) { return MdbcRec{__ldg(F.x + j), __ldg(F.area + j), __ldg(F.rho + j)}; };
+  for (int c = j0; c < j1; c += 32) {
+    uint32_t w = c + 32 <= F.n ? segment_mask_full(F.x, c, j1, xg.x, xg.y, P.thr)
+                               : segment_mask(F.x, c, j1, xg.x, xg.y, P.thr);
+    cnt += __popc(w);
+    while (w) {
+      int j[4];
+      bool ok[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        ok[t] = w != 0;
+        j[t] = ok[t] ? c - 1 + __ffs(w) : c;
+        w &= w - 1;   // 0 stays 0
+      }
+      const MdbcRec f0 = load(j[0]), f1 = load(j[1]), f2 = load(j[2]), f3 = load(j[3]);
+      use(f0);
+      if (ok[1]) use(f1);
+      if (ok[2]) use(f2);
+      if (ok[3]) use(f3);
+    }
+  }
+  return cnt;
 }
 
-__device__ __forceinline__ void mdbc_finish(int b, const float* s, int stride, int cnt, const WallView& W,
-                                            const SphParams& P) {
-  const auto v = [&](int k) { return s[k * stride]; };
+// Lane `sub` of wall b's kLanes; `live` false: a lane that only takes part in the sums.
+template <int kLanes>
+__device__ __forceinline__ void mdbc_body(int b, bool live, int sub, const FluidView& F, const WallView& W,
+                                          const sph_grid& g, const SphParams& P, int coff) {
+  const float2 xg = W.xg[b];
+  float s[kMdbcSums] = {};
+  int cnt = 0;
+  const int32_t* cs = F.cell_start + coff;
+  int x0 = 0, x1 = -1, y0 = 0, rows = 0;
+  if (live && grid_ok(g, P.cell_capacity)) {
+    const float fcx = ceilf(__fdiv_rn(__fsub_rn(xg.x, g.qmin[0]), g.hmax));
+    const float fcy = ceilf(__fdiv_rn(__fsub_rn(xg.y, g.qmin[1]), g.hmax));
+    if (fcx > -1e9f && fcx < 1e9f && fcy > -1e9f && fcy < 1e9f) {
+      const int cx = (int)fcx, cy = (int)fcy, r = P.search_radius;
+      x0 = max(cx - r, 0);
+      x1 = min(cx + r, g.cells_x - 1);
+      y0 = max(cy - r, 0);
+      rows = x0 <= x1 ? max(min(cy + r, g.cells_y - 1) - y0 + 1, 0) : 0;
+    }
+  }
+  const auto row_sums = [&](int q, float (&t)[kMdbcSums]) {
+    const int32_t* row = cs + (y0 + q) * g.cells_x;
+    return mdbc_row(xg, __ldg(row + x0), __ldg(row + x1 + 1), F, P, t);
+  };
+  if constexpr (kLanes == 1) {
+    for (int q = 0; q < rows; ++q) {
+      float t[kMdbcSums] = {};
+      cnt += row_sums(q, t);
+#pragma unroll
+      for (int k = 0; k < kMdbcSums; ++k) s[k] += t[k];
+    }
+  } else {
+    for (int q = 0; __any_sync(0xffffffffu, q < rows); q += kLanes) {
+      float t[kMdbcSums] = {};
+      int c = q + sub < rows ? row_sums(q + sub, t) : 0;
+#pragma unroll
+      for (int k = 0; k < kMdbcSums; ++k) {
+        s[k] += t[k];   // lane 0: the first row; the others' come in order
+#pragma unroll
+        for (int l = 1; l < kLanes; ++l) {
+          const float v = __shfl_sync(0xffffffffu, t[k], l, kLanes);
+          if (sub == 0) s[k] += v;
+        }
+      }
+#pragma unroll
+      for (int o = 1; o < kLanes; o <<= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+      cnt += c;
+    }
+  }
+  if (!live || sub != 0) return;
   double rho_b = 1.0;
   if (cnt > 10) {
-    const float A[3][3] = {{v(1), v(6), v(7)}, {v(4), v(8), v(9)}, {v(5), v(10), v(11)}};
-    const float bb[3] = {v(0), v(2), v(3)};
+    const float A[3][3] = {{s[1], s[6], s[7]}, {s[4], s[8], s[9]}, {s[5], s[10], s[11]}};
+    const float bb[3] = {s[0], s[2], s[3]};
     double res[3];
     pinv3_solve(A, bb, res);
-    const float2 xb = W.x[b], xg = W.xg[b];
+    const float2 xb = W.x[b];
     rho_b = (res[0] + ((double)xb.x - xg.x) * res[1] + ((double)xb.y - xg.y) * res[2]) / P.rho0;
   } else if (cnt > 0) {
-    rho_b = ((double)v(0) / (double)v(1)) / P.rho0;
+    rho_b = ((double)s[0] / (double)s[1]) / P.rho0;
   }
   const float rb = (float)fmax(rho_b, 1.0);
   W.rho[b] = rb;
   W.vol[b] = W.area[b] / rb;
   W.p[b] = tait(rb, P);
-}
-
-// One wall per thread.
-// `scene(b)`: grid, parameters and cell offset of wall b, or null for a wall of no scene.
-struct MdbcScene {
-  const sph_grid* g;
-  const SphParams* P;
-  int coff;
-};
-template <typename Scene>
-__device__ __forceinline__ void mdbc_wall(const FluidView& F, const WallView& W, Scene&& scene) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= W.n) return;
-  const MdbcScene S = scene(b);
-  if (!S.g) return;
-  float s[kMdbcSums] = {};
-  int cnt = 0;
-  mdbc_sums<1>(W.xg[b], 0, F, *S.g, *S.P, S.coff, s, cnt);
-  mdbc_finish(b, s, 1, cnt, W, *S.P);
-}
-
-// The walls of one block: kMdbcLanes lanes sum each wall, then one lane per wall (a single warp) runs the
-// double-precision solves: a warp's FP64 instruction costs the same for 1 lane as for 32.
-template <typename Scene>
-__device__ __forceinline__ void mdbc_block(const FluidView& F, const WallView& W, Scene&& scene) {
-  __shared__ float sums[kMdbcSums][kMdbcWalls];
-  __shared__ int found[kMdbcWalls];
-  const int slot = threadIdx.x / kMdbcLanes, sub = threadIdx.x % kMdbcLanes;
-  const int b = blockIdx.x * kMdbcWalls + slot;
-  float s[kMdbcSums] = {};
-  int cnt = 0;
-  if (b < W.n) {
-    const MdbcScene S = scene(b);
-    if (S.g) mdbc_sums<kMdbcLanes>(W.xg[b], sub, F, *S.g, *S.P, S.coff, s, cnt);
-  }
-#pragma unroll
-  for (int o = 1; o < kMdbcLanes; o <<= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-  if (sub == 0) found[slot] = cnt;
-#pragma unroll
-  for (int k = 0; k < kMdbcSums; ++k) {
-    s[k] = lane_sum<kMdbcLanes>(s[k]);
-    if (sub == 0) sums[k][slot] = s[k];
-  }
-  __syncthreads();
-  const int wall = blockIdx.x * kMdbcWalls + threadIdx.x;
-  if (threadIdx.x >= kMdbcWalls || wall >= W.n) return;
-  const MdbcScene S = scene(wall);
-  if (S.g) mdbc_finish(wall, &sums[0][threadIdx.x], kMdbcWalls, found[threadIdx.x], W, *S.P);
 }
 
 // ---------------------------------------------------------------------------- neighbor records
@@ -199,6 +217,11 @@ __device__ __forceinline__ PairG pair_g(float xi, float yi, float xj, float yj, 
 // sums the parts it can, ddiff = 2 sum_j (rho_j - rho_i) (x_ji . gradW) V_j / (|x_ji|^2 + eps)
 // - <grad rho>_i . sum_j V_j gradW_ij, and the diffusion pass subtracts
 // sum_j (<grad rho>_j V_j) . gradW_ij, the only part that needs the neighbors' gradients.
+struct WallRec {
+  float2 x;
+  float vol, rho, p;
+};
+
 struct Pass1 {
   float dpdt, ax, ay;
   float4 L;        // renormalization matrix, fluid + walls
@@ -206,12 +229,13 @@ struct Pass1 {
   float ddiff;     // deltaSPH: the pass-1 part of D_i
 };
 
-// kTpp lanes per particle (kCells only): lane `sub` sums its share of the pairs, the lanes
-// add their sums, and lane 0 finishes (walls, gravity, L^+); the other lanes return a zero
+// kTpp lanes per particle (kCells only): lane `sub` sums its share of the pairs and walls, the
+// lanes add their sums, and lane 0 finishes (gravity, L^+); the other lanes return a zero
 // record.  `live` false: a lane past the last particle, which only takes part in the sums.
 // kScheme: the density diffusion (0 none, 1 MOG, 2 deltaSPH) fixed at compile time, or -1:
-// read from P.diffusion.
-template <bool kCells, int kTpp = 1, int kScheme = -1>
+// read from P.diffusion.  kByFour (kCells, one lane): four pairs' records in flight at a time,
+// and the walls' bounds together; the same sums in the same order, for small launches.
+template <bool kCells, int kTpp = 1, int kScheme = -1, bool kByFour = false>
 __device__ __forceinline__ Pass1 pass1_body(int i, const FluidView& F, const Rec* __restrict__ rec,
                                             const WallView& W, const sph_grid& g,
                                             const SphParams& P, int coff, const Segments& S, int sub = 0,
@@ -224,8 +248,9 @@ __device__ __forceinline__ Pass1 pass1_body(int i, const FluidView& F, const Rec
   float dp_f = 0.f, mog = 0.f, bx = 0.f, by = 0.f;   // b = sum_j V_j gradW_ij (deltaSPH)
   float pax = 0.f, pay = 0.f, vax = 0.f, vay = 0.f, lax = 0.f, lay = 0.f;
   float l00 = 0.f, l01 = 0.f, l11 = 0.f, gfx = 0.f, gfy = 0.f;
-  auto fluid_pair = [&](int j) {
-    const float4 sj = __ldg(&rec[j].xv), qj = __ldg(&rec[j].q);
+  const auto load = [&](int j) { return Rec{__ldg(&rec[j].xv), __ldg(&rec[j].q)}; };
+  const auto fluid_pair = [&](const Rec& other) {
+    const float4 sj = other.xv, qj = other.q;
     const float rhoj = qj.x, Vj = qj.y, pVj = qj.z, mj = qj.w;
     const PairG e = pair_g(si.x, si.y, sj.x, sj.y, P);   // gradW = e.gd * d
     const float ux = sj.z - si.z, uy = sj.w - si.w;       // u_j - u_i
@@ -264,12 +289,17 @@ __device__ __forceinline__ Pass1 pass1_body(int i, const FluidView& F, const Rec
     }
   };
   if constexpr (kCells) {
-    if (live) stored_pairs<kTpp>(i, F, g, coff, P.search_radius, S.nseg, S.start, S.mask, si.x, si.y, P.thr,
-                                 fluid_pair, sub);
+    if constexpr (kByFour) {
+      stored_pairs_by_four(i, F, g, coff, P.search_radius, S.nseg, S.start, S.mask, si.x, si.y, P.thr, load,
+                           fluid_pair);
+    } else {
+      if (live) stored_pairs<kTpp>(i, F, g, coff, P.search_radius, S.nseg, S.start, S.mask, si.x, si.y, P.thr,
+                                   [&](int j) { fluid_pair(load(j)); }, sub);
+    }
   } else {
     static_assert(kTpp == 1, "CSR rows run one lane per particle");
     const int k0 = F.offsets[i], k1 = row_end(F, i, k0);
-    for (int k = k0; k < k1; ++k) fluid_pair(__ldg(F.cols + k));
+    for (int k = k0; k < k1; ++k) fluid_pair(load(__ldg(F.cols + k)));
   }
   if constexpr (kTpp > 1) {
     dp_f = lane_sum<kTpp>(dp_f);
@@ -287,44 +317,71 @@ __device__ __forceinline__ Pass1 pass1_body(int i, const FluidView& F, const Rec
     gfy = lane_sum<kTpp>(gfy);
     bx = lane_sum<kTpp>(bx);
     by = lane_sum<kTpp>(by);
-    if (sub != 0 || !live) return Pass1{};
   }
   float dp_w = 0.f, pwx = 0.f, pwy = 0.f, vwx = 0.f, vwy = 0.f;
   float w00 = 0.f, w01 = 0.f, w10 = 0.f, w11 = 0.f, gwx = 0.f, gwy = 0.f;
   if (W.n > 0) {
-    int cx, cy;
-    cell_of(F.keys[i] - (uint32_t)coff, g, &cx, &cy);
     const float thr = P.thr;
-    for_each_wall(
-        W, g, P.search_radius, cx, cy, si.x, si.y, thr,
-        [&](int b, float2 xb) {
-          const PairG e = pair_g(si.x, si.y, xb.x, xb.y, P);   // fluid side: d = x_f - x_b
-          const float Vb = W.vol[b], rhob = W.rho[b] * P.rho0, pb = W.p[b];
-          const float ud = -(si.z * e.dx + si.w * e.dy);       // (u_b - u_f) . d, walls at rest
-          dp_w -= e.gd * ud * Vb * rhob;
-          const float pf = (pi + pb) * Vb * e.gd;
-          pwx += pf * e.dx;
-          pwy += pf * e.dy;
-          if (P.boundary_diffusion) {
-            const float vf = fminf(-ud, 0.f) * rcp_normal(e.r2 + P.eps) * Vb * rhob *
-                             rcp_normal(rhoi + rhob) * e.gd;
-            vwx += vf * e.dx;
-            vwy += vf * e.dy;
-          }
-          if (renorm) {
-            const float t = Vb * e.gd;
-            const float tx = t * e.dx, ty = t * e.dy;
-            w00 -= tx * e.dx;
-            w01 -= tx * e.dy;
-            w10 -= ty * e.dx;
-            w11 -= ty * e.dy;
-            const float s = (rhob - rhoi) * 2.0f * t;
-            gwx += s * e.dx;
-            gwy += s * e.dy;
-          }
-        },
-        coff);
+    bool any = false;   // a wall of this lane's (kTpp > 1)
+    const auto load_wall = [&](int b) { return WallRec{__ldg(W.x + b), W.vol[b], W.rho[b], W.p[b]}; };
+    const auto wall_pair = [&](const WallRec& wall) {
+      any = true;
+      const PairG e = pair_g(si.x, si.y, wall.x.x, wall.x.y, P);   // fluid side: d = x_f - x_b
+      const float Vb = wall.vol, rhob = wall.rho * P.rho0, pb = wall.p;
+      const float ud = -(si.z * e.dx + si.w * e.dy);       // (u_b - u_f) . d, walls at rest
+      dp_w -= e.gd * ud * Vb * rhob;
+      const float pf = (pi + pb) * Vb * e.gd;
+      pwx += pf * e.dx;
+      pwy += pf * e.dy;
+      if (P.boundary_diffusion) {
+        const float vf = fminf(-ud, 0.f) * rcp_normal(e.r2 + P.eps) * Vb * rhob *
+                         rcp_normal(rhoi + rhob) * e.gd;
+        vwx += vf * e.dx;
+        vwy += vf * e.dy;
+      }
+      if (renorm) {
+        const float t = Vb * e.gd;
+        const float tx = t * e.dx, ty = t * e.dy;
+        w00 -= tx * e.dx;
+        w01 -= tx * e.dy;
+        w10 -= ty * e.dx;
+        w11 -= ty * e.dy;
+        const float s = (rhob - rhoi) * 2.0f * t;
+        gwx += s * e.dx;
+        gwy += s * e.dy;
+      }
+    };
+    if (kTpp == 1 || live) {
+      int cx, cy;
+      cell_of(F.keys[i] - (uint32_t)coff, g, &cx, &cy);
+      if constexpr (kByFour) {
+        for_each_wall_by_four(W, g, P.search_radius, cx, cy, si.x, si.y, thr, load_wall, wall_pair, coff);
+      } else if constexpr (kTpp == 1) {
+        for_each_wall(W, g, P.search_radius, cx, cy, si.x, si.y, thr,
+                      [&](int b, float2 xb) { wall_pair(WallRec{xb, W.vol[b], W.rho[b], W.p[b]}); }, coff);
+      } else {
+        for_each_wall_lanes<kTpp>(W, g, P.search_radius, cx, cy, si.x, si.y, thr, sub,
+                                  [&](int b, float2 xb) { wall_pair(WallRec{xb, W.vol[b], W.rho[b], W.p[b]}); },
+                                  coff);
+      }
+    }
+    if constexpr (kTpp > 1) {
+      if (__any_sync(0xffffffffu, any)) {
+        dp_w = lane_sum<kTpp>(dp_w);
+        pwx = lane_sum<kTpp>(pwx);
+        pwy = lane_sum<kTpp>(pwy);
+        vwx = lane_sum<kTpp>(vwx);
+        vwy = lane_sum<kTpp>(vwy);
+        w00 = lane_sum<kTpp>(w00);
+        w01 = lane_sum<kTpp>(w01);
+        w10 = lane_sum<kTpp>(w10);
+        w11 = lane_sum<kTpp>(w11);
+        gwx = lane_sum<kTpp>(gwx);
+        gwy = lane_sum<kTpp>(gwy);
+      }
+    }
   }
+  if (kTpp > 1 && (sub != 0 || !live)) return Pass1{};
   Pass1 o;
   o.dpdt = dp_f + dp_w;
   if (scheme == 1) o.dpdt += P.diff_k * (2.0f * mog);
@@ -371,30 +428,37 @@ __device__ __forceinline__ Pass1 pass1_body(int i, const FluidView& F, const Rec
 // so); otherwise it holds <grad rho> and V_j comes from the neighbor record (the same
 // product, so both give the same bits).  kCells: pairs from the segment lists instead of the
 // CSR row.
-template <bool kCells, int kTpp = 1, bool kHoldsGV = true>
+struct DiffRec {
+  float2 x, g;
+  float V;
+};
+
+template <bool kCells, int kTpp = 1, bool kHoldsGV = true, bool kByFour = false>
 __device__ __forceinline__ float diffusion_sum(int i, const FluidView& F, const Rec* __restrict__ rec,
                                                const SphParams& P, const float2* __restrict__ gbuf,
                                                const sph_grid& g, int coff, const Segments& S, int sub = 0,
                                                bool live = true) {
   const float2 xi = F.x[i];
   float acc = 0.f;
-  auto pair = [&](int j) {
-    const float2 xj = __ldg(F.x + j);
-    float2 gv = __ldg(gbuf + j);
-    if constexpr (!kHoldsGV) {
-      const float Vj = __ldg(&rec[j].q.y);
-      gv = make_float2(gv.x * Vj, gv.y * Vj);
-    }
+  const auto load = [&](int j) { return DiffRec{__ldg(F.x + j), __ldg(gbuf + j), kHoldsGV ? 0.f : __ldg(&rec[j].q.y)}; };
+  const auto pair = [&](const DiffRec& other) {
+    const float2 xj = other.x;
+    float2 gv = other.g;
+    if constexpr (!kHoldsGV) gv = make_float2(gv.x * other.V, gv.y * other.V);
     const PairG e = pair_g<false>(xi.x, xi.y, xj.x, xj.y, P);   // gk after the sum
     acc += (gv.x * e.dx + gv.y * e.dy) * e.gd;
   };
   if constexpr (kCells) {
-    if (live) stored_pairs<kTpp, true>(i, F, g, coff, P.search_radius, S.nseg, S.start, S.mask, xi.x, xi.y, P.thr,
-                                       pair, sub);
+    if constexpr (kByFour) {
+      stored_pairs_by_four(i, F, g, coff, P.search_radius, S.nseg, S.start, S.mask, xi.x, xi.y, P.thr, load, pair);
+    } else {
+      if (live) stored_pairs<kTpp, true>(i, F, g, coff, P.search_radius, S.nseg, S.start, S.mask, xi.x, xi.y, P.thr,
+                                         [&](int j) { pair(load(j)); }, sub);
+    }
   } else {
     static_assert(kTpp == 1, "CSR rows run one lane per particle");
     const int k0 = F.offsets[i], k1 = row_end(F, i, k0);
-    for (int k = k0; k < k1; ++k) pair(__ldg(F.cols + k));
+    for (int k = k0; k < k1; ++k) pair(load(__ldg(F.cols + k)));
   }
   return lane_sum<kTpp>(acc) * P.gk;
 }
@@ -415,9 +479,11 @@ __device__ __forceinline__ void sie_apply(int i, float2 xi, float2 vi, float rti
 }
 
 // ---------------------------------------------------------------------------- one scene
-__global__ void __launch_bounds__(kMdbcThreads) k_mdbc(FluidView F, WallView W, const sph_grid* __restrict__ gp,
-                                                       SphParams P) {
-  mdbc_block(F, W, [&](int) { return MdbcScene{gp, &P, 0}; });
+template <int kLanes>
+__global__ void __launch_bounds__(128) k_mdbc(FluidView F, WallView W, const sph_grid* __restrict__ gp, SphParams P) {
+  const int b = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+  if (kLanes == 1 && b >= W.n) return;
+  mdbc_body<kLanes>(min(b, W.n - 1), b < W.n, threadIdx.x % kLanes, F, W, *gp, P, 0);
 }
 
 __global__ void __launch_bounds__(256) k_prep(FluidView F, SphParams P, Rec* __restrict__ rec) {
@@ -426,24 +492,94 @@ __global__ void __launch_bounds__(256) k_prep(FluidView F, SphParams P, Rec* __r
   prep_body(i, F, P, rec);
 }
 
+// Neighbor record and segment list of particle i by kRowLanes lanes, for launches too small to
+// hide one thread's chain of candidate tests: a lane takes a cell row each, at the place that the
+// rows before it leave (a row's segments by its length, empty ones among them, so no lane waits
+// for another's tests).  `live` false: a lane that only takes part.  Records and segments of
+// 8,192 particles 6.1 -> 4.7 us, 16,384: 6.9 -> 5.1, 36,864: 7.0 -> 7.1, 65,536: 7.3 -> 9.6.
+constexpr int kRowLanes = 4;
+constexpr int kRowLanesMax = 32768;   // particles up to which it is faster
+
+__device__ __forceinline__ void prep_rows(int i, bool live, int sub, const FluidView& F, const sph_grid& g, int coff,
+                                          const SphParams& P, Rec* __restrict__ rec, int32_t* __restrict__ nseg,
+                                          int32_t* __restrict__ seg_start, uint32_t* __restrict__ seg_mask) {
+  const size_t n = (size_t)F.n;
+  int cx = 0, cy = -(1 << 20);
+  float2 xi = make_float2(0.f, 0.f);
+  if (live) {
+    cell_of(F.keys[i] - (uint32_t)coff, g, &cx, &cy);
+    xi = F.x[i];
+    if (sub == kRowLanes - 1) prep_body(i, F, P, rec);
+  }
+  const int r = P.search_radius;
+  const int x0 = max(cx - r, 0), x1 = min(cx + r, g.cells_x - 1), y0 = max(cy - r, 0);
+  const int rows = live && x0 <= x1 ? min(cy + r, g.cells_y - 1) - y0 + 1 : 0;
+  int first = 0;   // segments of the rows already placed
+  for (int q = 0; __any_sync(0xffffffffu, q < rows); q += kRowLanes) {
+    int b = 0, e = 0;
+    if (q + sub < rows) {
+      const int32_t* row = F.cell_start + coff + (y0 + q + sub) * g.cells_x;
+      b = __ldg(row + x0);
+      e = __ldg(row + x1 + 1);
+    }
+    const int mine = (e - b + 31) >> 5;
+    int k = mine, all = mine;
+#pragma unroll
+    for (int o = 1; o < kRowLanes; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, k, o, kRowLanes);
+      if (sub >= o) k += v;
+      all += __shfl_xor_sync(0xffffffffu, all, o);
+    }
+    k += first - mine;
+    first += all;
+    for (int c = b; c < e && k < kMaxSegments; c += 32, ++k) {
+      seg_start[k * n + i] = c;
+      seg_mask[k * n + i] = c + 32 <= F.n ? segment_mask_full(F.x, c, e, xi.x, xi.y, P.thr)
+                                          : segment_mask(F.x, c, e, xi.x, xi.y, P.thr);
+    }
+  }
+  if (live && sub == 0) nseg[i] = first <= kMaxSegments ? first : -1;
+}
+
+// Neighbor records and segment lists of one scene, kLanes (1 or kRowLanes) per particle.
+template <int kLanes>
+__global__ void __launch_bounds__(256) k_prep_cells(FluidView F, SphParams P, const sph_grid* __restrict__ gp,
+                                                    Rec* __restrict__ rec, int32_t* __restrict__ nseg,
+                                                    int32_t* __restrict__ seg_start,
+                                                    uint32_t* __restrict__ seg_mask) {
+  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes);
+  if constexpr (kLanes == 1) {
+    if (i >= F.n) return;
+    prep_body(i, F, P, rec);
+    segments_body(i, F, *gp, 0, P.search_radius, P.thr, nseg, seg_start, seg_mask);
+  } else {
+    prep_rows(i, i < F.n, threadIdx.x % kLanes, F, *gp, 0, P, rec, nseg, seg_start, seg_mask);
+  }
+}
+
+// One scene's right-hand side.
+template <bool kCells, int kScheme, bool kByFour>
 __global__ void __launch_bounds__(128) k_dsph_pass1(FluidView F, const Rec* __restrict__ rec, WallView W,
-                                                    const sph_grid* __restrict__ gp, SphParams P,
+                                                    const sph_grid* __restrict__ gp, SphParams P, Segments S,
                                                     float* __restrict__ dpdt, float2* __restrict__ acc,
                                                     float4* __restrict__ Lout, float2* __restrict__ grad_rho) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= F.n) return;
-  const Pass1 o = pass1_body<false>(i, F, rec, W, *gp, P, 0, Segments{});
-  dpdt[i] = P.diffusion == 2 ? o.dpdt + P.diff_k * o.ddiff : o.dpdt;
+  const Pass1 o = pass1_body<kCells, 1, kScheme, kByFour>(i, F, rec, W, *gp, P, 0, S);
+  dpdt[i] = (kScheme >= 0 ? kScheme : P.diffusion) == 2 ? o.dpdt + P.diff_k * o.ddiff : o.dpdt;
   acc[i] = make_float2(o.ax, o.ay);
   if (Lout) Lout[i] = o.L;
   if (grad_rho) grad_rho[i] = o.grad_rho;
 }
 
-__global__ void __launch_bounds__(128) k_dsph_diffusion(FluidView F, const Rec* __restrict__ rec, SphParams P,
-                                                        const float2* __restrict__ grad_rho, float* __restrict__ dpdt) {
+template <bool kCells, bool kByFour>
+__global__ void __launch_bounds__(128) k_dsph_diffusion(FluidView F, const Rec* __restrict__ rec,
+                                                        const sph_grid* __restrict__ gp, SphParams P, Segments S,
+                                                        const float2* __restrict__ grad_rho,
+                                                        float* __restrict__ dpdt) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= F.n) return;
-  dpdt[i] -= P.diff_k * diffusion_sum<false, 1, false>(i, F, rec, P, grad_rho, sph_grid{}, 0, Segments{});
+  dpdt[i] -= P.diff_k * diffusion_sum<kCells, 1, false, kByFour>(i, F, rec, P, grad_rho, *gp, 0, S);
 }
 
 __global__ void k_sie(int n, const float2* __restrict__ x, const float2* __restrict__ v,
@@ -457,22 +593,25 @@ __global__ void k_sie(int n, const float2* __restrict__ x, const float2* __restr
 
 // ---------------------------------------------------------------------------- batch of scenes
 // scenes[sid[i]] gives particle i's grid, parameters, cell-table offset and time step.
-struct BatchScene {
-  const SceneDev* scenes;
-  const int32_t* wsid;
-  __device__ __forceinline__ MdbcScene operator()(int b) const {
-    const int s = wsid[b];   // negative: wall of no scene (free slot of a pooled batch)
-    return s < 0 ? MdbcScene{nullptr, nullptr, 0} : MdbcScene{&scenes[s].g, &scenes[s].P, scenes[s].coff};
-  }
-};
-__global__ void __launch_bounds__(kMdbcThreads) k_batch_mdbc_lanes(FluidView F, WallView W,
-                                                                   const SceneDev* __restrict__ scenes,
-                                                                   const int32_t* __restrict__ wsid) {
-  mdbc_block(F, W, BatchScene{scenes, wsid});
-}
+template <int kLanes>
 __global__ void __launch_bounds__(128, 8) k_batch_mdbc(FluidView F, WallView W, const SceneDev* __restrict__ scenes,
                                                        const int32_t* __restrict__ wsid) {
-  mdbc_wall(F, W, BatchScene{scenes, wsid});
+  const int b = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+  const int sid = b < W.n ? wsid[b] : -1;   // -1: wall of no scene (free slot of a pooled batch)
+  if (kLanes == 1 && sid < 0) return;
+  const SceneDev& S = scenes[max(sid, 0)];
+  mdbc_body<kLanes>(min(b, W.n - 1), sid >= 0, threadIdx.x % kLanes, F, W, S.g, S.P, S.coff);
+}
+
+// Neighbor records and segment lists of a small batch.
+__global__ void __launch_bounds__(256) k_batch_prep_rows(FluidView F, const SceneDev* __restrict__ scenes,
+                                                         const int32_t* __restrict__ sid, Rec* __restrict__ rec,
+                                                         int32_t* __restrict__ nseg, int32_t* __restrict__ seg_start,
+                                                         uint32_t* __restrict__ seg_mask) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kRowLanes;
+  const int s = i < F.n ? sid[i] : -1;   // -1: particle of no scene
+  const SceneDev& S = scenes[max(s, 0)];
+  prep_rows(i, s >= 0, threadIdx.x % kRowLanes, F, S.g, S.coff, S.P, rec, nseg, seg_start, seg_mask);
 }
 
 // Neighbor records and, with pairs from the cell rows (nseg != NULL), the segment lists.
@@ -507,8 +646,8 @@ __device__ __forceinline__ void batch_update(int i, const FluidView& F, float ax
 // <grad rho> to k_batch_diffusion, which finishes and updates them.  kCells: pairs from the
 // segment lists; kTpp lanes per particle (kCells only).  With kTpp > 1 no lane leaves
 // before the lane sums: lanes past p_hi take part with nothing to add.
-template <bool kCells, int kTpp, int kScheme>
-__global__ void __launch_bounds__(128, 9) k_batch_pass1(FluidView F, const Rec* __restrict__ rec, WallView W,
+template <bool kCells, int kTpp, int kScheme, bool kByFour = false>
+__global__ void __launch_bounds__(128, kByFour ? 6 : 9) k_batch_pass1(FluidView F, const Rec* __restrict__ rec, WallView W,
                                                      const SceneDev* __restrict__ scenes,
                                                      const int32_t* __restrict__ sid, float* __restrict__ dpdt,
                                                      float2* __restrict__ acc, float2* __restrict__ grad_rho,
@@ -530,7 +669,8 @@ __global__ void __launch_bounds__(128, 9) k_batch_pass1(FluidView F, const Rec* 
   }
   const SceneDev& S = scenes[sid[i] < 0 ? 0 : sid[i]];
   const SphParams P = S.P;   // the fields the loop reads, in registers
-  const Pass1 o = pass1_body<kCells, kTpp, kScheme>(i, F, rec, W, S.g, P, S.coff, seg, sub, kTpp == 1 || live);
+  const Pass1 o = pass1_body<kCells, kTpp, kScheme, kByFour>(i, F, rec, W, S.g, P, S.coff, seg, sub,
+                                                             kTpp == 1 || live);
   if (kTpp > 1 && (!live || sub != 0)) return;
   if ((kScheme >= 0 ? kScheme : P.diffusion) == 2) {
     dpdt[i] = o.dpdt + P.diff_k * o.ddiff;
@@ -542,7 +682,7 @@ __global__ void __launch_bounds__(128, 9) k_batch_pass1(FluidView F, const Rec* 
   batch_update(i, F, o.ax, o.ay, o.dpdt, S, xo, vo, ro, status);
 }
 
-template <bool kCells, int kTpp>
+template <bool kCells, int kTpp, bool kByFour = false>
 __global__ void __launch_bounds__(128) k_batch_diffusion(FluidView F, const Rec* __restrict__ rec,
                                                          const SceneDev* __restrict__ scenes,
                                                          const int32_t* __restrict__ sid,
@@ -568,7 +708,8 @@ __global__ void __launch_bounds__(128) k_batch_diffusion(FluidView F, const Rec*
   const bool act = live && S.P.diffusion == 2;   // the same on all lanes of a particle
   if (kTpp == 1 && !act) return;
   const SphParams P = S.P;   // the fields the loop reads, in registers
-  const float sum = diffusion_sum<kCells, kTpp>(i, F, rec, P, grad_rho, S.g, S.coff, seg, sub, kTpp == 1 || act);
+  const float sum = diffusion_sum<kCells, kTpp, true, kByFour>(i, F, rec, P, grad_rho, S.g, S.coff, seg, sub,
+                                                               kTpp == 1 || act);
   if (kTpp > 1 && (!act || sub != 0)) return;
   const float d = dpdt[i] - P.diff_k * sum;
   const float2 a = acc[i];
@@ -642,8 +783,13 @@ sph_status_t sph_mdbc_wall_density(const sph_fluid_view* fluid, const sph_wall_v
   SPH_VIEW_CHECK(walls);
   SPH_REQUIRE(grid && params && params->support > 0.f, "mdbc: bad arguments");
   if (walls->n == 0) return SPH_OK;
-  k_mdbc<<<grid_for(walls->n, kMdbcWalls), kMdbcThreads, 0, as_stream(stream)>>>(to_fluid(fluid), to_walls(walls),
-                                                                                  grid, to_params(params));
+  const FluidView F = to_fluid(fluid);
+  const WallView W = to_walls(walls);
+  const SphParams P = to_params(params);
+  if (W.n <= kMdbcSplitWalls)
+    k_mdbc<4><<<grid_for(4 * walls->n, 128), 128, 0, as_stream(stream)>>>(F, W, grid, P);
+  else
+    k_mdbc<1><<<grid_for(walls->n, 128), 128, 0, as_stream(stream)>>>(F, W, grid, P);
   SPH_CHECK_LAUNCH("mdbc_wall_density");
   return SPH_OK;
 }
@@ -667,6 +813,12 @@ sph_status_t sph_deltasph_segment_lists(int64_t n, size_t* masks_offset, size_t*
 }
 
 }  // extern "C"
+
+// Particles of a launch up to which the force passes keep four pairs' records in flight per thread
+// (same sums, 78 instead of 56 registers): pass 1 and diffusion of one scene, us, without / with:
+// 8,100 particles 16.6 + 9.5 / 14.6 + 7.7, 36,864: 15.6 + 9.8 / 15.3 + 8.3, 65,536: 17.3 + 10.3 /
+// 18.1 + 9.7, 131,044: 21.9 + 12.3 / 27.8 + 13.2.
+constexpr int kByFourMax = 49152;
 
 // The neighbor records in caller scratch, 32-byte aligned.
 static bool records_from_scratch(void* scratch, size_t bytes, int64_t n, Rec** rec, Segments* seg = nullptr) {
@@ -695,19 +847,56 @@ sph_status_t sph_deltasph_forces(const sph_fluid_view* fluid, const sph_wall_vie
   SPH_REQUIRE(grid && params && dpdt && acc && params->support > 0.f, "deltasph_forces: bad arguments");
   SPH_REQUIRE(params->density_diffusion != 2 || grad_rho, "deltasph_forces: deltaSPH diffusion needs grad_rho");
   if (fluid->n == 0) return SPH_OK;
+  // no CSR list (offsets and cols NULL): the pairs come from the cell rows
+  const bool cells = !fluid->offsets && !fluid->cols;
+  SPH_REQUIRE(cells ? fluid->cell_start && fluid->keys : fluid->offsets && fluid->cols,
+              "deltasph_forces: give offsets and cols, or neither with keys and the cell table");
   Rec* rec;
-  SPH_REQUIRE(records_from_scratch(scratch, scratch_bytes, fluid->n, &rec),
+  Segments seg{};
+  SPH_REQUIRE(records_from_scratch(scratch, scratch_bytes, fluid->n, &rec, cells ? &seg : nullptr),
               "deltasph_forces: scratch smaller than sph_deltasph_scratch_bytes(n)");
   cudaStream_t st = as_stream(stream);
   const FluidView F = to_fluid(fluid);
   const WallView W = to_walls(walls);
   const SphParams P = to_params(params);
-  const int nb = grid_for(fluid->n, 128);
-  k_prep<<<grid_for(fluid->n, 256), 256, 0, st>>>(F, P, rec);
-  k_dsph_pass1<<<nb, 128, 0, st>>>(F, rec, W, grid, P, dpdt, reinterpret_cast<float2*>(acc),
-                                   reinterpret_cast<float4*>(L), reinterpret_cast<float2*>(grad_rho));
-  if (P.diffusion == 2)
-    k_dsph_diffusion<<<nb, 128, 0, st>>>(F, rec, P, reinterpret_cast<const float2*>(grad_rho), dpdt);
+  const int n = F.n;
+  float2* ac = reinterpret_cast<float2*>(acc);
+  float4* Lo = reinterpret_cast<float4*>(L);
+  float2* gr = reinterpret_cast<float2*>(grad_rho);
+  const int nb = grid_for(n, 128);
+#define SPH_PASS1(C, K, B4) k_dsph_pass1<C, K, B4><<<nb, 128, 0, st>>>(F, rec, W, grid, P, seg, dpdt, ac, Lo, gr)
+#define SPH_DIFFUSION(C, B4) k_dsph_diffusion<C, B4><<<nb, 128, 0, st>>>(F, rec, grid, P, seg, gr, dpdt)
+  if (!cells) {
+    k_prep<<<grid_for(n, 256), 256, 0, st>>>(F, P, rec);
+    SPH_PASS1(false, -1, false);
+    if (P.diffusion == 2) SPH_DIFFUSION(false, false);
+  } else {
+    int32_t* ns = const_cast<int32_t*>(seg.nseg);
+    int32_t* ss = const_cast<int32_t*>(seg.start);
+    uint32_t* sm = const_cast<uint32_t*>(seg.mask);
+    if (n <= kRowLanesMax)
+      k_prep_cells<kRowLanes><<<grid_for(kRowLanes * (int64_t)n, 256), 256, 0, st>>>(F, P, grid, rec, ns, ss, sm);
+    else
+      k_prep_cells<1><<<grid_for(n, 256), 256, 0, st>>>(F, P, grid, rec, ns, ss, sm);
+    const bool by_four = n <= kByFourMax;
+    if (P.diffusion == 2) {
+      if (by_four) {
+        SPH_PASS1(true, 2, true);
+        SPH_DIFFUSION(true, true);
+      } else {
+        SPH_PASS1(true, 2, false);
+        SPH_DIFFUSION(true, false);
+      }
+    } else if (by_four) {
+      SPH_PASS1(true, -1, true);
+    } else if (P.diffusion == 1) {
+      SPH_PASS1(true, 1, false);
+    } else {
+      SPH_PASS1(true, -1, false);
+    }
+  }
+#undef SPH_PASS1
+#undef SPH_DIFFUSION
   SPH_CHECK_LAUNCH("deltasph_forces");
   return SPH_OK;
 }
@@ -767,15 +956,21 @@ sph_status_t sph_batch_deltasph_step(const sph_fluid_view* fluid, const sph_wall
   const FluidView F = to_fluid(fluid);
   const WallView W = to_walls(walls);
   const SceneDev* S = static_cast<const SceneDev*>(scenes);
-  if (W.n > 0 && (phases & SPH_PHASE_WALLS))  {
+  if (W.n > 0 && (phases & SPH_PHASE_WALLS)) {
     if (W.n <= kMdbcSplitWalls)
-      k_batch_mdbc_lanes<<<grid_for(W.n, kMdbcWalls), kMdbcThreads, 0, st>>>(F, W, S, wall_sid);
+      k_batch_mdbc<4><<<grid_for(4 * (int64_t)W.n, 128), 128, 0, st>>>(F, W, S, wall_sid);
     else
-      k_batch_mdbc<<<grid_for(W.n, 128), 128, 0, st>>>(F, W, S, wall_sid);
+      k_batch_mdbc<1><<<grid_for(W.n, 128), 128, 0, st>>>(F, W, S, wall_sid);
   }
-  if (phases & SPH_PHASE_RECORDS)
-    k_batch_prep<<<grid_for(n, 256), 256, 0, st>>>(F, S, sid, rec, const_cast<int32_t*>(seg.nseg),
-                                                   const_cast<int32_t*>(seg.start), const_cast<uint32_t*>(seg.mask));
+  if (phases & SPH_PHASE_RECORDS) {
+    int32_t* ns = const_cast<int32_t*>(seg.nseg);
+    int32_t* ss = const_cast<int32_t*>(seg.start);
+    uint32_t* sm = const_cast<uint32_t*>(seg.mask);
+    if (cells && n <= kRowLanesMax)
+      k_batch_prep_rows<<<grid_for(kRowLanes * (int64_t)n, 256), 256, 0, st>>>(F, S, sid, rec, ns, ss, sm);
+    else
+      k_batch_prep<<<grid_for(n, 256), 256, 0, st>>>(F, S, sid, rec, ns, ss, sm);
+  }
   float2* xo = reinterpret_cast<float2*>(x_out);
   float2* vo = reinterpret_cast<float2*>(v_out);
   float2* gr = reinterpret_cast<float2*>(grad_rho);
@@ -784,15 +979,19 @@ sph_status_t sph_batch_deltasph_step(const sph_fluid_view* fluid, const sph_wall
   // or 4 lanes and a scheme of MOG, deltaSPH or read per scene
   auto pass1 = [&](int lo, int hi, int t, int scheme) {
     const int nb = grid_for((int64_t)(hi - lo) * t, 128);
-#define SPH_PASS1(C, T, K)                                                                                  \
-  k_batch_pass1<C, T, K><<<nb, 128, 0, st>>>(F, rec, W, S, sid, dpdt, ac, gr, C ? seg : Segments{}, xo, vo, \
-                                             rho_out, status, lo, hi)
+#define SPH_PASS1(C, T, K, ...)                                                                                \
+  k_batch_pass1<C, T, K, ##__VA_ARGS__><<<nb, 128, 0, st>>>(F, rec, W, S, sid, dpdt, ac, gr,                   \
+                                                            C ? seg : Segments{}, xo, vo, rho_out, status, lo, \
+                                                            hi)
     if (!cells) {
       SPH_PASS1(false, 1, -1);
       return;
     }
     const int k = scheme == 1 || scheme == 2 ? scheme : -1;
-    if (t == 1) {
+    if (t == 1 && hi - lo <= kByFourMax) {
+      if (k == 2) SPH_PASS1(true, 1, 2, true);
+      else SPH_PASS1(true, 1, -1, true);
+    } else if (t == 1) {
       if (k == 2) SPH_PASS1(true, 1, 2);
       else if (k == 1) SPH_PASS1(true, 1, 1);
       else SPH_PASS1(true, 1, -1);
@@ -816,6 +1015,9 @@ sph_status_t sph_batch_deltasph_step(const sph_fluid_view* fluid, const sph_wall
     if (!cells)
       k_batch_diffusion<false, 1><<<nb, 128, 0, st>>>(F, rec, S, sid, gr, Segments{}, dpdt, ac, xo, vo, rho_out,
                                                       status, lo, hi);
+    else if (t == 1 && hi - lo <= kByFourMax)
+      k_batch_diffusion<true, 1, true><<<nb, 128, 0, st>>>(F, rec, S, sid, gr, seg, dpdt, ac, xo, vo, rho_out,
+                                                           status, lo, hi);
     else if (t == 1)
       k_batch_diffusion<true, 1><<<nb, 128, 0, st>>>(F, rec, S, sid, gr, seg, dpdt, ac, xo, vo, rho_out, status, lo,
                                                      hi);

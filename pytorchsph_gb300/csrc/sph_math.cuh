@@ -591,6 +591,91 @@ __device__ __forceinline__ void stored_pairs(int i, const FluidView& F, const sp
   }
 }
 
+// for_each_wall with the walls of a cell row tested 32 at a time and the accepted ones' records
+// four in flight: use(load(b)) in the same order.
+template <typename Load, typename Use>
+__device__ __forceinline__ void for_each_wall_by_four(const WallView& W, const sph_grid& g, int r, int cx, int cy,
+                                                      float xf, float yf, float thr_b, Load&& load, Use&& use,
+                                                      int coff = 0) {
+  const int x0 = max(cx - r, 0), x1 = min(cx + r, g.cells_x - 1);
+  if (x0 > x1) return;
+  const int y0 = max(cy - r, 0), y1 = min(cy + r, g.cells_y - 1);
+  const int32_t* cs = W.cell_start + coff;
+  for (int yy = y0; yy <= y1; ++yy) {
+    const int32_t* row = cs + (int64_t)yy * g.cells_x;
+    const int b0 = __ldg(row + x0), b1 = __ldg(row + x1 + 1);
+    for (int c = b0; c < b1; c += 32) {
+      uint32_t w = c + 32 <= W.n ? segment_mask_full(W.x, c, b1, xf, yf, thr_b)
+                                 : segment_mask(W.x, c, b1, xf, yf, thr_b);
+      while (w) {
+        int j[4];
+        bool ok[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          ok[t] = w != 0;
+          j[t] = ok[t] ? c - 1 + __ffs(w) : c;
+          w &= w - 1;   // 0 stays 0
+        }
+        const auto f0 = load(j[0]), f1 = load(j[1]), f2 = load(j[2]), f3 = load(j[3]);
+        use(f0);
+        if (ok[1]) use(f1);
+        if (ok[2]) use(f2);
+        if (ok[3]) use(f3);
+      }
+    }
+  }
+}
+
+// stored_pairs in groups of four: use(load(j)) in the same order, the four records of a group in
+// flight together.  For scenes too small to hide a load's latency behind other warps.
+template <typename Load, typename Use>
+__device__ __forceinline__ void stored_pairs_by_four(int i, const FluidView& F, const sph_grid& g, int coff, int r,
+                                                     const int32_t* __restrict__ nseg,
+                                                     const int32_t* __restrict__ seg_start,
+                                                     const uint32_t* __restrict__ seg_mask, float xi, float yi,
+                                                     float thr, Load&& load, Use&& use) {
+  const int ns = nseg[i];
+  if (ns < 0 || ns > kMaxSegments) {
+    int cx, cy;
+    cell_of(F.keys[i] - (uint32_t)coff, g, &cx, &cy);
+    cell_pairs(F, g, r, coff, cx, cy, xi, yi, thr, [&](int j) { use(load(j)); });
+    return;
+  }
+  const size_t n = (size_t)F.n;
+  int j0 = i, j1 = i, j2 = i, j3 = i, k = 0, b = 0, bn = 0;
+  uint32_t w = 0, wn = 0;
+  if (ns > 0) {
+    bn = seg_start[i];
+    wn = seg_mask[i];
+  }
+  for (bool more = ns > 0; more;) {
+    int q = 0;   // the group's pairs, the last of them in j3
+    while (q < 4) {
+      while (w == 0 && k < ns) {
+        b = bn;
+        w = clip_segment(wn, bn, F.n);
+        if (++k < ns) {
+          bn = seg_start[k * n + i];
+          wn = seg_mask[k * n + i];
+        }
+      }
+      if (w == 0) break;
+      j0 = j1;
+      j1 = j2;
+      j2 = j3;
+      j3 = b - 1 + __ffs(w);
+      w &= w - 1;
+      ++q;
+    }
+    more = q == 4;
+    const auto r0 = load(j0), r1 = load(j1), r2 = load(j2), r3 = load(j3);
+    if (q > 3) use(r0);
+    if (q > 2) use(r1);
+    if (q > 1) use(r2);
+    if (q > 0) use(r3);
+  }
+}
+
 // Pairs from the segment lists S (kCells) instead of the CSR row.
 struct Segments {
   const int32_t* nseg;

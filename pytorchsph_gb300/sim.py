@@ -198,9 +198,10 @@ class Simulation:
         P.omega_fluid = c.omega_fluid
         return P
 
-    def _sort_keys(self, x, n, prefix, tie=None):
+    def _sort_keys(self, x, n, prefix, tie=None, rows=()):
         """Counting sort of `n` positions by cell key (inside a cell by `tie`, e.g. the
-        particle id, then index); returns (order, sorted_keys, cell_start)."""
+        particle id, then index); returns (order, sorted_keys, cell_start).  `rows`: (in, out)
+        pairs of at most 8 per-particle arrays moved into the sorted order by the same launches."""
         st = N.stream_ptr()
         ws = self.ws
         keys = ws.get(prefix + "keys", n)
@@ -211,8 +212,9 @@ class Simulation:
         N.call("sph_cell_keys", N.ptr(x), n, N.ptr(self.grid), self.cap, N.ptr(keys), None, N.ptr(hist),
                N.ptr(self.status), st)
         scratch = ws.bytes(prefix + "cs_scratch", self.lib.sph_counting_sort_scratch_bytes(n, self.cap))
-        N.call("sph_counting_sort_tie", N.ptr(keys), n, self.cap, N.ptr(hist), N.ptr(cs), N.ptr(tie), N.ptr(order),
-               N.ptr(skeys), N.ptr(self.status), N.ptr(scratch), scratch.numel() * 8, st)
+        k, eb, ins, outs = N.array_set(rows)
+        N.call("sph_counting_sort_permute", N.ptr(keys), n, self.cap, N.ptr(hist), N.ptr(cs), N.ptr(tie), N.ptr(order),
+               N.ptr(skeys), k, eb, ins, outs, N.ptr(self.status), N.ptr(scratch), scratch.numel() * 8, st)
         return order, skeys, cs
 
     def _permute(self, order, t):
@@ -254,14 +256,16 @@ class Simulation:
         """Re-sort every particle array by cell key and (pairs = "csr") build the neighbor list."""
         st = N.stream_ptr()
         n = self.n
-        order, skeys, cs = self._sort_keys(self.arr["x"], n, "f_", tie=self.arr["uid"])
-        for k in list(self.arr):
-            self.arr[k] = self._permute(order, self.arr[k])
-        for k in list(self.extra):
-            self.extra[k] = self._permute(order, self.extra[k])
+        old, extra = self.arr, self.extra
+        self.arr = {k: torch.empty_like(t) for k, t in old.items()}
+        order, skeys, cs = self._sort_keys(old["x"], n, "f_", tie=old["uid"],
+                                           rows=[(old[k], self.arr[k]) for k in old])
+        if extra:
+            self.extra = {k: torch.empty_like(t) for k, t in extra.items()}
+            N.permute_arrays(order, [(extra[k], self.extra[k]) for k in extra])
         self.skeys, self.cell_start = skeys, cs
         self.stepped = True
-        if self._cell_pairs():
+        if self.pairs == "cells":
             self.rho_fluid = None
             self.fluid_view = FluidViewC(N.ptr(self.arr["x"]), N.ptr(self.arr["v"]), N.ptr(self.arr["rho"]),
                                          N.ptr(self.arr["area"]), N.ptr(skeys), None, None, N.ptr(cs), n, 0)
@@ -287,9 +291,6 @@ class Simulation:
         self.fluid_view = FluidViewC(N.ptr(self.arr["x"]), N.ptr(self.arr["v"]), N.ptr(self.arr["rho"]),
                                      N.ptr(self.arr["area"]), N.ptr(skeys), N.ptr(offsets), N.ptr(self.cols), N.ptr(cs), n,
                                      self.pair_cap)
-
-    def _cell_pairs(self):
-        return self.pairs == "cells" and self.cfg.solver == "dfsph"
 
     def rhs(self, sync=True):
         """Evaluate one timestep() at the current state; returns (acc, vel, dpdt or None)."""
@@ -320,7 +321,7 @@ class Simulation:
              "wall_alpha": g("walpha", nb), "wall_source": g("wsrc", nb), "wall_pressure": g("wp", nb),
              "wall_residual": g("wres", nb), "wall_density_term": self.wall_term,
              "partials": g("partials", int(self.lib.sph_dfsph_partials_count()), torch.float64),
-             "errors": g("errors", maxit), "iters": g("iters", 1, torch.int32), "records": g("records", self.lib.sph_dfsph_records_count(n, self.nb, int(self._cell_pairs())))}
+             "errors": g("errors", maxit), "iters": g("iters", 1, torch.int32), "records": g("records", self.lib.sph_dfsph_records_count(n, self.nb, int(self.pairs == "cells")))}
         self.dfsph_arrays = b
         return DfsphBuffersC(*[N.ptr(b[k]) for k, _ in DfsphBuffersC._fields_])
 
