@@ -961,7 +961,7 @@ def run_diff_drop(args, dev, world, rank):
         peak, peak_src = hbm_peak()
         line["roofline"] = {"bound": "hbm", "kernel": "k_drop_adjoint (float32)", "achieved": None, "peak": peak,
                             "unit": "GB/s", "frac": None, "traffic": None, "peak_source": peak_src,
-                            "note": "the dual-number pair products bound this kernel, not HBM"}
+                            "note": "latency and the pair terms bound this kernel, not HBM"}
         line["e2e"] = {"value": None, "unit": "particle-steps/s", "h2d_bytes_per_step": None,
                        "d2h_bytes_per_step": None}
         line["gpu_launches"] = None

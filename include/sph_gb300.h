@@ -717,13 +717,36 @@ sph_status_t sph_drop_integrate(int32_t fp64, int64_t n, void* x, void* v, void*
                                 const void* dpdt, double dt, double rest_density, void* stream);
 /* Discrete adjoint of one step at state (x, v, rho) with the pairs of that state: from the
  * adjoint (lx1, lv1, lr1) of the next state, the adjoint (lx0, lv0, lr0) of this one and
- * dalpha[i] = particle i's share of dLoss/d(params->alpha) for this step.  Vector-Jacobian
- * products by forward-mode dual numbers per pair; each particle gathers over its own row
- * (no atomics). */
+ * dalpha[i] = particle i's share of dLoss/d(params->alpha) for this step.  Derivatives
+ * per pair in closed form (double) or by dual numbers (float); each particle gathers over its
+ * own row (no atomics). */
 sph_status_t sph_drop_adjoint(int32_t fp64, int64_t n, const int32_t* offsets, const int64_t* cols, const void* x,
                               const void* v, const void* rho, const void* area, const sph_params* params, double dt,
                               const void* lx1, const void* lv1, const void* lr1, void* lx0, void* lv0, void* lr0,
                               void* dalpha, void* stream);
+
+/* The same rollout without host waits: each step's search writes row offsets [n+1] and int32
+ * columns (original order) into buffers of a given capacity; a row past it is left unwritten,
+ * flags SPH_FLAG_PAIR_CAPACITY and reads as empty.  Rows come in cell order, or increasing when
+ * `unsorted` gives a second column buffer to sort from.  pair_capacity > 0.  grid:
+ * sph_grid_build with the domain given, so that it holds for every step.  scratch:
+ * sph_drop_search_scratch_bytes(n, cell_capacity), zeroed once before the first call. */
+size_t sph_drop_search_scratch_bytes(int64_t n, int32_t cell_capacity);
+sph_status_t sph_drop_search(const float* x32, const float* support, int64_t n, const sph_grid* grid,
+                             int32_t cell_capacity, int32_t* offsets, int64_t pair_capacity, int32_t* cols,
+                             int32_t* unsorted, int32_t* status, void* scratch, size_t scratch_bytes, void* stream);
+/* sph_drop_rhs and sph_drop_integrate in one launch, to other arrays than the state's, with the
+ * new positions in float32 (x32_out, may be NULL) for the next search. */
+sph_status_t sph_drop_step(int32_t fp64, int64_t n, const int32_t* offsets, const int32_t* cols,
+                           int64_t pair_capacity, const void* x, const void* v, const void* rho, const void* area,
+                           const sph_params* params, double dt, void* x_out, void* v_out, void* rho_out, float* x32_out,
+                           void* stream);
+/* sph_drop_adjoint over the pairs of sph_drop_search, with the step's shares added to dalpha. */
+sph_status_t sph_drop_adjoint_step(int32_t fp64, int64_t n, const int32_t* offsets, const int32_t* cols,
+                                   int64_t pair_capacity, const void* x, const void* v, const void* rho,
+                                   const void* area, const sph_params* params, double dt, const void* lx1,
+                                   const void* lv1, const void* lr1, void* lx0, void* lv0, void* lr0, void* dalpha,
+                                   void* stream);
 
 /* ---------------------------------------------------------------- DFSPH (a20-a25) */
 

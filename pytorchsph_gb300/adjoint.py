@@ -4,10 +4,12 @@ their discrete adjoint on the GPU, with checkpointing.
 The step is the reference's deltaSPH right-hand side (src/deltaSPH.py:146-200: point
 source or gravity, continuity, MOG density diffusion, Tait pressure, artificial and laminar
 viscosity) integrated by semi-implicit Euler (src/simulationBase.py:647-652).  Each step
-searches neighbors on the GPU (the reference predicate, pairs in (i, j) order), then runs
-`sph_drop_rhs` and `sph_drop_integrate`; the adjoint (`sph_drop_adjoint`) runs the steps
-backwards, recomputing each checkpoint segment's states forward first.  Scalars are float64
-(default) or float32; the search always sees float32 positions, as the reference's does.
+searches neighbors on the GPU (the reference predicate) and advances the state in one launch
+(`sph_drop_search`, `sph_drop_step`); the adjoint (`sph_drop_adjoint_step`) runs the steps
+backwards, recomputing each checkpoint segment's states forward first.  A rollout waits for
+the device before its first step (the grid) and after its last (the status).  Scalars are
+float64 (default) or float32; the search always sees float32 positions, as the reference's
+does.  `DropRollout.pairs` and `step` work on the reference's own (i, j)-ordered lists.
 
 Gradients are with respect to the initial velocity field and the artificial viscosity alpha.
 `DropRolloutFunction` puts the rollout behind torch.autograd: its forward records every
@@ -63,6 +65,10 @@ class DropRollout:
         self.acc = torch.empty((self.n, 2), dtype=self.dtype, device=self.dev)
         self.dpdt = torch.empty(self.n, dtype=self.dtype, device=self.dev)
         self.steps_run = 0
+        # pairs of a step: a support's area over a particle's, a quarter more for denser packing
+        a = float(np.mean(np.asarray(scene["area"], np.float64)))
+        per = np.pi * self.h * self.h / a if a > 0 else 32.0
+        self._pair_cap = int(self.n * min(max(1.25 * per + 8.0, 16.0), 512.0)) if np.isfinite(per) else 32 * self.n
 
     # ------------------------------------------------------------------ forward
     def pairs(self, x):
@@ -89,10 +95,78 @@ class DropRollout:
         self.steps_run += 1
         return off, cols
 
+    def _search_plan(self):
+        """A rollout's search: the grid (given domain and constant supports, so it holds for every
+        step), the cell capacity, the status word and the scratch."""
+        x32 = self.x0.to(torch.float32).contiguous()
+        cap = self.search.auto_cell_capacity(x32, self.support32, self.vmin, self.vmax)
+        grid = self.search.ws.get("grid", 8, torch.int32).clone()   # the one the cells were counted on
+        status = torch.zeros(1, dtype=torch.int32, device=self.dev)
+        size = N.load().sph_drop_search_scratch_bytes(self.n, cap)
+        return grid, cap, status, torch.zeros((size + 7) // 8, dtype=torch.int64, device=self.dev)
+
+    def _search_into(self, plan, x32, off, cols, unsorted):
+        """The pairs at x32 into (offsets, int32 columns); a float32 rollout's rows in increasing
+        order (through `unsorted`), the order its sums are defined in."""
+        grid, cap, status, scratch = plan
+        N.call("sph_drop_search", N.ptr(x32), N.ptr(self.support32), self.n, N.ptr(grid), cap, N.ptr(off),
+               cols.shape[0], N.ptr(cols), N.ptr(unsorted), N.ptr(status), N.ptr(scratch), scratch.numel() * 8,
+               N.stream_ptr())
+
+    def _advance(self, state, pr, x32=None):
+        """The state after one step with the pairs pr = (offsets, int32 columns)."""
+        x, v, rho = state
+        out = tuple(torch.empty_like(t) for t in state)
+        off, cols = pr
+        N.call("sph_drop_step", int(self.fp64), self.n, N.ptr(off), N.ptr(cols), cols.shape[0], N.ptr(x), N.ptr(v),
+               N.ptr(rho), N.ptr(self.area), ctypes.byref(self.P), self.dt, N.ptr(out[0]), N.ptr(out[1]),
+               N.ptr(out[2]), N.ptr(x32), N.stream_ptr())
+        self.steps_run += 1
+        return out
+
+    def _forward(self, v0, alpha, steps, checkpoints, record):
+        """(final state, checkpoints, pairs of every step), the steps without host waits.  The pair
+        buffers are sized from the particles' areas with headroom; a step that overflows them has
+        the rollout run again with twice as much."""
+        self.P.alpha = float(alpha)
+        start = (self.x0.clone(), v0.to(self.dtype).reshape(self.n, 2).clone(), self.rho0.clone())
+        if steps <= 0:
+            return start, {}, []
+        plan = self._search_plan()
+        status = plan[2]
+        x32_0 = self.x0.to(torch.float32).contiguous()
+        x32 = torch.empty_like(x32_0)
+        while True:
+            status.zero_()
+            cap = self._pair_cap
+            rows = steps if record else 1
+            offs = torch.empty((rows, self.n + 1), dtype=torch.int32, device=self.dev)
+            cols = torch.empty((rows, cap), dtype=torch.int32, device=self.dev)
+            unsorted = None if self.fp64 else torch.empty(cap, dtype=torch.int32, device=self.dev)
+            state, ck = start, {}
+            for k in range(steps):
+                if checkpoints and k % self.every == 0:
+                    ck[k] = state
+                pr = (offs[k if record else 0], cols[k if record else 0])
+                self._search_into(plan, x32 if k else x32_0, *pr, unsorted)
+                state = self._advance(state, pr, x32)
+            flags = int(status.item())
+            if not flags & N.SPH_FLAG_PAIR_CAPACITY:
+                break
+            if cap >= 2**31 - 1:
+                raise N.SPHError(f"neighbor search: {N.decode_flags(flags)}")
+            self._pair_cap = min(2 * cap, 2**31 - 1)
+        if flags:
+            raise N.SPHError(f"neighbor search: {N.decode_flags(flags)}")
+        return state, ck, [(offs[k], cols[k]) for k in range(rows)] if record else []
+
     def rollout(self, v0, alpha, steps, checkpoints=False, record_pairs=False):
         """Final positions after `steps` steps from (x0, v0, rho0) and the checkpoints (the states
         at every `checkpoint_every`-th step, when asked for); with record_pairs also the list of
-        every step's (offsets, columns)."""
+        every step's (offsets, columns), in the reference's (i, j) order."""
+        if not record_pairs:
+            state, ck, _ = self._forward(v0, alpha, steps, checkpoints, False)
+            return state[0], ck
         x = self.x0.clone()
         v = v0.to(self.dtype).reshape(self.n, 2).clone()
         rho = self.rho0.clone()
@@ -101,10 +175,8 @@ class DropRollout:
         for k in range(steps):
             if checkpoints and k % self.every == 0:
                 ck[k] = (x.clone(), v.clone(), rho.clone())
-            pr = self.step(x, v, rho, alpha)
-            if record_pairs:
-                pairs.append(pr)
-        return (x, ck, pairs) if record_pairs else (x, ck)
+            pairs.append(self.step(x, v, rho, alpha))
+        return x, ck, pairs
 
     # ------------------------------------------------------------------ adjoint
     def vjp(self, ck, alpha, steps, grad_x, pairs=None):
@@ -117,21 +189,25 @@ class DropRollout:
         lr = torch.zeros_like(self.rho0)
         nx, nv, nr = torch.empty_like(lx), torch.empty_like(lv), torch.empty_like(lr)
         dalpha = torch.zeros(self.n, dtype=self.dtype, device=self.dev)
-        da = torch.empty_like(dalpha)
         self.P.alpha = float(alpha)
         for s0 in sorted(ck, reverse=True):
             s1 = min(s0 + self.every, steps)
-            x, v, rho = (t.clone() for t in ck[s0])
+            state = ck[s0]
             seg = []
             for k in range(s0, s1):          # recompute the segment's states
-                state = (x.clone(), v.clone(), rho.clone())
-                pr = self.step(x, v, rho, alpha, pairs[k] if pairs is not None else None)
+                if pairs is not None:
+                    off, cols = pairs[k]
+                    pr = (off, cols if cols.dtype == torch.int32 else cols.to(torch.int32))
+                else:
+                    off, cols = self.pairs(state[0])
+                    pr = (off, cols.to(torch.int32))
                 seg.append((state, pr))
+                if k + 1 < s1:
+                    state = self._advance(state, pr)
             for (xs, vs, rs), (off, cols) in reversed(seg):
-                N.call("sph_drop_adjoint", int(self.fp64), self.n, N.ptr(off), N.ptr(cols), N.ptr(xs), N.ptr(vs),
-                       N.ptr(rs), N.ptr(self.area), ctypes.byref(self.P), self.dt, N.ptr(lx), N.ptr(lv), N.ptr(lr),
-                       N.ptr(nx), N.ptr(nv), N.ptr(nr), N.ptr(da), N.stream_ptr())
-                dalpha += da
+                N.call("sph_drop_adjoint_step", int(self.fp64), self.n, N.ptr(off), N.ptr(cols), cols.shape[0],
+                       N.ptr(xs), N.ptr(vs), N.ptr(rs), N.ptr(self.area), ctypes.byref(self.P), self.dt, N.ptr(lx),
+                       N.ptr(lv), N.ptr(lr), N.ptr(nx), N.ptr(nv), N.ptr(nr), N.ptr(dalpha), N.stream_ptr())
                 lx, nx = nx, lx
                 lv, nv = nv, lv
                 lr, nr = nr, lr
@@ -139,7 +215,7 @@ class DropRollout:
 
     def loss_and_grad(self, v0, alpha, target, steps):
         """Loss mean_i |x_T,i - target_i|^2 and its gradients with respect to v0 [n, 2] and alpha."""
-        xT, ck, pairs = self.rollout(v0, alpha, steps, checkpoints=True, record_pairs=True)
+        (xT, *_), ck, pairs = self._forward(v0, alpha, steps, True, True)
         diff = xT - target.to(self.dtype)
         loss = float((diff * diff).sum().item()) / self.n
         lv, da = self.vjp(ck, alpha, steps, (2.0 / self.n) * diff, pairs)
@@ -163,7 +239,7 @@ class DropRolloutFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, v0, alpha, rollout, steps):
         a = float(alpha)
-        xT, ck, pairs = rollout.rollout(v0.detach(), a, int(steps), checkpoints=True, record_pairs=True)
+        (xT, *_), ck, pairs = rollout._forward(v0.detach(), a, int(steps), True, True)
         ctx.rollout, ctx.ck, ctx.pairs, ctx.alpha, ctx.steps = rollout, ck, pairs, a, int(steps)
         ctx.v_dtype, ctx.a_dtype = v0.dtype, (alpha.dtype if isinstance(alpha, torch.Tensor) else torch.float64)
         ctx.a_device = alpha.device if isinstance(alpha, torch.Tensor) else v0.device

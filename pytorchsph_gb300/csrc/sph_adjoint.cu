@@ -1,20 +1,45 @@
 // Differentiable deltaSPH rollout of a free fluid (no walls): the right-hand side of
 // src/deltaSPH.py:146-200 with MOG density diffusion and gravity or the point source, the
 // semi-implicit Euler update (src/simulationBase.py:647-652), and the discrete adjoint of
-// one step — vector-Jacobian products by forward-mode dual numbers on each pair.
+// one step in closed form.
 //
-// Pairs are the reference's (i, j)-ordered list in original particle order (row offsets +
-// columns, as neighborSearchModule.search returns it); the list is symmetric because every
-// particle has the same support.  Particle i's adjoint gathers over its own row both
+// Pairs are row offsets + columns in original particle order; the list is symmetric because
+// every particle has the same support.  Particle i's adjoint gathers over its own row both
 //   (d f_ij / d in_i)^T lambda_out_i   (its own right-hand side)   and
 //   (d f_ji / d in_i)^T lambda_out_j   (its neighbors' right-hand sides),
-// so there are no atomics and the result does not depend on thread timing.  The same pair
-// function (template on the scalar type) gives the forward right-hand side, so forward and
-// adjoint differentiate one formula.  Scalars are float or double.
+// so there are no atomics and the result does not depend on thread timing.  Scalars are float
+// or double.
+//
+// What bounds it: in double the FP64 pipe (two operations a clock and SM), in float a small
+// rollout's latency.  kDropLanes lanes share a row in both.
+//   double: every quantity that both particles' terms share is formed once per pair, with one
+//     division for its three reciprocals, and the derivatives are written out (about 110
+//     operations a pair, where two sweeps of 5-component dual numbers took some 2,000).
+//   float: the pair function and its dual numbers, whose terms the lanes form side by side and
+//     add one after another in row order: a float32 gradient with respect to alpha is a sum
+//     that cancels to 1/70 of its terms, so its rounding is kept to that of one thread per
+//     row, bit for bit.
+// At 4,173 particles in double the right-hand side takes 32 µs (one thread per row: 179) and
+// the adjoint 55 (dual numbers: 819); at 16,173 in float 8.7 (31) and 25 (40).
 #include "sph_common.cuh"
 
 namespace sph {
 
+template <typename T>
+struct DropParams {
+  T inv_h, cg20;      // 1/h, 20 * 7/(pi h^3)
+  T rho0, tait_k;     // rho0 c0^2 / gamma (gamma = 7)
+  T eps;              // 0.1 h^2
+  T visc_unit;        // h c0 (artificial viscosity factor without alpha)
+  T alpha, nu;        // artificial and laminar (kinematic) viscosity
+  T diff_k;           // h delta c0 (MOG)
+  T gx, gy;           // constant gravity
+  int point_source;
+  T point_mag, cx, cy;
+  int mog;
+};
+
+// ---------------------------------------------------------------- float: pair function and dual numbers
 template <typename T, int K>
 struct Dual {
   T v;
@@ -141,20 +166,6 @@ __device__ __forceinline__ Dual<T, K> make_const(T c, const Dual<T, K>&) {
   return r;
 }
 
-template <typename T>
-struct DropParams {
-  T inv_h, cg20;      // 1/h, 20 * 7/(pi h^3)
-  T rho0, tait_k;     // rho0 c0^2 / gamma (gamma = 7)
-  T eps;              // 0.1 h^2
-  T visc_unit;        // h c0 (artificial viscosity factor without alpha)
-  T alpha, nu;        // artificial and laminar (kinematic) viscosity
-  T diff_k;           // h delta c0 (MOG)
-  T gx, gy;           // constant gravity
-  int point_source;
-  T point_mag, cx, cy;
-  int mog;
-};
-
 template <typename S>
 struct PairOut {
   S ax, ay, dp;
@@ -215,26 +226,167 @@ __device__ __forceinline__ bool apart(T xix, T xiy, T xjx, T xjy) {
   return dx * dx + dy * dy >= T(1e-14);   // the reference's e_ij is 0 below r = 1e-7
 }
 
-template <typename T, typename V2>
+// ---------------------------------------------------------------- lanes
+constexpr int kDropLanes = 8;
+
+// End of a row [k0, k1) of lists with a capacity (0: none): k0 unless the row lies inside it,
+// also after a count past 2^31 (a row is shorter than that, so one of a wrapped scan's rows
+// has a negative end and is caught).
+__device__ __forceinline__ int row_end(int k0, int k1, int64_t capacity) {
+  return capacity > 0 && (k0 < 0 || k1 < k0 || (int64_t)k1 > capacity) ? k0 : k1;
+}
+
+template <typename T>
+__device__ __forceinline__ T drop_sum(T v) {
+#pragma unroll
+  for (int o = 1; o < kDropLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// sum + the lanes' terms one after another (every lane of the group gets the result; the whole
+// warp must take part).
+__device__ __forceinline__ float drop_add_in_order(float sum, float term) {
+#pragma unroll
+  for (int l = 0; l < kDropLanes; ++l) {
+    const float v = __shfl_sync(0xffffffffu, term, l, kDropLanes);
+    sum += v;
+  }
+  return sum;
+}
+
+// Pairs of the longest row among a warp's groups (the loops of the lanes that add in order are
+// as long in the whole warp).
+__device__ __forceinline__ int drop_longest(int m) {
+#pragma unroll
+  for (int o = kDropLanes; o < 32; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  return m;
+}
+
+// ---------------------------------------------------------------- double: closed form
+// What both rows of a pair (i, j) share, d = x_i - x_j and w = v_i - v_j: the Wendland gradient
+// gradW_ij = gd d with gd = -20 c_g (1 - q)^3 / h (kernels.py:20-33), r, s = w . d, and the
+// reciprocals of R2 = r^2 + eps, rho_i + rho_j and rho~_j (from one division).
+struct DropPair {
+  double dx, dy, wx, wy, r2, r, gd, s, iR, irs, irj;
+};
+
+// False for a pair closer than r = 1e-7, where the reference's e_ij is zero (the particle itself).
+__device__ __forceinline__ bool drop_pair(double2 xi, double2 vi, double ri, double2 xj, double2 vj, double rj,
+                                          const DropParams<double>& P, DropPair& o) {
+  o.dx = xi.x - xj.x;
+  o.dy = xi.y - xj.y;
+  o.r2 = o.dx * o.dx + o.dy * o.dy;
+  if (!(o.r2 >= 1e-14)) return false;
+  o.r = sqrt(o.r2);
+  const double a = 1.0 - o.r * P.inv_h;
+  o.gd = -(P.cg20 * P.inv_h) * (a * a * a);
+  o.wx = vi.x - vj.x;
+  o.wy = vi.y - vj.y;
+  o.s = o.wx * o.dx + o.wy * o.dy;
+  const double R2 = o.r2 + P.eps, rs = P.rho0 * (ri + rj);
+  const double t = 1.0 / (R2 * rs * rj);
+  o.iR = t * (rs * rj);
+  o.irs = t * (R2 * rj);
+  o.irj = t * (R2 * rs);
+  return true;
+}
+
+// Sums of row i over the lanes' pairs [k0, k1) (double; pressure.py:31-38, diffusion.py:30-44,
+// laminar.py:30-46 with its index choices, momentum.py:31-38, densityDiffusion.py:74-82): with
+// rho = rho0 rho~, V = A / rho~, m = rho V = rho0 A,
+//   a_i  = -1/rho_i sum (p_i + p_j) V_j gd d + alpha h c0 sum min(s, 0) m_j irs iR gd d
+//          + 8 nu rho_i sum m_j gd r2 irs^2 iR w
+//   dp_i = sum m_j gd s - 2 h delta c0 sum (rho_j - rho_i) V_j gd r2 iR
+template <typename Col>
+__device__ __forceinline__ void drop_row(int k0, int k1, int sub, const Col* __restrict__ cols, double2 xi, double2 vi,
+                                         double ri, const double2* __restrict__ x, const double2* __restrict__ v,
+                                         const double* __restrict__ rt, const double* __restrict__ area,
+                                         const DropParams<double>& P, double& ax, double& ay, double& dp) {
+  using T = double;
+  const T rhoi = P.rho0 * ri, pi = tait7(ri, P);
+  T px = 0, py = 0, vx = 0, vy = 0, lx = 0, ly = 0, d1 = 0, d2 = 0;
+  for (int k = k0 + sub; k < k1; k += kDropLanes) {
+    const int j = (int)__ldg(cols + k);
+    const T rj = rt[j], Aj = area[j];
+    DropPair e;
+    if (!drop_pair(xi, vi, ri, x[j], v[j], rj, P, e)) continue;
+    const T mg = P.rho0 * Aj * e.gd, Vg = Aj * e.irj * e.gd;   // m_j gd, V_j gd
+    const T pf = (pi + tait7(rj, P)) * Vg;
+    px += pf * e.dx;
+    py += pf * e.dy;
+    const T g = mg * e.irs * e.iR;
+    const T vf = (e.s > T(0) ? T(0) : e.s) * g;
+    vx += vf * e.dx;
+    vy += vf * e.dy;
+    const T lf = e.r2 * e.irs * g;
+    lx += lf * e.wx;
+    ly += lf * e.wy;
+    d1 += mg * e.s;
+    d2 += (rj - ri) * Vg * (e.r2 * e.iR);
+  }
+  px = drop_sum(px);
+  py = drop_sum(py);
+  vx = drop_sum(vx);
+  vy = drop_sum(vy);
+  lx = drop_sum(lx);
+  ly = drop_sum(ly);
+  d1 = drop_sum(d1);
+  d2 = drop_sum(d2);
+  const T fp = T(-1) / rhoi, fv = P.alpha * P.visc_unit, fl = T(8) * P.nu * rhoi;
+  ax = fp * px + fv * vx + fl * lx;
+  ay = fp * py + fv * vy + fl * ly;
+  dp = P.mog ? d1 - P.diff_k * T(2) * P.rho0 * d2 : d1;
+}
+
+// The same sums in float, added in row order.
+template <typename Col>
+__device__ __forceinline__ void drop_row(int k0, int k1, int sub, const Col* __restrict__ cols, float2 xi, float2 vi,
+                                         float ri, const float2* __restrict__ x, const float2* __restrict__ v,
+                                         const float* __restrict__ rt, const float* __restrict__ area,
+                                         const DropParams<float>& P, float& ax, float& ay, float& dp) {
+  ax = ay = dp = 0.f;
+  const int m = k1 - k0, longest = drop_longest(m);
+  for (int q = 0; q < longest; q += kDropLanes) {
+    float tx = 0.f, ty = 0.f, td = 0.f;   // adding 0 where a lane has no pair changes no sum's value
+    if (q + sub < m) {
+      const int j = (int)__ldg(cols + k0 + q + sub);
+      const float2 xj = x[j], vj = v[j];
+      if (apart(xi.x, xi.y, xj.x, xj.y)) {
+        const PairOut<float> o =
+            pair_terms<float, float>(xi.x, xi.y, vi.x, vi.y, ri, xj.x, xj.y, vj.x, vj.y, rt[j], area[j], P);
+        tx = o.ax;
+        ty = o.ay;
+        td = o.dp;
+      }
+    }
+    ax = drop_add_in_order(ax, tx);
+    ay = drop_add_in_order(ay, ty);
+    dp = drop_add_in_order(dp, td);
+  }
+}
+
+// Right-hand side of every particle.  kStep: advance (x, v, rho) by semi-implicit Euler into xo, vo,
+// ro, with the new positions in float32 in x32 (may be NULL) for the next search; else write
+// acc and dpdt.
+template <typename T, typename V2, typename Col, bool kStep>
 __global__ void __launch_bounds__(128) k_drop_rhs(int n, const int32_t* __restrict__ offsets,
-                                                  const int64_t* __restrict__ cols, const V2* __restrict__ x,
-                                                  const V2* __restrict__ v, const T* __restrict__ rt,
-                                                  const T* __restrict__ area, DropParams<T> P, V2* __restrict__ acc,
-                                                  T* __restrict__ dpdt) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+                                                  const Col* __restrict__ cols, int64_t capacity,
+                                                  const V2* __restrict__ x, const V2* __restrict__ v,
+                                                  const T* __restrict__ rt, const T* __restrict__ area,
+                                                  DropParams<T> P, T dt, V2* __restrict__ acc, T* __restrict__ dpdt,
+                                                  V2* __restrict__ xo, V2* __restrict__ vo, T* __restrict__ ro,
+                                                  float2* __restrict__ x32) {
+  const int row = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kDropLanes);
+  const int sub = threadIdx.x % kDropLanes;
+  const bool live = row < n;
+  const int i = live ? row : n - 1;   // lanes past the last particle only take part in the sums
   const V2 xi = x[i], vi = v[i];
   const T ri = rt[i];
-  T ax = 0, ay = 0, dp = 0;
-  for (int k = offsets[i]; k < offsets[i + 1]; ++k) {
-    const int j = (int)cols[k];
-    const V2 xj = x[j], vj = v[j];
-    if (!apart(xi.x, xi.y, xj.x, xj.y)) continue;
-    const PairOut<T> o = pair_terms<T, T>(xi.x, xi.y, vi.x, vi.y, ri, xj.x, xj.y, vj.x, vj.y, rt[j], area[j], P);
-    ax += o.ax;
-    ay += o.ay;
-    dp += o.dp;
-  }
+  const int k0 = offsets[i];
+  const int k1 = row_end(k0, offsets[i + 1], capacity);
+  T ax, ay, dp;
+  drop_row(k0, k1, sub, cols, xi, vi, ri, x, v, rt, area, P, ax, ay, dp);
+  if (!live || sub != 0) return;
   if (P.point_source) {
     T dx = xi.x - P.cx, dy = xi.y - P.cy;
     const T d = sqrt(dx * dx + dy * dy);
@@ -248,9 +400,21 @@ __global__ void __launch_bounds__(128) k_drop_rhs(int n, const int32_t* __restri
     ax += P.gx;
     ay += P.gy;
   }
-  acc[i].x = ax;
-  acc[i].y = ay;
-  dpdt[i] = dp;
+  if constexpr (kStep) {
+    V2 vn, xn;
+    vn.x = vi.x + dt * ax;
+    vn.y = vi.y + dt * ay;
+    xn.x = xi.x + dt * (vi.x + dt * ax);
+    xn.y = xi.y + dt * (vi.y + dt * ay);
+    xo[i] = xn;
+    vo[i] = vn;
+    ro[i] = ri + dt * dp / P.rho0;
+    if (x32) x32[i] = make_float2((float)xn.x, (float)xn.y);
+  } else {
+    acc[i].x = ax;
+    acc[i].y = ay;
+    dpdt[i] = dp;
+  }
 }
 
 template <typename T, typename V2>
@@ -269,26 +433,96 @@ __global__ void k_drop_sie(int n, V2* __restrict__ x, V2* __restrict__ v, T* __r
   rt[i] = rt[i] + dt * dpdt[i] / rho0;
 }
 
-// One step of the adjoint: from (lx', lv', lr') of step k+1 and the state of step k, the
-// adjoint of step k and particle i's share of dL/d alpha.
-template <typename T, typename V2>
-__global__ void __launch_bounds__(128) k_drop_adjoint(int n, const int32_t* __restrict__ offsets,
-                                                      const int64_t* __restrict__ cols, const V2* __restrict__ x,
-                                                      const V2* __restrict__ v, const T* __restrict__ rt,
-                                                      const T* __restrict__ area, DropParams<T> P, T dt,
-                                                      const V2* __restrict__ lx1, const V2* __restrict__ lv1,
-                                                      const T* __restrict__ lr1, V2* __restrict__ lx0,
-                                                      V2* __restrict__ lv0, T* __restrict__ lr0,
-                                                      T* __restrict__ dalpha) {
-  using D = Dual<T, 5>;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// Sums of particle i's adjoint over the lanes' pairs (double).  With la, ld the adjoints of a_i
+// and dp_i (lb, le: of row j), the pair's terms of both rows sum to
+//   F = gd (p_i + p_j) Q1 + alpha h c0 gd min(s, 0) irs iR Q2 + 8 nu gd r2 irs^2 iR Q3
+//       + gd s Q4 - 2 h delta c0 gd r2 iR (rho_j - rho_i) Q5,
+//   Q1 = V_i/rho_j (lb.d) - V_j/rho_i (la.d),  Q2 = m_j (la.d) - m_i (lb.d),
+//   Q3 = m_j rho_i (la.w) - m_i rho_j (lb.w),  Q4 = m_j ld + m_i le,  Q5 = V_j ld - V_i le,
+// whose gradient with respect to d, w and rho~_i is particle i's share (m does not depend on
+// rho~; d gd / d r2 = 30 c_g (1 - q)^2 / (h^2 r)).
+template <typename Col>
+__device__ __forceinline__ void adjoint_row(int i, int k0, int k1, int sub, const Col* __restrict__ cols, double2 xi,
+                                            double2 vi, double ri, const double2* __restrict__ x,
+                                            const double2* __restrict__ v, const double* __restrict__ rt,
+                                            const double* __restrict__ area, const DropParams<double>& P, double dt,
+                                            const double2* __restrict__ lx1, const double2* __restrict__ lv1,
+                                            const double* __restrict__ lr1, double lax, double lay, double ld,
+                                            double (&g)[5], double& da) {
+  using T = double;
+  using V2 = double2;
   const T dt2 = dt * dt, sdp = dt / P.rho0;
-  const V2 xi = x[i], vi = v[i];
-  const T ri = rt[i];
-  // lambda of row i's outputs: acc via v' = v + dt a and x' = x + dt v + dt^2 a; dpdt via rho'
-  const V2 lxi1 = lx1[i], lvi1 = lv1[i];
-  const T lai_x = dt * lvi1.x + dt2 * lxi1.x, lai_y = dt * lvi1.y + dt2 * lxi1.y, ldi = sdp * lr1[i];
+  const T rhoi = P.rho0 * ri, iri = T(1) / ri, Vi = area[i] * iri, mi = P.rho0 * area[i], irhoi = iri / P.rho0;
+  const T ri2 = ri * ri, ri6 = ri2 * ri2 * ri2, pi = P.tait_k * (ri6 * ri - T(1)), dpi = T(7) * P.tait_k * ri6;
+  const T av = P.alpha * P.visc_unit, nu8 = T(8) * P.nu, df = P.mog ? T(-2) * P.diff_k * P.rho0 : T(0);
+  T gx = 0, gy = 0, gvx = 0, gvy = 0, gr = 0;
+  da = 0;
+  for (int k = k0 + sub; k < k1; k += kDropLanes) {
+    const int j = (int)__ldg(cols + k);
+    const T rj = rt[j], Aj = area[j];
+    DropPair e;
+    if (!drop_pair(xi, vi, ri, x[j], v[j], rj, P, e)) continue;
+    const V2 lxj1 = lx1[j], lvj1 = lv1[j];
+    const T lbx = dt * lvj1.x + dt2 * lxj1.x, lby = dt * lvj1.y + dt2 * lxj1.y, le = sdp * lr1[j];
+    const T rhoj = P.rho0 * rj, Vj = Aj * e.irj, mj = P.rho0 * Aj;
+    const T Pp = pi + tait7(rj, P);
+    const T ea = lax * e.dx + lay * e.dy, eb = lbx * e.dx + lby * e.dy;   // la . d, lb . d
+    const T fa = lax * e.wx + lay * e.wy, fb = lbx * e.wx + lby * e.wy;   // la . w, lb . w
+    const T cij = Vj * irhoi, cji = Vi * (e.irj / P.rho0);
+    const T Q1 = cji * eb - cij * ea;
+    const T Q2 = mj * ea - mi * eb;
+    const T mri = mj * rhoi, mrj = mi * rhoj;
+    const T Q3 = mri * fa - mrj * fb;
+    const T Q4 = mj * ld + mi * le;
+    const T Q5 = Vj * ld - Vi * le;
+    const T a = T(1) - e.r * P.inv_h;
+    const T g1 = T(1.5) * P.cg20 * P.inv_h * P.inv_h * (a * a) / e.r;   // d gd / d r2
+    const T gi = e.gd * e.iR, dgi = (g1 - gi) * e.iR;                   // gd iR and its d / d r2
+    const T rgi = e.r2 * gi, drgi = gi + e.r2 * dgi;                    // gd r2 iR
+    const bool closing = !(e.s > T(0));
+    const T s = closing ? e.s : T(0);
+    const T kv = av * e.irs, kl = nu8 * e.irs * e.irs, D = rj - ri;
+    // d F / d r2 with d and w held, times two
+    const T f2 = T(2) * (g1 * (Pp * Q1 + e.s * Q4) + kv * s * Q2 * dgi + (kl * Q3 + df * D * Q5) * drgi);
+    // d F / d (la . d), d F / d (lb . d), d F / d s
+    const T cp = e.gd * Pp, cv = kv * gi * s;
+    const T wa = cv * mj - cp * cij, wb = cp * cji - cv * mi;
+    const T ws = e.gd * Q4 + (closing ? kv * gi * Q2 : T(0));
+    const T la3 = kl * rgi * mri, lb3 = -kl * rgi * mrj;   // d F / d (la . w), d F / d (lb . w)
+    gx += f2 * e.dx + wa * lax + wb * lbx + ws * e.wx;
+    gy += f2 * e.dy + wa * lay + wb * lby + ws * e.wy;
+    gvx += ws * e.dx + la3 * lax + lb3 * lbx;
+    gvy += ws * e.dy + la3 * lay + lb3 * lby;
+    gr += e.gd * (dpi * Q1 + Pp * iri * (cij * ea - cji * eb)) - P.rho0 * e.irs * (cv * Q2) +
+          kl * rgi * (mj * P.rho0 * fa - T(2) * P.rho0 * e.irs * Q3) + df * rgi * (D * (Vi * iri) * le - Q5);
+    da += P.visc_unit * gi * e.irs * s * mj * ea;
+  }
+  gx = drop_sum(gx);
+  gy = drop_sum(gy);
+  gvx = drop_sum(gvx);
+  gvy = drop_sum(gvy);
+  gr = drop_sum(gr);
+  da = drop_sum(da);
+  g[0] = gx;
+  g[1] = gy;
+  g[2] = gvx;
+  g[3] = gvy;
+  g[4] = gr;
+}
+
+// The same sums in float by dual numbers, added in row order: of each pair the own row's share,
+// then the neighbor row's.
+template <typename Col>
+__device__ __forceinline__ void adjoint_row(int i, int k0, int k1, int sub, const Col* __restrict__ cols, float2 xi,
+                                            float2 vi, float ri, const float2* __restrict__ x,
+                                            const float2* __restrict__ v, const float* __restrict__ rt,
+                                            const float* __restrict__ area, const DropParams<float>& P, float dt,
+                                            const float2* __restrict__ lx1, const float2* __restrict__ lv1,
+                                            const float* __restrict__ lr1, float lax, float lay, float ld,
+                                            float (&g)[5], float& da) {
+  using T = float;
+  using D = Dual<T, 5>;
+  const T dt2 = dt * dt, sdp = dt / P.rho0;
   D Xx, Xy, Vx, Vy, R;   // particle i's inputs, seeded
   Xx = make_const(xi.x, Xx);
   Xy = make_const(xi.y, Xy);
@@ -300,32 +534,77 @@ __global__ void __launch_bounds__(128) k_drop_adjoint(int n, const int32_t* __re
   Vx.d[2] = T(1);
   Vy.d[3] = T(1);
   R.d[4] = T(1);
-  T g[5] = {0, 0, 0, 0, 0};
-  T da = 0;
-  for (int k = offsets[i]; k < offsets[i + 1]; ++k) {
-    const int j = (int)cols[k];
-    const V2 xj = x[j], vj = v[j];
-    if (!apart(xi.x, xi.y, xj.x, xj.y)) continue;
-    const T rj = rt[j];
-    const D Jx = make_const(xj.x, Xx), Jy = make_const(xj.y, Xx), Jvx = make_const(vj.x, Xx),
-            Jvy = make_const(vj.y, Xx), Jr = make_const(rj, Xx);
-    // row i, derivatives with respect to i
-    const PairOut<D> o = pair_terms<D, T>(Xx, Xy, Vx, Vy, R, Jx, Jy, Jvx, Jvy, Jr, area[j], P);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) g[c] += o.ax.d[c] * lai_x + o.ay.d[c] * lai_y + o.dp.d[c] * ldi;
-    da += o.vx.v * lai_x + o.vy.v * lai_y;
-    // row j, derivatives with respect to i (its column)
-    const V2 lxj1 = lx1[j], lvj1 = lv1[j];
-    const T laj_x = dt * lvj1.x + dt2 * lxj1.x, laj_y = dt * lvj1.y + dt2 * lxj1.y, ldj = sdp * lr1[j];
-    const PairOut<D> w = pair_terms<D, T>(Jx, Jy, Jvx, Jvy, Jr, Xx, Xy, Vx, Vy, R, area[i], P);
+  for (int c = 0; c < 5; ++c) g[c] = 0.f;
+  da = 0.f;
+  const int m = k1 - k0, longest = drop_longest(m);
+  for (int q = 0; q < longest; q += kDropLanes) {
+    T own[5] = {0, 0, 0, 0, 0}, other[5] = {0, 0, 0, 0, 0}, ta = 0;
+    if (q + sub < m) {
+      const int j = (int)__ldg(cols + k0 + q + sub);
+      const float2 xj = x[j], vj = v[j];
+      if (apart(xi.x, xi.y, xj.x, xj.y)) {
+        const T rj = rt[j];
+        const D Jx = make_const(xj.x, Xx), Jy = make_const(xj.y, Xx), Jvx = make_const(vj.x, Xx),
+                Jvy = make_const(vj.y, Xx), Jr = make_const(rj, Xx);
+        // row i, derivatives with respect to i
+        const PairOut<D> o = pair_terms<D, T>(Xx, Xy, Vx, Vy, R, Jx, Jy, Jvx, Jvy, Jr, area[j], P);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) g[c] += w.ax.d[c] * laj_x + w.ay.d[c] * laj_y + w.dp.d[c] * ldj;
+        for (int c = 0; c < 5; ++c) own[c] = o.ax.d[c] * lax + o.ay.d[c] * lay + o.dp.d[c] * ld;
+        ta = o.vx.v * lax + o.vy.v * lay;
+        // row j, derivatives with respect to i (its column)
+        const float2 lxj1 = lx1[j], lvj1 = lv1[j];
+        const T lbx = dt * lvj1.x + dt2 * lxj1.x, lby = dt * lvj1.y + dt2 * lxj1.y, le = sdp * lr1[j];
+        const PairOut<D> w = pair_terms<D, T>(Jx, Jy, Jvx, Jvy, Jr, Xx, Xy, Vx, Vy, R, area[i], P);
+#pragma unroll
+        for (int c = 0; c < 5; ++c) other[c] = w.ax.d[c] * lbx + w.ay.d[c] * lby + w.dp.d[c] * le;
+      }
+    }
+#pragma unroll
+    for (int l = 0; l < kDropLanes; ++l) {
+#pragma unroll
+      for (int c = 0; c < 5; ++c) {
+        const T a = __shfl_sync(0xffffffffu, own[c], l, kDropLanes);
+        const T b = __shfl_sync(0xffffffffu, other[c], l, kDropLanes);
+        g[c] += a;
+        g[c] += b;
+      }
+    }
+    da = drop_add_in_order(da, ta);
   }
+}
+
+// One step of the adjoint: from (lx', lv', lr') of step k+1 and the state of step k, the
+// adjoint of step k and particle i's share of dL/d alpha (added to dalpha when accumulate).
+template <typename T, typename V2, typename Col>
+__global__ void __launch_bounds__(128) k_drop_adjoint(int n, const int32_t* __restrict__ offsets,
+                                                      const Col* __restrict__ cols, int64_t capacity,
+                                                      const V2* __restrict__ x, const V2* __restrict__ v,
+                                                      const T* __restrict__ rt, const T* __restrict__ area,
+                                                      DropParams<T> P, T dt, const V2* __restrict__ lx1,
+                                                      const V2* __restrict__ lv1, const T* __restrict__ lr1,
+                                                      V2* __restrict__ lx0, V2* __restrict__ lv0,
+                                                      T* __restrict__ lr0, T* __restrict__ dalpha, int accumulate) {
+  const int row = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kDropLanes);
+  const int sub = threadIdx.x % kDropLanes;
+  const bool live = row < n;
+  const int i = live ? row : n - 1;
+  const T dt2 = dt * dt, sdp = dt / P.rho0;
+  const V2 xi = x[i], vi = v[i];
+  const T ri = rt[i];
+  // lambda of row i's outputs: acc via v' = v + dt a and x' = x + dt v + dt^2 a; dpdt via rho'
+  const V2 lxi1 = lx1[i], lvi1 = lv1[i];
+  const T lax = dt * lvi1.x + dt2 * lxi1.x, lay = dt * lvi1.y + dt2 * lxi1.y, ld = sdp * lr1[i];
+  const int k0 = offsets[i];
+  const int k1 = row_end(k0, offsets[i + 1], capacity);
+  T g[5], da;
+  adjoint_row(i, k0, k1, sub, cols, xi, vi, ri, x, v, rt, area, P, dt, lx1, lv1, lr1, lax, lay, ld, g, da);
+  if (!live || sub != 0) return;
   if (P.point_source) {  // a = -mag (x - c) away from the centre
     const T dx = xi.x - P.cx, dy = xi.y - P.cy;
     if (dx * dx + dy * dy > T(1e-14)) {
-      g[0] += -P.point_mag * lai_x;
-      g[1] += -P.point_mag * lai_y;
+      g[0] += -P.point_mag * lax;
+      g[1] += -P.point_mag * lay;
     }
   }
   V2 ox, ov;
@@ -336,7 +615,75 @@ __global__ void __launch_bounds__(128) k_drop_adjoint(int n, const int32_t* __re
   lx0[i] = ox;
   lv0[i] = ov;
   lr0[i] = lr1[i] + g[4];
-  dalpha[i] = da;
+  dalpha[i] = accumulate ? dalpha[i] + da : da;
+}
+
+// ---------------------------------------------------------------- pairs of one step
+// Row counts (kFill = false) or columns of the particles in cell-sorted order, kDropLanes lanes per
+// particle: the candidates are walked as one range per three cell rows, and a lane's hits
+// are placed by the group's ballot, so a row comes in cell order whatever the timing.
+template <bool kFill>
+__global__ void __launch_bounds__(128) k_drop_pairs(const float2* __restrict__ xs, const float* __restrict__ support,
+                                                    int n, const uint32_t* __restrict__ keys,
+                                                    const int32_t* __restrict__ cell_start,
+                                                    const sph_grid* __restrict__ gp, int32_t cap,
+                                                    const uint32_t* __restrict__ order, int32_t* __restrict__ counts,
+                                                    const int32_t* __restrict__ offsets, int64_t capacity,
+                                                    int32_t* __restrict__ cols, int32_t* status) {
+  const int s = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kDropLanes);
+  const int sub = threadIdx.x % kDropLanes;
+  if (s >= n) return;   // the lanes of one particle leave together
+  const unsigned group = ((1u << kDropLanes) - 1u) << ((threadIdx.x & 31) - sub);
+  const unsigned below = ((1u << (threadIdx.x & 31)) - 1u) & group;
+  const sph_grid g = *gp;
+  const uint32_t key = keys[s];
+  const int i = (int)order[s];
+  int found = 0;
+  int32_t* row_cols = nullptr;
+  if constexpr (kFill) {
+    const int k0 = offsets[i], k1 = offsets[i + 1];
+    if (k0 < 0 || k1 < k0 || (int64_t)k1 > capacity) {
+      if (sub == 0) flag(status, SPH_FLAG_PAIR_CAPACITY);
+      return;
+    }
+    row_cols = cols + k0;
+  }
+  if (grid_ok(g, cap) && key < (uint32_t)g.num_cells) {
+    const float2 xi = xs[s];
+    const float thr = grid_threshold(support[i], g);
+    const int cx = (int)(key % (uint32_t)g.cells_x), cy = (int)(key / (uint32_t)g.cells_x);
+    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, g.cells_x - 1);
+    const int y0 = max(cy - 1, 0), y1 = min(cy + 1, g.cells_y - 1);
+    int b[3], e[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const int32_t* row = cell_start + (int64_t)min(y0 + q, y1) * g.cells_x;
+      b[q] = __ldg(row + x0);
+      e[q] = y0 + q <= y1 ? __ldg(row + x1 + 1) : b[q];
+    }
+    const int n0 = e[0] - b[0], n1 = n0 + e[1] - b[1], n2 = n1 + e[2] - b[2];
+    for (int t0 = 0; t0 < n2; t0 += kDropLanes) {
+      const int t = t0 + sub;
+      const int j = t < n0 ? b[0] + t : t < n1 ? b[1] + t - n0 : b[2] + t - n1;
+      bool hit = false;
+      if (t < n2) {
+        const float2 xj = __ldg(xs + j);
+        hit = dist2_ref(xi.x, xi.y, xj.x, xj.y) <= thr;
+      }
+      if constexpr (kFill) {
+        const unsigned m = __ballot_sync(group, hit);
+        if (hit) row_cols[found + __popc(m & below)] = (int32_t)order[j];
+        found += __popc(m);
+      } else {
+        found += hit;
+      }
+    }
+  }
+  if constexpr (!kFill) {
+#pragma unroll
+    for (int o = 1; o < kDropLanes; o <<= 1) found += __shfl_xor_sync(group, found, o);
+    if (sub == 0) counts[i] = found;
+  }
 }
 
 template <typename T>
@@ -362,11 +709,191 @@ DropParams<T> drop_params(const sph_params* p, int mog) {
   return P;
 }
 
+// The columns of every row in increasing order, in -> out (distinct columns; rows past the
+// capacity are left out): one warp per row, a column's place the number of the row's columns
+// below it, counted over the warp's registers.
+__global__ void __launch_bounds__(256) k_sort_rows(int n, const int32_t* __restrict__ offsets, int64_t capacity,
+                                                   const int32_t* __restrict__ in, int32_t* __restrict__ out) {
+  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (i >= n) return;
+  const int b = offsets[i], m = row_end(b, offsets[i + 1], capacity) - b;
+  for (int t0 = 0; t0 < m; t0 += 32) {
+    const int t = t0 + lane;
+    const int j = t < m ? __ldg(in + b + t) : 0x7fffffff;
+    int r = 0;
+    for (int u0 = 0; u0 < m; u0 += 32) {
+      const int u = u0 + lane;
+      const int ju = u0 == t0 ? j : u < m ? __ldg(in + b + u) : 0x7fffffff;
+      const int len = min(m - u0, 32);
+      for (int k = 0; k < len; ++k) r += __shfl_sync(0xffffffffu, ju, k) < j;
+    }
+    if (t < m) out[b + r] = j;
+  }
+}
+
 }  // namespace sph
 
 using namespace sph;
 
+template <typename Col, bool kStep>
+static void launch_rhs(int32_t fp64, int64_t n, const int32_t* offsets, const Col* cols, int64_t capacity,
+                       const void* x, const void* v, const void* rho, const void* area, const sph_params* params,
+                       double dt, void* acc, void* dpdt, void* xo, void* vo, void* ro, float* x32, cudaStream_t st) {
+  const int mog = params->density_diffusion == 1;
+  const int nb = grid_for(n * kDropLanes, 128);
+  if (fp64)
+    k_drop_rhs<double, double2, Col, kStep><<<nb, 128, 0, st>>>(
+        (int)n, offsets, cols, capacity, static_cast<const double2*>(x), static_cast<const double2*>(v),
+        static_cast<const double*>(rho), static_cast<const double*>(area), drop_params<double>(params, mog), dt,
+        static_cast<double2*>(acc), static_cast<double*>(dpdt), static_cast<double2*>(xo), static_cast<double2*>(vo),
+        static_cast<double*>(ro), reinterpret_cast<float2*>(x32));
+  else
+    k_drop_rhs<float, float2, Col, kStep><<<nb, 128, 0, st>>>(
+        (int)n, offsets, cols, capacity, static_cast<const float2*>(x), static_cast<const float2*>(v),
+        static_cast<const float*>(rho), static_cast<const float*>(area), drop_params<float>(params, mog), (float)dt,
+        static_cast<float2*>(acc), static_cast<float*>(dpdt), static_cast<float2*>(xo), static_cast<float2*>(vo),
+        static_cast<float*>(ro), reinterpret_cast<float2*>(x32));
+}
+
+template <typename Col>
+static void launch_adjoint(int32_t fp64, int64_t n, const int32_t* offsets, const Col* cols, int64_t capacity,
+                           const void* x, const void* v, const void* rho, const void* area, const sph_params* params,
+                           double dt, const void* lx1, const void* lv1, const void* lr1, void* lx0, void* lv0,
+                           void* lr0, void* dalpha, int accumulate, cudaStream_t st) {
+  const int mog = params->density_diffusion == 1;
+  const int nb = grid_for(n * kDropLanes, 128);
+  if (fp64)
+    k_drop_adjoint<double, double2, Col><<<nb, 128, 0, st>>>(
+        (int)n, offsets, cols, capacity, static_cast<const double2*>(x), static_cast<const double2*>(v),
+        static_cast<const double*>(rho), static_cast<const double*>(area), drop_params<double>(params, mog), dt,
+        static_cast<const double2*>(lx1), static_cast<const double2*>(lv1), static_cast<const double*>(lr1),
+        static_cast<double2*>(lx0), static_cast<double2*>(lv0), static_cast<double*>(lr0),
+        static_cast<double*>(dalpha), accumulate);
+  else
+    k_drop_adjoint<float, float2, Col><<<nb, 128, 0, st>>>(
+        (int)n, offsets, cols, capacity, static_cast<const float2*>(x), static_cast<const float2*>(v),
+        static_cast<const float*>(rho), static_cast<const float*>(area), drop_params<float>(params, mog), (float)dt,
+        static_cast<const float2*>(lx1), static_cast<const float2*>(lv1), static_cast<const float*>(lr1),
+        static_cast<float2*>(lx0), static_cast<float2*>(lv0), static_cast<float*>(lr0), static_cast<float*>(dalpha),
+        accumulate);
+}
+
+// The scratch of sph_drop_search, in order: cell_count [cap + 1] (zero between calls), cell_start
+// [cap + 2], keys, order, sorted keys, counts [n], sorted positions float2 [n], the sort's and
+// the scan's scratch.
+struct DropScratch {
+  int32_t *cell_count, *cell_start, *counts;
+  uint32_t *keys, *order, *skeys;
+  float* xs;
+  void *sort, *scan;
+  size_t sort_bytes, scan_bytes;
+};
+
+static size_t drop_scratch(int64_t n, int32_t cap, char* base, DropScratch* s) {
+  size_t at = 0;
+  const auto take = [&](size_t bytes) {
+    char* p = base ? base + at : nullptr;
+    at += (bytes + 255) & ~(size_t)255;
+    return p;
+  };
+  DropScratch d;
+  d.cell_count = reinterpret_cast<int32_t*>(take(((size_t)cap + 1) * 4));
+  d.cell_start = reinterpret_cast<int32_t*>(take(((size_t)cap + 2) * 4));
+  d.keys = reinterpret_cast<uint32_t*>(take((size_t)n * 4));
+  d.order = reinterpret_cast<uint32_t*>(take((size_t)n * 4));
+  d.skeys = reinterpret_cast<uint32_t*>(take((size_t)n * 4));
+  d.counts = reinterpret_cast<int32_t*>(take((size_t)n * 4));
+  d.xs = reinterpret_cast<float*>(take((size_t)n * 8));
+  d.sort_bytes = sph_counting_sort_scratch_bytes(n, cap);
+  d.sort = take(d.sort_bytes);
+  d.scan_bytes = sph_scan_scratch_bytes(n);
+  d.scan = take(d.scan_bytes);
+  if (s) *s = d;
+  return at;
+}
+
+#define SPH_DROP_PARAMS(p)                                                \
+  ((p) && (p)->support > 0.f && (p)->gamma == 7.f &&                      \
+   ((p)->density_diffusion == 0 || (p)->density_diffusion == 1))
+
 extern "C" {
+
+size_t sph_drop_search_scratch_bytes(int64_t n, int32_t cell_capacity) {
+  return drop_scratch(n > 0 ? n : 0, cell_capacity > 0 ? cell_capacity : 0, nullptr, nullptr) + 256;
+}
+
+sph_status_t sph_drop_search(const float* x32, const float* support, int64_t n, const sph_grid* grid,
+                             int32_t cell_capacity, int32_t* offsets, int64_t pair_capacity, int32_t* cols,
+                             int32_t* unsorted, int32_t* status, void* scratch, size_t scratch_bytes, void* stream) {
+  SPH_REQUIRE(n >= 0 && n < (1LL << 31) && cell_capacity > 0 && grid && offsets && status && pair_capacity >= 0 &&
+                  (n == 0 || (x32 && support && cols && pair_capacity > 0 && unsorted != cols)),
+              "drop_search: bad arguments");
+  if (!scratch || scratch_bytes < sph_drop_search_scratch_bytes(n, cell_capacity)) {
+    set_error_text("drop_search: scratch smaller than sph_drop_search_scratch_bytes(n, cell_capacity)");
+    return SPH_ERR_SCRATCH_TOO_SMALL;
+  }
+  cudaStream_t st = as_stream(stream);
+  DropScratch d;
+  drop_scratch(n, cell_capacity, reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(scratch) + 255) & ~(uintptr_t)255),
+               &d);
+  if (n == 0) {
+    cudaMemsetAsync(offsets, 0, sizeof(int32_t), st);
+    SPH_CHECK_LAUNCH("drop_search");
+    return SPH_OK;
+  }
+  sph_status_t r = sph_cell_keys(x32, n, grid, cell_capacity, d.keys, nullptr, d.cell_count, status, stream);
+  if (r != SPH_OK) return r;
+  const int32_t eb[1] = {8};
+  const void* in[1] = {x32};
+  void* out[1] = {d.xs};
+  r = sph_counting_sort_permute(d.keys, n, cell_capacity, d.cell_count, d.cell_start, nullptr, d.order, d.skeys, 1, eb,
+                                in, out, status, d.sort, d.sort_bytes, stream);
+  if (r != SPH_OK) return r;
+  const int nb = grid_for(n * kDropLanes, 128);
+  const float2* xs = reinterpret_cast<const float2*>(d.xs);
+  k_drop_pairs<false><<<nb, 128, 0, st>>>(xs, support, (int)n, d.skeys, d.cell_start, grid, cell_capacity, d.order,
+                                          d.counts, nullptr, 0, nullptr, status);
+  SPH_CHECK_LAUNCH("drop_search(count)");
+  r = sph_exclusive_scan_i32(d.counts, offsets, n, d.scan, d.scan_bytes, stream);
+  if (r != SPH_OK) return r;
+  k_drop_pairs<true><<<nb, 128, 0, st>>>(xs, support, (int)n, d.skeys, d.cell_start, grid, cell_capacity, d.order,
+                                         nullptr, offsets, pair_capacity, unsorted ? unsorted : cols, status);
+  if (unsorted) k_sort_rows<<<grid_for(n, 8), 256, 0, st>>>((int)n, offsets, pair_capacity, unsorted, cols);
+  SPH_CHECK_LAUNCH("drop_search(fill)");
+  return SPH_OK;
+}
+
+sph_status_t sph_drop_step(int32_t fp64, int64_t n, const int32_t* offsets, const int32_t* cols,
+                           int64_t pair_capacity, const void* x, const void* v, const void* rho, const void* area,
+                           const sph_params* params, double dt, void* x_out, void* v_out, void* rho_out, float* x32_out,
+                           void* stream) {
+  SPH_REQUIRE(n >= 0 && n < (1LL << 31) && SPH_DROP_PARAMS(params) && params->rest_density > 0 &&
+                  (n == 0 || (pair_capacity > 0 && offsets && cols && x && v && rho && area && x_out && v_out && rho_out)),
+              "drop_step: bad arguments (gamma 7, MOG or no density diffusion)");
+  SPH_REQUIRE(n == 0 || (x_out != x && v_out != v && rho_out != rho), "drop_step: outputs must not alias inputs");
+  if (n == 0) return SPH_OK;
+  launch_rhs<int32_t, true>(fp64, n, offsets, cols, pair_capacity, x, v, rho, area, params, dt, nullptr, nullptr, x_out,
+                            v_out, rho_out, x32_out, as_stream(stream));
+  SPH_CHECK_LAUNCH("drop_step");
+  return SPH_OK;
+}
+
+sph_status_t sph_drop_adjoint_step(int32_t fp64, int64_t n, const int32_t* offsets, const int32_t* cols,
+                                   int64_t pair_capacity, const void* x, const void* v, const void* rho,
+                                   const void* area, const sph_params* params, double dt, const void* lx1,
+                                   const void* lv1, const void* lr1, void* lx0, void* lv0, void* lr0, void* dalpha,
+                                   void* stream) {
+  SPH_REQUIRE(n >= 0 && n < (1LL << 31) && SPH_DROP_PARAMS(params) &&
+                  (n == 0 || (pair_capacity > 0 && offsets && cols && x && v && rho && area && lx1 && lv1 && lr1 && lx0 && lv0 && lr0 &&
+                              dalpha)),
+              "drop_adjoint_step: bad arguments (gamma 7, MOG or no density diffusion)");
+  SPH_REQUIRE(lx0 != lx1 && lv0 != lv1 && lr0 != lr1, "drop_adjoint_step: outputs must not alias inputs");
+  if (n == 0) return SPH_OK;
+  launch_adjoint(fp64, n, offsets, cols, pair_capacity, x, v, rho, area, params, dt, lx1, lv1, lr1, lx0, lv0, lr0,
+                 dalpha, 1, as_stream(stream));
+  SPH_CHECK_LAUNCH("drop_adjoint_step");
+  return SPH_OK;
+}
 
 sph_status_t sph_drop_rhs(int32_t fp64, int64_t n, const int32_t* offsets, const int64_t* cols, const void* x,
                           const void* v, const void* rho, const void* area, const sph_params* params, void* acc,
@@ -376,19 +903,8 @@ sph_status_t sph_drop_rhs(int32_t fp64, int64_t n, const int32_t* offsets, const
                   (n == 0 || (offsets && cols && x && v && rho && area && acc && dpdt)),
               "drop_rhs: bad arguments (gamma 7, MOG or no density diffusion)");
   if (n == 0) return SPH_OK;
-  const int mog = params->density_diffusion == 1;
-  cudaStream_t st = as_stream(stream);
-  if (fp64) {
-    k_drop_rhs<double, double2><<<grid_for(n, 128), 128, 0, st>>>(
-        (int)n, offsets, cols, static_cast<const double2*>(x), static_cast<const double2*>(v),
-        static_cast<const double*>(rho), static_cast<const double*>(area), drop_params<double>(params, mog),
-        static_cast<double2*>(acc), static_cast<double*>(dpdt));
-  } else {
-    k_drop_rhs<float, float2><<<grid_for(n, 128), 128, 0, st>>>(
-        (int)n, offsets, cols, static_cast<const float2*>(x), static_cast<const float2*>(v),
-        static_cast<const float*>(rho), static_cast<const float*>(area), drop_params<float>(params, mog),
-        static_cast<float2*>(acc), static_cast<float*>(dpdt));
-  }
+  launch_rhs<int64_t, false>(fp64, n, offsets, cols, 0, x, v, rho, area, params, 0.0, acc, dpdt, nullptr, nullptr,
+                             nullptr, nullptr, as_stream(stream));
   SPH_CHECK_LAUNCH("drop_rhs");
   return SPH_OK;
 }
@@ -422,21 +938,8 @@ sph_status_t sph_drop_adjoint(int32_t fp64, int64_t n, const int32_t* offsets, c
               "drop_adjoint: bad arguments (gamma 7, MOG or no density diffusion)");
   SPH_REQUIRE(lx0 != lx1 && lv0 != lv1 && lr0 != lr1, "drop_adjoint: outputs must not alias inputs");
   if (n == 0) return SPH_OK;
-  const int mog = params->density_diffusion == 1;
-  cudaStream_t st = as_stream(stream);
-  if (fp64)
-    k_drop_adjoint<double, double2><<<grid_for(n, 128), 128, 0, st>>>(
-        (int)n, offsets, cols, static_cast<const double2*>(x), static_cast<const double2*>(v),
-        static_cast<const double*>(rho), static_cast<const double*>(area), drop_params<double>(params, mog), dt,
-        static_cast<const double2*>(lx1), static_cast<const double2*>(lv1), static_cast<const double*>(lr1),
-        static_cast<double2*>(lx0), static_cast<double2*>(lv0), static_cast<double*>(lr0),
-        static_cast<double*>(dalpha));
-  else
-    k_drop_adjoint<float, float2><<<grid_for(n, 128), 128, 0, st>>>(
-        (int)n, offsets, cols, static_cast<const float2*>(x), static_cast<const float2*>(v),
-        static_cast<const float*>(rho), static_cast<const float*>(area), drop_params<float>(params, mog), (float)dt,
-        static_cast<const float2*>(lx1), static_cast<const float2*>(lv1), static_cast<const float*>(lr1),
-        static_cast<float2*>(lx0), static_cast<float2*>(lv0), static_cast<float*>(lr0), static_cast<float*>(dalpha));
+  launch_adjoint(fp64, n, offsets, cols, 0, x, v, rho, area, params, dt, lx1, lv1, lr1, lx0, lv0, lr0, dalpha, 0,
+                 as_stream(stream));
   SPH_CHECK_LAUNCH("drop_adjoint");
   return SPH_OK;
 }
