@@ -825,7 +825,8 @@ sph_status_t sph_update_dt(int64_t n, const float* v, const float* acc, float su
  * and buildNeighborListUnsortedPerParticle (cppSrc/neighSearch.cpp:261-331): query points
  * (any order) against the reference-format hash table.  rows = query index, cols = sort[j].
  * Two passes: _count writes counts[m]; the caller scans them to offsets (int64 [m+1]);
- * _fill writes the pairs.  qmin is a device float[2]. */
+ * _fill writes the pairs (rows may be NULL: the offsets hold them).  qmin is a device
+ * float[2]. */
 sph_status_t sph_nl_hashed_query_count(const float* query_pos, const float* query_support, int64_t m,
                                        const float* sorted_pos, const int32_t* hash_table,
                                        const int32_t* cell_indices, const int32_t* cum_cell,
@@ -838,6 +839,10 @@ sph_status_t sph_nl_hashed_query_fill(const float* query_pos, const float* query
                                       const int32_t* cell_span, const int32_t* sort, const float* qmin,
                                       float hmax, int32_t cells_x, int32_t hash_len, int32_t search_radius,
                                       const int64_t* offsets, int32_t* rows, int32_t* cols, void* stream);
+/* The filled pairs of m rows in (row, column) order as int64 (the finalize of
+ * src/modules/neighborSearch.py:153-157). */
+sph_status_t sph_nl_pairs_in_order(int64_t m, const int64_t* offsets, const int32_t* cols, int64_t* rows_out,
+                                   int64_t* cols_out, void* stream);
 /* buildNeighborList (cppSrc/neighSearch.cpp:172-259): every occupied cell of the table
  * against its (2r+1)^2 neighbor cells; rows = sort[i], cols = sort[j].  One count per
  * cell (counts[num_cells]). */

@@ -61,6 +61,7 @@ SIGNATURES = {
     "sph_nl_hashed_query_count": (_I32, [_P, _P, _I64, _P, _P, _P, _P, _P, _P, _F32, _I32, _I32, _I32, _P, _P]),
     "sph_nl_hashed_query_fill": (_I32, [_P, _P, _I64, _P, _P, _P, _P, _P, _P, _P, _F32, _I32, _I32, _I32, _P,
                                         _P, _P, _P]),
+    "sph_nl_pairs_in_order": (_I32, [_I64, _P, _P, _P, _P, _P]),
     "sph_nl_hashed_cells_count": (_I32, [_P, _P, _P, _P, _P, _P, _I64, _I32, _I32, _I32, _P, _P]),
     "sph_nl_hashed_cells_fill": (_I32, [_P, _P, _P, _P, _P, _P, _P, _I64, _I32, _I32, _I32, _P, _P, _P, _P]),
     "sph_nl_hashed_asym_count": (_I32, [_P, _P, _P, _P, _P, _P, _I64, _P, _P, _P, _P, _P, _I32, _I32, _P, _P]),

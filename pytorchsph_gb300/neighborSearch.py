@@ -38,11 +38,12 @@ def _check_dtype(t, name, dtype):
         raise RuntimeError(f"{name} must have dtype {dtype}, got {t.dtype}")
 
 
-def _two_pass(count_fn, fill_fn, m, device):
+def _two_pass(count_fn, fill_fn, m, device, in_order=False):
+    """[rows, cols] int32 in the fill's order, or (in_order) int64 in (row, column) order."""
     st = N.stream_ptr()
     counts = torch.empty(max(m, 1), dtype=torch.int32, device=device)
     if m == 0:
-        e = torch.empty(0, dtype=torch.int32, device=device)
+        e = torch.empty(0, dtype=torch.int64 if in_order else torch.int32, device=device)
         return [e, e.clone()]
     count_fn(counts, st)
     offsets = torch.empty(m + 1, dtype=torch.int64, device=device)
@@ -51,8 +52,15 @@ def _two_pass(count_fn, fill_fn, m, device):
     scratch = torch.empty((sb + 7) // 8, dtype=torch.int64, device=device)
     N.call("sph_exclusive_scan_i32_to_i64", N.ptr(counts), N.ptr(offsets), m, N.ptr(scratch), scratch.numel() * 8, st)
     P = int(offsets[m].item())  # the reference reads the total back too (cppSrc/neighSearch_cuda.cu:267)
-    rows = torch.empty(P, dtype=torch.int32, device=device)
     cols = torch.empty(P, dtype=torch.int32, device=device)
+    if in_order:
+        i = torch.empty(P, dtype=torch.int64, device=device)
+        j = torch.empty(P, dtype=torch.int64, device=device)
+        if P > 0:
+            fill_fn(offsets, None, cols, st)
+            N.call("sph_nl_pairs_in_order", m, N.ptr(offsets), N.ptr(cols), N.ptr(i), N.ptr(j), st)
+        return [i, j]
+    rows = torch.empty(P, dtype=torch.int32, device=device)
     if P > 0:
         fill_fn(offsets, rows, cols, st)
     return [rows, cols]
@@ -83,7 +91,7 @@ def buildNeighborListCUDA(queryParticles_, support_, sortedParticles, sortedSupp
                   qMin_, hMax, cellsX, hashMapLength, searchRadius)
 
 
-def _query(qpos, qh, spos, table, ci, cc, cs, sort, qmin, hmax, cells_x, L, r):
+def _query(qpos, qh, spos, table, ci, cc, cs, sort, qmin, hmax, cells_x, L, r, in_order=False):
     m = qpos.shape[0]
     dev = qpos.device
     qmin = _qmin_device(qmin, dev)
@@ -97,7 +105,7 @@ def _query(qpos, qh, spos, table, ci, cc, cs, sort, qmin, hmax, cells_x, L, r):
                N.ptr(cc), N.ptr(cs), N.ptr(sort), N.ptr(qmin), float(hmax), int(cells_x), int(L), int(r),
                N.ptr(offsets), N.ptr(rows), N.ptr(cols), st)
 
-    return _two_pass(count, fill, m, dev)
+    return _two_pass(count, fill, m, dev, in_order)
 
 
 def buildNeighborList(queryParticles_, support_, hashTable_, cellIndices_, cumCell_, cellSpan_, sort_,

@@ -151,15 +151,11 @@ def constructNeighborhoodsCUDA(queryPositions, querySupports, hashMapLength: int
         hashMapLength = nextprime(queryPositions.shape[0])
     table, cli, cellOffsets, cellCounters = constructHashMap(sp, ss, sli, si, hashMapLength, cellCount)
     si = si.to(torch.int32)
-    i, j = _ext.buildNeighborListCUDA(_float32_cuda(queryPositions, "queryPositions"),
-                                      _float32_cuda(querySupports, "querySupports"), sp, ss, table, cli, cellOffsets,
-                                      cellCounters, si, qMin, hMax, cellCount, hashMapLength, searchRadius)
-    # the finalize of neighborSearch.py:153-157: stable sort by j, then by i
-    j, jj = torch.sort(j, dim=0, stable=True)
-    i = i[jj]
-    i, ii = torch.sort(i, dim=0, stable=True)
-    j = j[ii]
-    return (i.to(torch.int64), j.to(torch.int64), None, None, (qMin, hMax, si, sp, ss), (table, hashMapLength),
+    # the per-particle query of the extension, finalised in (i, j) order (neighborSearch.py:153-157)
+    i, j = _ext._query(_float32_cuda(queryPositions, "queryPositions"), _float32_cuda(querySupports, "querySupports"),
+                       sp, table, cli, cellOffsets, cellCounters, si, qMin, hMax, cellCount, hashMapLength,
+                       searchRadius, in_order=True)
+    return (i, j, None, None, (qMin, hMax, si, sp, ss), (table, hashMapLength),
             (cli, cellOffsets, cellCounters, cellCount))
 
 
