@@ -110,6 +110,10 @@ typedef struct sph_wall_view {
 int32_t sph_abi_version(void);
 const char* sph_last_error(void);
 const char* sph_status_string(sph_status_t status);
+/* Reads na words at a and nb at b (device; b may be NULL with nb = 0) into host[capacity] and
+ * waits for the stream once: a search's pair total and status without a wait for each. */
+sph_status_t sph_read_i32(const int32_t* a, int32_t na, const int32_t* b, int32_t nb, int32_t* host,
+                          int32_t capacity, void* stream);
 
 /* ---------------------------------------------------------------- primitives */
 

@@ -61,6 +61,7 @@ SIGNATURES = {
     "sph_nl_hashed_query_count": (_I32, [_P, _P, _I64, _P, _P, _P, _P, _P, _P, _F32, _I32, _I32, _I32, _P, _P]),
     "sph_nl_hashed_query_fill": (_I32, [_P, _P, _I64, _P, _P, _P, _P, _P, _P, _P, _F32, _I32, _I32, _I32, _P,
                                         _P, _P, _P]),
+    "sph_read_i32": (_I32, [_P, _I32, _P, _I32, _P, _I32, _P]),
     "sph_nl_pairs_in_order": (_I32, [_I64, _P, _P, _P, _P, _P]),
     "sph_nl_hashed_cells_count": (_I32, [_P, _P, _P, _P, _P, _P, _I64, _I32, _I32, _I32, _P, _P]),
     "sph_nl_hashed_cells_fill": (_I32, [_P, _P, _P, _P, _P, _P, _P, _I64, _I32, _I32, _I32, _P, _P, _P, _P]),
@@ -173,8 +174,11 @@ def library_path() -> str:
 def load(require_cuda: bool = True):
     """Load libsph_gb300.so; raises if it is missing (no CPU fallback exists)."""
     global _lib
-    if require_cuda and not torch.cuda.is_available():
+    # (an initialized CUDA context has a device; asking for one reads the environment, 3 us)
+    if require_cuda and not torch.cuda.is_initialized() and not torch.cuda.is_available():
         raise SPHError("pytorchsph_gb300 needs a CUDA device (GB300, sm_103a); there is no CPU path")
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             path = library_path()
@@ -198,8 +202,9 @@ def check(status: int, what: str = ""):
 
 
 def call(name: str, *args):
-    fn = getattr(load(), name)
-    check(fn(*args), name)
+    status = getattr(load(), name)(*args)
+    if status:
+        check(status, name)
 
 
 def ptr(t) -> int | None:
@@ -209,7 +214,24 @@ def ptr(t) -> int | None:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream.  torch.cuda.current_stream() also reads the
+    environment and builds a Stream object: 6 us of each call that launches 2 us of work."""
+    if not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+_host = threading.local()   # each thread's pinned words for read_i32
+
+
+def read_i32(a: torch.Tensor, b: torch.Tensor | None = None):
+    """The 32-bit words of one or two small device tensors on the host (at most 16 in all), with
+    one wait for the current stream."""
+    if not hasattr(_host, "words"):
+        _host.words = torch.empty(16, dtype=torch.int32, pin_memory=True)
+    na, nb = a.numel(), 0 if b is None else b.numel()
+    call("sph_read_i32", ptr(a), na, ptr(b), nb, ptr(_host.words), 16, stream_ptr())
+    return _host.words[:na + nb].tolist()
 
 
 def array_set(pairs):

@@ -100,7 +100,7 @@ class DropRollout:
         step), the cell capacity, the status word and the scratch."""
         x32 = self.x0.to(torch.float32).contiguous()
         cap = self.search.auto_cell_capacity(x32, self.support32, self.vmin, self.vmax)
-        grid = self.search.ws.get("grid", 8, torch.int32).clone()   # the one the cells were counted on
+        grid = self.search.grid_status()[0].clone()   # the one the cells were counted on
         status = torch.zeros(1, dtype=torch.int32, device=self.dev)
         size = N.load().sph_drop_search_scratch_bytes(self.n, cap)
         return grid, cap, status, torch.zeros((size + 7) // 8, dtype=torch.int64, device=self.dev)

@@ -382,6 +382,22 @@ const char* sph_status_string(sph_status_t s) {
   }
 }
 
+sph_status_t sph_read_i32(const int32_t* a, int32_t na, const int32_t* b, int32_t nb, int32_t* host,
+                          int32_t capacity, void* stream) {
+  SPH_REQUIRE(a && host && na > 0 && nb >= 0 && (nb == 0 || b) && (int64_t)na + nb <= capacity,
+              "read_i32: bad arguments");
+  cudaStream_t st = as_stream(stream);
+  cudaError_t e = cudaMemcpyAsync(host, a, (size_t)na * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess && nb > 0)
+    e = cudaMemcpyAsync(host + na, b, (size_t)nb * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    set_error("read_i32", e);
+    return SPH_ERR_CUDA;
+  }
+  return SPH_OK;
+}
+
 uint64_t sph_scan_timeouts(void) {
   unsigned long long v = 0;
   if (cudaMemcpyFromSymbol(&v, g_scan_timeouts, sizeof(v)) != cudaSuccess) return ~0ull;

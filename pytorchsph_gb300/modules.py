@@ -209,7 +209,8 @@ def pair_term(term, simulationState, P, pressure=None, L=None, grad_rho=None, ou
         "pred_accel", "pred_vel")], float(dt), n)
     w = WIDTH[term]
     if out is None:
-        out = torch.zeros((n,) if w == 1 else (n, w), dtype=torch.float32, device=st['fluidPosition'].device)
+        alloc = torch.zeros if accumulate else torch.empty   # every row is written
+        out = alloc((n,) if w == 1 else (n, w), dtype=torch.float32, device=st['fluidPosition'].device)
     N.call("sph_pair_term", TERM[term], ctypes.byref(inp), ctypes.byref(P), N.ptr(out), int(accumulate),
            N.stream_ptr())
     return out.view(n, 2, 2) if term == "normalization" else out
@@ -289,15 +290,17 @@ class neighborSearchModule(Module):
         sup = _f32(simulationState['fluidSupport'])
         if self.engine is None:
             self.engine = GridSearch(pos.device)
-        self.csr = self.engine.run(pos, sup, kernel_support=float(self.support), density=False,
-                                   min_coord=np.asarray(self.minDomain, np.float32),
-                                   max_coord=np.asarray(self.maxDomain, np.float32))
-        fluidNeighbors, fluidDistances, fluidRadialDistances = self.csr.to_coo(self.threshold)
+        csr = self.engine.run(pos, sup, kernel_support=float(self.support), density=False,
+                              min_coord=np.asarray(self.minDomain, np.float32),
+                              max_coord=np.asarray(self.maxDomain, np.float32), sync=False)
+        offsets = torch.empty(csr.n + 1, dtype=torch.int32, device=pos.device)
+        # (to_coo checks the search)
+        fluidNeighbors, fluidDistances, fluidRadialDistances = csr.to_coo(self.threshold, row_offsets=offsets)
+        self.csr = csr
         simulationState['fluidNeighbors'] = fluidNeighbors
         simulationState['fluidDistances'] = fluidDistances
         simulationState['fluidRadialDistances'] = fluidRadialDistances
-        simulationState.pop('fluidNeighborOffsets', None)
-        row_offsets(simulationState)
+        simulationState['fluidNeighborOffsets'] = offsets
         return fluidNeighbors, fluidDistances, fluidRadialDistances
 
     def searchExisting(self, queryPositions, querySupports, simulationState, simulation, searchRadius: int = 1):
@@ -547,11 +550,12 @@ def wall_term(term, pairs, P, n, nb, out=None, accumulate=False, dt=0.0, **array
                      *[N.ptr(keep.get(k)) for k in names], float(dt), n, nb)
     if out is None:
         dev = pairs.rows.device
+        alloc = torch.zeros if accumulate else torch.empty   # every row is written
         if WALL[term] >= 20:
-            out = torch.zeros(nb, dtype=torch.float32, device=dev)
+            out = alloc(nb, dtype=torch.float32, device=dev)
         else:
             w = WALL_WIDTH[term]
-            out = torch.zeros((n,) if w == 1 else (n, w), dtype=torch.float32, device=dev)
+            out = alloc((n,) if w == 1 else (n, w), dtype=torch.float32, device=dev)
     N.call("sph_wall_term", WALL[term], ctypes.byref(inp), ctypes.byref(P), N.ptr(out), int(accumulate),
            N.stream_ptr())
     return out

@@ -21,6 +21,7 @@ from __future__ import annotations
 import torch
 
 from . import _native as N
+from .search import _total
 
 __all__ = ["buildNeighborListCUDA", "buildNeighborList", "buildNeighborListAsymmetric",
            "buildNeighborListUnsortedPerParticle"]
@@ -51,7 +52,7 @@ def _two_pass(count_fn, fill_fn, m, device, in_order=False):
     sb = lib.sph_scan_scratch_bytes(m)
     scratch = torch.empty((sb + 7) // 8, dtype=torch.int64, device=device)
     N.call("sph_exclusive_scan_i32_to_i64", N.ptr(counts), N.ptr(offsets), m, N.ptr(scratch), scratch.numel() * 8, st)
-    P = int(offsets[m].item())  # the reference reads the total back too (cppSrc/neighSearch_cuda.cu:267)
+    P = _total(offsets)  # the reference reads the total back too (cppSrc/neighSearch_cuda.cu:267)
     cols = torch.empty(P, dtype=torch.int32, device=device)
     if in_order:
         i = torch.empty(P, dtype=torch.int64, device=device)

@@ -21,7 +21,7 @@ import torch
 
 from . import _native as N
 from . import neighborSearch as _ext
-from .search import MAX_CELLS, _f2, grid_from_bytes, next_prime
+from .search import MAX_CELLS, _f2, grid_from_words, next_prime
 
 __all__ = ["sortPositions", "constructHashMap", "constructNeighborhoods", "constructNeighborhoodsPreSorted",
            "constructNeighborhoodsCUDA", "constructNeighborhoodsPreSortedCUDA", "nextprime"]
@@ -50,6 +50,19 @@ def sortPositions(queryParticles, querySupport, supportScale: float = 1.0, qMin=
     """src/modules/neighborSearch.py:30-55: (sortedPositions, sortedSupport,
     sortedLinearIndices int32, sortingIndices int64, cellCount int, qMin float32 [2] (device),
     hMax float).  Reads the grid back to the host once (the reference's int() / float())."""
+    xy, sh, skeys, order, cells_x, qmin, hmax, status = _sort_positions(queryParticles, querySupport, supportScale,
+                                                                        qMin, qMax)
+    _check_sorted(int(status.item()))
+    return xy, sh, skeys, order.long(), cells_x, qmin, hmax
+
+
+def _check_sorted(flags):
+    if flags & (N.SPH_FLAG_OUT_OF_GRID | N.SPH_FLAG_NONFINITE):
+        raise RuntimeError("sortPositions: particles outside the grid given by qMin / qMax")
+
+
+def _sort_positions(queryParticles, querySupport, supportScale, qMin, qMax):
+    """sortPositions with int32 indices and the status word, unread, at the end."""
     if float(supportScale) != 1.0:
         raise RuntimeError("sortPositions: only supportScale = 1.0 is supported")
     pos = _float32_cuda(queryParticles, "queryParticles")
@@ -62,13 +75,14 @@ def sortPositions(queryParticles, querySupport, supportScale: float = 1.0, qMin=
     lib = N.load()
     dev = pos.device
     st = N.stream_ptr()
-    status = torch.zeros(1, dtype=torch.int32, device=dev)
-    grid = torch.empty(8, dtype=torch.int32, device=dev)
+    words = torch.zeros(9, dtype=torch.int32, device=dev)
+    grid, status = words[:8], words[8:]
     gs = torch.empty((lib.sph_grid_scratch_bytes(n) + 7) // 8, dtype=torch.int64, device=dev)
     N.call("sph_grid_build", N.ptr(pos), N.ptr(sup), n, _f2(_host2(qMin)), _f2(_host2(qMax)), MAX_CELLS,
            N.ptr(grid), N.ptr(status), N.ptr(gs), gs.numel() * 8, st)
-    info = grid_from_bytes(grid)
-    if int(status.item()) != 0:
+    *g, flags = N.read_i32(words)
+    info = grid_from_words(g)
+    if flags != 0:
         raise RuntimeError("sortPositions: non-finite input or a grid of more than 2^28 cells")
     cap = max(info["num_cells"], 1)
     keys = torch.empty(n, dtype=torch.int32, device=dev)
@@ -83,11 +97,8 @@ def sortPositions(queryParticles, querySupport, supportScale: float = 1.0, qMin=
     xy = torch.empty((n, 2), dtype=torch.float32, device=dev)
     sh = torch.empty(n, dtype=torch.float32, device=dev)
     N.call("sph_gather_sorted", N.ptr(order), n, N.ptr(pos), N.ptr(sup), None, N.ptr(xy), N.ptr(sh), None, st)
-    flags = int(status.item())
-    if flags & (N.SPH_FLAG_OUT_OF_GRID | N.SPH_FLAG_NONFINITE):
-        raise RuntimeError("sortPositions: particles outside the grid given by qMin / qMax")
-    qmin = torch.tensor(info["qmin"], dtype=torch.float32, device=dev)
-    return xy, sh, skeys, order.long(), int(info["cells_x"]), qmin, float(info["hmax"])
+    qmin = grid[:2].view(torch.float32).clone()
+    return xy, sh, skeys, order, int(info["cells_x"]), qmin, float(info["hmax"]), status
 
 
 def constructHashMap(sortedPositions, sortedSupport, sortedIndices, sort, hashMapLength: int, cellCount: int):
@@ -95,7 +106,11 @@ def constructHashMap(sortedPositions, sortedSupport, sortedIndices, sort, hashMa
     particle count of each cell), cellSpan (its first sorted index)), all int32 [C] in hash
     order.  The map is built on the device without a host wait; slicing the C occupied
     cells reads C back once (the reference's output shapes need it as well)."""
-    keys = sortedIndices
+    return _hash_map(sortedIndices, hashMapLength, cellCount)
+
+
+def _hash_map(keys, hashMapLength, cellCount, status=None):
+    """constructHashMap; a sort's status word is read with the number of cells."""
     if not isinstance(keys, torch.Tensor) or not keys.is_cuda:
         raise RuntimeError("sortedIndices must be a CUDA tensor")
     keys = keys.to(torch.int32).contiguous()
@@ -113,7 +128,8 @@ def constructHashMap(sortedPositions, sortedSupport, sortedIndices, sort, hashMa
     sc = torch.empty((lib.sph_hash_map_scratch_bytes(n, L) + 7) // 8, dtype=torch.int64, device=dev)
     N.call("sph_hash_map_build", N.ptr(keys), n, int(cellCount), L, N.ptr(table), N.ptr(ci), N.ptr(cum), N.ptr(span),
            N.ptr(C), N.ptr(sc), sc.numel() * 8, N.stream_ptr())
-    c = int(C.item())
+    c, flags = N.read_i32(C, status) if status is not None else (int(C.item()), 0)
+    _check_sorted(flags)
     return table, ci[:c], cum[:c], span[:c]
 
 
@@ -146,11 +162,11 @@ def constructNeighborhoodsPreSorted(queryPositions, querySupports, particleState
 def constructNeighborhoodsCUDA(queryPositions, querySupports, hashMapLength: int = -1, supportScale: float = 1.0,
                                minCoord=None, maxCoord=None, searchRadius: int = 1):
     """src/modules/neighborSearch.py:139-159: per-query search, pairs finalised in (i, j) order."""
-    sp, ss, sli, si, cellCount, qMin, hMax = sortPositions(queryPositions, querySupports, 1.0, minCoord, maxCoord)
+    sp, ss, sli, si, cellCount, qMin, hMax, status = _sort_positions(queryPositions, querySupports, 1.0, minCoord,
+                                                                     maxCoord)
     if hashMapLength == -1:
         hashMapLength = nextprime(queryPositions.shape[0])
-    table, cli, cellOffsets, cellCounters = constructHashMap(sp, ss, sli, si, hashMapLength, cellCount)
-    si = si.to(torch.int32)
+    table, cli, cellOffsets, cellCounters = _hash_map(sli, hashMapLength, cellCount, status)
     # the per-particle query of the extension, finalised in (i, j) order (neighborSearch.py:153-157)
     i, j = _ext._query(_float32_cuda(queryPositions, "queryPositions"), _float32_cuda(querySupports, "querySupports"),
                        sp, table, cli, cellOffsets, cellCounters, si, qMin, hMax, cellCount, hashMapLength,

@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import struct
 
 import torch
 
@@ -36,7 +37,7 @@ class Workspace:
         if b is None or b.numel() < numel or b.dtype != dtype:
             b = torch.empty(numel, dtype=dtype, device=self.device)
             self._bufs[name] = b
-        return b[:numel]
+        return b if b.numel() == numel else b[:numel]
 
     def zeros(self, name, numel, dtype=torch.int32):
         """Like get(), but zero-filled the first time the buffer is created."""
@@ -51,13 +52,21 @@ class Workspace:
         return self.get(name, (int(nbytes) + 7) // 8, torch.int64)
 
 
+def grid_from_words(words) -> dict:
+    """Decode the eight 32-bit words of an sph_grid."""
+    q0, q1, hmax, _, cx, cy, cells, _ = struct.unpack("<4f3if", struct.pack("<8i", *words))
+    return {"qmin": (q0, q1), "hmax": hmax, "cells_x": cx, "cells_y": cy, "num_cells": cells}
+
+
 def grid_from_bytes(t: torch.Tensor) -> dict:
     """Decode an sph_grid struct read back to the host."""
-    raw = t.detach().cpu().view(torch.int32)
-    f = raw[:4].view(torch.float32)
-    i = raw[4:8]
-    return {"qmin": (float(f[0]), float(f[1])), "hmax": float(f[2]), "cells_x": int(i[0]),
-            "cells_y": int(i[1]), "num_cells": int(i[2])}
+    return grid_from_words(t.detach().cpu().view(torch.int32)[:8].tolist())
+
+
+def _total(offsets: torch.Tensor) -> int:
+    """The last of int64 offsets on the host."""
+    low, high = N.read_i32(offsets[-1:].view(torch.int32))
+    return high << 32 | low & 0xffffffff
 
 
 def _f2(v):
@@ -85,12 +94,14 @@ class CSRNeighbors:
     def flags(self) -> int:
         return int(self.status.item())
 
-    def check(self):
-        f = self.flags()
+    def check(self) -> int:
+        """Raises for a flagged search; the number of pairs (one wait for both)."""
+        pairs, f = N.read_i32(self.offsets[self.n:], self.status)
         if f:
             raise N.SPHError(f"neighbor search: {N.decode_flags(f)}")
-        if self.num_pairs > self.pair_capacity:
+        if pairs > self.pair_capacity:
             raise N.SPHError("neighbor search: neighbor pair buffer too small")
+        return pairs
 
     def grid_info(self) -> dict:
         return grid_from_bytes(self.grid)
@@ -114,13 +125,15 @@ class CSRNeighbors:
         """rho in original particle order."""
         return self.to_original(self.rho)
 
-    def to_coo(self, grad_threshold: float = 1e-7, distances: bool = True):
+    def to_coo(self, grad_threshold: float = 1e-7, distances: bool = True, row_offsets=None):
         """(fluidNeighbors int64 [2,P], fluidDistances [P,2], fluidRadialDistances [P]) in the
-        reference layout (src/modules/neighborSearch.py:216-227), pairs ordered by (i, j)."""
-        self.check()
-        P = self.num_pairs
+        reference layout (src/modules/neighborSearch.py:216-227), pairs ordered by (i, j);
+        row_offsets (int32 [n+1]) takes the first pair of each i."""
+        P = self.check()
         dev = self.order.device
         if self.n == 0:
+            if row_offsets is not None:
+                row_offsets.zero_()
             return (torch.empty((2, 0), dtype=torch.int64, device=dev),
                     torch.empty((0, 2), dtype=torch.float32, device=dev) if distances else None,
                     torch.empty(0, dtype=torch.float32, device=dev) if distances else None)
@@ -131,6 +144,8 @@ class CSRNeighbors:
         scratch = torch.empty((N.load().sph_scan_scratch_bytes(self.n) + 7) // 8, dtype=torch.int64, device=dev)
         N.call("sph_exclusive_scan_i32_to_i64", N.ptr(cnt_orig), N.ptr(orig_off), self.n, N.ptr(scratch),
                scratch.numel() * 8, st)
+        if row_offsets is not None:
+            row_offsets.copy_(orig_off)
         pairs = torch.empty((2, P), dtype=torch.int64, device=dev)
         dist = torch.empty((P, 2), dtype=torch.float32, device=dev) if distances else None
         radial = torch.empty(P, dtype=torch.float32, device=dev) if distances else None
@@ -160,7 +175,7 @@ class CSRNeighbors:
         off = torch.empty(m + 1, dtype=torch.int64, device=dev)
         scratch = torch.empty((N.load().sph_scan_scratch_bytes(m) + 7) // 8, dtype=torch.int64, device=dev)
         N.call("sph_exclusive_scan_i32_to_i64", N.ptr(counts), N.ptr(off), m, N.ptr(scratch), scratch.numel() * 8, st)
-        P = int(off[m].item())
+        P = _total(off)
         rows = torch.empty(P, dtype=torch.int32, device=dev)
         cols = torch.empty(P, dtype=torch.int32, device=dev)
         if P:
@@ -197,12 +212,16 @@ class GridSearch:
             raise ValueError(cell_ratio)
         self.cell_ratio = int(cell_ratio)
 
+    def grid_status(self):
+        """The grid (8 words) and the status word, neighbors in one buffer."""
+        words = self.ws.get("grid_status", 9, torch.int32)
+        return words[:8], words[8:]
+
     def grid(self, pos, support, min_coord=None, max_coord=None, cell_capacity=MAX_CELLS):
         """Compute the search grid on the device; returns the device grid bytes."""
         lib = N.load()
         n = pos.shape[0]
-        grid = self.ws.get("grid", 8, torch.int32)
-        status = self.ws.get("status", 1, torch.int32)
+        grid, status = self.grid_status()
         scratch = self.ws.bytes("grid_scratch", lib.sph_grid_scratch_bytes(n))
         N.call("sph_grid_build_ratio", N.ptr(pos), N.ptr(support), n, _f2(min_coord), _f2(max_coord),
                self.cell_ratio, int(cell_capacity), N.ptr(grid), N.ptr(status), N.ptr(scratch), scratch.numel() * 8,
@@ -210,13 +229,15 @@ class GridSearch:
         return grid
 
     def auto_cell_capacity(self, pos, support, min_coord=None, max_coord=None) -> int:
-        """Number of grid cells (one host synchronisation)."""
-        status = self.ws.get("status", 1, torch.int32)
+        """Number of grid cells (one host synchronisation).  The grid stays in the workspace: one
+        with at most cell_capacity cells is the same for every such capacity."""
+        status = self.grid_status()[1]
         status.zero_()
-        g = self.grid(pos, support, min_coord, max_coord, MAX_CELLS)
-        info = grid_from_bytes(g)
-        flags = int(status.item())
-        status.zero_()
+        self.grid(pos, support, min_coord, max_coord, MAX_CELLS)
+        *words, flags = N.read_i32(self.ws.get("grid_status", 9, torch.int32))
+        info = grid_from_words(words)
+        if flags:
+            status.zero_()
         if flags & N.SPH_FLAG_NONFINITE:
             raise N.SPHError("neighbor search: non-finite positions or supports")
         if flags & N.SPH_FLAG_CELL_CAPACITY:
@@ -259,13 +280,15 @@ class GridSearch:
                                 offsets=i32(1), cols=i32(0), rho=f32(0) if density else None, grid=None,
                                 status=i32(1), cell_capacity=0, pair_capacity=0, kernel_support=kernel_support,
                                 search_radius=int(search_radius), cell_ratio=self.cell_ratio)
+        grid, status = self.grid_status()
         if cell_capacity is None:
-            cell_capacity = self.auto_cell_capacity(pos, support, min_coord, max_coord)
-        cap = int(cell_capacity)
-        status = ws.get("status", 1, torch.int32)
-        status.zero_()
-        mark("start")
-        grid = self.grid(pos, support, min_coord, max_coord, cap)
+            cap = self.auto_cell_capacity(pos, support, min_coord, max_coord)
+            mark("start")
+        else:
+            cap = int(cell_capacity)
+            status.zero_()
+            mark("start")
+            self.grid(pos, support, min_coord, max_coord, cap)
         keys = ws.get("keys", n)
         order = ws.get("order", n)
         skeys = ws.get("sorted_keys", n)
@@ -319,7 +342,7 @@ class GridSearch:
         N.call("sph_exclusive_scan_i32", N.ptr(counts), N.ptr(offsets), n, N.ptr(sc), sc.numel() * 8, st)
         mark("scan")
         if pair_capacity is None:
-            pair_capacity = int(offsets[n].item())
+            pair_capacity, = N.read_i32(offsets[n:])
         cols = ws.get("cols", pair_capacity)
         if self.segments:
             N.call("sph_nl_fill_segments", N.ptr(xy), N.ptr(sh), n, N.ptr(skeys), N.ptr(cell_start), N.ptr(grid), cap,
