@@ -203,87 +203,123 @@ __global__ void __launch_bounds__(256) k_nl_segments(const float2* __restrict__ 
   if (k > kSearchSegments) dense_list[atomicAdd(dense_count, 1)] = (int32_t)s;
 }
 
-// The CSR columns from the stored segments (no pair tests).  Rows of the dense list are left
-// to k_nl_fill_dense, which runs after this kernel (a staged block may copy placeholder
-// entries over them first).
-__global__ void __launch_bounds__(256) k_nl_fill_segments(const float2* __restrict__ xy,
-                                                          const float* __restrict__ sh, int64_t n,
-                                                          const uint32_t* __restrict__ keys,
-                                                          const int32_t* __restrict__ cell_start,
-                                                          const sph_grid* __restrict__ gp, int32_t cap, int r,
+// The CSR columns from the stored segments (no pair tests), one warp per 32 rows and no block
+// barrier.  The rows of a warp are one contiguous span of cols: it is built in the warp's
+// shared stage and stored flat, in whole lines.  A span past the stage is taken in 2, 4 .. 32
+// passes over as many fewer rows, and a row's segments are then dealt to that many lanes (the
+// lanes' bit counts place them), so all lanes expand masks whatever the rows' length; a row of
+// at most kSearchSegments x 32 columns always fits.  Bound by instruction issue (65 to 76 % of
+// the slots).  2^20 lattice particles (29.6 M columns): 37 µs; 1,000,003 with half of them in a
+// cluster (62 M): 99.  A stage of 8192 columns per block, and a warp per row for longer spans,
+// took 45 and 186; rows staged apart per lane and stored one by one 45 and 146.
+// A row that does not fit the column buffer is skipped with SPH_FLAG_PAIR_CAPACITY set; rows
+// of the dense list are left to k_nl_fill_dense, which runs after this kernel (a span may copy
+// placeholder entries over them first).
+__device__ __forceinline__ int highest_bit(uint32_t w) {
+  int b;
+  asm("bfind.u32 %0, %1;" : "=r"(b) : "r"(w));
+  return b;
+}
+
+constexpr int kRowStage = 1280;   // 40 columns a row: the usual rows in one pass
+static_assert(kRowStage >= kSearchSegments * 32, "one row has to fit");
+
+__global__ void __launch_bounds__(128) k_nl_fill_segments(int64_t n, const uint32_t* __restrict__ keys,
+                                                          const sph_grid* __restrict__ gp, int32_t cap,
                                                           const int32_t* __restrict__ offsets, int64_t pair_capacity,
                                                           int32_t* __restrict__ cols, int32_t* status,
                                                           const int32_t* __restrict__ nseg,
                                                           const int32_t* __restrict__ seg_start,
                                                           const uint32_t* __restrict__ seg_mask) {
+  __shared__ __align__(16) int32_t stages[4][kRowStage + 4];
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int64_t s0 = s - lane;
+  if (s0 >= n) return;   // the whole warp
+  int32_t* const stage = stages[threadIdx.x >> 5];
   const sph_grid g = *gp;
-  const uint32_t key = s < n ? keys[s] : 0xffffffffu;
-  const bool active = s < n && grid_ok(g, cap) && key < (uint32_t)g.num_cells;
-  const int ns = active ? nseg[s] : 0;
-  const int64_t b0 = (int64_t)blockIdx.x * blockDim.x, b1 = min(b0 + (int64_t)blockDim.x, n);
-  const int64_t span0 = offsets[b0], span1 = offsets[b1];
-  if (span0 >= 0 && span1 - span0 > kFillStage && span1 <= pair_capacity) {   // the same in the whole block
-    // Rows too long for one stage: each warp writes its 32 rows one after another, the lanes
-    // taking one candidate bit each; lane k holds segment k of the row, and the exclusive
-    // scan of the segments' bit counts places them, so a segment goes out as one contiguous
-    // store of its accepted candidates.  The next row's segments are loaded while a row is
-    // written.
-    const int lane = threadIdx.x & 31;
-    const uint32_t below = (1u << lane) - 1u;
-    const int64_t r0 = active ? offsets[s] : 0, r1 = active ? offsets[s + 1] : 0;
-    auto load_row = [&](int t, int& nst, int& c, uint32_t& m) {
-      nst = __shfl_sync(0xffffffffu, ns, t);
-      const int64_t st = __shfl_sync(0xffffffffu, s, t);
-      c = 0;
-      m = 0;
-      if (nst > 0 && nst <= kSearchSegments && lane < nst) {
-        c = seg_start[(int64_t)lane * n + st];
-        m = seg_mask[(int64_t)lane * n + st];
+  // this lane's row: first column, end, segments (none for a row that is not written)
+  const int lo = offsets[min(s, n)], hi = offsets[min(s + 1, n)];
+  int ns = 0;
+  if (s < n && grid_ok(g, cap) && keys[s] < (uint32_t)g.num_cells) {
+    ns = nseg[s];
+    if ((int64_t)hi > pair_capacity) {
+      flag(status, SPH_FLAG_PAIR_CAPACITY);
+      ns = 0;
+    }
+    if (ns < 0 || ns > kSearchSegments || lo < 0 || hi < lo || hi - lo > kRowStage) ns = 0;
+  }
+  // lanes per row: 1 << sh, the fewest whose passes' spans all fit
+  int sh = 0, first = lo, last = hi;
+  for (;; ++sh) {
+    const int rows = 32 >> sh;
+    first = __shfl_sync(0xffffffffu, lo, lane & -rows);
+    last = __shfl_sync(0xffffffffu, hi, lane | (rows - 1));
+    const bool fits = first >= 0 && last >= first && last - first <= kRowStage && (int64_t)last <= pair_capacity;
+    if (sh == 5 || __all_sync(0xffffffffu, fits)) break;
+  }
+  const int sub = lane & ((1 << sh) - 1);
+  for (int r0 = 0; r0 < 32; r0 += 32 >> sh) {
+    const int t = r0 + (lane >> sh);   // this lane's row of the pass
+    const int segs = __shfl_sync(0xffffffffu, ns, t);
+    const int o = __shfl_sync(0xffffffffu, lo, t), e = __shfl_sync(0xffffffffu, hi, t);
+    const int span0 = __shfl_sync(0xffffffffu, first, r0), span1 = __shfl_sync(0xffffffffu, last, r0);
+    const int longest = __reduce_max_sync(0xffffffffu, segs);
+    if (longest == 0) continue;
+    // columns stay inside the row and the span even if offsets and masks disagree
+    const int room = o >= span0 && e <= span1 ? e - o : 0;
+    int32_t* const mine = stage + (o - (span0 & ~3));   // the stage begins on span0's 16 bytes
+    int c_next = 0;
+    uint32_t w_next = 0;
+    const auto load = [&](int k) {
+      c_next = 0;
+      w_next = 0;
+      if (k < segs) {
+        c_next = seg_start[(int64_t)k * n + s0 + t];
+        w_next = seg_mask[(int64_t)k * n + s0 + t];
       }
     };
-    int nst_next, c_next;
-    uint32_t m_next;
-    load_row(0, nst_next, c_next, m_next);
-    for (int t = 0; t < 32; ++t) {
-      const int nst = nst_next, c = c_next;
-      uint32_t m = m_next;
-      if (t + 1 < 32) load_row(t + 1, nst_next, c_next, m_next);
-      if (nst <= 0 || nst > kSearchSegments) continue;   // nothing, or a dense row
-      const int64_t o = __shfl_sync(0xffffffffu, r0, t), e = __shfl_sync(0xffffffffu, r1, t);
-      m = clip_segment(m, c, (int)n);
-      const int cnt = __popc(m);
-      int incl = cnt;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += v;
-      }
-      const int excl = incl - cnt;
-      for (int k = 0; k < nst; ++k) {
-        const int ck = __shfl_sync(0xffffffffu, c, k);
-        const uint32_t mk = __shfl_sync(0xffffffffu, m, k);
-        const int bk = __shfl_sync(0xffffffffu, excl, k);
-        if ((mk >> lane) & 1u) {
-          const int64_t pos = o + bk + __popc(mk & below);
-          if (pos < e) cols[pos] = ck + lane;
+    load(sub);
+    int done = 0;   // columns of the row's earlier segments
+    for (int k = 0; k < longest; k += 1 << sh) {
+      const int c = c_next;
+      uint32_t w = clip_segment(w_next, c, (int)n);
+      load(k + (1 << sh) + sub);
+      int cnt = __popc(w);
+      int at = done;
+      if (sh) {   // the segments of the row's lower lanes come first
+        int incl = cnt;
+        for (int d = 1; d < 1 << sh; d <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, incl, d, 1 << sh);
+          if (sub >= d) incl += v;
         }
+        at += incl - cnt;
+        done += __shfl_sync(0xffffffffu, incl, (1 << sh) - 1, 1 << sh);
+      } else {
+        done += cnt;
       }
+      for (; at + cnt > room && cnt > 0; --cnt) w &= ~(1u << highest_bit(w));
+      for (int32_t* q = mine + at + cnt; w;) {   // from the last: the highest bit is one instruction
+        const int bit = highest_bit(w);
+        *--q = c + bit;
+        w ^= 1u << bit;
+      }
+      __syncwarp();
     }
-    return;
+    if (span0 >= 0 && span1 - span0 <= kRowStage && (int64_t)span1 <= pair_capacity) {
+      const int32_t* const from = stage - (span0 & ~3);
+      int a = span0, b = span0;   // [a, b): by 16 bytes
+      if ((reinterpret_cast<uintptr_t>(cols) & 15) == 0) {
+        a = min((span0 + 3) & ~3, span1);
+        b = max(span1 & ~3, a);
+      }
+      if (lane < a - span0) cols[span0 + lane] = from[span0 + lane];
+      for (int j = a + 4 * lane; j < b; j += 128)
+        *reinterpret_cast<int4*>(cols + j) = *reinterpret_cast<const int4*>(from + j);
+      for (int j = b + lane; j < span1; j += 32) cols[j] = from[j];
+    }
+    __syncwarp();
   }
-  staged_fill(s, n, active, offsets, pair_capacity, cols, status, [&](auto&& emit) {
-    if (ns < 0 || ns > kSearchSegments) return;   // a dense row
-    for (int k = 0; k < ns; ++k) {
-      const int c = seg_start[(int64_t)k * n + s];
-      uint32_t w = clip_segment(seg_mask[(int64_t)k * n + s], c, (int)n);
-      while (w) {
-        const int j = c - 1 + __ffs(w);
-        w &= w - 1;
-        emit(j);
-      }
-    }
-  });
 }
 
 // The rows of the dense list, one warp per particle: each sweep tests 32 candidates of a
@@ -587,9 +623,8 @@ sph_status_t sph_nl_fill_segments(const float* xy, const float* sorted_support, 
               "nl_fill_segments: scratch smaller than sph_nl_segments_scratch_bytes(n)");
   if (n == 0) return SPH_OK;
   cudaStream_t st = as_stream(stream);
-  k_nl_fill_segments<<<grid_for(n, 256), 256, 0, st>>>(reinterpret_cast<const float2*>(xy), sorted_support, n,
-                                                       sorted_keys, cell_start, grid, cell_capacity, search_radius,
-                                                       offsets, pair_capacity, cols, status, nseg, start, mask);
+  k_nl_fill_segments<<<grid_for(n, 128), 128, 0, st>>>(n, sorted_keys, grid, cell_capacity, offsets, pair_capacity,
+                                                       cols, status, nseg, start, mask);
   k_nl_fill_dense<<<kNumSMs * 8, 128, 0, st>>>(reinterpret_cast<const float2*>(xy), sorted_support, sorted_keys,
                                                cell_start, grid, cell_capacity, search_radius, offsets, pair_capacity,
                                                cols, status, dense_list, dense_count);
