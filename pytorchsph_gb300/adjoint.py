@@ -6,16 +6,15 @@ source or gravity, continuity, MOG density diffusion, Tait pressure, artificial 
 viscosity) integrated by semi-implicit Euler (src/simulationBase.py:647-652).  Each step
 searches neighbors on the GPU (the reference predicate) and advances the state in one launch
 (`sph_drop_search`, `sph_drop_step`); the adjoint (`sph_drop_adjoint_step`) runs the steps
-backwards, recomputing each checkpoint segment's states forward first.  A rollout waits for
-the device before its first step (the grid) and after its last (the status).  Scalars are
+backwards, over recorded states or (`vjp`) recomputing each checkpoint segment's states
+forward first.  A rollout waits for the device before its first step (the grid) and after its last (the status).  Scalars are
 float64 (default) or float32; the search always sees float32 positions, as the reference's
 does.  `DropRollout.pairs` and `step` work on the reference's own (i, j)-ordered lists.
 
 Gradients are with respect to the initial velocity field and the artificial viscosity alpha.
 `DropRolloutFunction` puts the rollout behind torch.autograd: its forward records every
-step's neighbor list and a checkpoint every `checkpoint_every` steps, and its backward
-recomputes each segment's states from its checkpoint with the recorded lists (no search)
-and runs the adjoint kernels backwards.
+step's neighbor list and state (a seventh of the list's memory), and its backward runs the
+adjoint kernels backwards over them.
 """
 from __future__ import annotations
 
@@ -105,67 +104,73 @@ class DropRollout:
         size = N.load().sph_drop_search_scratch_bytes(self.n, cap)
         return grid, cap, status, torch.zeros((size + 7) // 8, dtype=torch.int64, device=self.dev)
 
-    def _search_into(self, plan, x32, off, cols, unsorted):
-        """The pairs at x32 into (offsets, int32 columns); a float32 rollout's rows in increasing
-        order (through `unsorted`), the order its sums are defined in."""
-        grid, cap, status, scratch = plan
-        N.call("sph_drop_search", N.ptr(x32), N.ptr(self.support32), self.n, N.ptr(grid), cap, N.ptr(off),
-               cols.shape[0], N.ptr(cols), N.ptr(unsorted), N.ptr(status), N.ptr(scratch), scratch.numel() * 8,
-               N.stream_ptr())
-
-    def _advance(self, state, pr, x32=None):
+    def _advance(self, state, pr):
         """The state after one step with the pairs pr = (offsets, int32 columns)."""
-        x, v, rho = state
         out = tuple(torch.empty_like(t) for t in state)
         off, cols = pr
-        N.call("sph_drop_step", int(self.fp64), self.n, N.ptr(off), N.ptr(cols), cols.shape[0], N.ptr(x), N.ptr(v),
-               N.ptr(rho), N.ptr(self.area), ctypes.byref(self.P), self.dt, N.ptr(out[0]), N.ptr(out[1]),
-               N.ptr(out[2]), N.ptr(x32), N.stream_ptr())
+        N.call("sph_drop_step", int(self.fp64), self.n, N.ptr(off), N.ptr(cols), cols.shape[0], *map(N.ptr, state),
+               N.ptr(self.area), ctypes.byref(self.P), self.dt, *map(N.ptr, out), None, N.stream_ptr())
         self.steps_run += 1
         return out
 
-    def _forward(self, v0, alpha, steps, checkpoints, record):
-        """(final state, checkpoints, pairs of every step), the steps without host waits.  The pair
-        buffers are sized from the particles' areas with headroom; a step that overflows them has
-        the rollout run again with twice as much."""
+    def _forward(self, v0, alpha, steps, checkpoints=False, record=False):
+        """(final state, checkpoints, record of every step), the steps without host waits.
+
+        The pair buffers are sized from the particles' areas with headroom; a step that
+        overflows them has the rollout run again with twice as much.  A float32 rollout's
+        rows are put in increasing order, the order its sums are defined in.  A record holds
+        the pairs and the state of every step: the states take a seventh of the pairs' memory,
+        and the backward pass neither searches nor steps again."""
         self.P.alpha = float(alpha)
-        start = (self.x0.clone(), v0.to(self.dtype).reshape(self.n, 2).clone(), self.rho0.clone())
+        start = (self.x0.clone(), v0.to(self.dtype).reshape(self.n, 2).clone(memory_format=torch.contiguous_format),
+                 self.rho0.clone())
         if steps <= 0:
-            return start, {}, []
-        plan = self._search_plan()
-        status = plan[2]
-        x32_0 = self.x0.to(torch.float32).contiguous()
-        x32 = torch.empty_like(x32_0)
+            return start, {}, None
+        n, new = self.n, lambda *shape: torch.empty(shape, dtype=self.dtype, device=self.dev)
+        i32 = lambda *shape: torch.empty(shape, dtype=torch.int32, device=self.dev)
+        grid, cells, status, scratch = self._search_plan()
+        x32 = self.x0.to(torch.float32, copy=True).contiguous()
+        st, P, area = N.stream_ptr(), ctypes.byref(self.P), N.ptr(self.area)
+        sup, gp, sp, scr, scr_bytes, xp = (N.ptr(self.support32), N.ptr(grid), N.ptr(status), N.ptr(scratch),
+                                           scratch.numel() * 8, N.ptr(x32))
+        slots = steps - 1 if record else min(steps - 1, 2)   # of the states between the first and the last
         while True:
-            status.zero_()
             cap = self._pair_cap
             rows = steps if record else 1
-            offs = torch.empty((rows, self.n + 1), dtype=torch.int32, device=self.dev)
-            cols = torch.empty((rows, cap), dtype=torch.int32, device=self.dev)
-            unsorted = None if self.fp64 else torch.empty(cap, dtype=torch.int32, device=self.dev)
-            state, ck = start, {}
+            offs, cols = i32(rows, n + 1), i32(rows, cap)
+            unsorted = None if self.fp64 else i32(cap)
+            mid, end, ck = (new(slots, n, 2), new(slots, n, 2), new(slots, n)), tuple(map(torch.empty_like, start)), {}
+            at = lambda k: [N.ptr(t) for t in start] if k == 0 else [N.ptr(t) for t in end] if k == steps else \
+                [t.data_ptr() + (k - 1) % slots * t.stride(0) * t.element_size() for t in mid]
+            state = at(0)
             for k in range(steps):
                 if checkpoints and k % self.every == 0:
-                    ck[k] = state
-                pr = (offs[k if record else 0], cols[k if record else 0])
-                self._search_into(plan, x32 if k else x32_0, *pr, unsorted)
-                state = self._advance(state, pr, x32)
+                    ck[k] = tuple(t[(k - 1) % slots].clone() for t in mid) if k else start
+                r = k if record else 0
+                off, col = offs.data_ptr() + r * (n + 1) * 4, cols.data_ptr() + r * cap * 4
+                N.call("sph_drop_search", xp, sup, n, gp, cells, off, cap, col, N.ptr(unsorted), sp, scr, scr_bytes, st)
+                after = at(k + 1)
+                N.call("sph_drop_step", int(self.fp64), n, off, col, cap, *state, area, P, self.dt, *after, xp, st)
+                state = after
+            self.steps_run += steps
             flags = int(status.item())
             if not flags & N.SPH_FLAG_PAIR_CAPACITY:
                 break
             if cap >= 2**31 - 1:
                 raise N.SPHError(f"neighbor search: {N.decode_flags(flags)}")
             self._pair_cap = min(2 * cap, 2**31 - 1)
+            status.zero_()
+            x32.copy_(self.x0)
         if flags:
             raise N.SPHError(f"neighbor search: {N.decode_flags(flags)}")
-        return state, ck, [(offs[k], cols[k]) for k in range(rows)] if record else []
+        return end, ck, (start, mid, offs, cols) if record else None
 
     def rollout(self, v0, alpha, steps, checkpoints=False, record_pairs=False):
         """Final positions after `steps` steps from (x0, v0, rho0) and the checkpoints (the states
         at every `checkpoint_every`-th step, when asked for); with record_pairs also the list of
         every step's (offsets, columns), in the reference's (i, j) order."""
         if not record_pairs:
-            state, ck, _ = self._forward(v0, alpha, steps, checkpoints, False)
+            state, ck, _ = self._forward(v0, alpha, steps, checkpoints)
             return state[0], ck
         x = self.x0.clone()
         v = v0.to(self.dtype).reshape(self.n, 2).clone()
@@ -213,12 +218,31 @@ class DropRollout:
                 lr, nr = nr, lr
         return lv, dalpha.sum()
 
+    def _backward(self, record, alpha, steps, grad_x):
+        """vjp over a forward pass's record."""
+        lx = grad_x.to(self.dtype).reshape(self.n, 2).contiguous().clone()
+        cur = (lx, torch.zeros_like(lx), torch.zeros_like(self.rho0))
+        nxt = tuple(map(torch.empty_like, cur))
+        dalpha = torch.zeros(self.n, dtype=self.dtype, device=self.dev)
+        self.P.alpha = float(alpha)
+        st, P, area, da = N.stream_ptr(), ctypes.byref(self.P), N.ptr(self.area), N.ptr(dalpha)
+        a, b = [N.ptr(t) for t in cur], [N.ptr(t) for t in nxt]
+        for k in reversed(range(steps)):
+            start, mid, offs, cols = record
+            state = [t.data_ptr() + (k - 1) * t.stride(0) * t.element_size() for t in mid] if k else map(N.ptr, start)
+            cap = cols.shape[1]
+            N.call("sph_drop_adjoint_step", int(self.fp64), self.n, offs.data_ptr() + k * (self.n + 1) * 4,
+                   cols.data_ptr() + k * cap * 4, cap, *state, area, P, self.dt, *a, *b, da, st)
+            a, b = b, a
+            cur, nxt = nxt, cur
+        return cur[1], dalpha.sum()
+
     def loss_and_grad(self, v0, alpha, target, steps):
         """Loss mean_i |x_T,i - target_i|^2 and its gradients with respect to v0 [n, 2] and alpha."""
-        (xT, *_), ck, pairs = self._forward(v0, alpha, steps, True, True)
+        (xT, *_), _, record = self._forward(v0, alpha, steps, record=True)
         diff = xT - target.to(self.dtype)
         loss = float((diff * diff).sum().item()) / self.n
-        lv, da = self.vjp(ck, alpha, steps, (2.0 / self.n) * diff, pairs)
+        lv, da = self._backward(record, alpha, steps, (2.0 / self.n) * diff)
         return loss, lv, float(da.item())
 
     def loss(self, v0, alpha, target, steps):
@@ -231,23 +255,22 @@ class DropRolloutFunction(torch.autograd.Function):
     """Final positions x_T [n, 2] of a `steps`-step DropRollout as a differentiable function of
     the initial velocities v0 [n, 2] and the artificial viscosity alpha (0-d tensor).
 
-    Forward: the GPU rollout, recording each step's neighbor list and a checkpoint every
-    `rollout.every` steps.  Backward: DropRollout.vjp with the recorded lists (the adjoint
-    kernels of sph_drop_adjoint).  The rollout's precision (float32 or float64) is the
+    Forward: the GPU rollout, recording each step's neighbor list and state.  Backward: the
+    adjoint of each step over the record (sph_drop_adjoint_step).  The rollout's precision (float32 or float64) is the
     rollout's; gradients come back in the inputs' dtypes."""
 
     @staticmethod
     def forward(ctx, v0, alpha, rollout, steps):
         a = float(alpha)
-        (xT, *_), ck, pairs = rollout._forward(v0.detach(), a, int(steps), True, True)
-        ctx.rollout, ctx.ck, ctx.pairs, ctx.alpha, ctx.steps = rollout, ck, pairs, a, int(steps)
+        (xT, *_), _, ctx.record = rollout._forward(v0.detach(), a, int(steps), record=True)
+        ctx.rollout, ctx.alpha, ctx.steps = rollout, a, int(steps)
         ctx.v_dtype, ctx.a_dtype = v0.dtype, (alpha.dtype if isinstance(alpha, torch.Tensor) else torch.float64)
         ctx.a_device = alpha.device if isinstance(alpha, torch.Tensor) else v0.device
         return xT
 
     @staticmethod
     def backward(ctx, grad_x):
-        gv, ga = ctx.rollout.vjp(ctx.ck, ctx.alpha, ctx.steps, grad_x, ctx.pairs)
+        gv, ga = ctx.rollout._backward(ctx.record, ctx.alpha, ctx.steps, grad_x)
         gv = gv.to(ctx.v_dtype) if ctx.needs_input_grad[0] else None
         ga = ga.to(device=ctx.a_device, dtype=ctx.a_dtype) if ctx.needs_input_grad[1] else None
         return gv, ga, None, None
