@@ -310,6 +310,15 @@ sph_status_t sph_nl_query_fill(const float* query_pos, const float* query_suppor
                                int32_t cell_capacity, int32_t search_radius, const uint32_t* order,
                                const int64_t* offsets, int32_t* rows, int32_t* cols, void* stream);
 
+/* The fill with searchExisting's own outputs (src/modules/neighborSearch.py:231-252): int64 rows
+ * and original columns, unit vectors and distances / query support from `points` (original
+ * order, dist 8-byte aligned), and the row offsets as int32 [m+1]. */
+sph_status_t sph_nl_query_pairs(const float* query_pos, const float* query_support, int64_t m, const float* xy,
+                                const int32_t* cell_start, const sph_grid* grid, int32_t cell_capacity,
+                                int32_t search_radius, const uint32_t* order, const int64_t* offsets,
+                                const float* points, float threshold, int64_t* rows, int64_t* cols, float* dist,
+                                float* radial, int32_t* row_offsets, void* stream);
+
 /* ---------------------------------------------------------------- deltaSPH summations (a8-a19) */
 
 /* mDBC wall density (computeBoundaryDensitymDBC, src/modules/solidBoundary.py:561-617):

@@ -58,6 +58,7 @@ SIGNATURES = {
     "sph_invert_permutation": (_I32, [_P, _I64, _P, _P]),
     "sph_nl_query_count": (_I32, [_P, _P, _I64, _P, _P, _P, _I32, _I32, _P, _P]),
     "sph_nl_query_fill": (_I32, [_P, _P, _I64, _P, _P, _P, _I32, _I32, _P, _P, _P, _P, _P]),
+    "sph_nl_query_pairs": (_I32, [_P, _P, _I64, _P, _P, _P, _I32, _I32, _P, _P, _P, _F32] + [_P] * 6),
     "sph_nl_hashed_query_count": (_I32, [_P, _P, _I64, _P, _P, _P, _P, _P, _P, _F32, _I32, _I32, _I32, _P, _P]),
     "sph_nl_hashed_query_fill": (_I32, [_P, _P, _I64, _P, _P, _P, _P, _P, _P, _P, _F32, _I32, _I32, _I32, _P,
                                         _P, _P, _P]),

@@ -381,32 +381,88 @@ __device__ __forceinline__ bool query_cell(float x, float qmin, float hmax, int*
   return true;
 }
 
-template <bool kFill>
+// Where a query pair goes: sorted or original columns with 32-bit rows (sph_nl_query_fill), or
+// searchExisting's own outputs, with the row offsets as int32 (sph_nl_query_pairs).
+struct QueryPairs {
+  const uint32_t* order;
+  int32_t *rows, *cols;
+  int64_t *rows64, *cols64;
+  const float2* points;   // original order
+  float threshold;
+  float2* dist;
+  float* radial;
+  int32_t* row_offsets;
+};
+
+// Latency bounds the few thousand wall or ghost points of a scene, so kQueryLanes lanes share a
+// point's candidates and place their hits by ballot, in the order of one thread; the points
+// of a warp walk their cell rows in step.  The walls of a 30,621-particle block: 3.8 µs for
+// counting and 6 for filling with the geometry (one thread each: 4.8, and 8 + 2 for it).
+constexpr int kQueryLanes = 8;
+
+enum { kQueryCount, kQueryRows, kQueryModule };
+
+template <int kMode>
 __global__ void __launch_bounds__(128) k_nl_query(const float2* __restrict__ qpos, const float* __restrict__ qh, int64_t m,
                                                   const float2* __restrict__ xy,
                                                   const int32_t* __restrict__ cell_start,
                                                   const sph_grid* __restrict__ gp, int32_t cap, int r,
-                                                  const uint32_t* __restrict__ order, int32_t* __restrict__ counts,
-                                                  const int64_t* __restrict__ offsets, int32_t* __restrict__ rows,
-                                                  int32_t* __restrict__ cols) {
-  int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= m) return;
+                                                  int32_t* __restrict__ counts, const int64_t* __restrict__ offsets,
+                                                  const QueryPairs out) {
+  const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kQueryLanes;
+  const bool live = row < m;   // lanes past the last point take part in the warp's votes
+  const int64_t b = live ? row : m - 1;
+  const int lane = threadIdx.x & 31, sub = lane % kQueryLanes, base = lane - sub;
   const sph_grid g = *gp;
   int cnt = 0;
-  int64_t o = kFill ? offsets[b] : 0;
+  const int64_t o = kMode != kQueryCount ? offsets[b] : 0;
   const float2 xi = qpos[b];
-  const float thr = grid_threshold(qh[b], g);
-  int qx, qy;
-  if (grid_ok(g, cap) && query_cell(xi.x, g.qmin[0], g.hmax, &qx) && query_cell(xi.y, g.qmin[1], g.hmax, &qy)) {
-    scan_candidates(xy, cell_start, g, r, qx, qy, xi.x, xi.y, thr, [&](int j, float) {
-      if (kFill) {
-        rows[o + cnt] = (int32_t)b;
-        cols[o + cnt] = order ? (int32_t)order[j] : j;
-      }
-      ++cnt;
-    });
+  const float h = qh[b];
+  const float thr = grid_threshold(h, g);
+  int qx, qy, x0 = 0, x1 = -1, y0 = 0, y1 = -1;
+  if (live && grid_ok(g, cap) && query_cell(xi.x, g.qmin[0], g.hmax, &qx) && query_cell(xi.y, g.qmin[1], g.hmax, &qy)) {
+    x0 = max(qx - r, 0);
+    x1 = min(qx + r, g.cells_x - 1);
+    y0 = max(qy - r, 0);
+    y1 = x0 <= x1 ? min(qy + r, g.cells_y - 1) : y0 - 1;
   }
-  if (!kFill) counts[b] = cnt;
+  const int cell_rows = __reduce_max_sync(0xffffffffu, y1 - y0 + 1);
+  for (int q = 0; q < cell_rows; ++q) {
+    int j0 = 0, j1 = 0;
+    if (y0 + q <= y1) {
+      const int32_t* cells = cell_start + (int64_t)(y0 + q) * g.cells_x;
+      j0 = __ldg(cells + x0);
+      j1 = __ldg(cells + x1 + 1);
+    }
+    const int longest = __reduce_max_sync(0xffffffffu, j1 - j0);
+    for (int t = 0; t < longest; t += kQueryLanes) {
+      const int j = j0 + t + sub;
+      bool hit = false;
+      if (j < j1) {
+        const float2 pj = __ldg(xy + j);
+        hit = dist2_ref(xi.x, xi.y, pj.x, pj.y) <= thr;
+      }
+      const unsigned hits = __ballot_sync(0xffffffffu, hit) >> base & ((1u << kQueryLanes) - 1u);
+      if (kMode != kQueryCount && hit) {
+        const int64_t k = o + cnt + __popc(hits & ((1u << sub) - 1u));
+        const int c = out.order ? (int)out.order[j] : j;
+        if (kMode == kQueryRows) {
+          out.rows[k] = (int32_t)b;
+          out.cols[k] = c;
+        } else {
+          out.rows64[k] = b;
+          out.cols64[k] = c;
+          out.dist[k] = query_geometry(xi, out.points[c], h, out.threshold, out.radial + k);
+        }
+      }
+      cnt += __popc(hits);
+    }
+  }
+  if (kMode == kQueryCount && live && sub == 0) counts[b] = cnt;
+  if (kMode == kQueryModule && live && sub == 0) {
+    out.row_offsets[b] = (int32_t)o;
+    if (b == m - 1) out.row_offsets[m] = (int32_t)offsets[m];
+  }
 }
 
 // One warp per original particle i: its row of the (i, j)-ordered COO list, plus the
@@ -664,9 +720,9 @@ sph_status_t sph_nl_query_count(const float* query_pos, const float* query_suppo
   SPH_REQUIRE(m >= 0 && query_pos && query_support && xy && cell_start && grid && counts && search_radius >= 0,
               "nl_query: bad arguments");
   if (m == 0) return SPH_OK;
-  k_nl_query<false><<<grid_for(m, 128), 128, 0, as_stream(stream)>>>(
+  k_nl_query<kQueryCount><<<grid_for(m * kQueryLanes, 128), 128, 0, as_stream(stream)>>>(
       reinterpret_cast<const float2*>(query_pos), query_support, m, reinterpret_cast<const float2*>(xy), cell_start,
-      grid, cell_capacity, search_radius, nullptr, counts, nullptr, nullptr, nullptr);
+      grid, cell_capacity, search_radius, counts, nullptr, QueryPairs{});
   SPH_CHECK_LAUNCH("nl_query_count");
   return SPH_OK;
 }
@@ -679,10 +735,40 @@ sph_status_t sph_nl_query_fill(const float* query_pos, const float* query_suppor
                   search_radius >= 0,
               "nl_query: bad arguments");
   if (m == 0) return SPH_OK;
-  k_nl_query<true><<<grid_for(m, 128), 128, 0, as_stream(stream)>>>(
+  QueryPairs out{};
+  out.order = order;
+  out.rows = rows;
+  out.cols = cols;
+  k_nl_query<kQueryRows><<<grid_for(m * kQueryLanes, 128), 128, 0, as_stream(stream)>>>(
       reinterpret_cast<const float2*>(query_pos), query_support, m, reinterpret_cast<const float2*>(xy), cell_start,
-      grid, cell_capacity, search_radius, order, nullptr, offsets, rows, cols);
+      grid, cell_capacity, search_radius, nullptr, offsets, out);
   SPH_CHECK_LAUNCH("nl_query_fill");
+  return SPH_OK;
+}
+
+sph_status_t sph_nl_query_pairs(const float* query_pos, const float* query_support, int64_t m, const float* xy,
+                                const int32_t* cell_start, const sph_grid* grid, int32_t cell_capacity,
+                                int32_t search_radius, const uint32_t* order, const int64_t* offsets,
+                                const float* points, float threshold, int64_t* rows, int64_t* cols, float* dist,
+                                float* radial, int32_t* row_offsets, void* stream) {
+  SPH_REQUIRE(m >= 0 && query_pos && query_support && xy && cell_start && grid && order && offsets && points && rows &&
+                  cols && dist && radial && row_offsets && search_radius >= 0 &&
+                  (reinterpret_cast<uintptr_t>(dist) & 7) == 0,
+              "nl_query_pairs: bad arguments");
+  if (m == 0) return SPH_OK;
+  QueryPairs out{};
+  out.order = order;
+  out.rows64 = rows;
+  out.cols64 = cols;
+  out.points = reinterpret_cast<const float2*>(points);
+  out.threshold = threshold;
+  out.dist = reinterpret_cast<float2*>(dist);
+  out.radial = radial;
+  out.row_offsets = row_offsets;
+  k_nl_query<kQueryModule><<<grid_for(m * kQueryLanes, 128), 128, 0, as_stream(stream)>>>(
+      reinterpret_cast<const float2*>(query_pos), query_support, m, reinterpret_cast<const float2*>(xy), cell_start,
+      grid, cell_capacity, search_radius, nullptr, offsets, out);
+  SPH_CHECK_LAUNCH("nl_query_pairs");
   return SPH_OK;
 }
 

@@ -329,6 +329,15 @@ __device__ __forceinline__ float lane_sum(float v) {
   return v;
 }
 
+// Geometry of a query pair, src/modules/neighborSearch.py:244-251: d = x_q - x, r = |d|;
+// e = d / r (0 when r < threshold); q = r / h_q.
+__device__ __forceinline__ float2 query_geometry(float2 xq, float2 x, float hq, float threshold, float* radial) {
+  const float dx = xq.x - x.x, dy = xq.y - x.y;
+  const float d = sqrtf(dx * dx + dy * dy);
+  *radial = d / hq;
+  return d < threshold ? make_float2(0.f, 0.f) : make_float2(dx / d, dy / d);
+}
+
 // ---------------------------------------------------------------- candidate segments
 // The candidates of a particle in one cell row are a contiguous sorted range; it is tested
 // in segments of 32 candidates into bit masks (bit t: candidate c + t passes the pair test),

@@ -280,8 +280,7 @@ __global__ void k_row_offsets(const int64_t* __restrict__ rows, int64_t P, int n
   offsets[i] = (int32_t)lo;
 }
 
-// Distances of query pairs, src/modules/neighborSearch.py:244-251: d = x_q[row] - x[col],
-// r = |d|; e = d / r (0 when r < threshold); q = r / h_q[row].
+// Distances of query pairs (query_geometry).
 __global__ void k_pair_geometry(const int32_t* __restrict__ rows, const int32_t* __restrict__ cols, int64_t P,
                                 const float2* __restrict__ xq, const float2* __restrict__ xp,
                                 const float* __restrict__ hq, float threshold, float2* __restrict__ dist,
@@ -289,11 +288,7 @@ __global__ void k_pair_geometry(const int32_t* __restrict__ rows, const int32_t*
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= P) return;
   const int r = rows[k], c = cols[k];
-  const float2 a = xq[r], b = xp[c];
-  const float dx = a.x - b.x, dy = a.y - b.y;
-  const float d = sqrtf(dx * dx + dy * dy);
-  dist[k] = d < threshold ? make_float2(0.f, 0.f) : make_float2(dx / d, dy / d);
-  radial[k] = d / hq[r];
+  dist[k] = query_geometry(xq[r], xp[c], hq[r], threshold, radial + k);
 }
 
 }  // namespace sph

@@ -304,19 +304,14 @@ class neighborSearchModule(Module):
         return fluidNeighbors, fluidDistances, fluidRadialDistances
 
     def searchExisting(self, queryPositions, querySupports, simulationState, simulation, searchRadius: int = 1):
+        return self.searchExistingRows(queryPositions, querySupports, simulationState, searchRadius)[:3]
+
+    def searchExistingRows(self, queryPositions, querySupports, simulationState, searchRadius: int = 1):
+        """searchExisting with the pairs' int32 row offsets [queries + 1]."""
         if self.csr is None:
             raise N.SPHError("searchExisting needs a prior search() of the fluid")
-        q = _f32(queryPositions)
-        hq = _f32(querySupports)
-        rows, cols = self.csr.query(q, hq, searchRadius)
-        P = rows.shape[0]
-        dist = torch.empty((P, 2), dtype=torch.float32, device=q.device)
-        radial = torch.empty(P, dtype=torch.float32, device=q.device)
-        N.call("sph_pair_geometry", N.ptr(rows), N.ptr(cols), P, N.ptr(q),
-               N.ptr(_f32(simulationState['fluidPosition'])), N.ptr(hq), float(self.threshold), N.ptr(dist),
-               N.ptr(radial), N.stream_ptr())
-        fluidNeighbors = torch.stack([rows.long(), cols.long()], dim=0)
-        return fluidNeighbors, dist, radial
+        return self.csr.query_pairs(_f32(queryPositions), _f32(querySupports),
+                                    _f32(simulationState['fluidPosition']), self.threshold, searchRadius)
 
 
 # ----------------------------------------------------------------------------- summations
@@ -517,9 +512,10 @@ class gravityModule(Module):
 # ----------------------------------------------------------------------------- solid walls
 class _WallPairs:
     """A wall -> fluid pair list of searchExisting (rows = wall, cols = fluid particle) with
-    its grouping by wall (row offsets) and by fluid particle (sph_transpose_pairs)."""
+    its grouping by wall (row offsets, given or found) and, for the sums of the fluid side, by
+    fluid particle (sph_transpose_pairs)."""
 
-    def __init__(self, neighbors, dist, radial, nb, n):
+    def __init__(self, neighbors, dist, radial, nb, n, woff=None, by_fluid=True):
         self.rows = neighbors[0].contiguous()
         self.cols = neighbors[1].contiguous()
         self.dist = _f32(dist)
@@ -527,13 +523,19 @@ class _WallPairs:
         P = self.rows.shape[0]
         dev = self.rows.device
         st = N.stream_ptr()
-        self.woff = torch.empty(nb + 1, dtype=torch.int32, device=dev)
-        N.call("sph_row_offsets", N.ptr(self.rows), P, nb, N.ptr(self.woff), st)
-        self.foff = torch.empty(n + 1, dtype=torch.int32, device=dev)
-        self.fpairs = torch.empty(max(P, 1), dtype=torch.int32, device=dev)
-        scr = torch.empty((N.load().sph_transpose_pairs_scratch_bytes(n) + 7) // 8, dtype=torch.int64, device=dev)
-        N.call("sph_transpose_pairs", N.ptr(self.cols), P, n, N.ptr(self.foff), N.ptr(self.fpairs), N.ptr(scr),
-               scr.numel() * 8, st)
+        if P >= 1 << 31:
+            raise N.SPHError("wall pairs: at most 2^31-1 pairs")
+        if woff is None:
+            woff = torch.empty(nb + 1, dtype=torch.int32, device=dev)
+            N.call("sph_row_offsets", N.ptr(self.rows), P, nb, N.ptr(woff), st)
+        self.woff = woff
+        self.foff = self.fpairs = None
+        if by_fluid:
+            self.foff = torch.empty(n + 1, dtype=torch.int32, device=dev)
+            self.fpairs = torch.empty(max(P, 1), dtype=torch.int32, device=dev)
+            scr = torch.empty((N.load().sph_transpose_pairs_scratch_bytes(n) + 7) // 8, dtype=torch.int64, device=dev)
+            N.call("sph_transpose_pairs", N.ptr(self.cols), P, n, N.ptr(self.foff), N.ptr(self.fpairs), N.ptr(scr),
+                   scr.numel() * 8, st)
 
 
 def wall_term(term, pairs, P, n, nb, out=None, accumulate=False, dt=0.0, **arrays):
@@ -715,20 +717,25 @@ class solidBoundaryModule(BoundaryModule):
             return
         n = simulationState['fluidPosition'].shape[0]
         ns = simulation.neighborSearch
+
+        def find(positions, supports, radius):
+            # row offsets come along unless the caller's search has a searchExisting of its own
+            if getattr(ns.searchExisting, '__func__', None) is neighborSearchModule.searchExisting:
+                return ns.searchExistingRows(positions, supports, simulationState, radius)
+            return (*ns.searchExisting(positions, supports, simulationState, simulation, searchRadius=radius), None)
+
+        *bf, bf_rows = find(self.boundaryPositions, self.boundarySupport, 1)
         (self.boundaryToFluidNeighbors, self.boundaryToFluidNeighborDistances,
-         self.boundaryToFluidNeighborRadialDistances) = ns.searchExisting(
-            self.boundaryPositions, self.boundarySupport, simulationState, simulation)
+         self.boundaryToFluidNeighborRadialDistances) = bf
         # the ghost pair list; the deltaMLS and MLSPressure wall pressures query it from the wall
         # positions instead (solidBoundary.py:639-640), and mDBC then uses those pairs too
         query = self.boundaryPositions if self.boundaryPressureScheme in ('deltaMLS', 'MLSPressure') \
             else self.boundaryGhostPositions
+        *gf, gf_rows = find(query, self.boundarySupport * self.MLSscale, self.MLSscale)
         (self.ghostToFluidNeighbors, self.ghostToFluidNeighborDistances,
-         self.ghostToFluidNeighborRadialDistances) = ns.searchExisting(
-            query, self.boundarySupport * self.MLSscale, simulationState, simulation, searchRadius=self.MLSscale)
-        self._bf = _WallPairs(self.boundaryToFluidNeighbors, self.boundaryToFluidNeighborDistances,
-                              self.boundaryToFluidNeighborRadialDistances, self.numPtcls, n)
-        self._gf = _WallPairs(self.ghostToFluidNeighbors, self.ghostToFluidNeighborDistances,
-                              self.ghostToFluidNeighborRadialDistances, self.numPtcls, n)
+         self.ghostToFluidNeighborRadialDistances) = gf
+        self._bf = _WallPairs(*bf, self.numPtcls, n, bf_rows)
+        self._gf = _WallPairs(*gf, self.numPtcls, n, gf_rows, by_fluid=False)   # wall-side sums only
 
     def _wall_volume(self):
         out = torch.empty_like(self.boundaryVolume)

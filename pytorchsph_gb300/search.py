@@ -160,29 +160,52 @@ class CSRNeighbors:
         src/modules/neighborSearch.py:231-252): rows = query index, cols = particle index
         (original order by default), predicate |x_q - x_j| < support_q.  search_radius counts
         supports, as in GridSearch.run (the grid's cells are support / cell_ratio)."""
-        r = self.search_radius if search_radius is None else int(search_radius) * getattr(self, "cell_ratio", 1)
+        r, qpos, qsupport, off = self._query_offsets(qpos, qsupport, search_radius)
         m = qpos.shape[0]
-        dev = self.order.device
-        st = N.stream_ptr()
-        qpos = qpos.contiguous()
-        qsupport = qsupport.contiguous()
-        counts = torch.empty(max(m, 1), dtype=torch.int32, device=dev)
-        if m == 0:
-            e = torch.empty(0, dtype=torch.int32, device=dev)
-            return e, e.clone()
-        N.call("sph_nl_query_count", N.ptr(qpos), N.ptr(qsupport), m, N.ptr(self.xy), N.ptr(self.cell_start),
-               N.ptr(self.grid), self.cell_capacity, r, N.ptr(counts), st)
-        off = torch.empty(m + 1, dtype=torch.int64, device=dev)
-        scratch = torch.empty((N.load().sph_scan_scratch_bytes(m) + 7) // 8, dtype=torch.int64, device=dev)
-        N.call("sph_exclusive_scan_i32_to_i64", N.ptr(counts), N.ptr(off), m, N.ptr(scratch), scratch.numel() * 8, st)
-        P = _total(off)
-        rows = torch.empty(P, dtype=torch.int32, device=dev)
-        cols = torch.empty(P, dtype=torch.int32, device=dev)
+        P = _total(off) if m else 0
+        rows = torch.empty(P, dtype=torch.int32, device=self.order.device)
+        cols = torch.empty(P, dtype=torch.int32, device=self.order.device)
         if P:
             N.call("sph_nl_query_fill", N.ptr(qpos), N.ptr(qsupport), m, N.ptr(self.xy), N.ptr(self.cell_start),
                    N.ptr(self.grid), self.cell_capacity, r, N.ptr(self.order) if original_indices else None,
-                   N.ptr(off), N.ptr(rows), N.ptr(cols), st)
+                   N.ptr(off), N.ptr(rows), N.ptr(cols), N.stream_ptr())
         return rows, cols
+
+    def query_pairs(self, qpos, qsupport, points, threshold, search_radius: int | None = None):
+        """query() in the reference's layout: (neighbors int64 [2, P], unit vectors [P, 2],
+        distances / query support [P]) by `points` (original order), and int32 row offsets."""
+        r, qpos, qsupport, off = self._query_offsets(qpos, qsupport, search_radius)
+        m = qpos.shape[0]
+        P = _total(off) if m else 0
+        dev = self.order.device
+        pairs = torch.empty((2, P), dtype=torch.int64, device=dev)
+        dist = torch.empty((P, 2), dtype=torch.float32, device=dev)
+        radial = torch.empty(P, dtype=torch.float32, device=dev)
+        rows = (torch.empty if P else torch.zeros)(m + 1, dtype=torch.int32, device=dev)
+        if P:
+            N.call("sph_nl_query_pairs", N.ptr(qpos), N.ptr(qsupport), m, N.ptr(self.xy), N.ptr(self.cell_start),
+                   N.ptr(self.grid), self.cell_capacity, r, N.ptr(self.order), N.ptr(off), N.ptr(points),
+                   float(threshold), N.ptr(pairs[0]), N.ptr(pairs[1]), N.ptr(dist), N.ptr(radial), N.ptr(rows),
+                   N.stream_ptr())
+        return pairs, dist, radial, rows
+
+    def _query_offsets(self, qpos, qsupport, search_radius):
+        """(radius in cells, contiguous inputs, scanned int64 counts [m + 1]) of a query."""
+        r = self.search_radius if search_radius is None else int(search_radius) * getattr(self, "cell_ratio", 1)
+        m = qpos.shape[0]
+        dev = self.order.device
+        qpos = qpos.contiguous()
+        qsupport = qsupport.contiguous()
+        off = torch.empty(m + 1, dtype=torch.int64, device=dev)
+        if m:
+            st = N.stream_ptr()
+            counts = torch.empty(m, dtype=torch.int32, device=dev)
+            N.call("sph_nl_query_count", N.ptr(qpos), N.ptr(qsupport), m, N.ptr(self.xy), N.ptr(self.cell_start),
+                   N.ptr(self.grid), self.cell_capacity, r, N.ptr(counts), st)
+            scratch = torch.empty((N.load().sph_scan_scratch_bytes(m) + 7) // 8, dtype=torch.int64, device=dev)
+            N.call("sph_exclusive_scan_i32_to_i64", N.ptr(counts), N.ptr(off), m, N.ptr(scratch),
+                   scratch.numel() * 8, st)
+        return r, qpos, qsupport, off
 
 
 class GridSearch:
