@@ -368,8 +368,9 @@ class Simulation:
         try:
             with torch.cuda.graph(g):
                 self._step_kernels()
-                for k, t in inputs.items():
-                    t.copy_(self.arr[k])
+                moved = [(self.arr[k], t) for k, t in inputs.items() if self.arr[k].data_ptr() != t.data_ptr()]
+                for k in range(0, len(moved), 8):   # one launch for the state
+                    N.permute_arrays(None, moved[k:k + 8])
         except Exception:
             self.arr, self.last = inputs, last
             raise
@@ -406,7 +407,9 @@ class Simulation:
         elif c.integration == "RK4":
             if not cont:
                 raise N.SPHError("RK4 is implemented for the continuum-density deltaSPH solver")
-            self.extra = {"x0": self.arr["x"].clone(), "v0": self.arr["v"].clone(), "r0": self.arr["rho"].clone()}
+            keep = {"x0": self.arr["x"], "v0": self.arr["v"], "r0": self.arr["rho"]}
+            self.extra = {k: torch.empty_like(t) for k, t in keep.items()}
+            N.permute_arrays(None, [(t, self.extra[k]) for k, t in keep.items()])
             self.extra["su"] = torch.empty_like(self.arr["x"])
             self.extra["sa"] = torch.empty_like(self.arr["x"])
             self.extra["sd"] = torch.empty_like(self.arr["rho"])
