@@ -305,46 +305,135 @@ __device__ __forceinline__ uint64_t cell_rank(uint32_t x, const uint32_t* __rest
   return tie ? (((uint64_t)__ldg(tie + x)) << 32) | x : (uint64_t)x;
 }
 
-// Per-slot fix-up of ascending (tie, index) order inside every cell, and the sorted keys.
-// After the scatter, cell c's particles fill [cell_start[c], cell_start[c+1]) in atomic
-// order; the thread of slot t counts the cell's particles that rank below its own and
-// writes its particle to that place (k comparisons per particle, L1-resident).  Cells larger
-// than kSmallCell are queued for k_cell_fix_large by the thread of their first slot.
-// The sentinel cell (the key cell_capacity: particles outside every grid, or of no scene in
-// a pooled batch) keeps the scatter order: nothing reads its order.
-__global__ void __launch_bounds__(256) k_cell_fix(const uint32_t* __restrict__ keys, int64_t n,
-                                                  const int32_t* __restrict__ cell_start,
-                                                  const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ tie,
-                                                  uint32_t* __restrict__ order, uint32_t* __restrict__ sorted_keys,
-                                                  int32_t* __restrict__ big_list, int32_t* __restrict__ big_count,
-                                                  const ArraySet rows, uint32_t sentinel) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const uint32_t x = tmp[t];
-  const uint32_t c = __ldg(keys + x);
-  sorted_keys[t] = c;
-  if (c == sentinel) {
-    order[t] = x;
-    copy_rows(rows, t, x);
-    return;
-  }
-  const int b = __ldg(cell_start + c), e = __ldg(cell_start + c + 1);
-  if (e - b > kSmallCell) {
-    if (t == b) big_list[atomicAdd(big_count, 1)] = (int32_t)c;
-    return;
-  }
-  const uint64_t mine = cell_rank(x, tie);
-  int rank = 0;
-  for (int u = b; u < e; ++u) rank += cell_rank(__ldg(tmp + u), tie) < mine;
-  order[b + rank] = x;
-  copy_rows(rows, b + rank, x);
-}
-
-// One block per large cell, its (tie, index) ranks in shared memory: up to kRankSortMax
+// One large cell by a whole block, its (tie, index) ranks in shared memory: up to kRankSortMax
 // entries each thread counts the smaller ranks of its entries (one barrier); above that a
 // bitonic sort, up to kBlockSortMax entries.  Bigger cells keep the atomic scatter order
 // (their pair set is unchanged; only the order inside that cell is not reproducible) and
 // flag SPH_FLAG_CELL_ORDER.
+__device__ __forceinline__ void fix_large_cell(int b, int e, const uint32_t* __restrict__ tmp,
+                                               const uint32_t* __restrict__ tie, uint32_t* __restrict__ order,
+                                               int32_t* status, const ArraySet& rows, uint64_t* s) {
+  const int k = e - b;
+  if (k > kBlockSortMax) {
+    for (int t = threadIdx.x; t < k; t += blockDim.x) {
+      order[b + t] = tmp[b + t];
+      copy_rows(rows, b + t, tmp[b + t]);
+    }
+    if (threadIdx.x == 0) flag(status, SPH_FLAG_CELL_ORDER);
+    return;
+  }
+  if (k <= kRankSortMax) {
+    for (int t = threadIdx.x; t < k; t += blockDim.x) s[t] = cell_rank(tmp[b + t], tie);
+    __syncthreads();
+    for (int t = threadIdx.x; t < k; t += blockDim.x) {
+      const uint64_t mine = s[t];
+      int rank = 0;
+#pragma unroll 4
+      for (int u = 0; u < k; ++u) rank += s[u] < mine;   // every lane reads the same word
+      order[b + rank] = (uint32_t)(mine & 0xffffffffu);
+      copy_rows(rows, b + rank, (uint32_t)(mine & 0xffffffffu));
+    }
+    __syncthreads();
+    return;
+  }
+  int p2 = 1;
+  while (p2 < k) p2 <<= 1;
+  for (int t = threadIdx.x; t < p2; t += blockDim.x) s[t] = t < k ? cell_rank(tmp[b + t], tie) : ~0ull;
+  __syncthreads();
+  for (int size = 2; size <= p2; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int t = threadIdx.x; t < p2; t += blockDim.x) {
+        int u = t ^ stride;
+        if (u > t) {
+          bool up = (t & size) == 0;
+          uint64_t a = s[t], bb = s[u];
+          if ((a > bb) == up) {
+            s[t] = bb;
+            s[u] = a;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
+  for (int t = threadIdx.x; t < k; t += blockDim.x) {
+    order[b + t] = (uint32_t)(s[t] & 0xffffffffu);
+    copy_rows(rows, b + t, (uint32_t)(s[t] & 0xffffffffu));
+  }
+  __syncthreads();
+}
+
+// Per-slot fix-up of ascending (tie, index) order inside every cell, and the sorted keys.
+// After the scatter, cell c's particles fill [cell_start[c], cell_start[c+1]) in atomic
+// order; the thread of slot t counts the cell's particles that rank below its own and
+// writes its particle to that place (k comparisons per particle, L1-resident).  The rows to
+// move are loaded while the cell is ranked: bound by the latency of its loads, a serving step of
+// 3.1 M particles takes 50 µs (64 with each row's load behind the one before).
+// A cell larger than kSmallCell is left, by the thread of its first slot, to
+//   kInBlock: its block, after the block's other slots.  This saves the launch for them, mostly
+//     without work, and its list's memset (2.7 µs of every step at 150,000 particles), and
+//     pays with the block's barriers and 16 KB of shared memory;
+//   else: k_cell_fix_large.  At 260,100 particles the block variant takes 6.0 µs against 4.6 + 1.9
+//     and the memset, at 2^20 20 against 15 + 2, at 3.1 M 82 against 50 + 2.
+// kFixInBlock is the line between them.
+// The sentinel cell (the key cell_capacity: particles outside every grid, or of no scene in
+// a pooled batch) keeps the scatter order: nothing reads its order.
+constexpr int64_t kFixInBlock = 1 << 18;
+constexpr int kFixThreads = 256;
+constexpr int kFixLarge = kFixThreads / (kSmallCell + 1) + 1;   // large cells that begin in one block
+
+template <bool kInBlock>
+__global__ void __launch_bounds__(kFixThreads) k_cell_fix(const uint32_t* __restrict__ keys, int64_t n,
+                                                          const int32_t* __restrict__ cell_start,
+                                                          const uint32_t* __restrict__ tmp,
+                                                          const uint32_t* __restrict__ tie,
+                                                          uint32_t* __restrict__ order,
+                                                          uint32_t* __restrict__ sorted_keys,
+                                                          int32_t* __restrict__ big_list,
+                                                          int32_t* __restrict__ big_count, int32_t* status,
+                                                          const ArraySet rows, uint32_t sentinel) {
+  __shared__ int large[kFixLarge];
+  __shared__ int num_large;
+  if constexpr (kInBlock) {
+    if (threadIdx.x == 0) num_large = 0;
+    __syncthreads();
+  }
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) {
+    const uint32_t x = tmp[t];
+    const uint32_t c = __ldg(keys + x);
+    sorted_keys[t] = c;
+    if (c == sentinel) {
+      order[t] = x;
+      copy_rows(rows, t, x);
+    } else {
+      const int b = __ldg(cell_start + c), e = __ldg(cell_start + c + 1);
+      if (e - b > kSmallCell) {
+        if (t == b) {
+          if constexpr (kInBlock)
+            large[atomicAdd(&num_large, 1)] = (int)c;
+          else
+            big_list[atomicAdd(big_count, 1)] = (int32_t)c;
+        }
+      } else {
+        const FourRows head = load_rows(rows, 0, x);
+        const uint64_t mine = cell_rank(x, tie);
+        int rank = 0;
+        for (int u = b; u < e; ++u) rank += cell_rank(__ldg(tmp + u), tie) < mine;
+        order[b + rank] = x;
+        store_rows(rows, 0, b + rank, head);
+        copy_rows(rows, b + rank, x, 4);
+      }
+    }
+  }
+  if constexpr (kInBlock) {
+    __shared__ uint64_t ranks[kBlockSortMax];
+    __syncthreads();
+    for (int q = 0; q < num_large; ++q)
+      fix_large_cell(cell_start[large[q]], cell_start[large[q] + 1], tmp, tie, order, status, rows, ranks);
+  }
+}
+
 __global__ void __launch_bounds__(512) k_cell_fix_large(const int32_t* __restrict__ cell_start,
                                                         const uint32_t* __restrict__ tmp,
                                                         const uint32_t* __restrict__ tie,
@@ -352,60 +441,10 @@ __global__ void __launch_bounds__(512) k_cell_fix_large(const int32_t* __restric
                                                         const int32_t* __restrict__ big_list,
                                                         const int32_t* __restrict__ big_count, int32_t* status,
                                                         const ArraySet rows) {
-  __shared__ uint64_t s[kBlockSortMax];
+  __shared__ uint64_t ranks[kBlockSortMax];
   const int nbig = *big_count;
-  for (int q = blockIdx.x; q < nbig; q += gridDim.x) {
-    const int c = big_list[q];
-    const int b = cell_start[c], e = cell_start[c + 1];
-    const int k = e - b;
-    if (k > kBlockSortMax) {
-      for (int t = threadIdx.x; t < k; t += blockDim.x) {
-        order[b + t] = tmp[b + t];
-        copy_rows(rows, b + t, tmp[b + t]);
-      }
-      if (threadIdx.x == 0) flag(status, SPH_FLAG_CELL_ORDER);
-      continue;
-    }
-    if (k <= kRankSortMax) {
-      for (int t = threadIdx.x; t < k; t += blockDim.x) s[t] = cell_rank(tmp[b + t], tie);
-      __syncthreads();
-      for (int t = threadIdx.x; t < k; t += blockDim.x) {
-        const uint64_t mine = s[t];
-        int rank = 0;
-#pragma unroll 4
-        for (int u = 0; u < k; ++u) rank += s[u] < mine;   // every lane reads the same word
-        order[b + rank] = (uint32_t)(mine & 0xffffffffu);
-        copy_rows(rows, b + rank, (uint32_t)(mine & 0xffffffffu));
-      }
-      __syncthreads();
-      continue;
-    }
-    int p2 = 1;
-    while (p2 < k) p2 <<= 1;
-    for (int t = threadIdx.x; t < p2; t += blockDim.x) s[t] = t < k ? cell_rank(tmp[b + t], tie) : ~0ull;
-    __syncthreads();
-    for (int size = 2; size <= p2; size <<= 1) {
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        for (int t = threadIdx.x; t < p2; t += blockDim.x) {
-          int u = t ^ stride;
-          if (u > t) {
-            bool up = (t & size) == 0;
-            uint64_t a = s[t], bb = s[u];
-            if ((a > bb) == up) {
-              s[t] = bb;
-              s[u] = a;
-            }
-          }
-        }
-        __syncthreads();
-      }
-    }
-    for (int t = threadIdx.x; t < k; t += blockDim.x) {
-      order[b + t] = (uint32_t)(s[t] & 0xffffffffu);
-      copy_rows(rows, b + t, (uint32_t)(s[t] & 0xffffffffu));
-    }
-    __syncthreads();
-  }
+  for (int q = blockIdx.x; q < nbig; q += gridDim.x)
+    fix_large_cell(cell_start[big_list[q]], cell_start[big_list[q] + 1], tmp, tie, order, status, rows, ranks);
 }
 
 // cell_start[c] = lower_bound(sorted_keys, c) for c = 0..cap+1 (used after the LSD radix sort).
@@ -650,9 +689,8 @@ sph_status_t sph_batch_cell_keys(const float* pos, int64_t n, const int32_t* sid
 
 size_t sph_counting_sort_scratch_bytes(int64_t n, int32_t cell_capacity) {
   size_t b = (size_t)(n < 1 ? 1 : n) * sizeof(uint32_t) + 256;          // scatter target
-  b += ((size_t)cell_capacity + 1) * sizeof(int32_t) + 256;              // large-cell list
-  b += 256;                                                               // large-cell count
   b += sph_scan_scratch_bytes((int64_t)cell_capacity + 1) + 256;
+  if (n > kFixInBlock) b += ((size_t)cell_capacity + 1) * sizeof(int32_t) + 512;   // large-cell list and count
   return b;
 }
 
@@ -682,19 +720,25 @@ static sph_status_t counting_sort_impl(const uint32_t* keys, int64_t n, int32_t 
     return r;
   };
   uint32_t* tmp = reinterpret_cast<uint32_t*>(take((size_t)(n < 1 ? 1 : n) * sizeof(uint32_t)));
-  int32_t* big_list = reinterpret_cast<int32_t*>(take(((size_t)cell_capacity + 1) * sizeof(int32_t)));
-  int32_t* big_count = reinterpret_cast<int32_t*>(take(sizeof(int32_t)));
   size_t scan_b = sph_scan_scratch_bytes((int64_t)cell_capacity + 1);
   void* scan_s = take(scan_b);
   const int64_t slots = (int64_t)cell_capacity + 1;  // cells 0..cap-1 and the sentinel cap
   sph_status_t s = sph_exclusive_scan_i32(cell_count, cell_start, slots, scan_s, scan_b, stream);
   if (s != SPH_OK) return s;
   if (n == 0) return SPH_OK;
-  cudaMemsetAsync(big_count, 0, sizeof(int32_t), st);
   k_count_scatter<<<grid_for(n, 256), 256, 0, st>>>(keys, n, cell_start, cell_count, tmp, (uint32_t)cell_capacity);
-  k_cell_fix<<<grid_for(n, 256), 256, 0, st>>>(keys, n, cell_start, tmp, tie, order, sorted_keys, big_list,
-                                               big_count, rows, (uint32_t)cell_capacity);
-  k_cell_fix_large<<<4 * kNumSMs, 512, 0, st>>>(cell_start, tmp, tie, order, big_list, big_count, status, rows);
+  const int nb = grid_for(n, kFixThreads);
+  if (n <= kFixInBlock) {
+    k_cell_fix<true><<<nb, kFixThreads, 0, st>>>(keys, n, cell_start, tmp, tie, order, sorted_keys, nullptr, nullptr,
+                                                 status, rows, (uint32_t)cell_capacity);
+  } else {
+    int32_t* big_list = reinterpret_cast<int32_t*>(take(((size_t)cell_capacity + 1) * sizeof(int32_t)));
+    int32_t* big_count = reinterpret_cast<int32_t*>(take(sizeof(int32_t)));
+    cudaMemsetAsync(big_count, 0, sizeof(int32_t), st);
+    k_cell_fix<false><<<nb, kFixThreads, 0, st>>>(keys, n, cell_start, tmp, tie, order, sorted_keys, big_list, big_count,
+                                                  status, rows, (uint32_t)cell_capacity);
+    k_cell_fix_large<<<4 * kNumSMs, 512, 0, st>>>(cell_start, tmp, tie, order, big_list, big_count, status, rows);
+  }
   SPH_CHECK_LAUNCH("counting_sort");
   return SPH_OK;
 }

@@ -139,22 +139,60 @@ inline bool array_set_from(int32_t count, const int32_t* elem_bytes, const void*
   return true;
 }
 
-__device__ __forceinline__ void copy_rows(const ArraySet& a, int64_t dst, int64_t src) {
+// Rows of arrays first .. first + 3, all four loads in flight before the first store: copied one
+// after another each row waits for its own load.
+struct FourRows {
+  uint4 v[4];
+};
+
+__device__ __forceinline__ FourRows load_rows(const ArraySet& a, int first, int64_t src) {
+  FourRows r;
 #pragma unroll
-  for (int k = 0; k < kMaxArrays; ++k) {
+  for (int q = 0; q < 4; ++q) {
+    const int k = first + q;
     if (k >= a.count) break;
     switch (a.bytes[k]) {
       case 4:
-        static_cast<uint32_t*>(a.out[k])[dst] = static_cast<const uint32_t*>(a.in[k])[src];
+        r.v[q].x = __ldg(static_cast<const uint32_t*>(a.in[k]) + src);
         break;
-      case 8:
-        static_cast<uint2*>(a.out[k])[dst] = static_cast<const uint2*>(a.in[k])[src];
+      case 8: {
+        const uint2 w = __ldg(static_cast<const uint2*>(a.in[k]) + src);
+        r.v[q].x = w.x;
+        r.v[q].y = w.y;
         break;
+      }
       default:
-        static_cast<uint4*>(a.out[k])[dst] = static_cast<const uint4*>(a.in[k])[src];
+        r.v[q] = __ldg(static_cast<const uint4*>(a.in[k]) + src);
         break;
     }
   }
+  return r;
+}
+
+__device__ __forceinline__ void store_rows(const ArraySet& a, int first, int64_t dst, const FourRows& r) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int k = first + q;
+    if (k >= a.count) break;
+    switch (a.bytes[k]) {
+      case 4:
+        static_cast<uint32_t*>(a.out[k])[dst] = r.v[q].x;
+        break;
+      case 8:
+        static_cast<uint2*>(a.out[k])[dst] = make_uint2(r.v[q].x, r.v[q].y);
+        break;
+      default:
+        static_cast<uint4*>(a.out[k])[dst] = r.v[q];
+        break;
+    }
+  }
+}
+
+// Rows from array `first` on.
+__device__ __forceinline__ void copy_rows(const ArraySet& a, int64_t dst, int64_t src, int first = 0) {
+#pragma unroll
+  for (int k = 0; k < kMaxArrays; k += 4)
+    if (k >= first && k < a.count) store_rows(a, k, dst, load_rows(a, k, src));
 }
 
 __device__ __forceinline__ void flag(int32_t* status, int32_t f) {
