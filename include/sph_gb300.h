@@ -347,6 +347,11 @@ sph_status_t sph_deltasph_segment_lists(int64_t n, size_t* masks_offset, size_t*
 sph_status_t sph_deltasph_forces(const sph_fluid_view* fluid, const sph_wall_view* walls, const sph_grid* grid,
                                  const sph_params* params, float* dpdt, float* acc, float* L, float* grad_rho,
                                  void* scratch, size_t scratch_bytes, void* stream);
+/* sph_mdbc_wall_density, then sph_deltasph_forces; for small scenes with pairs from the cell
+ * rows the walls' densities share a launch with the neighbor records. */
+sph_status_t sph_deltasph_wall_forces(const sph_fluid_view* fluid, const sph_wall_view* walls, const sph_grid* grid,
+                                      const sph_params* params, float* dpdt, float* acc, float* L, float* grad_rho,
+                                      void* scratch, size_t scratch_bytes, void* stream);
 /* semiImplicitEuler (src/simulationBase.py:647-652): v' = v + dt a, x' = x + dt (v + dt a),
  * rho' = rho + dt dpdt / rest_density when continuum_density.  dt is a device float. */
 sph_status_t sph_integrate_semi_implicit_euler(int64_t n, const float* x, const float* v, const float* rho,
@@ -357,6 +362,17 @@ sph_status_t sph_integrate_semi_implicit_euler(int64_t n, const float* x, const 
 sph_status_t sph_rk_axpy(int64_t n, const float* x0, const float* v0, const float* rho0_field, const float* ku,
                          const float* ka, const float* kd, const float* dt, float c, float rest_density, float* x_out,
                          float* v_out, float* rho_out, int32_t* status, void* stream);
+/* sph_integrate_semi_implicit_euler that also adds dt to *time (device double, may be NULL). */
+sph_status_t sph_integrate_step(int64_t n, const float* x, const float* v, const float* rho, const float* acc,
+                                const float* dpdt, const float* dt, float rest_density, int32_t continuum_density,
+                                float* x_out, float* v_out, float* rho_out, int32_t* status, double* time,
+                                void* stream);
+/* One RK4 stage: sph_rk_accumulate of k, then sph_rk_axpy of k, or (last) of the sums; adds dt to
+ * *time (device double, may be NULL). */
+sph_status_t sph_rk_stage(int64_t n, const float* x0, const float* v0, const float* rho0_field, const float* ku,
+                          const float* ka, const float* kd, float w, int32_t init, int32_t last, float* su, float* sa,
+                          float* sd, const float* dt, float c, float rest_density, float* x_out, float* v_out,
+                          float* rho_out, int32_t* status, double* time, void* stream);
 /* s = w*k (init) or s += w*k for the RK4 sums of (velocity, acceleration, dpdt). */
 sph_status_t sph_rk_accumulate(int64_t n, const float* ku, const float* ka, const float* kd, float w, int32_t init,
                                float* su, float* sa, float* sd, void* stream);

@@ -117,6 +117,9 @@ SIGNATURES.update({  # simulation kernels
     "sph_deltasph_forces": (_I32, [_P] * 8 + [_P, _SZ, _P]),
     "sph_integrate_semi_implicit_euler": (_I32, [_I64] + [_P] * 6 +
                                           [_F32, _I32] + [_P] * 5),
+    "sph_deltasph_wall_forces": (_I32, [_P] * 8 + [_P, _SZ, _P]),
+    "sph_integrate_step": (_I32, [_I64] + [_P] * 6 + [_F32, _I32] + [_P] * 6),
+    "sph_rk_stage": (_I32, [_I64] + [_P] * 6 + [_F32, _I32, _I32] + [_P] * 4 + [_F32, _F32] + [_P] * 6),
     "sph_rk_axpy": (_I32, [_I64] + [_P] * 7 + [_F32, _F32] +
                     [_P] * 5),
     "sph_rk_accumulate": (_I32, [_I64] + [_P] * 3 + [_F32, _I32] +

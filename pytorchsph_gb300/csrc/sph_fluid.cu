@@ -557,6 +557,30 @@ __global__ void __launch_bounds__(256) k_prep_cells(FluidView F, SphParams P, co
   }
 }
 
+// The walls' densities and the records of one scene in one launch: the first wall_blocks blocks
+// take four lanes per wall, the others the records.  Both only read the sorted state; the
+// walls are a chain of latencies (a cell row, its candidates, a solve in double) in a few blocks.
+// 8,192 particles with 1,380 walls: 9.4 us (9.4 + 4.4 one after the other).
+template <int kLanes>
+__global__ void __launch_bounds__(128) k_walls_and_prep(FluidView F, WallView W, SphParams P,
+                                                        const sph_grid* __restrict__ gp, Rec* __restrict__ rec,
+                                                        int32_t* __restrict__ nseg, int32_t* __restrict__ seg_start,
+                                                        uint32_t* __restrict__ seg_mask, int wall_blocks) {
+  if ((int)blockIdx.x < wall_blocks) {
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) / 4;
+    mdbc_body<4>(min(b, W.n - 1), b < W.n, threadIdx.x % 4, F, W, *gp, P, 0);
+    return;
+  }
+  const int i = (int)(((int64_t)(blockIdx.x - wall_blocks) * blockDim.x + threadIdx.x) / kLanes);
+  if constexpr (kLanes == 1) {
+    if (i >= F.n) return;
+    prep_body(i, F, P, rec);
+    segments_body(i, F, *gp, 0, P.search_radius, P.thr, nseg, seg_start, seg_mask);
+  } else {
+    prep_rows(i, i < F.n, threadIdx.x % kLanes, F, *gp, 0, P, rec, nseg, seg_start, seg_mask);
+  }
+}
+
 // One scene's right-hand side.
 template <bool kCells, int kScheme, bool kByFour>
 __global__ void __launch_bounds__(128) k_dsph_pass1(FluidView F, const Rec* __restrict__ rec, WallView W,
@@ -585,9 +609,10 @@ __global__ void __launch_bounds__(128) k_dsph_diffusion(FluidView F, const Rec* 
 __global__ void k_sie(int n, const float2* __restrict__ x, const float2* __restrict__ v,
                       const float* __restrict__ rho, const float2* __restrict__ a, const float* __restrict__ dpdt,
                       const float* __restrict__ dt_ptr, float rho0, int continuum, float2* __restrict__ xo,
-                      float2* __restrict__ vo, float* __restrict__ ro, int32_t* status) {
+                      float2* __restrict__ vo, float* __restrict__ ro, int32_t* status, double* time) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  if (time && i == 0) *time += (double)*dt_ptr;
   sie_apply(i, x[i], v[i], rho[i], a[i], continuum ? dpdt[i] : 0.f, *dt_ptr, rho0, continuum, xo, vo, ro, status);
 }
 
@@ -736,6 +761,48 @@ __global__ void k_rk_axpy(int n, const float2* __restrict__ x0, const float2* __
     flag(status, SPH_FLAG_NONFINITE);
 }
 
+// A whole RK4 stage: s (+)= w k, then out = base + c dt k, or the step's end from the sums (last).
+// One launch where a sum and an update were two of about 1.3 us.
+__global__ void k_rk_stage(int n, const float2* __restrict__ x0, const float2* __restrict__ v0,
+                           const float* __restrict__ r0, const float2* __restrict__ ku, const float2* __restrict__ ka,
+                           const float* __restrict__ kd, float w, int init, int last, float2* __restrict__ su,
+                           float2* __restrict__ sa, float* __restrict__ sd, const float* __restrict__ dt_ptr, float c,
+                           float rho0, float2* __restrict__ xo, float2* __restrict__ vo, float* __restrict__ ro,
+                           int32_t* status, double* time) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float dt = *dt_ptr;
+  if (time && i == 0) *time += (double)dt;
+  float2 u = ku[i], a = ka[i];
+  float d = kd[i];
+  float2 pu = make_float2(w * u.x, w * u.y), pa = make_float2(w * a.x, w * a.y);
+  float pd = w * d;
+  if (!init) {
+    const float2 cu = su[i], ca = sa[i];
+    pu = make_float2(cu.x + w * u.x, cu.y + w * u.y);
+    pa = make_float2(ca.x + w * a.x, ca.y + w * a.y);
+    pd = sd[i] + w * d;
+  }
+  su[i] = pu;
+  sa[i] = pa;
+  sd[i] = pd;
+  if (last) {
+    u = pu;
+    a = pa;
+    d = pd;
+  }
+  const float h = c * dt;
+  const float2 x = x0[i], v = v0[i];
+  const float2 xn = make_float2(x.x + h * u.x, x.y + h * u.y);
+  const float2 vn = make_float2(v.x + h * a.x, v.y + h * a.y);
+  const float rn = r0[i] + h * d / rho0;
+  xo[i] = xn;
+  vo[i] = vn;
+  ro[i] = rn;
+  if (!isfinite(xn.x) || !isfinite(xn.y) || !isfinite(vn.x) || !isfinite(vn.y) || !isfinite(rn))
+    flag(status, SPH_FLAG_NONFINITE);
+}
+
 // s (+)= w * k for the RK4 sums; init = 1 overwrites.
 __global__ void k_rk_accum(int n, const float2* __restrict__ ku, const float2* __restrict__ ka,
                            const float* __restrict__ kd, float w, int init, float2* __restrict__ su,
@@ -820,6 +887,12 @@ sph_status_t sph_deltasph_segment_lists(int64_t n, size_t* masks_offset, size_t*
 // 18.1 + 9.7, 131,044: 21.9 + 12.3 / 27.8 + 13.2.
 constexpr int kByFourMax = 49152;
 
+// Particles up to which the walls' densities run beside the records (k_walls_and_prep; its
+// registers cost the records some of their warps), us, beside / one after the other, the walls of a
+// tank twice as wide and high: 49,152: 9.1 / 15.8, 153,863: 12.0 / 20.0, 262,144: 14.6 / 24.2,
+// 1,024,000: 43.0 / 50.1.
+constexpr int kWallsBesideMax = 1 << 20;
+
 // The neighbor records in caller scratch, 32-byte aligned.
 static bool records_from_scratch(void* scratch, size_t bytes, int64_t n, Rec** rec, Segments* seg = nullptr) {
   if (!scratch) return false;
@@ -839,14 +912,14 @@ static bool records_from_scratch(void* scratch, size_t bytes, int64_t n, Rec** r
 
 extern "C" {
 
-sph_status_t sph_deltasph_forces(const sph_fluid_view* fluid, const sph_wall_view* walls, const sph_grid* grid,
-                                 const sph_params* params, float* dpdt, float* acc, float* L, float* grad_rho,
-                                 void* scratch, size_t scratch_bytes, void* stream) {
+static sph_status_t forces(const sph_fluid_view* fluid, const sph_wall_view* walls, const sph_grid* grid,
+                           const sph_params* params, float* dpdt, float* acc, float* L, float* grad_rho, void* scratch,
+                           size_t scratch_bytes, bool with_walls, void* stream) {
   SPH_VIEW_CHECK(fluid);
   SPH_VIEW_CHECK(walls);
   SPH_REQUIRE(grid && params && dpdt && acc && params->support > 0.f, "deltasph_forces: bad arguments");
   SPH_REQUIRE(params->density_diffusion != 2 || grad_rho, "deltasph_forces: deltaSPH diffusion needs grad_rho");
-  if (fluid->n == 0) return SPH_OK;
+  if (fluid->n == 0) return with_walls ? sph_mdbc_wall_density(fluid, walls, grid, params, stream) : SPH_OK;
   // no CSR list (offsets and cols NULL): the pairs come from the cell rows
   const bool cells = !fluid->offsets && !fluid->cols;
   SPH_REQUIRE(cells ? fluid->cell_start && fluid->keys : fluid->offsets && fluid->cols,
@@ -866,6 +939,11 @@ sph_status_t sph_deltasph_forces(const sph_fluid_view* fluid, const sph_wall_vie
   const int nb = grid_for(n, 128);
 #define SPH_PASS1(C, K, B4) k_dsph_pass1<C, K, B4><<<nb, 128, 0, st>>>(F, rec, W, grid, P, seg, dpdt, ac, Lo, gr)
 #define SPH_DIFFUSION(C, B4) k_dsph_diffusion<C, B4><<<nb, 128, 0, st>>>(F, rec, grid, P, seg, gr, dpdt)
+  const bool beside = cells && with_walls && W.n > 0 && W.n <= kMdbcSplitWalls && n <= kWallsBesideMax;
+  if (with_walls && !beside) {
+    const sph_status_t r = sph_mdbc_wall_density(fluid, walls, grid, params, stream);
+    if (r != SPH_OK) return r;
+  }
   if (!cells) {
     k_prep<<<grid_for(n, 256), 256, 0, st>>>(F, P, rec);
     SPH_PASS1(false, -1, false);
@@ -874,7 +952,13 @@ sph_status_t sph_deltasph_forces(const sph_fluid_view* fluid, const sph_wall_vie
     int32_t* ns = const_cast<int32_t*>(seg.nseg);
     int32_t* ss = const_cast<int32_t*>(seg.start);
     uint32_t* sm = const_cast<uint32_t*>(seg.mask);
-    if (n <= kRowLanesMax)
+    const int wb = beside ? grid_for(4 * (int64_t)W.n, 128) : 0;
+    if (beside && n <= kRowLanesMax)
+      k_walls_and_prep<kRowLanes><<<wb + grid_for(kRowLanes * (int64_t)n, 128), 128, 0, st>>>(F, W, P, grid, rec, ns, ss,
+                                                                                           sm, wb);
+    else if (beside)
+      k_walls_and_prep<1><<<wb + grid_for(n, 128), 128, 0, st>>>(F, W, P, grid, rec, ns, ss, sm, wb);
+    else if (n <= kRowLanesMax)
       k_prep_cells<kRowLanes><<<grid_for(kRowLanes * (int64_t)n, 256), 256, 0, st>>>(F, P, grid, rec, ns, ss, sm);
     else
       k_prep_cells<1><<<grid_for(n, 256), 256, 0, st>>>(F, P, grid, rec, ns, ss, sm);
@@ -901,10 +985,22 @@ sph_status_t sph_deltasph_forces(const sph_fluid_view* fluid, const sph_wall_vie
   return SPH_OK;
 }
 
-sph_status_t sph_integrate_semi_implicit_euler(int64_t n, const float* x, const float* v, const float* rho,
-                                               const float* acc, const float* dpdt, const float* dt,
-                                               float rest_density, int32_t continuum_density, float* x_out,
-                                               float* v_out, float* rho_out, int32_t* status, void* stream) {
+sph_status_t sph_deltasph_forces(const sph_fluid_view* fluid, const sph_wall_view* walls, const sph_grid* grid,
+                                 const sph_params* params, float* dpdt, float* acc, float* L, float* grad_rho,
+                                 void* scratch, size_t scratch_bytes, void* stream) {
+  return forces(fluid, walls, grid, params, dpdt, acc, L, grad_rho, scratch, scratch_bytes, false, stream);
+}
+
+sph_status_t sph_deltasph_wall_forces(const sph_fluid_view* fluid, const sph_wall_view* walls, const sph_grid* grid,
+                                      const sph_params* params, float* dpdt, float* acc, float* L, float* grad_rho,
+                                      void* scratch, size_t scratch_bytes, void* stream) {
+  return forces(fluid, walls, grid, params, dpdt, acc, L, grad_rho, scratch, scratch_bytes, true, stream);
+}
+
+sph_status_t sph_integrate_step(int64_t n, const float* x, const float* v, const float* rho, const float* acc,
+                                const float* dpdt, const float* dt, float rest_density, int32_t continuum_density,
+                                float* x_out, float* v_out, float* rho_out, int32_t* status, double* time,
+                                void* stream) {
   SPH_REQUIRE(n >= 0 && n < (1LL << 31) && x && v && rho && acc && dt && x_out && v_out && rho_out,
               "integrate_semi_implicit_euler: bad arguments");
   SPH_REQUIRE(!continuum_density || dpdt, "integrate_semi_implicit_euler: continuum density needs dpdt");
@@ -912,9 +1008,17 @@ sph_status_t sph_integrate_semi_implicit_euler(int64_t n, const float* x, const 
   k_sie<<<grid_for(n, 256), 256, 0, as_stream(stream)>>>(
       (int)n, reinterpret_cast<const float2*>(x), reinterpret_cast<const float2*>(v), rho,
       reinterpret_cast<const float2*>(acc), dpdt, dt, rest_density, continuum_density, reinterpret_cast<float2*>(x_out),
-      reinterpret_cast<float2*>(v_out), rho_out, status);
+      reinterpret_cast<float2*>(v_out), rho_out, status, time);
   SPH_CHECK_LAUNCH("integrate_semi_implicit_euler");
   return SPH_OK;
+}
+
+sph_status_t sph_integrate_semi_implicit_euler(int64_t n, const float* x, const float* v, const float* rho,
+                                               const float* acc, const float* dpdt, const float* dt,
+                                               float rest_density, int32_t continuum_density, float* x_out,
+                                               float* v_out, float* rho_out, int32_t* status, void* stream) {
+  return sph_integrate_step(n, x, v, rho, acc, dpdt, dt, rest_density, continuum_density, x_out, v_out, rho_out, status,
+                            nullptr, stream);
 }
 
 sph_status_t sph_batch_deltasph_step(const sph_fluid_view* fluid, const sph_wall_view* walls, const void* scenes,
@@ -1057,6 +1161,23 @@ sph_status_t sph_rk_axpy(int64_t n, const float* x0, const float* v0, const floa
       reinterpret_cast<const float2*>(ku), reinterpret_cast<const float2*>(ka), kd, dt, c, rest_density,
       reinterpret_cast<float2*>(x_out), reinterpret_cast<float2*>(v_out), rho_out, status);
   SPH_CHECK_LAUNCH("rk_axpy");
+  return SPH_OK;
+}
+
+sph_status_t sph_rk_stage(int64_t n, const float* x0, const float* v0, const float* rho0_field, const float* ku,
+                          const float* ka, const float* kd, float w, int32_t init, int32_t last, float* su, float* sa,
+                          float* sd, const float* dt, float c, float rest_density, float* x_out, float* v_out,
+                          float* rho_out, int32_t* status, double* time, void* stream) {
+  SPH_REQUIRE(n >= 0 && n < (1LL << 31) && x0 && v0 && rho0_field && ku && ka && kd && su && sa && sd && dt && x_out &&
+                  v_out && rho_out,
+              "rk_stage: bad arguments");
+  if (n == 0) return SPH_OK;
+  k_rk_stage<<<grid_for(n, 256), 256, 0, as_stream(stream)>>>(
+      (int)n, reinterpret_cast<const float2*>(x0), reinterpret_cast<const float2*>(v0), rho0_field,
+      reinterpret_cast<const float2*>(ku), reinterpret_cast<const float2*>(ka), kd, w, init, last,
+      reinterpret_cast<float2*>(su), reinterpret_cast<float2*>(sa), sd, dt, c, rest_density,
+      reinterpret_cast<float2*>(x_out), reinterpret_cast<float2*>(v_out), rho_out, status, time);
+  SPH_CHECK_LAUNCH("rk_stage");
   return SPH_OK;
 }
 

@@ -301,13 +301,10 @@ class Simulation:
         if self.cfg.solver == "dfsph":
             return self._dfsph_rhs(acc, st)
         dpdt = torch.empty(n, dtype=torch.float32, device=self.device)
-        if self.nb:
-            N.call("sph_mdbc_wall_density", _ref(self.fluid_view), _ref(self.wall_view), N.ptr(self.grid),
-                   _ref(self.params), st)
         gr = self.ws.get("grad_rho", 2 * n, torch.float32) if self.cfg.density_diffusion == "deltaSPH" else None
         scr = self.ws.bytes("forces_scratch", self.lib.sph_deltasph_scratch_bytes(n))
-        N.call("sph_deltasph_forces", _ref(self.fluid_view), _ref(self.wall_view), N.ptr(self.grid), _ref(self.params),
-               N.ptr(dpdt), N.ptr(acc), None, N.ptr(gr), N.ptr(scr), scr.numel() * 8, st)
+        N.call("sph_deltasph_wall_forces", _ref(self.fluid_view), _ref(self.wall_view), N.ptr(self.grid),
+               _ref(self.params), N.ptr(dpdt), N.ptr(acc), None, N.ptr(gr), N.ptr(scr), scr.numel() * 8, st)
         self.last = {"acc": acc, "dpdt": dpdt}
         return acc, self.arr["v"], dpdt
 
@@ -398,9 +395,9 @@ class Simulation:
             xo = torch.empty_like(self.arr["x"])
             vo = torch.empty_like(self.arr["v"])
             ro = torch.empty_like(self.arr["rho"])
-            N.call("sph_integrate_semi_implicit_euler", n, N.ptr(self.arr["x"]), N.ptr(vel), N.ptr(self.arr["rho"]),
+            N.call("sph_integrate_step", n, N.ptr(self.arr["x"]), N.ptr(vel), N.ptr(self.arr["rho"]),
                    N.ptr(acc), N.ptr(dpdt), N.ptr(self.dt), c.rest_density, int(cont), N.ptr(xo), N.ptr(vo),
-                   N.ptr(ro), N.ptr(self.status), st)
+                   N.ptr(ro), N.ptr(self.status), N.ptr(self.time), st)
             self.last["eval"] = {"x": self.arr["x"], "v": self.arr["v"], "rho": self.arr["rho"]}
             self.arr["x"], self.arr["v"], self.arr["rho"] = xo, vo, ro
             self.last["acc_final"] = acc
@@ -413,33 +410,25 @@ class Simulation:
             self.extra["su"] = torch.empty_like(self.arr["x"])
             self.extra["sa"] = torch.empty_like(self.arr["x"])
             self.extra["sd"] = torch.empty_like(self.arr["rho"])
-            for k, (cstage, w) in enumerate([(0.5, 1.0), (0.5, 2.0), (1.0, 2.0), (None, 1.0)]):
+            for k, (cstage, w) in enumerate([(0.5, 1.0), (0.5, 2.0), (1.0, 2.0), (1.0 / 6.0, 1.0)]):
                 acc, vel, dpdt = self.rhs(sync)
                 e = self.extra
-                N.call("sph_rk_accumulate", n, N.ptr(vel), N.ptr(acc), N.ptr(dpdt), w, int(k == 0), N.ptr(e["su"]),
-                       N.ptr(e["sa"]), N.ptr(e["sd"]), st)
-                if cstage is not None:
-                    xo = torch.empty_like(self.arr["x"])
-                    vo = torch.empty_like(self.arr["v"])
-                    ro = torch.empty_like(self.arr["rho"])
-                    N.call("sph_rk_axpy", n, N.ptr(e["x0"]), N.ptr(e["v0"]), N.ptr(e["r0"]), N.ptr(vel), N.ptr(acc),
-                           N.ptr(dpdt), N.ptr(self.dt), cstage, c.rest_density, N.ptr(xo), N.ptr(vo), N.ptr(ro),
-                           N.ptr(self.status), st)
-                    self.arr["x"], self.arr["v"], self.arr["rho"] = xo, vo, ro
-            e = self.extra
-            xo = torch.empty_like(self.arr["x"])
-            vo = torch.empty_like(self.arr["v"])
-            ro = torch.empty_like(self.arr["rho"])
-            N.call("sph_rk_axpy", n, N.ptr(e["x0"]), N.ptr(e["v0"]), N.ptr(e["r0"]), N.ptr(e["su"]), N.ptr(e["sa"]),
-                   N.ptr(e["sd"]), N.ptr(self.dt), 1.0 / 6.0, c.rest_density, N.ptr(xo), N.ptr(vo), N.ptr(ro),
-                   N.ptr(self.status), st)
-            self.last["eval"] = {"x": self.arr["x"], "v": self.arr["v"], "rho": self.arr["rho"]}
-            self.arr["x"], self.arr["v"], self.arr["rho"] = xo, vo, ro
+                xo = torch.empty_like(self.arr["x"])
+                vo = torch.empty_like(self.arr["v"])
+                ro = torch.empty_like(self.arr["rho"])
+                N.call("sph_rk_stage", n, N.ptr(e["x0"]), N.ptr(e["v0"]), N.ptr(e["r0"]), N.ptr(vel), N.ptr(acc),
+                       N.ptr(dpdt), w, int(k == 0), int(k == 3), N.ptr(e["su"]), N.ptr(e["sa"]), N.ptr(e["sd"]),
+                       N.ptr(self.dt), cstage, c.rest_density, N.ptr(xo), N.ptr(vo), N.ptr(ro), N.ptr(self.status),
+                       N.ptr(self.time) if k == 3 else None, st)
+                if k == 3:
+                    self.last["eval"] = {"x": self.arr["x"], "v": self.arr["v"], "rho": self.arr["rho"]}
+                self.arr["x"], self.arr["v"], self.arr["rho"] = xo, vo, ro
             self.last["acc_final"] = e["sa"]
             self.extra = {}
         else:
             raise N.SPHError(f"integration scheme {c.integration!r} is not on the GB300 path")
-        self.time += self.dt
+        if n == 0:
+            self.time += self.dt   # (the integrator's launch adds it)
         if not c.fixed_dt:
             self.last["dt_used"] = self.dt.clone()
             sc = self.ws.bytes("dt_scratch", self.lib.sph_dt_scratch_bytes())
