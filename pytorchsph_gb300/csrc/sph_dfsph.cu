@@ -177,10 +177,10 @@ __device__ __forceinline__ void wall_fluid_pairs(int b, const FluidView& F, cons
 // is stored whenever it holds four new ones.
 struct ListWriter {
   const DfsphBufs& B;
-  int i, n, lanes, k;
+  int i, n, shift, k;   // 1 << shift lanes per particle
   int4 four;
   __device__ __forceinline__ void store(int c) {
-    if (c < kListChunks) B.list[((size_t)(c / lanes) * n + i) * lanes + c % lanes] = four;
+    if (c < kListChunks) B.list[(((size_t)(c >> shift) * n + i) << shift) + (c & ((1 << shift) - 1))] = four;
   }
   __device__ __forceinline__ void add(int j) {
     four = make_int4(four.y, four.z, four.w, j);
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(128) k_dfsph_fluid_density(FluidView F, WallVi
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= F.n) return;
   const sph_grid g = *gp;
-  ListWriter out{B, i, F.n, lanes, 0, make_int4(i, i, i, i)};
+  ListWriter out{B, i, F.n, 31 - __clz(lanes), 0, make_int4(i, i, i, i)};
   float rf;
   int fluid_chunks = 0;
   if constexpr (kCells) {
@@ -243,11 +243,23 @@ __global__ void __launch_bounds__(128) k_dfsph_fluid_density(FluidView F, WallVi
     cell_of(F.keys[i], g, &cx, &cy);
     const float2 xi = F.x[i];
     const float thr = P.thr;
-    for_each_wall(W, g, P.search_radius, cx, cy, xi.x, xi.y, thr, [&](int b, float2 xb) {
+    const auto wall = [&](int b, float2 xb, float area) {
       const Geo e = geo(xb.x, xb.y, xi.x, xi.y, P.inv_h);
-      rw += kW(e.q, P.c_w) * W.area[b];
+      rw += kW(e.q, P.c_w) * area;
       if (kCells) out.add(b);
-    });
+    };
+    if constexpr (kCells) {   // the walls of a row tested together: the particles beside walls end last
+      struct At {
+        int b;
+        float2 x;
+        float area;
+      };
+      for_each_wall_by_four(
+          W, g, P.search_radius, cx, cy, xi.x, xi.y, thr, [&](int b) { return At{b, __ldg(W.x + b), __ldg(W.area + b)}; },
+          [&](const At& a) { wall(a.b, a.x, a.area); });
+    } else {
+      for_each_wall(W, g, P.search_radius, cx, cy, xi.x, xi.y, thr, [&](int b, float2 xb) { wall(b, xb, W.area[b]); });
+    }
   }
   if constexpr (kCells) {
     out.fill_up(-1);
