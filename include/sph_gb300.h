@@ -754,25 +754,27 @@ sph_status_t sph_drop_adjoint(int32_t fp64, int64_t n, const int32_t* offsets, c
                               const void* lx1, const void* lv1, const void* lr1, void* lx0, void* lv0, void* lr0,
                               void* dalpha, void* stream);
 
-/* The same rollout without host waits: each step's search writes row offsets [n+1] and int32
- * columns (original order) into buffers of a given capacity; a row past it is left unwritten,
- * flags SPH_FLAG_PAIR_CAPACITY and reads as empty.  Rows come in cell order, or increasing when
- * `unsorted` gives a second column buffer to sort from.  pair_capacity > 0.  grid:
+/* The same rollout without host waits: each step's search writes the columns (original order) of
+ * particle i to the row_capacity slots of row i and their number to counts[i]; a row that does
+ * not fit is left empty and flags SPH_FLAG_PAIR_CAPACITY.  Rows come in cell order, or (ordered)
+ * increasing; with more than 512 slots that needs `unordered`, a second array of columns.  grid:
  * sph_grid_build with the domain given, so that it holds for every step.  scratch:
  * sph_drop_search_scratch_bytes(n, cell_capacity), zeroed once before the first call. */
 size_t sph_drop_search_scratch_bytes(int64_t n, int32_t cell_capacity);
 sph_status_t sph_drop_search(const float* x32, const float* support, int64_t n, const sph_grid* grid,
-                             int32_t cell_capacity, int32_t* offsets, int64_t pair_capacity, int32_t* cols,
-                             int32_t* unsorted, int32_t* status, void* scratch, size_t scratch_bytes, void* stream);
+                             int32_t cell_capacity, int32_t* counts, int32_t row_capacity, int32_t* cols,
+                             int32_t ordered, int32_t* unordered, int32_t* status, void* scratch, size_t scratch_bytes,
+                             void* stream);
 /* sph_drop_rhs and sph_drop_integrate in one launch, to other arrays than the state's, with the
- * new positions in float32 (x32_out, may be NULL) for the next search. */
-sph_status_t sph_drop_step(int32_t fp64, int64_t n, const int32_t* offsets, const int32_t* cols,
-                           int64_t pair_capacity, const void* x, const void* v, const void* rho, const void* area,
+ * new positions in float32 (x32_out, may be NULL) for the next search.  row_info: the counts of
+ * sph_drop_search, or with row_capacity 0 the offsets [n+1] of a CSR list. */
+sph_status_t sph_drop_step(int32_t fp64, int64_t n, const int32_t* row_info, const int32_t* cols,
+                           int32_t row_capacity, const void* x, const void* v, const void* rho, const void* area,
                            const sph_params* params, double dt, void* x_out, void* v_out, void* rho_out, float* x32_out,
                            void* stream);
-/* sph_drop_adjoint over the pairs of sph_drop_search, with the step's shares added to dalpha. */
-sph_status_t sph_drop_adjoint_step(int32_t fp64, int64_t n, const int32_t* offsets, const int32_t* cols,
-                                   int64_t pair_capacity, const void* x, const void* v, const void* rho,
+/* sph_drop_adjoint over the pairs of sph_drop_step, with the step's shares added to dalpha. */
+sph_status_t sph_drop_adjoint_step(int32_t fp64, int64_t n, const int32_t* row_info, const int32_t* cols,
+                                   int32_t row_capacity, const void* x, const void* v, const void* rho,
                                    const void* area, const sph_params* params, double dt, const void* lx1,
                                    const void* lv1, const void* lr1, void* lx0, void* lv0, void* lr0, void* dalpha,
                                    void* stream);

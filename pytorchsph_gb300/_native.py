@@ -127,9 +127,9 @@ SIGNATURES.update({  # simulation kernels
     "sph_permute": (_I32, [_P, _I64, _I32] + [_P] * 3),
     "sph_permute_arrays": (_I32, [_P, _I64, _I32, _P, _P, _P, _P]),
     "sph_drop_search_scratch_bytes": (_SZ, [_I64, _I32]),
-    "sph_drop_search": (_I32, [_P, _P, _I64, _P, _I32, _P, _I64, _P, _P, _P, _P, _SZ, _P]),
-    "sph_drop_step": (_I32, [_I32, _I64, _P, _P, _I64, _P, _P, _P, _P, _P, _F64] + [_P] * 5),
-    "sph_drop_adjoint_step": (_I32, [_I32, _I64, _P, _P, _I64, _P, _P, _P, _P, _P, _F64] + [_P] * 8),
+    "sph_drop_search": (_I32, [_P, _P, _I64, _P, _I32, _P, _I32, _P, _I32, _P, _P, _P, _SZ, _P]),
+    "sph_drop_step": (_I32, [_I32, _I64, _P, _P, _I32, _P, _P, _P, _P, _P, _F64] + [_P] * 5),
+    "sph_drop_adjoint_step": (_I32, [_I32, _I64, _P, _P, _I32, _P, _P, _P, _P, _P, _F64] + [_P] * 8),
     "sph_dfsph_partials_count": (_SZ, []),
     "sph_dfsph_records_count": (_SZ, [_I64, _I64, _I32]),
     "sph_dfsph_wall_wall_term": (_I32, [_P] * 5),

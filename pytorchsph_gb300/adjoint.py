@@ -13,7 +13,7 @@ does.  `DropRollout.pairs` and `step` work on the reference's own (i, j)-ordered
 
 Gradients are with respect to the initial velocity field and the artificial viscosity alpha.
 `DropRolloutFunction` puts the rollout behind torch.autograd: its forward records every
-step's neighbor list and state (a seventh of the list's memory), and its backward runs the
+step's neighbor list and state (a tenth of the list's memory), and its backward runs the
 adjoint kernels backwards over them.
 """
 from __future__ import annotations
@@ -64,10 +64,10 @@ class DropRollout:
         self.acc = torch.empty((self.n, 2), dtype=self.dtype, device=self.dev)
         self.dpdt = torch.empty(self.n, dtype=self.dtype, device=self.dev)
         self.steps_run = 0
-        # pairs of a step: a support's area over a particle's, a quarter more for denser packing
+        # slots of a row: a support's area over a particle's, a quarter more for denser packing
         a = float(np.mean(np.asarray(scene["area"], np.float64)))
         per = np.pi * self.h * self.h / a if a > 0 else 32.0
-        self._pair_cap = int(self.n * min(max(1.25 * per + 8.0, 16.0), 512.0)) if np.isfinite(per) else 32 * self.n
+        self._row_cap = int(min(max(1.25 * per + 8.0, 16.0), 512.0)) + 7 & ~7 if np.isfinite(per) else 32
 
     # ------------------------------------------------------------------ forward
     def pairs(self, x):
@@ -108,7 +108,7 @@ class DropRollout:
         """The state after one step with the pairs pr = (offsets, int32 columns)."""
         out = tuple(torch.empty_like(t) for t in state)
         off, cols = pr
-        N.call("sph_drop_step", int(self.fp64), self.n, N.ptr(off), N.ptr(cols), cols.shape[0], *map(N.ptr, state),
+        N.call("sph_drop_step", int(self.fp64), self.n, N.ptr(off), N.ptr(cols), 0, *map(N.ptr, state),
                N.ptr(self.area), ctypes.byref(self.P), self.dt, *map(N.ptr, out), None, N.stream_ptr())
         self.steps_run += 1
         return out
@@ -116,11 +116,11 @@ class DropRollout:
     def _forward(self, v0, alpha, steps, checkpoints=False, record=False):
         """(final state, checkpoints, record of every step), the steps without host waits.
 
-        The pair buffers are sized from the particles' areas with headroom; a step that
-        overflows them has the rollout run again with twice as much.  A float32 rollout's
-        rows are put in increasing order, the order its sums are defined in.  A record holds
-        the pairs and the state of every step: the states take a seventh of the pairs' memory,
-        and the backward pass neither searches nor steps again."""
+        The rows' slots are sized from the particles' areas with headroom; a step that overflows
+        one has the rollout run again with twice as many.  A float32 rollout's rows are in
+        increasing order, the order its sums are defined in.  A record holds the pairs and the
+        state of every step: the states take a tenth of the pairs' memory, and the backward
+        pass neither searches nor steps again."""
         self.P.alpha = float(alpha)
         start = (self.x0.clone(), v0.to(self.dtype).reshape(self.n, 2).clone(memory_format=torch.contiguous_format),
                  self.rho0.clone())
@@ -135,10 +135,11 @@ class DropRollout:
                                            scratch.numel() * 8, N.ptr(x32))
         slots = steps - 1 if record else min(steps - 1, 2)   # of the states between the first and the last
         while True:
-            cap = self._pair_cap
+            cap = self._row_cap
             rows = steps if record else 1
-            offs, cols = i32(rows, n + 1), i32(rows, cap)
-            unsorted = None if self.fp64 else i32(cap)
+            counts, cols = i32(rows, n), i32(rows, n * cap)
+            # (rows that one block cannot order by itself are ordered from a second array)
+            second = None if self.fp64 or cap <= 512 else i32(n * cap)
             mid, end, ck = (new(slots, n, 2), new(slots, n, 2), new(slots, n)), tuple(map(torch.empty_like, start)), {}
             at = lambda k: [N.ptr(t) for t in start] if k == 0 else [N.ptr(t) for t in end] if k == steps else \
                 [t.data_ptr() + (k - 1) % slots * t.stride(0) * t.element_size() for t in mid]
@@ -147,23 +148,24 @@ class DropRollout:
                 if checkpoints and k % self.every == 0:
                     ck[k] = tuple(t[(k - 1) % slots].clone() for t in mid) if k else start
                 r = k if record else 0
-                off, col = offs.data_ptr() + r * (n + 1) * 4, cols.data_ptr() + r * cap * 4
-                N.call("sph_drop_search", xp, sup, n, gp, cells, off, cap, col, N.ptr(unsorted), sp, scr, scr_bytes, st)
+                num, col = counts.data_ptr() + r * n * 4, cols.data_ptr() + r * n * cap * 4
+                N.call("sph_drop_search", xp, sup, n, gp, cells, num, cap, col, int(not self.fp64), N.ptr(second), sp, scr,
+                       scr_bytes, st)
                 after = at(k + 1)
-                N.call("sph_drop_step", int(self.fp64), n, off, col, cap, *state, area, P, self.dt, *after, xp, st)
+                N.call("sph_drop_step", int(self.fp64), n, num, col, cap, *state, area, P, self.dt, *after, xp, st)
                 state = after
             self.steps_run += steps
             flags = int(status.item())
             if not flags & N.SPH_FLAG_PAIR_CAPACITY:
                 break
-            if cap >= 2**31 - 1:
+            if cap >= n:
                 raise N.SPHError(f"neighbor search: {N.decode_flags(flags)}")
-            self._pair_cap = min(2 * cap, 2**31 - 1)
+            self._row_cap = min(2 * cap, n)
             status.zero_()
             x32.copy_(self.x0)
         if flags:
             raise N.SPHError(f"neighbor search: {N.decode_flags(flags)}")
-        return end, ck, (start, mid, offs, cols) if record else None
+        return end, ck, (start, mid, counts, cols, cap) if record else None
 
     def rollout(self, v0, alpha, steps, checkpoints=False, record_pairs=False):
         """Final positions after `steps` steps from (x0, v0, rho0) and the checkpoints (the states
@@ -210,7 +212,7 @@ class DropRollout:
                 if k + 1 < s1:
                     state = self._advance(state, pr)
             for (xs, vs, rs), (off, cols) in reversed(seg):
-                N.call("sph_drop_adjoint_step", int(self.fp64), self.n, N.ptr(off), N.ptr(cols), cols.shape[0],
+                N.call("sph_drop_adjoint_step", int(self.fp64), self.n, N.ptr(off), N.ptr(cols), 0,
                        N.ptr(xs), N.ptr(vs), N.ptr(rs), N.ptr(self.area), ctypes.byref(self.P), self.dt, N.ptr(lx),
                        N.ptr(lv), N.ptr(lr), N.ptr(nx), N.ptr(nv), N.ptr(nr), N.ptr(dalpha), N.stream_ptr())
                 lx, nx = nx, lx
@@ -228,11 +230,10 @@ class DropRollout:
         st, P, area, da = N.stream_ptr(), ctypes.byref(self.P), N.ptr(self.area), N.ptr(dalpha)
         a, b = [N.ptr(t) for t in cur], [N.ptr(t) for t in nxt]
         for k in reversed(range(steps)):
-            start, mid, offs, cols = record
+            start, mid, counts, cols, cap = record
             state = [t.data_ptr() + (k - 1) * t.stride(0) * t.element_size() for t in mid] if k else map(N.ptr, start)
-            cap = cols.shape[1]
-            N.call("sph_drop_adjoint_step", int(self.fp64), self.n, offs.data_ptr() + k * (self.n + 1) * 4,
-                   cols.data_ptr() + k * cap * 4, cap, *state, area, P, self.dt, *a, *b, da, st)
+            N.call("sph_drop_adjoint_step", int(self.fp64), self.n, counts.data_ptr() + k * self.n * 4,
+                   cols.data_ptr() + k * self.n * cap * 4, cap, *state, area, P, self.dt, *a, *b, da, st)
             a, b = b, a
             cur, nxt = nxt, cur
         return cur[1], dalpha.sum()

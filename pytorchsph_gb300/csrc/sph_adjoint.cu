@@ -3,8 +3,8 @@
 // semi-implicit Euler update (src/simulationBase.py:647-652), and the discrete adjoint of
 // one step in closed form.
 //
-// Pairs are row offsets + columns in original particle order; the list is symmetric because
-// every particle has the same support.  Particle i's adjoint gathers over its own row both
+// Pairs are rows of columns in original particle order (CSR, or a rollout's rows of fixed slots);
+// the list is symmetric because every particle has the same support.  Particle i's adjoint gathers over its own row both
 //   (d f_ij / d in_i)^T lambda_out_i   (its own right-hand side)   and
 //   (d f_ji / d in_i)^T lambda_out_j   (its neighbors' right-hand sides),
 // so there are no atomics and the result does not depend on thread timing.  Scalars are float
@@ -229,12 +229,19 @@ __device__ __forceinline__ bool apart(T xix, T xiy, T xjx, T xjy) {
 // ---------------------------------------------------------------- lanes
 constexpr int kDropLanes = 8;
 
-// End of a row [k0, k1) of lists with a capacity (0: none): k0 unless the row lies inside it,
-// also after a count past 2^31 (a row is shorter than that, so one of a wrapped scan's rows
-// has a negative end and is caught).
-__device__ __forceinline__ int row_end(int k0, int k1, int64_t capacity) {
-  return capacity > 0 && (k0 < 0 || k1 < k0 || (int64_t)k1 > capacity) ? k0 : k1;
-}
+// The columns of row i: a rollout's own rows of `room` slots each (row_info holds their counts), or
+// with room 0 a CSR list (row_info holds its offsets).
+template <typename Col>
+struct DropRows {
+  const int32_t* row_info;
+  const Col* cols;
+  int room;
+  __device__ __forceinline__ const Col* row(int i, int& m) const {
+    const int a = row_info[i];
+    m = room ? min(a, room) : row_info[i + 1] - a;
+    return cols + (room ? (int64_t)i * room : (int64_t)a);
+  }
+};
 
 template <typename T>
 __device__ __forceinline__ T drop_sum(T v) {
@@ -291,21 +298,21 @@ __device__ __forceinline__ bool drop_pair(double2 xi, double2 vi, double ri, dou
   return true;
 }
 
-// Sums of row i over the lanes' pairs [k0, k1) (double; pressure.py:31-38, diffusion.py:30-44,
+// Sums of row i (m columns) over the lanes' pairs (double; pressure.py:31-38, diffusion.py:30-44,
 // laminar.py:30-46 with its index choices, momentum.py:31-38, densityDiffusion.py:74-82): with
 // rho = rho0 rho~, V = A / rho~, m = rho V = rho0 A,
 //   a_i  = -1/rho_i sum (p_i + p_j) V_j gd d + alpha h c0 sum min(s, 0) m_j irs iR gd d
 //          + 8 nu rho_i sum m_j gd r2 irs^2 iR w
 //   dp_i = sum m_j gd s - 2 h delta c0 sum (rho_j - rho_i) V_j gd r2 iR
 template <typename Col>
-__device__ __forceinline__ void drop_row(int k0, int k1, int sub, const Col* __restrict__ cols, double2 xi, double2 vi,
+__device__ __forceinline__ void drop_row(int m, int sub, const Col* __restrict__ cols, double2 xi, double2 vi,
                                          double ri, const double2* __restrict__ x, const double2* __restrict__ v,
                                          const double* __restrict__ rt, const double* __restrict__ area,
                                          const DropParams<double>& P, double& ax, double& ay, double& dp) {
   using T = double;
   const T rhoi = P.rho0 * ri, pi = tait7(ri, P);
   T px = 0, py = 0, vx = 0, vy = 0, lx = 0, ly = 0, d1 = 0, d2 = 0;
-  for (int k = k0 + sub; k < k1; k += kDropLanes) {
+  for (int k = sub; k < m; k += kDropLanes) {
     const int j = (int)__ldg(cols + k);
     const T rj = rt[j], Aj = area[j];
     DropPair e;
@@ -340,16 +347,16 @@ __device__ __forceinline__ void drop_row(int k0, int k1, int sub, const Col* __r
 
 // The same sums in float, added in row order.
 template <typename Col>
-__device__ __forceinline__ void drop_row(int k0, int k1, int sub, const Col* __restrict__ cols, float2 xi, float2 vi,
+__device__ __forceinline__ void drop_row(int m, int sub, const Col* __restrict__ cols, float2 xi, float2 vi,
                                          float ri, const float2* __restrict__ x, const float2* __restrict__ v,
                                          const float* __restrict__ rt, const float* __restrict__ area,
                                          const DropParams<float>& P, float& ax, float& ay, float& dp) {
   ax = ay = dp = 0.f;
-  const int m = k1 - k0, longest = drop_longest(m);
+  const int longest = drop_longest(m);
   for (int q = 0; q < longest; q += kDropLanes) {
     float tx = 0.f, ty = 0.f, td = 0.f;   // adding 0 where a lane has no pair changes no sum's value
     if (q + sub < m) {
-      const int j = (int)__ldg(cols + k0 + q + sub);
+      const int j = (int)__ldg(cols + q + sub);
       const float2 xj = x[j], vj = v[j];
       if (apart(xi.x, xi.y, xj.x, xj.y)) {
         const PairOut<float> o =
@@ -369,8 +376,7 @@ __device__ __forceinline__ void drop_row(int k0, int k1, int sub, const Col* __r
 // ro, with the new positions in float32 in x32 (may be NULL) for the next search; else write
 // acc and dpdt.
 template <typename T, typename V2, typename Col, bool kStep>
-__global__ void __launch_bounds__(128) k_drop_rhs(int n, const int32_t* __restrict__ offsets,
-                                                  const Col* __restrict__ cols, int64_t capacity,
+__global__ void __launch_bounds__(128) k_drop_rhs(int n, DropRows<Col> rows,
                                                   const V2* __restrict__ x, const V2* __restrict__ v,
                                                   const T* __restrict__ rt, const T* __restrict__ area,
                                                   DropParams<T> P, T dt, V2* __restrict__ acc, T* __restrict__ dpdt,
@@ -382,10 +388,10 @@ __global__ void __launch_bounds__(128) k_drop_rhs(int n, const int32_t* __restri
   const int i = live ? row : n - 1;   // lanes past the last particle only take part in the sums
   const V2 xi = x[i], vi = v[i];
   const T ri = rt[i];
-  const int k0 = offsets[i];
-  const int k1 = row_end(k0, offsets[i + 1], capacity);
+  int m;
+  const Col* cols = rows.row(i, m);
   T ax, ay, dp;
-  drop_row(k0, k1, sub, cols, xi, vi, ri, x, v, rt, area, P, ax, ay, dp);
+  drop_row(m, sub, cols, xi, vi, ri, x, v, rt, area, P, ax, ay, dp);
   if (!live || sub != 0) return;
   if (P.point_source) {
     T dx = xi.x - P.cx, dy = xi.y - P.cy;
@@ -442,7 +448,7 @@ __global__ void k_drop_sie(int n, V2* __restrict__ x, V2* __restrict__ v, T* __r
 // whose gradient with respect to d, w and rho~_i is particle i's share (m does not depend on
 // rho~; d gd / d r2 = 30 c_g (1 - q)^2 / (h^2 r)).
 template <typename Col>
-__device__ __forceinline__ void adjoint_row(int i, int k0, int k1, int sub, const Col* __restrict__ cols, double2 xi,
+__device__ __forceinline__ void adjoint_row(int i, int m, int sub, const Col* __restrict__ cols, double2 xi,
                                             double2 vi, double ri, const double2* __restrict__ x,
                                             const double2* __restrict__ v, const double* __restrict__ rt,
                                             const double* __restrict__ area, const DropParams<double>& P, double dt,
@@ -457,7 +463,7 @@ __device__ __forceinline__ void adjoint_row(int i, int k0, int k1, int sub, cons
   const T av = P.alpha * P.visc_unit, nu8 = T(8) * P.nu, df = P.mog ? T(-2) * P.diff_k * P.rho0 : T(0);
   T gx = 0, gy = 0, gvx = 0, gvy = 0, gr = 0;
   da = 0;
-  for (int k = k0 + sub; k < k1; k += kDropLanes) {
+  for (int k = sub; k < m; k += kDropLanes) {
     const int j = (int)__ldg(cols + k);
     const T rj = rt[j], Aj = area[j];
     DropPair e;
@@ -513,7 +519,7 @@ __device__ __forceinline__ void adjoint_row(int i, int k0, int k1, int sub, cons
 // The same sums in float by dual numbers, added in row order: of each pair the own row's share,
 // then the neighbor row's.
 template <typename Col>
-__device__ __forceinline__ void adjoint_row(int i, int k0, int k1, int sub, const Col* __restrict__ cols, float2 xi,
+__device__ __forceinline__ void adjoint_row(int i, int m, int sub, const Col* __restrict__ cols, float2 xi,
                                             float2 vi, float ri, const float2* __restrict__ x,
                                             const float2* __restrict__ v, const float* __restrict__ rt,
                                             const float* __restrict__ area, const DropParams<float>& P, float dt,
@@ -537,11 +543,11 @@ __device__ __forceinline__ void adjoint_row(int i, int k0, int k1, int sub, cons
 #pragma unroll
   for (int c = 0; c < 5; ++c) g[c] = 0.f;
   da = 0.f;
-  const int m = k1 - k0, longest = drop_longest(m);
+  const int longest = drop_longest(m);
   for (int q = 0; q < longest; q += kDropLanes) {
     T own[5] = {0, 0, 0, 0, 0}, other[5] = {0, 0, 0, 0, 0}, ta = 0;
     if (q + sub < m) {
-      const int j = (int)__ldg(cols + k0 + q + sub);
+      const int j = (int)__ldg(cols + q + sub);
       const float2 xj = x[j], vj = v[j];
       if (apart(xi.x, xi.y, xj.x, xj.y)) {
         const T rj = rt[j];
@@ -577,8 +583,7 @@ __device__ __forceinline__ void adjoint_row(int i, int k0, int k1, int sub, cons
 // One step of the adjoint: from (lx', lv', lr') of step k+1 and the state of step k, the
 // adjoint of step k and particle i's share of dL/d alpha (added to dalpha when accumulate).
 template <typename T, typename V2, typename Col>
-__global__ void __launch_bounds__(128) k_drop_adjoint(int n, const int32_t* __restrict__ offsets,
-                                                      const Col* __restrict__ cols, int64_t capacity,
+__global__ void __launch_bounds__(128) k_drop_adjoint(int n, DropRows<Col> rows,
                                                       const V2* __restrict__ x, const V2* __restrict__ v,
                                                       const T* __restrict__ rt, const T* __restrict__ area,
                                                       DropParams<T> P, T dt, const V2* __restrict__ lx1,
@@ -595,10 +600,10 @@ __global__ void __launch_bounds__(128) k_drop_adjoint(int n, const int32_t* __re
   // lambda of row i's outputs: acc via v' = v + dt a and x' = x + dt v + dt^2 a; dpdt via rho'
   const V2 lxi1 = lx1[i], lvi1 = lv1[i];
   const T lax = dt * lvi1.x + dt2 * lxi1.x, lay = dt * lvi1.y + dt2 * lxi1.y, ld = sdp * lr1[i];
-  const int k0 = offsets[i];
-  const int k1 = row_end(k0, offsets[i + 1], capacity);
+  int m;
+  const Col* cols = rows.row(i, m);
   T g[5], da;
-  adjoint_row(i, k0, k1, sub, cols, xi, vi, ri, x, v, rt, area, P, dt, lx1, lv1, lr1, lax, lay, ld, g, da);
+  adjoint_row(i, m, sub, cols, xi, vi, ri, x, v, rt, area, P, dt, lx1, lv1, lr1, lax, lay, ld, g, da);
   if (!live || sub != 0) return;
   if (P.point_source) {  // a = -mag (x - c) away from the centre
     const T dx = xi.x - P.cx, dy = xi.y - P.cy;
@@ -619,70 +624,95 @@ __global__ void __launch_bounds__(128) k_drop_adjoint(int n, const int32_t* __re
 }
 
 // ---------------------------------------------------------------- pairs of one step
-// Row counts (kFill = false) or columns of the particles in cell-sorted order, kDropLanes lanes per
-// particle: the candidates are walked as one range per three cell rows, and a lane's hits
-// are placed by the group's ballot, so a row comes in cell order whatever the timing.
-template <bool kFill>
-__global__ void __launch_bounds__(128) k_drop_pairs(const float2* __restrict__ xs, const float* __restrict__ support,
-                                                    int n, const uint32_t* __restrict__ keys,
-                                                    const int32_t* __restrict__ cell_start,
-                                                    const sph_grid* __restrict__ gp, int32_t cap,
-                                                    const uint32_t* __restrict__ order, int32_t* __restrict__ counts,
-                                                    const int32_t* __restrict__ offsets, int64_t capacity,
-                                                    int32_t* __restrict__ cols, int32_t* status) {
-  const int s = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kDropLanes);
-  const int sub = threadIdx.x % kDropLanes;
-  if (s >= n) return;   // the lanes of one particle leave together
-  const unsigned group = ((1u << kDropLanes) - 1u) << ((threadIdx.x & 31) - sub);
-  const unsigned below = ((1u << (threadIdx.x & 31)) - 1u) & group;
+// The columns of the particles in cell-sorted order, kDropLanes lanes per particle, into rows of
+// `room` slots: no count, no scan and no second test of the candidates (with those and a launch
+// of its own for the order a search took 25 us more than its sort at 16,173 particles, this
+// one 8).  The candidates are walked as one range per three cell rows, and a lane's hits are placed by the group's ballot, so a row
+// comes in cell order whatever the timing.  kOrdered: through shared memory in increasing
+// order, a column's place the number of the row's columns below it.  A row with more
+// columns than slots is left empty and flags SPH_FLAG_PAIR_CAPACITY.
+constexpr int kDropBlock = 128, kDropBlockRows = kDropBlock / kDropLanes;
+constexpr int kDropOrderedRoom = 512;   // slots up to which a block's rows fit in shared memory
+
+template <bool kOrdered>
+__global__ void __launch_bounds__(kDropBlock) k_drop_pairs(const float2* __restrict__ xs,
+                                                           const float* __restrict__ support, int n,
+                                                           const uint32_t* __restrict__ keys,
+                                                           const int32_t* __restrict__ cell_start,
+                                                           const sph_grid* __restrict__ gp, int32_t cap,
+                                                           const uint32_t* __restrict__ order, int room,
+                                                           int32_t* __restrict__ counts, int32_t* __restrict__ cols,
+                                                           int32_t* status) {
+  extern __shared__ int32_t drop_stage[];   // kOrdered: kDropBlockRows rows of room + 1
+  const int64_t particle = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kDropLanes;
+  const bool live = particle < n;   // lanes past the last particle take part in the warp's votes
+  const int s = live ? (int)particle : n - 1;
+  const int lane = threadIdx.x & 31, sub = lane % kDropLanes, base = lane - sub;
   const sph_grid g = *gp;
   const uint32_t key = keys[s];
   const int i = (int)order[s];
-  int found = 0;
-  int32_t* row_cols = nullptr;
-  if constexpr (kFill) {
-    const int k0 = offsets[i], k1 = offsets[i + 1];
-    if (k0 < 0 || k1 < k0 || (int64_t)k1 > capacity) {
-      if (sub == 0) flag(status, SPH_FLAG_PAIR_CAPACITY);
-      return;
-    }
-    row_cols = cols + k0;
-  }
-  if (grid_ok(g, cap) && key < (uint32_t)g.num_cells) {
-    const float2 xi = xs[s];
-    const float thr = grid_threshold(support[i], g);
+  int32_t* const out = cols + (int64_t)i * room;
+  int32_t* const row = kOrdered ? drop_stage + (threadIdx.x / kDropLanes) * (room + 1) : out;
+  const float2 xi = xs[s];
+  const float thr = grid_threshold(support[i], g);
+  int b[3] = {}, n0 = 0, n1 = 0, n2 = 0;   // the cell rows' first candidates, and candidates up to each one's end
+  if (live && grid_ok(g, cap) && key < (uint32_t)g.num_cells) {
     const int cx = (int)(key % (uint32_t)g.cells_x), cy = (int)(key / (uint32_t)g.cells_x);
     const int x0 = max(cx - 1, 0), x1 = min(cx + 1, g.cells_x - 1);
     const int y0 = max(cy - 1, 0), y1 = min(cy + 1, g.cells_y - 1);
-    int b[3], e[3];
+    int e[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      const int32_t* row = cell_start + (int64_t)min(y0 + q, y1) * g.cells_x;
-      b[q] = __ldg(row + x0);
-      e[q] = y0 + q <= y1 ? __ldg(row + x1 + 1) : b[q];
+      const int32_t* first = cell_start + (int64_t)min(y0 + q, y1) * g.cells_x;
+      b[q] = __ldg(first + x0);
+      e[q] = y0 + q <= y1 ? __ldg(first + x1 + 1) : b[q];
     }
-    const int n0 = e[0] - b[0], n1 = n0 + e[1] - b[1], n2 = n1 + e[2] - b[2];
-    for (int t0 = 0; t0 < n2; t0 += kDropLanes) {
-      const int t = t0 + sub;
-      const int j = t < n0 ? b[0] + t : t < n1 ? b[1] + t - n0 : b[2] + t - n1;
-      bool hit = false;
-      if (t < n2) {
-        const float2 xj = __ldg(xs + j);
-        hit = dist2_ref(xi.x, xi.y, xj.x, xj.y) <= thr;
-      }
-      if constexpr (kFill) {
-        const unsigned m = __ballot_sync(group, hit);
-        if (hit) row_cols[found + __popc(m & below)] = (int32_t)order[j];
-        found += __popc(m);
-      } else {
-        found += hit;
-      }
-    }
+    n0 = e[0] - b[0];
+    n1 = n0 + e[1] - b[1];
+    n2 = n1 + e[2] - b[2];
   }
-  if constexpr (!kFill) {
+  int found = 0;
+  const int longest = __reduce_max_sync(0xffffffffu, n2);
+  for (int t0 = 0; t0 < longest; t0 += kDropLanes) {
+    const int t = t0 + sub;
+    const int j = t < n0 ? b[0] + t : t < n1 ? b[1] + t - n0 : b[2] + t - n1;
+    bool hit = false;
+    if (t < n2) {
+      const float2 xj = __ldg(xs + j);
+      hit = dist2_ref(xi.x, xi.y, xj.x, xj.y) <= thr;
+    }
+    const unsigned hits = __ballot_sync(0xffffffffu, hit) >> base & ((1u << kDropLanes) - 1u);
+    const int at = found + __popc(hits & ((1u << sub) - 1u));
+    if (hit && at < room) row[at] = (int32_t)order[j];
+    found += __popc(hits);
+  }
+  if (found > room) {
+    if (sub == 0) flag(status, SPH_FLAG_PAIR_CAPACITY);
+    found = 0;
+  }
+  if (live && sub == 0) counts[i] = found;
+  if constexpr (kOrdered) {
+    constexpr int kKeep = 4;   // columns a lane places at a time
+    const int most = __reduce_max_sync(0xffffffffu, found);
+    __syncwarp();
+    for (int t0 = 0; t0 < most; t0 += kKeep * kDropLanes) {
+      int32_t v[kKeep];
+      int place[kKeep] = {};
 #pragma unroll
-    for (int o = 1; o < kDropLanes; o <<= 1) found += __shfl_xor_sync(group, found, o);
-    if (sub == 0) counts[i] = found;
+      for (int q = 0; q < kKeep; ++q) {
+        const int t = t0 + q * kDropLanes + sub;
+        v[q] = t < found ? row[t] : 0x7fffffff;
+      }
+#pragma unroll 4
+      for (int u = 0; u < most; ++u) {
+        const int32_t c = u < found ? row[u] : 0x7fffffff;
+#pragma unroll
+        for (int q = 0; q < kKeep; ++q) place[q] += c < v[q];
+      }
+#pragma unroll
+      for (int q = 0; q < kKeep; ++q)
+        if (t0 + q * kDropLanes + sub < found) out[place[q]] = v[q];
+    }
   }
 }
 
@@ -709,25 +739,25 @@ DropParams<T> drop_params(const sph_params* p, int mog) {
   return P;
 }
 
-// The columns of every row in increasing order, in -> out (distinct columns; rows past the
-// capacity are left out): one warp per row, a column's place the number of the row's columns
-// below it, counted over the warp's registers.
-__global__ void __launch_bounds__(256) k_sort_rows(int n, const int32_t* __restrict__ offsets, int64_t capacity,
-                                                   const int32_t* __restrict__ in, int32_t* __restrict__ out) {
+// The columns of every row in increasing order, in -> out (distinct columns): one warp per row, for
+// rows of more slots than shared memory takes.
+__global__ void __launch_bounds__(256) k_order_rows(int n, int room, const int32_t* __restrict__ counts,
+                                                    const int32_t* __restrict__ in, int32_t* __restrict__ out) {
   const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (i >= n) return;
-  const int b = offsets[i], m = row_end(b, offsets[i + 1], capacity) - b;
+  const int m = min(counts[i], room);
+  const int32_t* const row = in + (int64_t)i * room;
   for (int t0 = 0; t0 < m; t0 += 32) {
     const int t = t0 + lane;
-    const int j = t < m ? __ldg(in + b + t) : 0x7fffffff;
+    const int j = t < m ? __ldg(row + t) : 0x7fffffff;
     int r = 0;
     for (int u0 = 0; u0 < m; u0 += 32) {
       const int u = u0 + lane;
-      const int ju = u0 == t0 ? j : u < m ? __ldg(in + b + u) : 0x7fffffff;
+      const int ju = u0 == t0 ? j : u < m ? __ldg(row + u) : 0x7fffffff;
       const int len = min(m - u0, 32);
       for (int k = 0; k < len; ++k) r += __shfl_sync(0xffffffffu, ju, k) < j;
     }
-    if (t < m) out[b + r] = j;
+    if (t < m) out[(int64_t)i * room + r] = j;
   }
 }
 
@@ -736,42 +766,42 @@ __global__ void __launch_bounds__(256) k_sort_rows(int n, const int32_t* __restr
 using namespace sph;
 
 template <typename Col, bool kStep>
-static void launch_rhs(int32_t fp64, int64_t n, const int32_t* offsets, const Col* cols, int64_t capacity,
-                       const void* x, const void* v, const void* rho, const void* area, const sph_params* params,
+static void launch_rhs(int32_t fp64, int64_t n, const DropRows<Col>& rows, const void* x, const void* v,
+                       const void* rho, const void* area, const sph_params* params,
                        double dt, void* acc, void* dpdt, void* xo, void* vo, void* ro, float* x32, cudaStream_t st) {
   const int mog = params->density_diffusion == 1;
   const int nb = grid_for(n * kDropLanes, 128);
   if (fp64)
     k_drop_rhs<double, double2, Col, kStep><<<nb, 128, 0, st>>>(
-        (int)n, offsets, cols, capacity, static_cast<const double2*>(x), static_cast<const double2*>(v),
+        (int)n, rows, static_cast<const double2*>(x), static_cast<const double2*>(v),
         static_cast<const double*>(rho), static_cast<const double*>(area), drop_params<double>(params, mog), dt,
         static_cast<double2*>(acc), static_cast<double*>(dpdt), static_cast<double2*>(xo), static_cast<double2*>(vo),
         static_cast<double*>(ro), reinterpret_cast<float2*>(x32));
   else
     k_drop_rhs<float, float2, Col, kStep><<<nb, 128, 0, st>>>(
-        (int)n, offsets, cols, capacity, static_cast<const float2*>(x), static_cast<const float2*>(v),
+        (int)n, rows, static_cast<const float2*>(x), static_cast<const float2*>(v),
         static_cast<const float*>(rho), static_cast<const float*>(area), drop_params<float>(params, mog), (float)dt,
         static_cast<float2*>(acc), static_cast<float*>(dpdt), static_cast<float2*>(xo), static_cast<float2*>(vo),
         static_cast<float*>(ro), reinterpret_cast<float2*>(x32));
 }
 
 template <typename Col>
-static void launch_adjoint(int32_t fp64, int64_t n, const int32_t* offsets, const Col* cols, int64_t capacity,
-                           const void* x, const void* v, const void* rho, const void* area, const sph_params* params,
+static void launch_adjoint(int32_t fp64, int64_t n, const DropRows<Col>& rows, const void* x, const void* v,
+                           const void* rho, const void* area, const sph_params* params,
                            double dt, const void* lx1, const void* lv1, const void* lr1, void* lx0, void* lv0,
                            void* lr0, void* dalpha, int accumulate, cudaStream_t st) {
   const int mog = params->density_diffusion == 1;
   const int nb = grid_for(n * kDropLanes, 128);
   if (fp64)
     k_drop_adjoint<double, double2, Col><<<nb, 128, 0, st>>>(
-        (int)n, offsets, cols, capacity, static_cast<const double2*>(x), static_cast<const double2*>(v),
+        (int)n, rows, static_cast<const double2*>(x), static_cast<const double2*>(v),
         static_cast<const double*>(rho), static_cast<const double*>(area), drop_params<double>(params, mog), dt,
         static_cast<const double2*>(lx1), static_cast<const double2*>(lv1), static_cast<const double*>(lr1),
         static_cast<double2*>(lx0), static_cast<double2*>(lv0), static_cast<double*>(lr0),
         static_cast<double*>(dalpha), accumulate);
   else
     k_drop_adjoint<float, float2, Col><<<nb, 128, 0, st>>>(
-        (int)n, offsets, cols, capacity, static_cast<const float2*>(x), static_cast<const float2*>(v),
+        (int)n, rows, static_cast<const float2*>(x), static_cast<const float2*>(v),
         static_cast<const float*>(rho), static_cast<const float*>(area), drop_params<float>(params, mog), (float)dt,
         static_cast<const float2*>(lx1), static_cast<const float2*>(lv1), static_cast<const float*>(lr1),
         static_cast<float2*>(lx0), static_cast<float2*>(lv0), static_cast<float*>(lr0), static_cast<float*>(dalpha),
@@ -779,14 +809,13 @@ static void launch_adjoint(int32_t fp64, int64_t n, const int32_t* offsets, cons
 }
 
 // The scratch of sph_drop_search, in order: cell_count [cap + 1] (zero between calls), cell_start
-// [cap + 2], keys, order, sorted keys, counts [n], sorted positions float2 [n], the sort's and
-// the scan's scratch.
+// [cap + 2], keys, order, sorted keys [n], sorted positions float2 [n], the sort's scratch.
 struct DropScratch {
-  int32_t *cell_count, *cell_start, *counts;
+  int32_t *cell_count, *cell_start;
   uint32_t *keys, *order, *skeys;
   float* xs;
-  void *sort, *scan;
-  size_t sort_bytes, scan_bytes;
+  void* sort;
+  size_t sort_bytes;
 };
 
 static size_t drop_scratch(int64_t n, int32_t cap, char* base, DropScratch* s) {
@@ -802,12 +831,9 @@ static size_t drop_scratch(int64_t n, int32_t cap, char* base, DropScratch* s) {
   d.keys = reinterpret_cast<uint32_t*>(take((size_t)n * 4));
   d.order = reinterpret_cast<uint32_t*>(take((size_t)n * 4));
   d.skeys = reinterpret_cast<uint32_t*>(take((size_t)n * 4));
-  d.counts = reinterpret_cast<int32_t*>(take((size_t)n * 4));
   d.xs = reinterpret_cast<float*>(take((size_t)n * 8));
   d.sort_bytes = sph_counting_sort_scratch_bytes(n, cap);
   d.sort = take(d.sort_bytes);
-  d.scan_bytes = sph_scan_scratch_bytes(n);
-  d.scan = take(d.scan_bytes);
   if (s) *s = d;
   return at;
 }
@@ -823,24 +849,22 @@ size_t sph_drop_search_scratch_bytes(int64_t n, int32_t cell_capacity) {
 }
 
 sph_status_t sph_drop_search(const float* x32, const float* support, int64_t n, const sph_grid* grid,
-                             int32_t cell_capacity, int32_t* offsets, int64_t pair_capacity, int32_t* cols,
-                             int32_t* unsorted, int32_t* status, void* scratch, size_t scratch_bytes, void* stream) {
-  SPH_REQUIRE(n >= 0 && n < (1LL << 31) && cell_capacity > 0 && grid && offsets && status && pair_capacity >= 0 &&
-                  (n == 0 || (x32 && support && cols && pair_capacity > 0 && unsorted != cols)),
+                             int32_t cell_capacity, int32_t* counts, int32_t row_capacity, int32_t* cols,
+                             int32_t ordered, int32_t* unordered, int32_t* status, void* scratch, size_t scratch_bytes,
+                             void* stream) {
+  SPH_REQUIRE(n >= 0 && n < (1LL << 31) && cell_capacity > 0 && grid && status && row_capacity > 0 &&
+                  (n == 0 || (x32 && support && cols && counts)) &&
+                  (!ordered || row_capacity <= kDropOrderedRoom || (unordered && unordered != cols)),
               "drop_search: bad arguments");
   if (!scratch || scratch_bytes < sph_drop_search_scratch_bytes(n, cell_capacity)) {
     set_error_text("drop_search: scratch smaller than sph_drop_search_scratch_bytes(n, cell_capacity)");
     return SPH_ERR_SCRATCH_TOO_SMALL;
   }
+  if (n == 0) return SPH_OK;
   cudaStream_t st = as_stream(stream);
   DropScratch d;
-  drop_scratch(n, cell_capacity, reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(scratch) + 255) & ~(uintptr_t)255),
-               &d);
-  if (n == 0) {
-    cudaMemsetAsync(offsets, 0, sizeof(int32_t), st);
-    SPH_CHECK_LAUNCH("drop_search");
-    return SPH_OK;
-  }
+  char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(scratch) + 255) & ~(uintptr_t)255);
+  drop_scratch(n, cell_capacity, base, &d);
   sph_status_t r = sph_cell_keys(x32, n, grid, cell_capacity, d.keys, nullptr, d.cell_count, status, stream);
   if (r != SPH_OK) return r;
   const int32_t eb[1] = {8};
@@ -849,48 +873,50 @@ sph_status_t sph_drop_search(const float* x32, const float* support, int64_t n, 
   r = sph_counting_sort_permute(d.keys, n, cell_capacity, d.cell_count, d.cell_start, nullptr, d.order, d.skeys, 1, eb,
                                 in, out, status, d.sort, d.sort_bytes, stream);
   if (r != SPH_OK) return r;
-  const int nb = grid_for(n * kDropLanes, 128);
+  const int nb = grid_for(n * kDropLanes, kDropBlock);
   const float2* xs = reinterpret_cast<const float2*>(d.xs);
-  k_drop_pairs<false><<<nb, 128, 0, st>>>(xs, support, (int)n, d.skeys, d.cell_start, grid, cell_capacity, d.order,
-                                          d.counts, nullptr, 0, nullptr, status);
-  SPH_CHECK_LAUNCH("drop_search(count)");
-  r = sph_exclusive_scan_i32(d.counts, offsets, n, d.scan, d.scan_bytes, stream);
-  if (r != SPH_OK) return r;
-  k_drop_pairs<true><<<nb, 128, 0, st>>>(xs, support, (int)n, d.skeys, d.cell_start, grid, cell_capacity, d.order,
-                                         nullptr, offsets, pair_capacity, unsorted ? unsorted : cols, status);
-  if (unsorted) k_sort_rows<<<grid_for(n, 8), 256, 0, st>>>((int)n, offsets, pair_capacity, unsorted, cols);
-  SPH_CHECK_LAUNCH("drop_search(fill)");
+  const bool in_block = ordered && row_capacity <= kDropOrderedRoom;
+  if (in_block)
+    k_drop_pairs<true><<<nb, kDropBlock, kDropBlockRows * (row_capacity + 1) * sizeof(int32_t), st>>>(
+        xs, support, (int)n, d.skeys, d.cell_start, grid, cell_capacity, d.order, row_capacity, counts, cols, status);
+  else
+    k_drop_pairs<false><<<nb, kDropBlock, 0, st>>>(xs, support, (int)n, d.skeys, d.cell_start, grid, cell_capacity,
+                                                   d.order, row_capacity, counts, ordered ? unordered : cols, status);
+  if (ordered && !in_block)
+    k_order_rows<<<grid_for(n, 8), 256, 0, st>>>((int)n, row_capacity, counts, unordered, cols);
+  SPH_CHECK_LAUNCH("drop_search");
   return SPH_OK;
 }
 
-sph_status_t sph_drop_step(int32_t fp64, int64_t n, const int32_t* offsets, const int32_t* cols,
-                           int64_t pair_capacity, const void* x, const void* v, const void* rho, const void* area,
+sph_status_t sph_drop_step(int32_t fp64, int64_t n, const int32_t* row_info, const int32_t* cols,
+                           int32_t row_capacity, const void* x, const void* v, const void* rho, const void* area,
                            const sph_params* params, double dt, void* x_out, void* v_out, void* rho_out, float* x32_out,
                            void* stream) {
   SPH_REQUIRE(n >= 0 && n < (1LL << 31) && SPH_DROP_PARAMS(params) && params->rest_density > 0 &&
-                  (n == 0 || (pair_capacity > 0 && offsets && cols && x && v && rho && area && x_out && v_out && rho_out)),
+                  (n == 0 || (row_capacity >= 0 && row_info && cols && x && v && rho && area && x_out && v_out &&
+                              rho_out)),
               "drop_step: bad arguments (gamma 7, MOG or no density diffusion)");
   SPH_REQUIRE(n == 0 || (x_out != x && v_out != v && rho_out != rho), "drop_step: outputs must not alias inputs");
   if (n == 0) return SPH_OK;
-  launch_rhs<int32_t, true>(fp64, n, offsets, cols, pair_capacity, x, v, rho, area, params, dt, nullptr, nullptr, x_out,
-                            v_out, rho_out, x32_out, as_stream(stream));
+  launch_rhs<int32_t, true>(fp64, n, DropRows<int32_t>{row_info, cols, row_capacity}, x, v, rho, area, params, dt,
+                            nullptr, nullptr, x_out, v_out, rho_out, x32_out, as_stream(stream));
   SPH_CHECK_LAUNCH("drop_step");
   return SPH_OK;
 }
 
-sph_status_t sph_drop_adjoint_step(int32_t fp64, int64_t n, const int32_t* offsets, const int32_t* cols,
-                                   int64_t pair_capacity, const void* x, const void* v, const void* rho,
+sph_status_t sph_drop_adjoint_step(int32_t fp64, int64_t n, const int32_t* row_info, const int32_t* cols,
+                                   int32_t row_capacity, const void* x, const void* v, const void* rho,
                                    const void* area, const sph_params* params, double dt, const void* lx1,
                                    const void* lv1, const void* lr1, void* lx0, void* lv0, void* lr0, void* dalpha,
                                    void* stream) {
   SPH_REQUIRE(n >= 0 && n < (1LL << 31) && SPH_DROP_PARAMS(params) &&
-                  (n == 0 || (pair_capacity > 0 && offsets && cols && x && v && rho && area && lx1 && lv1 && lr1 && lx0 && lv0 && lr0 &&
-                              dalpha)),
+                  (n == 0 || (row_capacity >= 0 && row_info && cols && x && v && rho && area && lx1 && lv1 && lr1 &&
+                              lx0 && lv0 && lr0 && dalpha)),
               "drop_adjoint_step: bad arguments (gamma 7, MOG or no density diffusion)");
   SPH_REQUIRE(lx0 != lx1 && lv0 != lv1 && lr0 != lr1, "drop_adjoint_step: outputs must not alias inputs");
   if (n == 0) return SPH_OK;
-  launch_adjoint(fp64, n, offsets, cols, pair_capacity, x, v, rho, area, params, dt, lx1, lv1, lr1, lx0, lv0, lr0,
-                 dalpha, 1, as_stream(stream));
+  launch_adjoint(fp64, n, DropRows<int32_t>{row_info, cols, row_capacity}, x, v, rho, area, params, dt, lx1, lv1, lr1,
+                 lx0, lv0, lr0, dalpha, 1, as_stream(stream));
   SPH_CHECK_LAUNCH("drop_adjoint_step");
   return SPH_OK;
 }
@@ -903,8 +929,8 @@ sph_status_t sph_drop_rhs(int32_t fp64, int64_t n, const int32_t* offsets, const
                   (n == 0 || (offsets && cols && x && v && rho && area && acc && dpdt)),
               "drop_rhs: bad arguments (gamma 7, MOG or no density diffusion)");
   if (n == 0) return SPH_OK;
-  launch_rhs<int64_t, false>(fp64, n, offsets, cols, 0, x, v, rho, area, params, 0.0, acc, dpdt, nullptr, nullptr,
-                             nullptr, nullptr, as_stream(stream));
+  launch_rhs<int64_t, false>(fp64, n, DropRows<int64_t>{offsets, cols, 0}, x, v, rho, area, params, 0.0, acc, dpdt,
+                             nullptr, nullptr, nullptr, nullptr, as_stream(stream));
   SPH_CHECK_LAUNCH("drop_rhs");
   return SPH_OK;
 }
@@ -938,8 +964,8 @@ sph_status_t sph_drop_adjoint(int32_t fp64, int64_t n, const int32_t* offsets, c
               "drop_adjoint: bad arguments (gamma 7, MOG or no density diffusion)");
   SPH_REQUIRE(lx0 != lx1 && lv0 != lv1 && lr0 != lr1, "drop_adjoint: outputs must not alias inputs");
   if (n == 0) return SPH_OK;
-  launch_adjoint(fp64, n, offsets, cols, 0, x, v, rho, area, params, dt, lx1, lv1, lr1, lx0, lv0, lr0, dalpha, 0,
-                 as_stream(stream));
+  launch_adjoint(fp64, n, DropRows<int64_t>{offsets, cols, 0}, x, v, rho, area, params, dt, lx1, lv1, lr1, lx0, lv0,
+                 lr0, dalpha, 0, as_stream(stream));
   SPH_CHECK_LAUNCH("drop_adjoint");
   return SPH_OK;
 }

@@ -1,6 +1,7 @@
 """A drop rollout's own neighbor lists and steps (lanes per row, rows past a capacity run
-again), against the step on the reference's (i, j)-ordered lists and, for the adjoint, against
-autograd through a dense float64 restatement of the step.
+again, rows ordered in a block or from a second array), against the step on the reference's
+(i, j)-ordered lists and, for the adjoint, against autograd through a dense float64
+restatement of the step.
 
 Tolerances.  float32 rows are summed in the same order by both, so states are equal.  float64
 rows are summed in another order: a step moves x by dt^2 a, whose terms are below 1e-2 of
@@ -55,17 +56,17 @@ def dense_rollout(sc, v, alpha, dt, steps):
 
 @pytest.mark.parametrize("n", [1, 2, 7, 9, 33, 130])
 @pytest.mark.parametrize("fp64", [True, False])
-@pytest.mark.parametrize("capacity", [None, 1])
+@pytest.mark.parametrize("capacity", [None, 1, 600])
 def test_rollout_and_adjoint(cuda, n, fp64, capacity):
     from pytorchsph_gb300.adjoint import DropRollout
     sc = blob(n, n)
     dt = 0.1 * sc["h"] / C0
     r = DropRollout(sc, C0, dt, fp64=fp64, checkpoint_every=2, device=cuda)
     if capacity:
-        r._pair_cap = capacity
+        r._row_cap = capacity
     v0 = torch.as_tensor(sc["vel"], dtype=r.dtype, device=cuda)
     xT, _ = r.rollout(v0, 0.05, STEPS)
-    assert r._pair_cap >= n
+    assert r._row_cap > 1 or n == 1
     x, v, rho = r.x0.clone(), v0.clone(), r.rho0.clone()
     for _ in range(STEPS):
         r.step(x, v, rho, 0.05)
