@@ -158,8 +158,8 @@ __global__ void __launch_bounds__(256) k_nl_fill(const float2* __restrict__ xy, 
 // tested in segments of 32 candidates (segment_mask); the non-empty segments are stored for
 // k_nl_fill_segments, the count is their bit count, and the density visits the set bits in
 // order, the order of k_nl_count, so both give the same sums.  A particle with more than
-// kSearchSegments segments gets nseg[s] = -1 and goes on the dense list, whose rows
-// k_nl_fill_dense writes one warp per particle.
+// kSearchSegments segments gets nseg[s] = -1 and goes on the dense list, whose rows the fill
+// writes one warp per particle.
 __global__ void __launch_bounds__(256) k_nl_segments(const float2* __restrict__ xy, const float* __restrict__ sh,
                                                      const float* __restrict__ sa, int64_t n,
                                                      const uint32_t* __restrict__ keys,
@@ -203,6 +203,57 @@ __global__ void __launch_bounds__(256) k_nl_segments(const float2* __restrict__ 
   if (k > kSearchSegments) dense_list[atomicAdd(dense_count, 1)] = (int32_t)s;
 }
 
+// The rows of the dense list, one warp per particle: each sweep tests 32 candidates of a
+// cell row at once, and the accepted ones are written in order through a ballot, so the row
+// goes out in coalesced stores.  A row that does not fit the column buffer is skipped with
+// SPH_FLAG_PAIR_CAPACITY set.
+struct DenseRows {
+  const float2* xy;
+  const float* sh;
+  const int32_t* cell_start;
+  int r;
+  const int32_t* list;
+  const int32_t* count;
+};
+
+__device__ __noinline__ void fill_dense_rows(const DenseRows D, const uint32_t* __restrict__ keys, const sph_grid& g,
+                                             const int32_t* __restrict__ offsets, int64_t pair_capacity,
+                                             int32_t* __restrict__ cols, int32_t* status, int nd) {
+  const int lane = threadIdx.x & 31;
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  for (int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); q < nd; q += warps) {
+    const int s = D.list[q];
+    int o = offsets[s];
+    const int end = offsets[s + 1];
+    if ((int64_t)end > pair_capacity || o < 0) {
+      if (lane == 0) flag(status, SPH_FLAG_PAIR_CAPACITY);
+      continue;
+    }
+    const uint32_t key = keys[s];
+    const float2 pi = D.xy[s];
+    const float thr = grid_threshold(D.sh[s], g);
+    const int cx = (int)(key % (uint32_t)g.cells_x), cy = (int)(key / (uint32_t)g.cells_x);
+    const int x0 = max(cx - D.r, 0), x1 = min(cx + D.r, g.cells_x - 1);
+    const int y0 = max(cy - D.r, 0), y1 = min(cy + D.r, g.cells_y - 1);
+    for (int yy = y0; yy <= y1 && x0 <= x1; ++yy) {
+      const int row = yy * g.cells_x;
+      const int b = __ldg(D.cell_start + row + x0), e = __ldg(D.cell_start + row + x1 + 1);
+      for (int c = b; c < e; c += 32) {
+        const int j = c + lane;
+        bool hit = false;
+        if (j < e) {
+          const float2 pj = __ldg(D.xy + j);
+          hit = dist2_ref(pi.x, pi.y, pj.x, pj.y) <= thr;
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, hit);
+        const int pos = o + __popc(m & ((1u << lane) - 1u));
+        if (hit && pos < end) cols[pos] = j;
+        o += __popc(m);
+      }
+    }
+  }
+}
+
 // The CSR columns from the stored segments (no pair tests), one warp per 32 rows and no block
 // barrier.  The rows of a warp are one contiguous span of cols: it is built in the warp's
 // shared stage and stored flat, in whole lines.  A span past the stage is taken in 2, 4 .. 32
@@ -212,9 +263,10 @@ __global__ void __launch_bounds__(256) k_nl_segments(const float2* __restrict__ 
 // the slots).  2^20 lattice particles (29.6 M columns): 37 µs; 1,000,003 with half of them in a
 // cluster (62 M): 99.  A stage of 8192 columns per block, and a warp per row for longer spans,
 // took 45 and 186; rows staged apart per lane and stored one by one 45 and 146.
-// A row that does not fit the column buffer is skipped with SPH_FLAG_PAIR_CAPACITY set; rows
-// of the dense list are left to k_nl_fill_dense, which runs after this kernel (a span may copy
-// placeholder entries over them first).
+// A row that does not fit the column buffer is skipped with SPH_FLAG_PAIR_CAPACITY set.  The rows of
+// the dense list are dealt to all warps at the end (a launch of their own took 2 us of every
+// search, mostly for an empty list); a warp that has one among its rows takes those one by
+// one, so that no span copies placeholders over it.
 __device__ __forceinline__ int highest_bit(uint32_t w) {
   int b;
   asm("bfind.u32 %0, %1;" : "=r"(b) : "r"(w));
@@ -230,19 +282,22 @@ __global__ void __launch_bounds__(128) k_nl_fill_segments(int64_t n, const uint3
                                                           int32_t* __restrict__ cols, int32_t* status,
                                                           const int32_t* __restrict__ nseg,
                                                           const int32_t* __restrict__ seg_start,
-                                                          const uint32_t* __restrict__ seg_mask) {
+                                                          const uint32_t* __restrict__ seg_mask,
+                                                          const DenseRows dense) {
   __shared__ __align__(16) int32_t stages[4][kRowStage + 4];
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const int64_t s0 = s - lane;
-  if (s0 >= n) return;   // the whole warp
   int32_t* const stage = stages[threadIdx.x >> 5];
   const sph_grid g = *gp;
+  const int nd = __ldg(dense.count);
   // this lane's row: first column, end, segments (none for a row that is not written)
   const int lo = offsets[min(s, n)], hi = offsets[min(s + 1, n)];
   int ns = 0;
+  bool is_dense = false;
   if (s < n && grid_ok(g, cap) && keys[s] < (uint32_t)g.num_cells) {
     ns = nseg[s];
+    is_dense = ns < 0;
     if ((int64_t)hi > pair_capacity) {
       flag(status, SPH_FLAG_PAIR_CAPACITY);
       ns = 0;
@@ -250,7 +305,7 @@ __global__ void __launch_bounds__(128) k_nl_fill_segments(int64_t n, const uint3
     if (ns < 0 || ns > kSearchSegments || lo < 0 || hi < lo || hi - lo > kRowStage) ns = 0;
   }
   // lanes per row: 1 << sh, the fewest whose passes' spans all fit
-  int sh = 0, first = lo, last = hi;
+  int sh = __any_sync(0xffffffffu, is_dense) ? 5 : 0, first = lo, last = hi;
   for (;; ++sh) {
     const int rows = 32 >> sh;
     first = __shfl_sync(0xffffffffu, lo, lane & -rows);
@@ -320,55 +375,7 @@ __global__ void __launch_bounds__(128) k_nl_fill_segments(int64_t n, const uint3
     }
     __syncwarp();
   }
-}
-
-// The rows of the dense list, one warp per particle: each sweep tests 32 candidates of a
-// cell row at once, and the accepted ones are written in order through a ballot, so the row
-// goes out in coalesced stores.  A row that does not fit the column buffer is skipped with
-// SPH_FLAG_PAIR_CAPACITY set.
-__global__ void __launch_bounds__(128) k_nl_fill_dense(const float2* __restrict__ xy, const float* __restrict__ sh,
-                                                       const uint32_t* __restrict__ keys,
-                                                       const int32_t* __restrict__ cell_start,
-                                                       const sph_grid* __restrict__ gp, int32_t cap, int r,
-                                                       const int32_t* __restrict__ offsets, int64_t pair_capacity,
-                                                       int32_t* __restrict__ cols, int32_t* status,
-                                                       const int32_t* __restrict__ dense_list,
-                                                       const int32_t* __restrict__ dense_count) {
-  const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  const int nd = *dense_count;
-  const sph_grid g = *gp;
-  for (int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); q < nd; q += warps) {
-    const int s = dense_list[q];
-    int o = offsets[s];
-    const int end = offsets[s + 1];
-    if ((int64_t)end > pair_capacity || o < 0) {
-      if (lane == 0) flag(status, SPH_FLAG_PAIR_CAPACITY);
-      continue;
-    }
-    const uint32_t key = keys[s];
-    const float2 pi = xy[s];
-    const float thr = grid_threshold(sh[s], g);
-    const int cx = (int)(key % (uint32_t)g.cells_x), cy = (int)(key / (uint32_t)g.cells_x);
-    const int x0 = max(cx - r, 0), x1 = min(cx + r, g.cells_x - 1);
-    const int y0 = max(cy - r, 0), y1 = min(cy + r, g.cells_y - 1);
-    for (int yy = y0; yy <= y1 && x0 <= x1; ++yy) {
-      const int row = yy * g.cells_x;
-      const int b = __ldg(cell_start + row + x0), e = __ldg(cell_start + row + x1 + 1);
-      for (int c = b; c < e; c += 32) {
-        const int j = c + lane;
-        bool hit = false;
-        if (j < e) {
-          const float2 pj = __ldg(xy + j);
-          hit = dist2_ref(pi.x, pi.y, pj.x, pj.y) <= thr;
-        }
-        const uint32_t m = __ballot_sync(0xffffffffu, hit);
-        const int pos = o + __popc(m & ((1u << lane) - 1u));
-        if (hit && pos < end) cols[pos] = j;
-        o += __popc(m);
-      }
-    }
-  }
+  if (nd > 0) fill_dense_rows(dense, keys, g, offsets, pair_capacity, cols, status, nd);
 }
 
 // Query points (any order, e.g. wall or ghost particles) against the sorted grid, with
@@ -679,11 +686,10 @@ sph_status_t sph_nl_fill_segments(const float* xy, const float* sorted_support, 
               "nl_fill_segments: scratch smaller than sph_nl_segments_scratch_bytes(n)");
   if (n == 0) return SPH_OK;
   cudaStream_t st = as_stream(stream);
+  const DenseRows dense{reinterpret_cast<const float2*>(xy), sorted_support, cell_start, search_radius, dense_list,
+                        dense_count};
   k_nl_fill_segments<<<grid_for(n, 128), 128, 0, st>>>(n, sorted_keys, grid, cell_capacity, offsets, pair_capacity,
-                                                       cols, status, nseg, start, mask);
-  k_nl_fill_dense<<<kNumSMs * 8, 128, 0, st>>>(reinterpret_cast<const float2*>(xy), sorted_support, sorted_keys,
-                                               cell_start, grid, cell_capacity, search_radius, offsets, pair_capacity,
-                                               cols, status, dense_list, dense_count);
+                                                       cols, status, nseg, start, mask, dense);
   SPH_CHECK_LAUNCH("nl_fill_segments");
   return SPH_OK;
 }
