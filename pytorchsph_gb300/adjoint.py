@@ -24,7 +24,7 @@ import numpy as np
 import torch
 
 from . import _native as N
-from .search import GridSearch
+from .search import MAX_CELLS, GridSearch, _f2, grid_from_words
 from .sim import SphParamsC
 
 
@@ -94,15 +94,20 @@ class DropRollout:
         self.steps_run += 1
         return off, cols
 
-    def _search_plan(self):
+    def _search_plan(self, x32):
         """A rollout's search: the grid (given domain and constant supports, so it holds for every
-        step), the cell capacity, the status word and the scratch."""
-        x32 = self.x0.to(torch.float32).contiguous()
-        cap = self.search.auto_cell_capacity(x32, self.support32, self.vmin, self.vmax)
-        grid = self.search.grid_status()[0].clone()   # the one the cells were counted on
-        status = torch.zeros(1, dtype=torch.int32, device=self.dev)
-        size = N.load().sph_drop_search_scratch_bytes(self.n, cap)
-        return grid, cap, status, torch.zeros((size + 7) // 8, dtype=torch.int64, device=self.dev)
+        step) with the status word behind it, the cell capacity and the scratch."""
+        lib, st = N.load(), N.stream_ptr()
+        words = torch.zeros(9, dtype=torch.int32, device=self.dev)
+        part = torch.empty((lib.sph_grid_scratch_bytes(self.n) + 7) // 8, dtype=torch.int64, device=self.dev)
+        N.call("sph_grid_build", N.ptr(x32), N.ptr(self.support32), self.n, _f2(self.vmin), _f2(self.vmax), MAX_CELLS,
+               N.ptr(words), N.ptr(words) + 32, N.ptr(part), part.numel() * 8, st)
+        *grid, flags = N.read_i32(words)
+        if flags:
+            raise N.SPHError(f"neighbor search: {N.decode_flags(flags)}")
+        cells = max(grid_from_words(grid)["num_cells"], 1)
+        size = lib.sph_drop_search_scratch_bytes(self.n, cells)
+        return words, cells, torch.zeros((size + 7) // 8, dtype=torch.int64, device=self.dev)
 
     def _advance(self, state, pr):
         """The state after one step with the pairs pr = (offsets, int32 columns)."""
@@ -128,10 +133,11 @@ class DropRollout:
             return start, {}, None
         n, new = self.n, lambda *shape: torch.empty(shape, dtype=self.dtype, device=self.dev)
         i32 = lambda *shape: torch.empty(shape, dtype=torch.int32, device=self.dev)
-        grid, cells, status, scratch = self._search_plan()
         x32 = self.x0.to(torch.float32, copy=True).contiguous()
+        words, cells, scratch = self._search_plan(x32)
+        status = words[8:]
         st, P, area = N.stream_ptr(), ctypes.byref(self.P), N.ptr(self.area)
-        sup, gp, sp, scr, scr_bytes, xp = (N.ptr(self.support32), N.ptr(grid), N.ptr(status), N.ptr(scratch),
+        sup, gp, sp, scr, scr_bytes, xp = (N.ptr(self.support32), N.ptr(words), N.ptr(status), N.ptr(scratch),
                                            scratch.numel() * 8, N.ptr(x32))
         slots = steps - 1 if record else min(steps - 1, 2)   # of the states between the first and the last
         while True:
