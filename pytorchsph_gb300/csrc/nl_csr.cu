@@ -474,14 +474,14 @@ __global__ void __launch_bounds__(128) k_nl_query(const float2* __restrict__ qpo
 
 // One warp per original particle i: its row of the (i, j)-ordered COO list, plus the
 // reference's fluidDistances / fluidRadialDistances (src/modules/neighborSearch.py:218-223).
-// A lane holds one pair; its place in the row is the number of the row's columns below its
-// own (they are distinct), counted over the warp's registers 32 columns at a time, so rows of
-// any length sort without scratch.  The lanes' columns are loaded, and the row's four outputs
-// stored, as contiguous pieces, where one thread per row moved every column through global
-// memory once per inversion: 558 -> 103 us for 260,017 particles, 7.2 M pairs (201 MB of
-// pairs and distances stored).  Bound by instruction issue (81 % of the slots): the count,
-// and the correctly rounded root and divisions.  Tiles in shared memory instead of shuffles
-// gave the same time.
+// A lane holds one pair.  Up to 32 columns are sorted in the lanes (bitonic; a column's sorted
+// place comes back from rank); in a longer row a column's place is the number of the row's
+// columns below it (they are distinct), counted over the warp's registers 32 columns at a
+// time.  No scratch, and the row's loads and four outputs are contiguous pieces, where one
+// thread per row moved every column through global memory once per inversion: 558 us for
+// 260,017 particles, 7.2 M pairs (201 MB of pairs and distances stored); counting in all
+// rows 103, sorting the short ones 85.  Bound by instruction issue: the sort, and the
+// correctly rounded root and divisions.
 __global__ void __launch_bounds__(256) k_nl_to_coo(const float2* __restrict__ xy, int64_t n,
                                                    const uint32_t* __restrict__ order,
                                                    const uint32_t* __restrict__ rank,
@@ -499,6 +499,37 @@ __global__ void __launch_bounds__(256) k_nl_to_coo(const float2* __restrict__ xy
   int64_t* prow = pairs;
   int64_t* pcol = pairs + P;
   const float2 pi = xy[s];
+  const auto write = [&](int64_t k, uint32_t jo, int32_t c) {
+    prow[k] = i;
+    pcol[k] = (int64_t)jo;
+    if (dist || radial) {
+      const float2 pj = __ldg(xy + c);
+      const float dx = pi.x - pj.x, dy = pi.y - pj.y;
+      const float rr = sqrtf(dx * dx + dy * dy);
+      if (dist) {
+        const float2 e = rr < thr ? make_float2(0.f, 0.f) : make_float2(dx / rr, dy / rr);
+        if ((reinterpret_cast<uintptr_t>(dist) & 7) == 0) {
+          reinterpret_cast<float2*>(dist)[k] = e;
+        } else {
+          dist[2 * k] = e.x;
+          dist[2 * k + 1] = e.y;
+        }
+      }
+      if (radial) radial[k] = rr / support;
+    }
+  };
+  if (m <= 32) {
+    uint32_t jo = lane < m ? __ldg(order + __ldg(cols + b + lane)) : 0xffffffffu;
+#pragma unroll
+    for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+      for (int d = k >> 1; d > 0; d >>= 1) {
+        const uint32_t v = __shfl_xor_sync(0xffffffffu, jo, d);
+        jo = ((lane & k) == 0) == ((lane & d) == 0) ? min(jo, v) : max(jo, v);
+      }
+    if (lane < m) write(o + lane, jo, (int32_t)__ldg(rank + jo));
+    return;
+  }
   for (int t0 = 0; t0 < m; t0 += 32) {
     const int t = t0 + lane;
     const int32_t c = t < m ? __ldg(cols + b + t) : 0;
@@ -510,24 +541,7 @@ __global__ void __launch_bounds__(256) k_nl_to_coo(const float2* __restrict__ xy
       const int len = min(m - u0, 32);
       for (int k = 0; k < len; ++k) r += __shfl_sync(0xffffffffu, ju, k) < jo;
     }
-    if (t >= m) continue;
-    prow[o + r] = i;
-    pcol[o + r] = (int64_t)jo;
-    if (dist || radial) {
-      const float2 pj = __ldg(xy + c);
-      const float dx = pi.x - pj.x, dy = pi.y - pj.y;
-      const float rr = sqrtf(dx * dx + dy * dy);
-      if (dist) {
-        const float2 e = rr < thr ? make_float2(0.f, 0.f) : make_float2(dx / rr, dy / rr);
-        if ((reinterpret_cast<uintptr_t>(dist) & 7) == 0) {
-          reinterpret_cast<float2*>(dist)[o + r] = e;
-        } else {
-          dist[2 * (o + r)] = e.x;
-          dist[2 * (o + r) + 1] = e.y;
-        }
-      }
-      if (radial) radial[o + r] = rr / support;
-    }
+    if (t < m) write(o + r, jo, c);
   }
 }
 
