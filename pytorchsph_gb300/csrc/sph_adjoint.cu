@@ -4,14 +4,15 @@
 // one step in closed form.
 //
 // Pairs are rows of columns in original particle order (CSR, or a rollout's rows of fixed slots);
-// the list is symmetric because every particle has the same support.  Particle i's adjoint gathers over its own row both
+// the list is symmetric because every particle has the same support.  Particle i's adjoint
+// gathers over its own row both
 //   (d f_ij / d in_i)^T lambda_out_i   (its own right-hand side)   and
 //   (d f_ji / d in_i)^T lambda_out_j   (its neighbors' right-hand sides),
 // so there are no atomics and the result does not depend on thread timing.  Scalars are float
 // or double.
 //
 // What bounds it: in double the FP64 pipe (two operations a clock and SM), in float a small
-// rollout's latency.  kDropLanes lanes share a row in both.
+// rollout's latency.  4 or 8 lanes share a row in both (drop_lanes).
 //   double: every quantity that both particles' terms share is formed once per pair, with one
 //     division for its three reciprocals, and the derivatives are written out (about 110
 //     operations a pair, where two sweeps of 5-component dual numbers took some 2,000).
@@ -19,8 +20,8 @@
 //     add one after another in row order: a float32 gradient with respect to alpha is a sum
 //     that cancels to 1/70 of its terms, so its rounding is kept to that of one thread per
 //     row, bit for bit.
-// At 4,173 particles in double the right-hand side takes 32 µs (one thread per row: 179) and
-// the adjoint 55 (dual numbers: 819); at 16,173 in float 8.7 (31) and 25 (40).
+// At 4,173 particles in double the right-hand side takes 26.6 µs (one thread per row: 179) and
+// the adjoint 48.5 (dual numbers: 819); at 16,173 in float 9 (31) and 21 (40).
 #include "sph_common.cuh"
 
 namespace sph {
@@ -28,7 +29,7 @@ namespace sph {
 template <typename T>
 struct DropParams {
   T inv_h, cg20;      // 1/h, 20 * 7/(pi h^3)
-  T rho0, tait_k;     // rho0 c0^2 / gamma (gamma = 7)
+  T rho0, inv_rho0, tait_k;   // tait_k = rho0 c0^2 / gamma (gamma = 7)
   T eps;              // 0.1 h^2
   T visc_unit;        // h c0 (artificial viscosity factor without alpha)
   T alpha, nu;        // artificial and laminar (kinematic) viscosity
@@ -227,7 +228,6 @@ __device__ __forceinline__ bool apart(T xix, T xiy, T xjx, T xjy) {
 }
 
 // ---------------------------------------------------------------- lanes
-constexpr int kDropLanes = 8;
 
 // The columns of row i: a rollout's own rows of `room` slots each (row_info holds their counts), or
 // with room 0 a CSR list (row_info holds its offsets).
@@ -243,19 +243,20 @@ struct DropRows {
   }
 };
 
-template <typename T>
+template <int kLanes, typename T>
 __device__ __forceinline__ T drop_sum(T v) {
 #pragma unroll
-  for (int o = 1; o < kDropLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 1; o < kLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
 // sum + the lanes' terms one after another (every lane of the group gets the result; the whole
 // warp must take part).
+template <int kLanes>
 __device__ __forceinline__ float drop_add_in_order(float sum, float term) {
 #pragma unroll
-  for (int l = 0; l < kDropLanes; ++l) {
-    const float v = __shfl_sync(0xffffffffu, term, l, kDropLanes);
+  for (int l = 0; l < kLanes; ++l) {
+    const float v = __shfl_sync(0xffffffffu, term, l, kLanes);
     sum += v;
   }
   return sum;
@@ -263,18 +264,19 @@ __device__ __forceinline__ float drop_add_in_order(float sum, float term) {
 
 // Pairs of the longest row among a warp's groups (the loops of the lanes that add in order are
 // as long in the whole warp).
+template <int kLanes>
 __device__ __forceinline__ int drop_longest(int m) {
 #pragma unroll
-  for (int o = kDropLanes; o < 32; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  for (int o = kLanes; o < 32; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
   return m;
 }
 
 // ---------------------------------------------------------------- double: closed form
 // What both rows of a pair (i, j) share, d = x_i - x_j and w = v_i - v_j: the Wendland gradient
 // gradW_ij = gd d with gd = -20 c_g (1 - q)^3 / h (kernels.py:20-33), r, s = w . d, and the
-// reciprocals of R2 = r^2 + eps, rho_i + rho_j and rho~_j (from one division).
+// reciprocals of r (one rsqrt), and of R2 = r^2 + eps, rho_i + rho_j and rho~_j (one division).
 struct DropPair {
-  double dx, dy, wx, wy, r2, r, gd, s, iR, irs, irj;
+  double dx, dy, wx, wy, r2, ir, r, gd, s, iR, irs, irj;
 };
 
 // False for a pair closer than r = 1e-7, where the reference's e_ij is zero (the particle itself).
@@ -284,7 +286,8 @@ __device__ __forceinline__ bool drop_pair(double2 xi, double2 vi, double ri, dou
   o.dy = xi.y - xj.y;
   o.r2 = o.dx * o.dx + o.dy * o.dy;
   if (!(o.r2 >= 1e-14)) return false;
-  o.r = sqrt(o.r2);
+  o.ir = rsqrt(o.r2);
+  o.r = o.r2 * o.ir;
   const double a = 1.0 - o.r * P.inv_h;
   o.gd = -(P.cg20 * P.inv_h) * (a * a * a);
   o.wx = vi.x - vj.x;
@@ -304,7 +307,7 @@ __device__ __forceinline__ bool drop_pair(double2 xi, double2 vi, double ri, dou
 //   a_i  = -1/rho_i sum (p_i + p_j) V_j gd d + alpha h c0 sum min(s, 0) m_j irs iR gd d
 //          + 8 nu rho_i sum m_j gd r2 irs^2 iR w
 //   dp_i = sum m_j gd s - 2 h delta c0 sum (rho_j - rho_i) V_j gd r2 iR
-template <typename Col>
+template <int kLanes, typename Col>
 __device__ __forceinline__ void drop_row(int m, int sub, const Col* __restrict__ cols, double2 xi, double2 vi,
                                          double ri, const double2* __restrict__ x, const double2* __restrict__ v,
                                          const double* __restrict__ rt, const double* __restrict__ area,
@@ -312,7 +315,7 @@ __device__ __forceinline__ void drop_row(int m, int sub, const Col* __restrict__
   using T = double;
   const T rhoi = P.rho0 * ri, pi = tait7(ri, P);
   T px = 0, py = 0, vx = 0, vy = 0, lx = 0, ly = 0, d1 = 0, d2 = 0;
-  for (int k = sub; k < m; k += kDropLanes) {
+  for (int k = sub; k < m; k += kLanes) {
     const int j = (int)__ldg(cols + k);
     const T rj = rt[j], Aj = area[j];
     DropPair e;
@@ -331,14 +334,14 @@ __device__ __forceinline__ void drop_row(int m, int sub, const Col* __restrict__
     d1 += mg * e.s;
     d2 += (rj - ri) * Vg * (e.r2 * e.iR);
   }
-  px = drop_sum(px);
-  py = drop_sum(py);
-  vx = drop_sum(vx);
-  vy = drop_sum(vy);
-  lx = drop_sum(lx);
-  ly = drop_sum(ly);
-  d1 = drop_sum(d1);
-  d2 = drop_sum(d2);
+  px = drop_sum<kLanes>(px);
+  py = drop_sum<kLanes>(py);
+  vx = drop_sum<kLanes>(vx);
+  vy = drop_sum<kLanes>(vy);
+  lx = drop_sum<kLanes>(lx);
+  ly = drop_sum<kLanes>(ly);
+  d1 = drop_sum<kLanes>(d1);
+  d2 = drop_sum<kLanes>(d2);
   const T fp = T(-1) / rhoi, fv = P.alpha * P.visc_unit, fl = T(8) * P.nu * rhoi;
   ax = fp * px + fv * vx + fl * lx;
   ay = fp * py + fv * vy + fl * ly;
@@ -346,14 +349,14 @@ __device__ __forceinline__ void drop_row(int m, int sub, const Col* __restrict__
 }
 
 // The same sums in float, added in row order.
-template <typename Col>
+template <int kLanes, typename Col>
 __device__ __forceinline__ void drop_row(int m, int sub, const Col* __restrict__ cols, float2 xi, float2 vi,
                                          float ri, const float2* __restrict__ x, const float2* __restrict__ v,
                                          const float* __restrict__ rt, const float* __restrict__ area,
                                          const DropParams<float>& P, float& ax, float& ay, float& dp) {
   ax = ay = dp = 0.f;
-  const int longest = drop_longest(m);
-  for (int q = 0; q < longest; q += kDropLanes) {
+  const int longest = drop_longest<kLanes>(m);
+  for (int q = 0; q < longest; q += kLanes) {
     float tx = 0.f, ty = 0.f, td = 0.f;   // adding 0 where a lane has no pair changes no sum's value
     if (q + sub < m) {
       const int j = (int)__ldg(cols + q + sub);
@@ -366,24 +369,24 @@ __device__ __forceinline__ void drop_row(int m, int sub, const Col* __restrict__
         td = o.dp;
       }
     }
-    ax = drop_add_in_order(ax, tx);
-    ay = drop_add_in_order(ay, ty);
-    dp = drop_add_in_order(dp, td);
+    ax = drop_add_in_order<kLanes>(ax, tx);
+    ay = drop_add_in_order<kLanes>(ay, ty);
+    dp = drop_add_in_order<kLanes>(dp, td);
   }
 }
 
 // Right-hand side of every particle.  kStep: advance (x, v, rho) by semi-implicit Euler into xo, vo,
 // ro, with the new positions in float32 in x32 (may be NULL) for the next search; else write
 // acc and dpdt.
-template <typename T, typename V2, typename Col, bool kStep>
+template <int kLanes, typename T, typename V2, typename Col, bool kStep>
 __global__ void __launch_bounds__(128) k_drop_rhs(int n, DropRows<Col> rows,
                                                   const V2* __restrict__ x, const V2* __restrict__ v,
                                                   const T* __restrict__ rt, const T* __restrict__ area,
                                                   DropParams<T> P, T dt, V2* __restrict__ acc, T* __restrict__ dpdt,
                                                   V2* __restrict__ xo, V2* __restrict__ vo, T* __restrict__ ro,
                                                   float2* __restrict__ x32) {
-  const int row = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kDropLanes);
-  const int sub = threadIdx.x % kDropLanes;
+  const int row = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes);
+  const int sub = threadIdx.x % kLanes;
   const bool live = row < n;
   const int i = live ? row : n - 1;   // lanes past the last particle only take part in the sums
   const V2 xi = x[i], vi = v[i];
@@ -391,7 +394,7 @@ __global__ void __launch_bounds__(128) k_drop_rhs(int n, DropRows<Col> rows,
   int m;
   const Col* cols = rows.row(i, m);
   T ax, ay, dp;
-  drop_row(m, sub, cols, xi, vi, ri, x, v, rt, area, P, ax, ay, dp);
+  drop_row<kLanes>(m, sub, cols, xi, vi, ri, x, v, rt, area, P, ax, ay, dp);
   if (!live || sub != 0) return;
   if (P.point_source) {
     T dx = xi.x - P.cx, dy = xi.y - P.cy;
@@ -447,7 +450,7 @@ __global__ void k_drop_sie(int n, V2* __restrict__ x, V2* __restrict__ v, T* __r
 //   Q3 = m_j rho_i (la.w) - m_i rho_j (lb.w),  Q4 = m_j ld + m_i le,  Q5 = V_j ld - V_i le,
 // whose gradient with respect to d, w and rho~_i is particle i's share (m does not depend on
 // rho~; d gd / d r2 = 30 c_g (1 - q)^2 / (h^2 r)).
-template <typename Col>
+template <int kLanes, typename Col>
 __device__ __forceinline__ void adjoint_row(int i, int m, int sub, const Col* __restrict__ cols, double2 xi,
                                             double2 vi, double ri, const double2* __restrict__ x,
                                             const double2* __restrict__ v, const double* __restrict__ rt,
@@ -458,12 +461,12 @@ __device__ __forceinline__ void adjoint_row(int i, int m, int sub, const Col* __
   using T = double;
   using V2 = double2;
   const T dt2 = dt * dt, sdp = dt / P.rho0;
-  const T rhoi = P.rho0 * ri, iri = T(1) / ri, Vi = area[i] * iri, mi = P.rho0 * area[i], irhoi = iri / P.rho0;
+  const T rhoi = P.rho0 * ri, iri = T(1) / ri, Vi = area[i] * iri, mi = P.rho0 * area[i], irhoi = iri * P.inv_rho0;
   const T ri2 = ri * ri, ri6 = ri2 * ri2 * ri2, pi = P.tait_k * (ri6 * ri - T(1)), dpi = T(7) * P.tait_k * ri6;
   const T av = P.alpha * P.visc_unit, nu8 = T(8) * P.nu, df = P.mog ? T(-2) * P.diff_k * P.rho0 : T(0);
   T gx = 0, gy = 0, gvx = 0, gvy = 0, gr = 0;
   da = 0;
-  for (int k = sub; k < m; k += kDropLanes) {
+  for (int k = sub; k < m; k += kLanes) {
     const int j = (int)__ldg(cols + k);
     const T rj = rt[j], Aj = area[j];
     DropPair e;
@@ -474,7 +477,7 @@ __device__ __forceinline__ void adjoint_row(int i, int m, int sub, const Col* __
     const T Pp = pi + tait7(rj, P);
     const T ea = lax * e.dx + lay * e.dy, eb = lbx * e.dx + lby * e.dy;   // la . d, lb . d
     const T fa = lax * e.wx + lay * e.wy, fb = lbx * e.wx + lby * e.wy;   // la . w, lb . w
-    const T cij = Vj * irhoi, cji = Vi * (e.irj / P.rho0);
+    const T cij = Vj * irhoi, cji = Vi * (e.irj * P.inv_rho0);
     const T Q1 = cji * eb - cij * ea;
     const T Q2 = mj * ea - mi * eb;
     const T mri = mj * rhoi, mrj = mi * rhoj;
@@ -482,7 +485,7 @@ __device__ __forceinline__ void adjoint_row(int i, int m, int sub, const Col* __
     const T Q4 = mj * ld + mi * le;
     const T Q5 = Vj * ld - Vi * le;
     const T a = T(1) - e.r * P.inv_h;
-    const T g1 = T(1.5) * P.cg20 * P.inv_h * P.inv_h * (a * a) / e.r;   // d gd / d r2
+    const T g1 = T(1.5) * P.cg20 * P.inv_h * P.inv_h * (a * a) * e.ir;   // d gd / d r2
     const T gi = e.gd * e.iR, dgi = (g1 - gi) * e.iR;                   // gd iR and its d / d r2
     const T rgi = e.r2 * gi, drgi = gi + e.r2 * dgi;                    // gd r2 iR
     const bool closing = !(e.s > T(0));
@@ -503,12 +506,12 @@ __device__ __forceinline__ void adjoint_row(int i, int m, int sub, const Col* __
           kl * rgi * (mj * P.rho0 * fa - T(2) * P.rho0 * e.irs * Q3) + df * rgi * (D * (Vi * iri) * le - Q5);
     da += P.visc_unit * gi * e.irs * s * mj * ea;
   }
-  gx = drop_sum(gx);
-  gy = drop_sum(gy);
-  gvx = drop_sum(gvx);
-  gvy = drop_sum(gvy);
-  gr = drop_sum(gr);
-  da = drop_sum(da);
+  gx = drop_sum<kLanes>(gx);
+  gy = drop_sum<kLanes>(gy);
+  gvx = drop_sum<kLanes>(gvx);
+  gvy = drop_sum<kLanes>(gvy);
+  gr = drop_sum<kLanes>(gr);
+  da = drop_sum<kLanes>(da);
   g[0] = gx;
   g[1] = gy;
   g[2] = gvx;
@@ -518,7 +521,7 @@ __device__ __forceinline__ void adjoint_row(int i, int m, int sub, const Col* __
 
 // The same sums in float by dual numbers, added in row order: of each pair the own row's share,
 // then the neighbor row's.
-template <typename Col>
+template <int kLanes, typename Col>
 __device__ __forceinline__ void adjoint_row(int i, int m, int sub, const Col* __restrict__ cols, float2 xi,
                                             float2 vi, float ri, const float2* __restrict__ x,
                                             const float2* __restrict__ v, const float* __restrict__ rt,
@@ -543,8 +546,8 @@ __device__ __forceinline__ void adjoint_row(int i, int m, int sub, const Col* __
 #pragma unroll
   for (int c = 0; c < 5; ++c) g[c] = 0.f;
   da = 0.f;
-  const int longest = drop_longest(m);
-  for (int q = 0; q < longest; q += kDropLanes) {
+  const int longest = drop_longest<kLanes>(m);
+  for (int q = 0; q < longest; q += kLanes) {
     T own[5] = {0, 0, 0, 0, 0}, other[5] = {0, 0, 0, 0, 0}, ta = 0;
     if (q + sub < m) {
       const int j = (int)__ldg(cols + q + sub);
@@ -567,22 +570,22 @@ __device__ __forceinline__ void adjoint_row(int i, int m, int sub, const Col* __
       }
     }
 #pragma unroll
-    for (int l = 0; l < kDropLanes; ++l) {
+    for (int l = 0; l < kLanes; ++l) {
 #pragma unroll
       for (int c = 0; c < 5; ++c) {
-        const T a = __shfl_sync(0xffffffffu, own[c], l, kDropLanes);
-        const T b = __shfl_sync(0xffffffffu, other[c], l, kDropLanes);
+        const T a = __shfl_sync(0xffffffffu, own[c], l, kLanes);
+        const T b = __shfl_sync(0xffffffffu, other[c], l, kLanes);
         g[c] += a;
         g[c] += b;
       }
     }
-    da = drop_add_in_order(da, ta);
+    da = drop_add_in_order<kLanes>(da, ta);
   }
 }
 
 // One step of the adjoint: from (lx', lv', lr') of step k+1 and the state of step k, the
 // adjoint of step k and particle i's share of dL/d alpha (added to dalpha when accumulate).
-template <typename T, typename V2, typename Col>
+template <int kLanes, typename T, typename V2, typename Col>
 __global__ void __launch_bounds__(128) k_drop_adjoint(int n, DropRows<Col> rows,
                                                       const V2* __restrict__ x, const V2* __restrict__ v,
                                                       const T* __restrict__ rt, const T* __restrict__ area,
@@ -590,8 +593,8 @@ __global__ void __launch_bounds__(128) k_drop_adjoint(int n, DropRows<Col> rows,
                                                       const V2* __restrict__ lv1, const T* __restrict__ lr1,
                                                       V2* __restrict__ lx0, V2* __restrict__ lv0,
                                                       T* __restrict__ lr0, T* __restrict__ dalpha, int accumulate) {
-  const int row = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kDropLanes);
-  const int sub = threadIdx.x % kDropLanes;
+  const int row = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes);
+  const int sub = threadIdx.x % kLanes;
   const bool live = row < n;
   const int i = live ? row : n - 1;
   const T dt2 = dt * dt, sdp = dt / P.rho0;
@@ -603,7 +606,7 @@ __global__ void __launch_bounds__(128) k_drop_adjoint(int n, DropRows<Col> rows,
   int m;
   const Col* cols = rows.row(i, m);
   T g[5], da;
-  adjoint_row(i, m, sub, cols, xi, vi, ri, x, v, rt, area, P, dt, lx1, lv1, lr1, lax, lay, ld, g, da);
+  adjoint_row<kLanes>(i, m, sub, cols, xi, vi, ri, x, v, rt, area, P, dt, lx1, lv1, lr1, lax, lay, ld, g, da);
   if (!live || sub != 0) return;
   if (P.point_source) {  // a = -mag (x - c) away from the centre
     const T dx = xi.x - P.cx, dy = xi.y - P.cy;
@@ -627,11 +630,12 @@ __global__ void __launch_bounds__(128) k_drop_adjoint(int n, DropRows<Col> rows,
 // The columns of the particles in cell-sorted order, kDropLanes lanes per particle, into rows of
 // `room` slots: no count, no scan and no second test of the candidates (with those and a launch
 // of its own for the order a search took 25 us more than its sort at 16,173 particles, this
-// one 8).  The candidates are walked as one range per three cell rows, and a lane's hits are placed by the group's ballot, so a row
+// one 8).  The candidates are walked as one range per three cell rows, and a lane's hits are
+// placed by the group's ballot, so a row
 // comes in cell order whatever the timing.  kOrdered: through shared memory in increasing
 // order, a column's place the number of the row's columns below it.  A row with more
 // columns than slots is left empty and flags SPH_FLAG_PAIR_CAPACITY.
-constexpr int kDropBlock = 128, kDropBlockRows = kDropBlock / kDropLanes;
+constexpr int kDropLanes = 8, kDropBlock = 128, kDropBlockRows = kDropBlock / kDropLanes;
 constexpr int kDropOrderedRoom = 512;   // slots up to which a block's rows fit in shared memory
 
 template <bool kOrdered>
@@ -723,6 +727,7 @@ DropParams<T> drop_params(const sph_params* p, int mog) {
   P.inv_h = T(1.0 / h);
   P.cg20 = T(20.0 * 7.0 / 3.14159265358979323846 / (h * h * h));
   P.rho0 = T(p->rest_density);
+  P.inv_rho0 = T(1.0 / p->rest_density);
   P.tait_k = T((double)p->rest_density * p->c0 * p->c0 / p->gamma);
   P.eps = T(h * h * 0.1);
   P.visc_unit = T(h * p->c0);
@@ -765,47 +770,56 @@ __global__ void __launch_bounds__(256) k_order_rows(int n, int room, const int32
 
 using namespace sph;
 
-template <typename Col, bool kStep>
-static void launch_rhs(int32_t fp64, int64_t n, const DropRows<Col>& rows, const void* x, const void* v,
-                       const void* rho, const void* area, const sph_params* params,
-                       double dt, void* acc, void* dpdt, void* xo, void* vo, void* ro, float* x32, cudaStream_t st) {
-  const int mog = params->density_diffusion == 1;
-  const int nb = grid_for(n * kDropLanes, 128);
-  if (fp64)
-    k_drop_rhs<double, double2, Col, kStep><<<nb, 128, 0, st>>>(
-        (int)n, rows, static_cast<const double2*>(x), static_cast<const double2*>(v),
-        static_cast<const double*>(rho), static_cast<const double*>(area), drop_params<double>(params, mog), dt,
-        static_cast<double2*>(acc), static_cast<double*>(dpdt), static_cast<double2*>(xo), static_cast<double2*>(vo),
-        static_cast<double*>(ro), reinterpret_cast<float2*>(x32));
-  else
-    k_drop_rhs<float, float2, Col, kStep><<<nb, 128, 0, st>>>(
-        (int)n, rows, static_cast<const float2*>(x), static_cast<const float2*>(v),
-        static_cast<const float*>(rho), static_cast<const float*>(area), drop_params<float>(params, mog), (float)dt,
-        static_cast<float2*>(acc), static_cast<float*>(dpdt), static_cast<float2*>(xo), static_cast<float2*>(vo),
-        static_cast<float*>(ro), reinterpret_cast<float2*>(x32));
+// Lanes per row: 8 while that gives every SM at most one block, then fewer rows' sums and ends weigh
+// more than the shorter rows.  us with 8 / 4 lanes, right-hand side and adjoint:
+//   double  2,000 particles 18.4 / 26.3, 27.5 / 48.4; 4,173: 31.3 / 26.6, 50.4 / 48.5;
+//           8,000: 59.9 / 45.1, 99 / 91; 16,173: 103 / 85, 171 / 174
+//   float   4,173 particles 7.2 / 10.3, 10.4 / 13.5; 8,000: 7.6 / 10.9, 13.6 / 15.7;
+//           16,173: 9.0 / 11.4, 25.2 / 21.4
+static int drop_lanes(bool fp64, bool adjoint, int64_t n) {
+  if (fp64) return n * 8 <= 128 * kNumSMs ? 8 : 4;
+  return adjoint && n > 12288 ? 4 : 8;
 }
 
-template <typename Col>
-static void launch_adjoint(int32_t fp64, int64_t n, const DropRows<Col>& rows, const void* x, const void* v,
-                           const void* rho, const void* area, const sph_params* params,
-                           double dt, const void* lx1, const void* lv1, const void* lr1, void* lx0, void* lv0,
-                           void* lr0, void* dalpha, int accumulate, cudaStream_t st) {
-  const int mog = params->density_diffusion == 1;
-  const int nb = grid_for(n * kDropLanes, 128);
+template <int kLanes, typename T, typename V2, bool kStep, typename Col>
+static void rhs_as(int64_t n, const DropRows<Col>& rows, const void* x, const void* v, const void* rho,
+                   const void* area, const sph_params* params, double dt, void* acc, void* dpdt, void* xo, void* vo, void* ro, float* x32,
+                   cudaStream_t st) {
+  k_drop_rhs<kLanes, T, V2, Col, kStep><<<grid_for(n * kLanes, 128), 128, 0, st>>>(
+      (int)n, rows, static_cast<const V2*>(x), static_cast<const V2*>(v), static_cast<const T*>(rho),
+      static_cast<const T*>(area), drop_params<T>(params, params->density_diffusion == 1), (T)dt, static_cast<V2*>(acc),
+      static_cast<T*>(dpdt), static_cast<V2*>(xo), static_cast<V2*>(vo), static_cast<T*>(ro),
+      reinterpret_cast<float2*>(x32));
+}
+
+template <int kLanes, typename T, typename V2, typename Col>
+static void adjoint_as(int64_t n, const DropRows<Col>& rows, const void* x, const void* v, const void* rho,
+                       const void* area, const sph_params* params, double dt, const void* lx1, const void* lv1,
+                       const void* lr1, void* lx0, void* lv0, void* lr0, void* dalpha, int accumulate,
+                       cudaStream_t st) {
+  k_drop_adjoint<kLanes, T, V2, Col><<<grid_for(n * kLanes, 128), 128, 0, st>>>(
+      (int)n, rows, static_cast<const V2*>(x), static_cast<const V2*>(v), static_cast<const T*>(rho),
+      static_cast<const T*>(area), drop_params<T>(params, params->density_diffusion == 1), (T)dt,
+      static_cast<const V2*>(lx1), static_cast<const V2*>(lv1), static_cast<const T*>(lr1), static_cast<V2*>(lx0),
+      static_cast<V2*>(lv0), static_cast<T*>(lr0), static_cast<T*>(dalpha), accumulate);
+}
+
+template <bool kStep, typename Col, typename... Args>
+static void launch_rhs(int32_t fp64, int64_t n, Args... args) {
+  const bool four = drop_lanes(fp64, false, n) == 4;
   if (fp64)
-    k_drop_adjoint<double, double2, Col><<<nb, 128, 0, st>>>(
-        (int)n, rows, static_cast<const double2*>(x), static_cast<const double2*>(v),
-        static_cast<const double*>(rho), static_cast<const double*>(area), drop_params<double>(params, mog), dt,
-        static_cast<const double2*>(lx1), static_cast<const double2*>(lv1), static_cast<const double*>(lr1),
-        static_cast<double2*>(lx0), static_cast<double2*>(lv0), static_cast<double*>(lr0),
-        static_cast<double*>(dalpha), accumulate);
+    four ? rhs_as<4, double, double2, kStep, Col>(n, args...) : rhs_as<8, double, double2, kStep, Col>(n, args...);
   else
-    k_drop_adjoint<float, float2, Col><<<nb, 128, 0, st>>>(
-        (int)n, rows, static_cast<const float2*>(x), static_cast<const float2*>(v),
-        static_cast<const float*>(rho), static_cast<const float*>(area), drop_params<float>(params, mog), (float)dt,
-        static_cast<const float2*>(lx1), static_cast<const float2*>(lv1), static_cast<const float*>(lr1),
-        static_cast<float2*>(lx0), static_cast<float2*>(lv0), static_cast<float*>(lr0), static_cast<float*>(dalpha),
-        accumulate);
+    four ? rhs_as<4, float, float2, kStep, Col>(n, args...) : rhs_as<8, float, float2, kStep, Col>(n, args...);
+}
+
+template <typename Col, typename... Args>
+static void launch_adjoint(int32_t fp64, int64_t n, Args... args) {
+  const bool four = drop_lanes(fp64, true, n) == 4;
+  if (fp64)
+    four ? adjoint_as<4, double, double2, Col>(n, args...) : adjoint_as<8, double, double2, Col>(n, args...);
+  else
+    four ? adjoint_as<4, float, float2, Col>(n, args...) : adjoint_as<8, float, float2, Col>(n, args...);
 }
 
 // The scratch of sph_drop_search, in order: cell_count [cap + 1] (zero between calls), cell_start
@@ -898,7 +912,7 @@ sph_status_t sph_drop_step(int32_t fp64, int64_t n, const int32_t* row_info, con
               "drop_step: bad arguments (gamma 7, MOG or no density diffusion)");
   SPH_REQUIRE(n == 0 || (x_out != x && v_out != v && rho_out != rho), "drop_step: outputs must not alias inputs");
   if (n == 0) return SPH_OK;
-  launch_rhs<int32_t, true>(fp64, n, DropRows<int32_t>{row_info, cols, row_capacity}, x, v, rho, area, params, dt,
+  launch_rhs<true, int32_t>(fp64, n, DropRows<int32_t>{row_info, cols, row_capacity}, x, v, rho, area, params, dt,
                             nullptr, nullptr, x_out, v_out, rho_out, x32_out, as_stream(stream));
   SPH_CHECK_LAUNCH("drop_step");
   return SPH_OK;
@@ -915,8 +929,8 @@ sph_status_t sph_drop_adjoint_step(int32_t fp64, int64_t n, const int32_t* row_i
               "drop_adjoint_step: bad arguments (gamma 7, MOG or no density diffusion)");
   SPH_REQUIRE(lx0 != lx1 && lv0 != lv1 && lr0 != lr1, "drop_adjoint_step: outputs must not alias inputs");
   if (n == 0) return SPH_OK;
-  launch_adjoint(fp64, n, DropRows<int32_t>{row_info, cols, row_capacity}, x, v, rho, area, params, dt, lx1, lv1, lr1,
-                 lx0, lv0, lr0, dalpha, 1, as_stream(stream));
+  launch_adjoint<int32_t>(fp64, n, DropRows<int32_t>{row_info, cols, row_capacity}, x, v, rho, area, params, dt, lx1,
+                          lv1, lr1, lx0, lv0, lr0, dalpha, 1, as_stream(stream));
   SPH_CHECK_LAUNCH("drop_adjoint_step");
   return SPH_OK;
 }
@@ -929,7 +943,7 @@ sph_status_t sph_drop_rhs(int32_t fp64, int64_t n, const int32_t* offsets, const
                   (n == 0 || (offsets && cols && x && v && rho && area && acc && dpdt)),
               "drop_rhs: bad arguments (gamma 7, MOG or no density diffusion)");
   if (n == 0) return SPH_OK;
-  launch_rhs<int64_t, false>(fp64, n, DropRows<int64_t>{offsets, cols, 0}, x, v, rho, area, params, 0.0, acc, dpdt,
+  launch_rhs<false, int64_t>(fp64, n, DropRows<int64_t>{offsets, cols, 0}, x, v, rho, area, params, 0.0, acc, dpdt,
                              nullptr, nullptr, nullptr, nullptr, as_stream(stream));
   SPH_CHECK_LAUNCH("drop_rhs");
   return SPH_OK;
@@ -964,8 +978,8 @@ sph_status_t sph_drop_adjoint(int32_t fp64, int64_t n, const int32_t* offsets, c
               "drop_adjoint: bad arguments (gamma 7, MOG or no density diffusion)");
   SPH_REQUIRE(lx0 != lx1 && lv0 != lv1 && lr0 != lr1, "drop_adjoint: outputs must not alias inputs");
   if (n == 0) return SPH_OK;
-  launch_adjoint(fp64, n, DropRows<int64_t>{offsets, cols, 0}, x, v, rho, area, params, dt, lx1, lv1, lr1, lx0, lv0,
-                 lr0, dalpha, 0, as_stream(stream));
+  launch_adjoint<int64_t>(fp64, n, DropRows<int64_t>{offsets, cols, 0}, x, v, rho, area, params, dt, lx1, lv1, lr1,
+                          lx0, lv0, lr0, dalpha, 0, as_stream(stream));
   SPH_CHECK_LAUNCH("drop_adjoint");
   return SPH_OK;
 }

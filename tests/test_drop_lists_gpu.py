@@ -99,3 +99,26 @@ def test_out_of_domain_is_refused(cuda):
         r.rollout(v0, 0.0, 3)
     r.rollout(torch.zeros_like(v0), 0.0, 0)
     assert r.rollout(v0 * 1e-3, 0.0, 1)[0].shape == (33, 2)
+
+
+@pytest.mark.parametrize("n", [2432, 2433, 12288, 12289])
+@pytest.mark.parametrize("fp64", [True, False])
+def test_lanes_by_size(cuda, n, fp64):
+    """Sizes on both sides of the lanes' limits: the rollout against the (i, j)-ordered step (the same
+    bits in float32), and the gradient of the sum of positions, which one step at rest moves
+    as dt to each component (pressure and viscosity are pair forces of equal masses: they
+    sum to zero within 30 roundings of dt^2 a, below 1e-5 of dt; gravity's point source
+    takes dt^2 off)."""
+    from pytorchsph_gb300.adjoint import DropRollout
+    sc = blob(n, n)
+    dt = 0.1 * sc["h"] / C0
+    r = DropRollout(sc, C0, dt, fp64=fp64, device=cuda)
+    v0 = torch.as_tensor(sc["vel"], dtype=r.dtype, device=cuda)
+    xT, _ = r.rollout(v0, 0.05, 2)
+    x, v, rho = r.x0.clone(), v0.clone(), r.rho0.clone()
+    for _ in range(2):
+        r.step(x, v, rho, 0.05)
+    assert torch.equal(xT, x) if not fp64 else float((xT - x).abs().max()) <= 1e-12 * float(x.abs().max())
+    (_, *_), _, record = r._forward(v0, 0.05, 1, record=True)
+    gv, _ = r._backward(record, 0.05, 1, torch.ones((n, 2), dtype=r.dtype, device=cuda))
+    assert float((gv.mean(0) - dt).abs().max()) <= 1e-3 * dt
