@@ -757,12 +757,18 @@ __global__ void __launch_bounds__(256) k_dt_partials(int n, const float2* __rest
 
 __global__ void k_dt_final(int nparts, const float* __restrict__ part, float h, float kinematic, float cfl, float c0,
                            int acoustic_from_c0, float dt_min, float dt_max, float* __restrict__ dt) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  // one warp over the parts (one thread took 14 us of every step for the 304 of a large scene)
   float vmax = 0.f, amin = INFINITY;
-  for (int k = 0; k < nparts; ++k) {
+  for (int k = threadIdx.x; k < nparts; k += 32) {
     vmax = fmaxf(vmax, part[2 * k]);
     amin = fminf(amin, part[2 * k + 1]);
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+    amin = fminf(amin, __shfl_xor_sync(0xffffffffu, amin, o));
+  }
+  if (threadIdx.x != 0) return;
   const double visc = 0.125 * (double)h * h / kinematic;
   const double accdt = 0.25 * (double)amin;
   const double vdt = acoustic_from_c0 ? (double)cfl * h / c0 : 0.4 * (double)h / vmax;
