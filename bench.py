@@ -631,16 +631,16 @@ def run_search_density(args, dev, world, rank):
         marks("end")
         return r
 
-    # grid (bounds, final), keys, sort, gather, count, scan, fill, dense rows, scatter; a scan
-    # is one kernel (the zeroing of its tile words is a memset); counting sort: scan,
-    # scatter, in-cell fix of small and of large cells, which also gather the positions,
+    # grid (bounds, final), keys, sort, count, scan, fill, scatter; a scan is one kernel (the
+    # zeroing of its tile words is a memset); counting sort: scan, scatter, in-cell fix of
+    # small and (above 2^18 particles) of large cells, which also gather the positions,
     # supports and areas; radix: per digit histogram, scan, scatter, then the cell starts
     # and the gather
     if args.sort == "counting":
-        sort_launches = 4
+        sort_launches = 3 + (n > 1 << 18)
     else:
         sort_launches = ((N.load().sph_key_bits(cells) + args.digit_bits - 1) // args.digit_bits) * 3 + 1 + 1
-    launches_per_step = 2 + 1 + sort_launches + 1 + 1 + 1 + 1 + 1
+    launches_per_step = 2 + 1 + sort_launches + 1 + 1 + 1 + 1
     s = torch.cuda.Stream(dev)
     s.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(s):
@@ -831,7 +831,7 @@ def run_dambreak(args, dev, world, rank):
             sync_ranks(world)
         sim.check()
         ms = max_over_ranks(st.elapsed_time(en) / args.steps, world)
-        n, launches = sim.n, 40
+        n, launches = sim.n, 22   # sort 4, densities 2, solves 2 x (v*, prepare, solve), walls, viscosity, update, dt
         config = {"workload": args.workload, "particles": n, "walls": sim.nb,
                   "solver": "DFSPH, divergence + density solves, semi-implicit Euler, adaptive dt",
                   "density_iters_last": int(sim.last["density_iters"].item()),

@@ -485,7 +485,7 @@ class SceneBatch:
     # update 1 for a group with deltaSPH scenes).  A scan is one kernel (above 16,384 items its tile words
     # are zeroed by a memset first, which is not a kernel).
     def launches_per_step(self):
-        sort = 1 + 3
+        sort = 1 + 2 + (self.n > 1 << 18)   # scan, scatter, in-cell fix, large cells
         csr = 1 + 1 + 1 if self.pairs == "csr" else 0
         p1 = sum(1 for lo, hi, _, _ in self.groups if hi > lo)
         dif = sum(1 for lo, hi, _, k in self.groups if hi > lo and k not in (0, 1)) if self.any_renorm else 0
@@ -1047,7 +1047,7 @@ class SceneArena(SceneBatch):
                 for slot, d in self.slots.items()}
 
     def launches_per_step(self):
-        return 1 + 4 + 1 + 1 + 1 + (1 if self.any_renorm else 0)
+        return 1 + 3 + (self.n > 1 << 18) + 1 + 1 + 1 + (1 if self.any_renorm else 0)
 
 
 def estimate_bytes(scene, pairs: str = "cells") -> int:
