@@ -5,7 +5,8 @@
 //   * sph_counting_sort — single-digit radix (counting) sort where the digit is the whole
 //     cell key: a global per-cell histogram (atomics, filled by sph_cell_keys), one
 //     exclusive scan that is directly the cell begin table, an atomic scatter, and a
-//     per-cell fix-up that restores index order inside each cell.  ~6 launches.
+//     per-cell fix-up that restores index order inside each cell.  Three launches, and a
+//     fourth for large cells above 2^18 particles; the scan's tile words are a memset.
 //   * sph_radix_sort_pairs (scan_sort.cu) — multi-pass LSD radix sort with 1..8-bit
 //     digits; its cell table comes from sph_cell_starts (binary search per cell).
 #include <cstdio>
@@ -274,14 +275,36 @@ __global__ void k_count_scatter(const uint32_t* __restrict__ keys, int64_t n, co
   if (sent) tmp[cell_start[sentinel] + s_left - 1 - base - __popc(b & ((1u << lane) - 1u))] = (uint32_t)i;
 }
 
-constexpr int kRankSortMax = 1024;   // large cells up to this size are ranked in shared memory
+constexpr int kRankSortMax = 320;   // large cells up to this size are ranked in shared memory
 constexpr int kSmallCell = 48;    // cells up to this size are ordered by ranking, one thread per particle
 constexpr int kBlockSortMax = 2048;  // larger cells: one block, bitonic sort in shared memory
+constexpr int kFixThreads = 256;     // a block's threads, at least
 
 // Sort key inside a cell: the particle's index, or (tie[index], index) when a tie key is
 // given (e.g. a particle id, which makes the order independent of the previous order).
 __device__ __forceinline__ uint64_t cell_rank(uint32_t x, const uint32_t* __restrict__ tie) {
   return tie ? (((uint64_t)__ldg(tie + x)) << 32) | x : (uint64_t)x;
+}
+
+// One pass of a bitonic sort of the p2 words s by the block: thread t compares its pairs (i, i +
+// stride), kPairs of them in flight (kPairs blockDim >= p2 / 2).
+template <int kPairs>
+__device__ __forceinline__ void bitonic_pass(uint64_t* s, int p2, int size, int stride) {
+  int i[kPairs];
+  uint64_t lo[kPairs], hi[kPairs];
+#pragma unroll
+  for (int q = 0; q < kPairs; ++q) {
+    const int p = threadIdx.x + q * (int)blockDim.x;
+    i[q] = p < p2 / 2 ? 2 * p - (p & (stride - 1)) : -1;
+    lo[q] = i[q] >= 0 ? s[i[q]] : 0;
+    hi[q] = i[q] >= 0 ? s[i[q] + stride] : 0;
+  }
+#pragma unroll
+  for (int q = 0; q < kPairs; ++q)
+    if (i[q] >= 0 && (lo[q] > hi[q]) == ((i[q] & size) == 0)) {
+      s[i[q]] = hi[q];
+      s[i[q] + stride] = lo[q];
+    }
 }
 
 // One large cell by a whole block, its (tie, index) ranks in shared memory: up to kRankSortMax
@@ -321,17 +344,12 @@ __device__ __forceinline__ void fix_large_cell(int b, int e, const uint32_t* __r
   __syncthreads();
   for (int size = 2; size <= p2; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int t = threadIdx.x; t < p2; t += blockDim.x) {
-        int u = t ^ stride;
-        if (u > t) {
-          bool up = (t & size) == 0;
-          uint64_t a = s[t], bb = s[u];
-          if ((a > bb) == up) {
-            s[t] = bb;
-            s[u] = a;
-          }
-        }
-      }
+      if (p2 <= 2 * blockDim.x)
+        bitonic_pass<1>(s, p2, size, stride);
+      else if (p2 <= 4 * blockDim.x)
+        bitonic_pass<2>(s, p2, size, stride);
+      else
+        bitonic_pass<kBlockSortMax / (2 * kFixThreads)>(s, p2, size, stride);
       __syncthreads();
     }
   }
@@ -354,11 +372,13 @@ __device__ __forceinline__ void fix_large_cell(int b, int e, const uint32_t* __r
 //     pays with the block's barriers and 16 KB of shared memory;
 //   else: k_cell_fix_large.  At 260,100 particles the block variant takes 6.0 µs against 4.6 + 1.9
 //     and the memset, at 2^20 20 against 15 + 2, at 3.1 M 82 against 50 + 2.
-// kFixInBlock is the line between them.
+// kFixInBlock is the line between them.  A block that has large cells ranks those of up to
+// kRankSortMax entries together and sorts longer ones one by one: 100,000 particles in cells of
+// 100 / 300 / 1,000 / 2,000 take 7 / 13 / 22 / 33 µs (one cell after the other and ranks up to 1,024
+// 10 / 19 / 92 / 58; the launch of their own 10 / 14 / 34 / 36 with the small cells').
 // The sentinel cell (the key cell_capacity: particles outside every grid, or of no scene in
 // a pooled batch) keeps the scatter order: nothing reads its order.
 constexpr int64_t kFixInBlock = 1 << 18;
-constexpr int kFixThreads = 256;
 constexpr int kFixLarge = kFixThreads / (kSmallCell + 1) + 1;   // large cells that begin in one block
 
 template <bool kInBlock>
@@ -371,7 +391,7 @@ __global__ void __launch_bounds__(kFixThreads) k_cell_fix(const uint32_t* __rest
                                                           int32_t* __restrict__ big_list,
                                                           int32_t* __restrict__ big_count, int32_t* status,
                                                           const ArraySet rows, uint32_t sentinel) {
-  __shared__ int large[kFixLarge];
+  __shared__ int large_b[kFixLarge], large_k[kFixLarge], part[kFixLarge + 1];
   __shared__ int num_large;
   if constexpr (kInBlock) {
     if (threadIdx.x == 0) num_large = 0;
@@ -389,10 +409,13 @@ __global__ void __launch_bounds__(kFixThreads) k_cell_fix(const uint32_t* __rest
       const int b = __ldg(cell_start + c), e = __ldg(cell_start + c + 1);
       if (e - b > kSmallCell) {
         if (t == b) {
-          if constexpr (kInBlock)
-            large[atomicAdd(&num_large, 1)] = (int)c;
-          else
+          if constexpr (kInBlock) {
+            const int q = atomicAdd(&num_large, 1);
+            large_b[q] = b;
+            large_k[q] = e - b;
+          } else {
             big_list[atomicAdd(big_count, 1)] = (int32_t)c;
+          }
         }
       } else {
         const FourRows head = load_rows(rows, 0, x);
@@ -408,10 +431,42 @@ __global__ void __launch_bounds__(kFixThreads) k_cell_fix(const uint32_t* __rest
   if constexpr (kInBlock) {
     __shared__ uint64_t ranks[kBlockSortMax];
     __syncthreads();
-    for (int q = 0; q < num_large; ++q)
-      fix_large_cell(cell_start[large[q]], cell_start[large[q] + 1], tmp, tie, order, status, rows, ranks);
+    const int cells = num_large;
+    if (cells == 0) return;
+    // the cells that are ranked, all at once: entries part[q] .. part[q + 1] - 1 are those of cell q
+    if (threadIdx.x == 0) {
+      int sum = 0;
+      for (int q = 0; q < cells; ++q) {
+        part[q] = sum;
+        sum += large_k[q] <= kRankSortMax ? large_k[q] : 0;
+      }
+      part[cells] = sum;
+    }
+    __syncthreads();
+    const int ranked = part[cells];
+    for (int u = threadIdx.x, q = 0; u < ranked; u += kFixThreads) {
+      while (part[q + 1] <= u) ++q;
+      ranks[u] = cell_rank(__ldg(tmp + large_b[q] + u - part[q]), tie);
+    }
+    __syncthreads();
+    for (int u = threadIdx.x, q = 0; u < ranked; u += kFixThreads) {
+      while (part[q + 1] <= u) ++q;
+      const uint64_t mine = ranks[u];
+      const int first = part[q], end = part[q + 1];
+      int rank = 0;
+#pragma unroll 8
+      for (int v = first; v < end; ++v) rank += ranks[v] < mine;
+      order[large_b[q] + rank] = (uint32_t)(mine & 0xffffffffu);
+      copy_rows(rows, large_b[q] + rank, (uint32_t)(mine & 0xffffffffu));
+    }
+    __syncthreads();
+    for (int q = 0; q < cells; ++q)
+      if (large_k[q] > kRankSortMax)
+        fix_large_cell(large_b[q], large_b[q] + large_k[q], tmp, tie, order, status, rows, ranks);
   }
 }
+
+static_assert(kFixLarge * kRankSortMax <= kBlockSortMax, "the ranked cells of a block fit its shared words");
 
 __global__ void __launch_bounds__(512) k_cell_fix_large(const int32_t* __restrict__ cell_start,
                                                         const uint32_t* __restrict__ tmp,

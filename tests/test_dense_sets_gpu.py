@@ -1,0 +1,70 @@
+"""Sets with many particles in a cell or a row: order and speed.
+
+Order is compared with a stable sort on the host (integers, equal).  Speed is compared with
+another call on the same device over the same number of particles or pairs, as a ratio with
+at least a factor of 1.5 between the bar and what the calls take."""
+import numpy as np
+import pytest
+import torch
+
+import test_cell_fix_gpu as cells
+
+pytestmark = pytest.mark.gpu
+
+
+def time_us(f, runs=5, repeats=10):
+    """The shortest of `repeats` means over `runs` calls, on the device."""
+    for _ in range(3):
+        f()
+    best = float("inf")
+    for _ in range(repeats):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        a.record()
+        for _ in range(runs):
+            f()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b) * 1e3 / runs)
+    return best
+
+
+def graph_of(f):
+    f()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        f()
+    return g.replay
+
+
+@pytest.mark.parametrize("sizes", [[320, 321, 49], [320] * 9, [512, 513, 320, 1024], [300] * 200 + [7] * 50,
+                                   [49, 319, 1, 2048, 64, 1], [512] * 520 + [320] * 30])
+@pytest.mark.parametrize("with_tie", [False, True])
+def test_cell_order(cuda, sizes, with_tie):
+    """Cells around the block's limits: 320 entries ranked with the block's others, then bitonic
+    passes with one, two or four pairs a thread."""
+    cells.test_order(cuda, sizes, with_tie)
+
+
+def test_sort_of_large_cells_in_time(cuda):
+    """100,000 particles in cells of 1,000 against cells of 9.  The scatter's atomics on 100 words take
+    about 16 us more, the ranks about 20; four times the small cells' 19 us is held."""
+    from pytorchsph_gb300 import _native as N
+    n, took = 100000, {}
+    for size in (9, 1000):
+        cap = -(-n // size)
+        rng = np.random.default_rng(size)
+        keys = torch.from_numpy(rng.permutation(np.arange(n) // size).astype(np.int32)).to(cuda)
+        full = torch.bincount(keys.long(), minlength=cap + 1).to(torch.int32)
+        i32 = lambda m: torch.empty(m, dtype=torch.int32, device=cuda)
+        count, start, order, skeys, status = full.clone(), i32(cap + 2), i32(n), i32(n), torch.zeros_like(full[:1])
+        scratch = torch.empty(N.load().sph_counting_sort_scratch_bytes(n, cap) // 8 + 1, dtype=torch.int64, device=cuda)
+
+        def sort():
+            count.copy_(full)
+            N.call("sph_counting_sort", N.ptr(keys), n, cap, N.ptr(count), N.ptr(start), N.ptr(order), N.ptr(skeys),
+                   N.ptr(status), N.ptr(scratch), scratch.numel() * 8, N.stream_ptr())
+        took[size] = time_us(graph_of(sort))
+        assert torch.equal(order.long(), torch.argsort(keys.long(), stable=True))
+    assert took[1000] < 4 * took[9], took
