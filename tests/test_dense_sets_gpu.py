@@ -68,3 +68,39 @@ def test_sort_of_large_cells_in_time(cuda):
         took[size] = time_us(graph_of(sort))
         assert torch.equal(order.long(), torch.argsort(keys.long(), stable=True))
     assert took[1000] < 4 * took[9], took
+
+
+def clusters(n, size, seed=0):
+    """n particles in clusters of `size` within a support (0.1) of each other, in random order."""
+    rng = np.random.default_rng(seed)
+    c = np.arange(n) // size
+    pos = np.stack([c % 64, c // 64], 1) * 1.0 + rng.uniform(0, 0.05, (n, 2))
+    return torch.from_numpy(rng.permutation(pos).astype(np.float32)).cuda()
+
+
+def test_fill_of_dense_rows_in_time(cuda):
+    """8,192 rows of 1,024 columns, all on the dense list: the fill stores 34 MB and repeats the
+    count's candidate tests a warp per row (a third of the count's time); twice it is held."""
+    from pytorchsph_gb300 import _native as N
+    from pytorchsph_gb300.search import GridSearch
+    n = 8192
+    pos, sup = clusters(n, 1024), torch.full((n,), 0.1, device=cuda)
+    s = GridSearch(cuda)
+    r = s.run(pos, sup, density=False)
+    assert r.num_pairs == n * 1024
+    seg = s.ws.bytes("segments", N.load().sph_nl_segments_scratch_bytes(n))
+    head = (N.ptr(r.xy), N.ptr(r.sh))
+    grid = (n, N.ptr(r.keys), N.ptr(r.cell_start), N.ptr(r.grid), r.cell_capacity, 1)
+
+    def count():
+        N.call("sph_nl_count_segments", *head, None, *grid, 0.0, N.ptr(r.counts), None, N.ptr(seg), seg.numel() * 8,
+               N.stream_ptr())
+
+    def fill():
+        N.call("sph_nl_fill_segments", *head, *grid, N.ptr(r.offsets), r.pair_capacity, N.ptr(r.cols), N.ptr(r.status),
+               N.ptr(seg), seg.numel() * 8, N.stream_ptr())
+    want = r.cols.clone()
+    counted = time_us(graph_of(count))
+    r.cols.zero_()
+    filled = time_us(graph_of(fill))
+    assert torch.equal(r.cols, want) and filled < 2 * counted, (filled, counted)
