@@ -277,34 +277,13 @@ __global__ void k_count_scatter(const uint32_t* __restrict__ keys, int64_t n, co
 
 constexpr int kRankSortMax = 320;   // large cells up to this size are ranked in shared memory
 constexpr int kSmallCell = 48;    // cells up to this size are ordered by ranking, one thread per particle
-constexpr int kBlockSortMax = 2048;  // larger cells: one block, bitonic sort in shared memory
+constexpr int kBlockSortMax = kBlockSortWords;  // larger cells: one block, bitonic sort in shared memory
 constexpr int kFixThreads = 256;     // a block's threads, at least
 
 // Sort key inside a cell: the particle's index, or (tie[index], index) when a tie key is
 // given (e.g. a particle id, which makes the order independent of the previous order).
 __device__ __forceinline__ uint64_t cell_rank(uint32_t x, const uint32_t* __restrict__ tie) {
   return tie ? (((uint64_t)__ldg(tie + x)) << 32) | x : (uint64_t)x;
-}
-
-// One pass of a bitonic sort of the p2 words s by the block: thread t compares its pairs (i, i +
-// stride), kPairs of them in flight (kPairs blockDim >= p2 / 2).
-template <int kPairs>
-__device__ __forceinline__ void bitonic_pass(uint64_t* s, int p2, int size, int stride) {
-  int i[kPairs];
-  uint64_t lo[kPairs], hi[kPairs];
-#pragma unroll
-  for (int q = 0; q < kPairs; ++q) {
-    const int p = threadIdx.x + q * (int)blockDim.x;
-    i[q] = p < p2 / 2 ? 2 * p - (p & (stride - 1)) : -1;
-    lo[q] = i[q] >= 0 ? s[i[q]] : 0;
-    hi[q] = i[q] >= 0 ? s[i[q] + stride] : 0;
-  }
-#pragma unroll
-  for (int q = 0; q < kPairs; ++q)
-    if (i[q] >= 0 && (lo[q] > hi[q]) == ((i[q] & size) == 0)) {
-      s[i[q]] = hi[q];
-      s[i[q] + stride] = lo[q];
-    }
 }
 
 // One large cell by a whole block, its (tie, index) ranks in shared memory: up to kRankSortMax
@@ -342,17 +321,7 @@ __device__ __forceinline__ void fix_large_cell(int b, int e, const uint32_t* __r
   while (p2 < k) p2 <<= 1;
   for (int t = threadIdx.x; t < p2; t += blockDim.x) s[t] = t < k ? cell_rank(tmp[b + t], tie) : ~0ull;
   __syncthreads();
-  for (int size = 2; size <= p2; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      if (p2 <= 2 * blockDim.x)
-        bitonic_pass<1>(s, p2, size, stride);
-      else if (p2 <= 4 * blockDim.x)
-        bitonic_pass<2>(s, p2, size, stride);
-      else
-        bitonic_pass<kBlockSortMax / (2 * kFixThreads)>(s, p2, size, stride);
-      __syncthreads();
-    }
-  }
+  block_sort(s, p2);
   for (int t = threadIdx.x; t < k; t += blockDim.x) {
     order[b + t] = (uint32_t)(s[t] & 0xffffffffu);
     copy_rows(rows, b + t, (uint32_t)(s[t] & 0xffffffffu));

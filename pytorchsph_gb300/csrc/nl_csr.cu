@@ -486,49 +486,55 @@ __global__ void __launch_bounds__(128) k_nl_query(const float2* __restrict__ qpo
 // A lane holds one pair.  Up to 32 columns are sorted in the lanes (bitonic; a column's sorted
 // place comes back from rank); in a longer row a column's place is the number of the row's
 // columns below it (they are distinct), counted over the warp's registers 32 columns at a
-// time.  No scratch, and the row's loads and four outputs are contiguous pieces, where one
-// thread per row moved every column through global memory once per inversion: 558 us for
-// 260,017 particles, 7.2 M pairs (201 MB of pairs and distances stored); counting in all
-// rows 103, sorting the short ones 85.  Bound by instruction issue: the sort, and the
-// correctly rounded root and divisions.
-__global__ void __launch_bounds__(256) k_nl_to_coo(const float2* __restrict__ xy, int64_t n,
-                                                   const uint32_t* __restrict__ order,
-                                                   const uint32_t* __restrict__ rank,
-                                                   const int32_t* __restrict__ offsets,
-                                                   const int32_t* __restrict__ cols,
-                                                   const int64_t* __restrict__ orig_offsets, float thr, float support,
-                                                   int64_t* __restrict__ pairs, int64_t P, float* __restrict__ dist,
-                                                   float* __restrict__ radial) {
+// time; rows past kLongRow are left to k_nl_to_coo_long.  No scratch, and the row's loads and four
+// outputs are contiguous pieces, where one thread per row moved every column through global
+// memory once per inversion: 558 us for 260,017 particles, 7.2 M pairs (201 MB of pairs and
+// distances stored); counting in all rows 103, sorting the short ones 85.  Bound by instruction
+// issue: the sort, and the correctly rounded root and divisions.
+struct CooRows {
+  const float2* xy;
+  const uint32_t* order;
+  const uint32_t* rank;
+  const int32_t* offsets;
+  const int32_t* cols;
+  const int64_t* orig_offsets;
+  float thr, support;
+  int64_t *prow, *pcol;
+  float *dist, *radial;
+};
+
+// Pair k: original particles i at pi and jo, which is c in sorted order.
+__device__ __forceinline__ void write_pair(const CooRows& R, int64_t i, float2 pi, int64_t k, uint32_t jo, int32_t c) {
+  R.prow[k] = i;
+  R.pcol[k] = (int64_t)jo;
+  if (R.dist || R.radial) {
+    const float2 pj = __ldg(R.xy + c);
+    const float dx = pi.x - pj.x, dy = pi.y - pj.y;
+    const float rr = sqrtf(dx * dx + dy * dy);
+    if (R.dist) {
+      const float2 e = rr < R.thr ? make_float2(0.f, 0.f) : make_float2(dx / rr, dy / rr);
+      if ((reinterpret_cast<uintptr_t>(R.dist) & 7) == 0) {
+        reinterpret_cast<float2*>(R.dist)[k] = e;
+      } else {
+        R.dist[2 * k] = e.x;
+        R.dist[2 * k + 1] = e.y;
+      }
+    }
+    if (R.radial) R.radial[k] = rr / R.support;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_nl_to_coo(int64_t n, const CooRows R) {
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (i >= n) return;
-  const uint32_t s = rank[i];
-  const int32_t b = offsets[s], m = offsets[s + 1] - b;
-  const int64_t o = orig_offsets[i];
-  int64_t* prow = pairs;
-  int64_t* pcol = pairs + P;
-  const float2 pi = xy[s];
-  const auto write = [&](int64_t k, uint32_t jo, int32_t c) {
-    prow[k] = i;
-    pcol[k] = (int64_t)jo;
-    if (dist || radial) {
-      const float2 pj = __ldg(xy + c);
-      const float dx = pi.x - pj.x, dy = pi.y - pj.y;
-      const float rr = sqrtf(dx * dx + dy * dy);
-      if (dist) {
-        const float2 e = rr < thr ? make_float2(0.f, 0.f) : make_float2(dx / rr, dy / rr);
-        if ((reinterpret_cast<uintptr_t>(dist) & 7) == 0) {
-          reinterpret_cast<float2*>(dist)[k] = e;
-        } else {
-          dist[2 * k] = e.x;
-          dist[2 * k + 1] = e.y;
-        }
-      }
-      if (radial) radial[k] = rr / support;
-    }
-  };
+  const uint32_t s = __ldg(R.rank + i);
+  const int32_t b = __ldg(R.offsets + s), m = __ldg(R.offsets + s + 1) - b;
+  if (m > kLongRow) return;
+  const int64_t o = __ldg(R.orig_offsets + i);
+  const float2 pi = __ldg(R.xy + s);
   if (m <= 32) {
-    uint32_t jo = lane < m ? __ldg(order + __ldg(cols + b + lane)) : 0xffffffffu;
+    uint32_t jo = lane < m ? __ldg(R.order + __ldg(R.cols + b + lane)) : 0xffffffffu;
 #pragma unroll
     for (int k = 2; k <= 32; k <<= 1)
 #pragma unroll
@@ -536,22 +542,37 @@ __global__ void __launch_bounds__(256) k_nl_to_coo(const float2* __restrict__ xy
         const uint32_t v = __shfl_xor_sync(0xffffffffu, jo, d);
         jo = ((lane & k) == 0) == ((lane & d) == 0) ? min(jo, v) : max(jo, v);
       }
-    if (lane < m) write(o + lane, jo, (int32_t)__ldg(rank + jo));
+    if (lane < m) write_pair(R, i, pi, o + lane, jo, (int32_t)__ldg(R.rank + jo));
     return;
   }
   for (int t0 = 0; t0 < m; t0 += 32) {
     const int t = t0 + lane;
-    const int32_t c = t < m ? __ldg(cols + b + t) : 0;
-    const uint32_t jo = t < m ? __ldg(order + c) : 0xffffffffu;
+    const int32_t c = t < m ? __ldg(R.cols + b + t) : 0;
+    const uint32_t jo = t < m ? __ldg(R.order + c) : 0xffffffffu;
     int r = 0;
     for (int u0 = 0; u0 < m; u0 += 32) {
       const int u = u0 + lane;
-      const uint32_t ju = u0 == t0 ? jo : (u < m ? __ldg(order + __ldg(cols + b + u)) : 0xffffffffu);
+      const uint32_t ju = u0 == t0 ? jo : (u < m ? __ldg(R.order + __ldg(R.cols + b + u)) : 0xffffffffu);
       const int len = min(m - u0, 32);
       for (int k = 0; k < len; ++k) r += __shfl_sync(0xffffffffu, ju, k) < jo;
     }
-    if (t < m) write(o + r, jo, c);
+    if (t < m) write_pair(R, i, pi, o + r, jo, c);
   }
+}
+
+// The rows past kLongRow, a warp each.
+__global__ void __launch_bounds__(256) k_nl_to_coo_long(int64_t n, const CooRows R) {
+  __shared__ uint32_t words[8][kWarpSortWords];
+  const int lane = threadIdx.x & 31;
+  for_long_rows(n, [&](int64_t s) { return R.offsets[s + 1] - R.offsets[s]; }, [&](int64_t s, int m) {
+    const int64_t i = R.order[s], o = R.orig_offsets[i];
+    const float2 pi = R.xy[s];
+    warp_sort_row(R.cols + R.offsets[s], R.order, m, R.pcol + o, words[threadIdx.x >> 5]);
+    for (int t = lane; t < m; t += 32) {
+      const uint32_t jo = (uint32_t)R.pcol[o + t];
+      write_pair(R, i, pi, o + t, jo, (int32_t)__ldg(R.rank + jo));
+    }
+  });
 }
 
 // ---------------------------------------------------------------------------- batch of scenes
@@ -737,9 +758,11 @@ sph_status_t sph_nl_to_coo(const float* xy, int64_t n, const uint32_t* order, co
                            float* radial, void* stream) {
   SPH_REQUIRE(n >= 0 && xy && order && rank && offsets && cols && orig_offsets && pairs, "nl_to_coo: bad arguments");
   if (n == 0) return SPH_OK;
-  k_nl_to_coo<<<grid_for(n, 8), 256, 0, as_stream(stream)>>>(reinterpret_cast<const float2*>(xy), n, order, rank,
-                                                                offsets, cols, orig_offsets, grad_threshold,
-                                                                kernel_support, pairs, num_pairs, dist, radial);
+  const CooRows R{reinterpret_cast<const float2*>(xy), order, rank, offsets, cols, orig_offsets, grad_threshold,
+                  kernel_support, pairs, pairs + num_pairs, dist, radial};
+  cudaStream_t st = as_stream(stream);
+  k_nl_to_coo<<<grid_for(n, 8), 256, 0, st>>>(n, R);
+  if (num_pairs > kLongRow) k_nl_to_coo_long<<<std::min(grid_for(n, 8), kLongRowBlocks), 256, 0, st>>>(n, R);
   SPH_CHECK_LAUNCH("nl_to_coo");
   return SPH_OK;
 }

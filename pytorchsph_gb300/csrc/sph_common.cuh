@@ -195,6 +195,137 @@ __device__ __forceinline__ void copy_rows(const ArraySet& a, int64_t dst, int64_
     if (k >= first && k < a.count) store_rows(a, k, dst, load_rows(a, k, src));
 }
 
+// ---------------------------------------------------------------- bitonic sorts in shared memory
+// One step of a bitonic sort of the p2 shared words s (a power of two) by `threads` threads, of which
+// this is number t: each pair (a, a ^ x), a = the p-th index without the bit `half`, is put in
+// increasing order.  x = 2 half - 1 (the step that begins a merge) or half.  A thread's
+// kPairs pairs are in flight together (kPairs threads >= p2 / 2).
+template <int kPairs, typename W>
+__device__ __forceinline__ void compare_pairs(W* s, int p2, int half, int x, int t, int threads) {
+  int a[kPairs];
+  W lo[kPairs], hi[kPairs];
+#pragma unroll
+  for (int q = 0; q < kPairs; ++q) {
+    const int p = t + q * threads;
+    a[q] = p < p2 / 2 ? 2 * p - (p & (half - 1)) : -1;
+    lo[q] = a[q] >= 0 ? s[a[q]] : 0;
+    hi[q] = a[q] >= 0 ? s[a[q] ^ x] : 0;
+  }
+#pragma unroll
+  for (int q = 0; q < kPairs; ++q)
+    if (lo[q] > hi[q]) {   // (never without a pair)
+      s[a[q]] = hi[q];
+      s[a[q] ^ x] = lo[q];
+    }
+}
+
+// The p2 words in increasing order, by a block (after a barrier; ends with one).
+constexpr int kBlockSortWords = 2048;   // of a block of at least 256 threads: 4 pairs each
+
+template <typename W>
+__device__ __forceinline__ void block_sort(W* s, int p2) {
+  const auto step = [&](int half, int x) {
+    if (p2 <= 2 * (int)blockDim.x)
+      compare_pairs<1>(s, p2, half, x, threadIdx.x, blockDim.x);
+    else if (p2 <= 4 * (int)blockDim.x)
+      compare_pairs<2>(s, p2, half, x, threadIdx.x, blockDim.x);
+    else
+      compare_pairs<4>(s, p2, half, x, threadIdx.x, blockDim.x);
+    __syncthreads();
+  };
+  for (int size = 2; size <= p2; size <<= 1) {
+    step(size >> 1, size - 1);
+    for (int stride = size >> 2; stride > 0; stride >>= 1) step(stride, stride);
+  }
+}
+
+// The columns in[0, len), renumbered by `order` (may be NULL), in increasing order to row[0, len), by
+// a warp with kWarpSortWords shared words s.  Pieces of kWarpSortWords are sorted in s, then
+// merged: steps over longer distances in `row` itself, the others in s again.  A place past the
+// end of the row counts as the largest value and never moves.
+constexpr int kWarpSortWords = 256;   // 4 pairs a lane
+
+static __device__ __noinline__ void warp_sort_row(const int32_t* __restrict__ in, const uint32_t* __restrict__ order,
+                                                  int len, int64_t* row, uint32_t* s) {
+  constexpr int kW = kWarpSortWords;
+  const int lane = threadIdx.x & 31;
+  const auto step = [&](int half, int x) {
+    compare_pairs<kW / 64>(s, kW, half, x, lane, 32);
+    __syncwarp();
+  };
+  for (int base = 0; base < len; base += kW) {
+#pragma unroll
+    for (int q = 0; q < kW; q += 32) {
+      const int t = base + q + lane;
+      const uint32_t c = t < len ? (uint32_t)in[t] : 0u;
+      s[q + lane] = t >= len ? 0xffffffffu : order ? __ldg(order + c) : c;
+    }
+    __syncwarp();
+    for (int size = 2; size <= kW; size <<= 1) {
+      step(size >> 1, size - 1);
+      for (int stride = size >> 2; stride > 0; stride >>= 1) step(stride, stride);
+    }
+    for (int t = lane; t < min(len - base, kW); t += 32) row[base + t] = s[t];
+    __syncwarp();
+  }
+  for (int64_t size = 2 * kW; size / 2 < len; size *= 2) {
+    const int64_t pairs = (len + size - 1) / size * (size / 2);
+    for (int64_t half = size / 2; half >= kW; half /= 2) {
+      const int64_t x = half == size / 2 ? size - 1 : half;
+#pragma unroll 4
+      for (int64_t p = lane; p < pairs; p += 32) {
+        const int64_t a = 2 * p - (p & (half - 1)), b = a ^ x;
+        if (b < len) {
+          const int64_t lo = row[a], hi = row[b];
+          if (lo > hi) {
+            row[a] = hi;
+            row[b] = lo;
+          }
+        }
+      }
+      __syncwarp();
+    }
+    for (int base = 0; base < len; base += kW) {
+#pragma unroll
+      for (int q = 0; q < kW; q += 32) {
+        const int t = base + q + lane;
+        s[q + lane] = t < len ? (uint32_t)row[t] : 0xffffffffu;
+      }
+      __syncwarp();
+      for (int stride = kW / 2; stride > 0; stride >>= 1) step(stride, stride);
+      for (int t = lane; t < min(len - base, kW); t += 32) row[base + t] = s[t];
+      __syncwarp();
+    }
+  }
+}
+
+// Rows past kLongRow columns are sorted by a kernel of their own: counting the smaller columns of each
+// in a warp's registers, which the others do, is quadratic.  65,536 rows of 99 / 139 / 199 / 399
+// columns with their distances take 212 / 348 / 671 / 2,376 us that way and 218 / 239 / 261 / 612
+// sorted, 8,192 rows of 2,048 8.2 and 0.6 ms.  In the counting kernel itself the sort's shared words
+// cost short rows 7 to 10 %; the launch without a long row takes 2.9 us, at 260,017 rows 5.2
+// (5.8 with twice the blocks).
+constexpr int kLongRow = 112;
+constexpr int kLongRowBlocks = 4 * kNumSMs;   // of 256 threads
+
+// use(row, length) by a whole warp for every long row of n; the rows are dealt one to a warp at a
+// time, so that neighboring long rows go to different warps.
+template <typename Length, typename Use>
+__device__ __forceinline__ void for_long_rows(int64_t n, Length&& length, Use&& use) {
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  for (int64_t r0 = warp; r0 < n; r0 += 32 * warps) {
+    const int64_t mine = r0 + lane * warps;
+    const int len = mine < n ? length(mine) : 0;
+    for (unsigned w = __ballot_sync(0xffffffffu, len > kLongRow); w; w &= w - 1) {
+      const int l = __ffs(w) - 1;
+      use(r0 + l * warps, __shfl_sync(0xffffffffu, len, l));
+      __syncwarp();
+    }
+  }
+}
+
 __device__ __forceinline__ void flag(int32_t* status, int32_t f) {
   if (status) atomicOr(status, f);
 }

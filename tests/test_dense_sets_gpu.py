@@ -8,6 +8,7 @@ import pytest
 import torch
 
 import test_cell_fix_gpu as cells
+import test_pair_rows_gpu as rows
 
 pytestmark = pytest.mark.gpu
 
@@ -104,3 +105,34 @@ def test_fill_of_dense_rows_in_time(cuda):
     r.cols.zero_()
     filled = time_us(graph_of(fill))
     assert torch.equal(r.cols, want) and filled < 2 * counted, (filled, counted)
+
+
+@pytest.mark.parametrize("m", [111, 112, 113, 255, 256, 257, 511, 513, 1025, 2040])
+def test_coo_rows(cuda, m):
+    """Rows around the length from which they are sorted, and the sort's pieces of 256."""
+    rows.test_coo_rows_of_length_m(cuda, m)
+
+
+def sorts_of(pairs):
+    """Two stable sorts of a pair list, by column and by row (src/modules/neighborSearch.py:153-157)."""
+    i, j = (t.to(torch.int32) for t in pairs)
+    perm = torch.randperm(len(i), device=i.device)
+    i, j = i[perm], j[perm]
+
+    def f():
+        b, at = torch.sort(j, stable=True)
+        a, at2 = torch.sort(i[at], stable=True)
+        return a, b[at2]
+    return f
+
+
+def test_coo_of_long_rows_in_time(cuda):
+    """8,192 rows of 2,048 columns against two sorts of the same 16.8 M pairs without their distances."""
+    from pytorchsph_gb300.search import GridSearch
+    n = 8192
+    r = GridSearch(cuda).run(clusters(n, 2048), torch.full((n,), 0.1, device=cuda), kernel_support=0.1, density=False)
+    pairs = r.to_coo()[0]
+    key = pairs[0] * n + pairs[1]
+    assert bool((key[1:] > key[:-1]).all()) and len(key) == n * 2048
+    taken, sorts = time_us(lambda: r.to_coo()), time_us(sorts_of(pairs))
+    assert taken < sorts, (taken, sorts)
