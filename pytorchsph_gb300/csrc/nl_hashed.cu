@@ -124,8 +124,9 @@ __global__ void __launch_bounds__(128) k_hashed_query(
 // increasing order, one warp per row.  The rows are in order already, so two sorts of the
 // whole pair list, by column and by row, come down to this.  Up to 32 columns are sorted in the
 // lanes (bitonic, 15 exchanges); of a longer row each column's place is the number of the
-// row's columns below it (equal columns by their place in the row): 24 µs for 65,537 rows of 28,
-// 11.7 with the short rows in the lanes; the two sorts took some 280 with their copies.
+// row's columns below it (equal columns by their place in the row), and rows past kLongRow are left
+// to k_long_pairs_in_order: 24 µs for 65,537 rows of 28, 11.7 with the short rows in the lanes; the
+// two sorts took some 280 with their copies.
 __global__ void __launch_bounds__(256) k_pairs_in_order(int64_t m, const int64_t* __restrict__ offsets,
                                                         const int32_t* __restrict__ in, int64_t* __restrict__ rows,
                                                         int64_t* __restrict__ cols) {
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(256) k_pairs_in_order(int64_t m, const int64_t
   if (b >= m) return;
   const int64_t o = offsets[b];
   const int len = (int)(offsets[b + 1] - o);
+  if (len > kLongRow) return;
   if (len <= 32) {
     int32_t j = lane < len ? __ldg(in + o + lane) : 0x7fffffff;   // columns are below 2^31 - 1
 #pragma unroll
@@ -167,6 +169,18 @@ __global__ void __launch_bounds__(256) k_pairs_in_order(int64_t m, const int64_t
       cols[o + r] = j;
     }
   }
+}
+
+// The rows past kLongRow, a warp each.
+__global__ void __launch_bounds__(256) k_long_pairs_in_order(int64_t m, const int64_t* __restrict__ offsets,
+                                                             const int32_t* __restrict__ in,
+                                                             int64_t* __restrict__ rows, int64_t* __restrict__ cols) {
+  __shared__ uint32_t words[8][kWarpSortWords];
+  for_long_rows(m, [&](int64_t b) { return (int)(offsets[b + 1] - offsets[b]); }, [&](int64_t b, int len) {
+    const int64_t o = offsets[b];
+    warp_sort_row(in + o, nullptr, len, cols + o, words[threadIdx.x >> 5]);
+    for (int t = threadIdx.x & 31; t < len; t += 32) rows[o + t] = b;
+  });
 }
 
 template <bool kFill>
@@ -285,7 +299,10 @@ sph_status_t sph_nl_pairs_in_order(int64_t m, const int64_t* offsets, const int3
                                    int64_t* cols_out, void* stream) {
   SPH_REQUIRE(m >= 0 && (m == 0 || (offsets && cols && rows_out && cols_out)), "nl_pairs_in_order: bad arguments");
   if (m == 0) return SPH_OK;
-  k_pairs_in_order<<<grid_for(m, 8), 256, 0, as_stream(stream)>>>(m, offsets, cols, rows_out, cols_out);
+  cudaStream_t st = as_stream(stream);
+  const int nb = grid_for(m, 8);
+  k_pairs_in_order<<<nb, 256, 0, st>>>(m, offsets, cols, rows_out, cols_out);
+  k_long_pairs_in_order<<<std::min(nb, kLongRowBlocks), 256, 0, st>>>(m, offsets, cols, rows_out, cols_out);
   SPH_CHECK_LAUNCH("nl_pairs_in_order");
   return SPH_OK;
 }

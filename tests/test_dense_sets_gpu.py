@@ -136,3 +136,37 @@ def test_coo_of_long_rows_in_time(cuda):
     assert bool((key[1:] > key[:-1]).all()) and len(key) == n * 2048
     taken, sorts = time_us(lambda: r.to_coo()), time_us(sorts_of(pairs))
     assert taken < sorts, (taken, sorts)
+
+
+@pytest.mark.parametrize("m", [112, 113, 256, 257, 2049, 5000])
+def test_constructed_pairs_of_long_rows(cuda, m):
+    """constructNeighborhoodsCUDA with rows of m columns beside rows of one: (i, j) order and equal to all
+    pairs (the points of a cluster are within a support of each other)."""
+    from pytorchsph_gb300 import neighborhoods
+    rng = np.random.default_rng(m)
+    x = np.concatenate([rng.uniform(0, 0.05, (m, 2)), np.stack([np.arange(40) + 1.0, np.zeros(40)], 1)])
+    perm = rng.permutation(len(x))
+    x, inside = x[perm].astype(np.float32), (np.arange(len(x)) < m)[perm]
+    i, j, *_ = neighborhoods.constructNeighborhoodsCUDA(torch.from_numpy(x).to(cuda),
+                                                        torch.full((len(x),), 0.1, device=cuda))
+    c = np.flatnonzero(inside)
+    one = np.flatnonzero(~inside)
+    rows = np.concatenate([np.repeat(c, m), one])
+    cols = np.concatenate([np.tile(c, m), one])
+    want = np.lexsort((cols, rows))
+    assert np.array_equal(i.cpu().numpy(), rows[want]) and np.array_equal(j.cpu().numpy(), cols[want])
+
+
+def test_constructed_pairs_of_long_rows_in_time(cuda):
+    """8,192 rows of 4,096 columns: the order against two sorts of the 33.6 M pairs."""
+    from pytorchsph_gb300 import _native as N, neighborhoods
+    n, m = 8192, 4096
+    i, j, *_ = neighborhoods.constructNeighborhoodsCUDA(clusters(n, m), torch.full((n,), 0.1, device=cuda))
+    assert len(i) == n * m
+    off = torch.arange(0, n * m + 1, m, device=cuda)
+    cols = j.view(n, m)[:, torch.randperm(m, device=cuda)].to(torch.int32).contiguous()
+    a, b = torch.empty_like(i), torch.empty_like(j)
+    taken = time_us(lambda: N.call("sph_nl_pairs_in_order", n, N.ptr(off), N.ptr(cols), N.ptr(a), N.ptr(b),
+                                   N.stream_ptr()))
+    sorts = time_us(sorts_of((i, j)))
+    assert torch.equal(a, i) and torch.equal(b, j) and taken < sorts, (taken, sorts)
