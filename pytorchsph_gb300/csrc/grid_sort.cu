@@ -602,10 +602,14 @@ __global__ void k_bucket_emit(const int32_t* __restrict__ num_cells, int64_t n, 
 }
 
 // Counting takes one pass over the cells and the buckets where the radix sort takes three to four
-// over all n slots: 65,537 particles with the next prime as length, 17 µs in 8 launches against
-// 65 in 20.  It needs the table not to be much longer than the particles (its scan), and not
-// much shorter: with L >= n / 4 the cells of one bucket, which are compared with each other, stay few
-// (a grid has at most 2^28 cells, of which about one in L falls in a bucket).
+// over all n slots.  Its tables and their scan are as long as the hash table, and the cells of one
+// bucket are compared with each other, so it is kept to n / 4 <= L <= 16 n.  A bucket is longer than
+// cells / L: 3 x + 5 y takes some 8 sqrt(C) values over a square of C occupied cells, so a bucket holds
+// sqrt(C) / 8 of them on average whatever L is, 14 at C = 13,000 and 170 at 1.9 M.  (All cells of a
+// line 3 x + 5 y = constant share one bucket: C^2 comparisons, as many as the queries through
+// that table make.)  The whole call, us, counting / radix: with 9 particles per cell and L = n 65,537
+// particles 88 / 177, 2^20: 112 / 210, 2^24: 534 / 1,083; with one particle per cell 94 / 184, 145 /
+// 237, 1,256 / 1,445; 2^20 with L = n / 4 107 / 202, with 16 n 224 / 251.
 static bool hash_by_counting(int64_t n, int32_t L) { return L >= n / 4 && (int64_t)L <= 16 * n; }
 
 static int key_bits_for(int64_t v) {
