@@ -20,8 +20,8 @@
 //     add one after another in row order: a float32 gradient with respect to alpha is a sum
 //     that cancels to 1/70 of its terms, so its rounding is kept to that of one thread per
 //     row, bit for bit.
-// At 4,173 particles in double the right-hand side takes 26.6 µs (one thread per row: 179) and
-// the adjoint 48.5 (dual numbers: 819); at 16,173 in float 9 (31) and 21 (40).
+// At 3,985 particles in double the right-hand side takes 23 µs (one thread per row: 179) and
+// the adjoint 44 (dual numbers: 819); at 16,173 in float 9.4 (31) and 20 (40).
 #include "sph_common.cuh"
 
 namespace sph {
@@ -770,15 +770,19 @@ __global__ void __launch_bounds__(256) k_order_rows(int n, int room, const int32
 
 using namespace sph;
 
-// Lanes per row: 8 while that gives every SM at most one block, then fewer rows' sums and ends weigh
-// more than the shorter rows.  us with 8 / 4 lanes, right-hand side and adjoint:
-//   double  2,000 particles 18.4 / 26.3, 27.5 / 48.4; 4,173: 31.3 / 26.6, 50.4 / 48.5;
-//           8,000: 59.9 / 45.1, 99 / 91; 16,173: 103 / 85, 171 / 174
-//   float   4,173 particles 7.2 / 10.3, 10.4 / 13.5; 8,000: 7.6 / 10.9, 13.6 / 15.7;
-//           16,173: 9.0 / 11.4, 25.2 / 21.4
+// Lanes per row, 8 while the launch has few blocks per SM, then 4: a row's sums and end are paid once per
+// lane.  The line lies where the two measured the same: in double (bound by the FP64 pipe) at one
+// block per SM, in float at ten for the right-hand side and four for the adjoint.  us with 8 / 4
+// lanes, right-hand side and adjoint:
+//   double   1,917 particles 18.5 / 22.9, 27.5 / 43.9;   2,893: 31.2 / 23.8, 50.3 / 45.0;
+//            5,877: 45.9 / 39.5, 74.7 / 82.2;  8,029: 60.3 / 40.9, 99 / 85;  16,173: 104 / 79, 172 / 165;
+//            65,049: 393 / 264, 655 / 564
+//   float    3,985 particles 7.4 / 10.2, 10.2 / 12.2;  8,029: 8.1 / 10.7, 13.5 / 14.3;
+//            12,093: 8.4 / 11.0, 22.2 / 17.0;  16,173: 9.4 / 11.5, 24.9 / 20.2;  23,709: 12.2 / 12.1,
+//            34.6 / 31.9;  65,049: 27.5 / 24.2, 81 / 67;  130,429: 52 / 43, 166 / 129
 static int drop_lanes(bool fp64, bool adjoint, int64_t n) {
-  if (fp64) return n * 8 <= 128 * kNumSMs ? 8 : 4;
-  return adjoint && n > 12288 ? 4 : 8;
+  const int blocks = fp64 ? 1 : adjoint ? 4 : 10;   // per SM
+  return n * 8 <= (int64_t)blocks * 128 * kNumSMs ? 8 : 4;
 }
 
 template <int kLanes, typename T, typename V2, bool kStep, typename Col>
