@@ -804,6 +804,8 @@ typedef struct sph_dfsph_buffers {
   int32_t* iters;           /* [1] iterations run */
   float* records;           /* [sph_dfsph_records_count()], 16-byte aligned: per-particle pair records of the Jacobi
                                sweeps and, with pairs from the cell rows, neighbor lists */
+  int32_t list_capacity;    /* with pairs from the cell rows: neighbors (fluid and walls) a particle's list has room
+                               for; 0: 48.  A particle with more tests its cell rows in every sweep */
 } sph_dfsph_buffers;
 
 /* The DFSPH calls below take their pairs from the CSR list of the fluid view, or, when the view
@@ -811,8 +813,8 @@ typedef struct sph_dfsph_buffers {
  * particle's neighbor list in bufs->records for the calls of the same step, and sums rho_fluid
  * itself where that is NULL. */
 
-/* Floats of sph_dfsph_buffers.records: 9 n with a CSR list; more with pairs from the cell
- * rows, for the neighbor lists. */
+/* Floats of sph_dfsph_buffers.records: 9 n with a CSR list (cell_rows 0); more with pairs from the
+ * cell rows, for neighbor lists of list_capacity cell_rows (1: list_capacity 0). */
 size_t sph_dfsph_records_count(int64_t n, int64_t nb, int32_t cell_rows);
 
 size_t sph_dfsph_partials_count(void);

@@ -46,15 +46,21 @@ struct DfsphBufs {
   float* fdt;         // dt^2 A_act
   // pairs from the cell rows (kCells kernels): neighbor lists made by the density pass
   int4* list;         // [list_slots(n)] four neighbors each, see fluid_pairs
-  int32_t* chunks;    // of particle i: fluid chunks + 256 x wall chunks, or -1: more than kListChunks in all
-  int4* wlist;        // [kWallChunks nb] the walls' fluid neighbors, four each
-  int32_t* wchunks;   // chunks of wall b, or -1: more than kWallChunks
+  int32_t* chunks;    // of particle i: fluid chunks + 256 x wall chunks, or -1: more than list_chunks in all
+  int4* wlist;        // [wall_chunks nb] the walls' fluid neighbors, four each
+  int32_t* wchunks;   // chunks of wall b, or -1: more than wall_chunks
+  int list_chunks, wall_chunks;   // a particle's and a wall's places for chunks
 };
 
-// Neighbor list chunks (of four) per particle.  A lattice at support 3 dx has 29 neighbors; a
-// fluid packed 1.6 times as densely still fits.
-constexpr int kListChunks = 12;
-constexpr int kWallChunks = 8;    // the first wall layer sees about 14 fluid neighbors
+// Neighbor list chunks (of four) per particle: the caller's list_capacity, which it takes from support and
+// area with headroom.  A particle whose list does not fit tests its cell rows again in every sweep:
+// one right-hand side of 262,144 particles at support 3 / 4 / 5 dx takes 648 / 566 / 796 us with
+// lists that fit and 662 / 1,165 / 1,609 with room for 48 (over CSR rows 960 / 900 / 1,308).
+constexpr int kListChunks = 12;      // list_capacity 0: a lattice at support 3 dx (29) 1.6 times as dense
+constexpr int kMaxListChunks = 255;  // `chunks` holds the fluid's in 8 bits
+
+// A wall's fluid neighbors are less than half a particle's (the first layer sees about 14 at 3 dx).
+static int wall_chunks(int list_chunks) { return (2 * list_chunks + 2) / 3; }
 
 // The fluid pairs of particle i for lane `sub` of its kTpp lanes: use(load(j)) for its share of
 // the neighbor list (kCells) or of the CSR row.  A list is kept in chunks of four neighbors,
@@ -163,13 +169,13 @@ __device__ __forceinline__ void wall_fluid_pairs(int b, const FluidView& F, cons
     wall_candidates(F, g, P, xb, sub, use);
     return;
   }
-  static_assert(kWallChunks == kWallLanes, "one chunk per lane");
-  if (sub >= chunks) return;
-  const int4 j = __ldg(B.wlist + (size_t)b * kWallChunks + sub);
-  if (j.x >= 0) use(j.x);
-  if (j.y >= 0) use(j.y);
-  if (j.z >= 0) use(j.z);
-  if (j.w >= 0) use(j.w);
+  for (int c = sub; c < chunks; c += kWallLanes) {
+    const int4 j = __ldg(B.wlist + (size_t)b * B.wall_chunks + c);
+    if (j.x >= 0) use(j.x);
+    if (j.y >= 0) use(j.y);
+    if (j.z >= 0) use(j.z);
+    if (j.w >= 0) use(j.w);
+  }
 }
 
 // ---------------------------------------------------------------- densities
@@ -180,7 +186,7 @@ struct ListWriter {
   int i, n, shift, k;   // 1 << shift lanes per particle
   int4 four;
   __device__ __forceinline__ void store(int c) {
-    if (c < kListChunks) B.list[(((size_t)(c >> shift) * n + i) << shift) + (c & ((1 << shift) - 1))] = four;
+    if (c < B.list_chunks) B.list[(((size_t)(c >> shift) * n + i) << shift) + (c & ((1 << shift) - 1))] = four;
   }
   __device__ __forceinline__ void add(int j) {
     four = make_int4(four.y, four.z, four.w, j);
@@ -264,7 +270,7 @@ __global__ void __launch_bounds__(128) k_dfsph_fluid_density(FluidView F, WallVi
   if constexpr (kCells) {
     out.fill_up(-1);
     const int all = out.k / 4;
-    B.chunks[i] = all <= kListChunks ? fluid_chunks + 256 * (all - fluid_chunks) : -1;
+    B.chunks[i] = all <= B.list_chunks ? fluid_chunks + 256 * (all - fluid_chunks) : -1;
   }
   const float A = F.area[i];
   const float r = rf + rw;
@@ -301,12 +307,12 @@ __global__ void __launch_bounds__(128) k_dfsph_wall_density(FluidView F, WallVie
     }
     at -= found;
     if (b < W.n) {
-      int32_t* list = reinterpret_cast<int32_t*>(B.wlist + (size_t)b * kWallChunks);
-      if (all <= 4 * kWallChunks) {
+      int32_t* list = reinterpret_cast<int32_t*>(B.wlist + (size_t)b * B.wall_chunks);
+      if (all <= 4 * B.wall_chunks) {
         wall_candidates(F, g, P, xb, sub, [&](int j) { list[at++] = j; });
         for (int k = all + sub; k < (all + 3) / 4 * 4; k += kWallLanes) list[k] = -1;
       }
-      if (sub == 0) B.wchunks[b] = all <= 4 * kWallChunks ? (all + 3) / 4 : -1;
+      if (sub == 0) B.wchunks[b] = all <= 4 * B.wall_chunks ? (all + 3) / 4 : -1;
     }
   }
   if (b >= W.n || sub != 0) return;
@@ -794,11 +800,16 @@ using namespace sph;
 // the error's sum was cut to one warp); 262,144: - / - / 724 / 702.
 static int dfsph_lanes(int64_t n) { return n <= 8192 ? 8 : n <= 32768 ? 4 : n <= 196608 ? 2 : 1; }
 
-// List slots (int4) of n particles: a particle's chunks are dealt to its lanes, so their number is
-// rounded up to the lanes (chunk c < kListChunks lies below (c / lanes + 1) lanes n).
-static size_t list_slots(int64_t n) {
+// Chunks for a list_capacity (0: kListChunks).
+static int list_chunks(int32_t capacity) {
+  return capacity <= 0 ? kListChunks : std::min((capacity + 3) / 4, kMaxListChunks);
+}
+
+// List slots (int4) of n particles with c chunks: a particle's chunks are dealt to its lanes, so their
+// number is rounded up to the lanes (chunk k < c lies below (k / lanes + 1) lanes n).
+static size_t list_slots(int64_t n, int c) {
   const int lanes = dfsph_lanes(n);
-  return (size_t)n * ((kListChunks + lanes - 1) / lanes * lanes);
+  return (size_t)n * ((c + lanes - 1) / lanes * lanes);
 }
 
 // n: the fluid count, which places the pair records (and, with pairs from the cell rows, the
@@ -829,8 +840,10 @@ static DfsphBufs to_bufs(const sph_dfsph_buffers* b, int64_t n, int64_t nb, bool
   B.fdt = B.rec_p ? b->records + 8 * n : nullptr;
   // the lists start 16-byte aligned: 9 n floats rounded up to a multiple of four
   B.list = cells && B.rec_p ? reinterpret_cast<int4*>(b->records + (9 * n + 3) / 4 * 4) : nullptr;
-  B.wlist = B.list ? B.list + list_slots(n) : nullptr;
-  B.chunks = B.list ? reinterpret_cast<int32_t*>(B.wlist + kWallChunks * nb) : nullptr;
+  B.list_chunks = cells ? list_chunks(b->list_capacity) : 0;
+  B.wall_chunks = wall_chunks(B.list_chunks);
+  B.wlist = B.list ? B.list + list_slots(n, B.list_chunks) : nullptr;
+  B.chunks = B.list ? reinterpret_cast<int32_t*>(B.wlist + B.wall_chunks * nb) : nullptr;
   B.wchunks = B.list ? B.chunks + n : nullptr;
   return B;
 }
@@ -865,7 +878,8 @@ extern "C" {
 size_t sph_dfsph_records_count(int64_t n, int64_t nb, int32_t cell_rows) {
   if (n < 0 || nb < 0) return 0;
   if (!cell_rows) return (size_t)n * 9;
-  return (size_t)(9 * n + 3) / 4 * 4 + 4 * list_slots(n) + (size_t)n + (size_t)nb * (4 * kWallChunks + 1);
+  const int c = list_chunks(cell_rows == 1 ? 0 : cell_rows);
+  return (size_t)(9 * n + 3) / 4 * 4 + 4 * list_slots(n, c) + (size_t)n + (size_t)nb * (4 * wall_chunks(c) + 1);
 }
 
 size_t sph_dfsph_partials_count(void) { return (size_t)kNumSMs * 8; }

@@ -53,7 +53,7 @@ class DfsphBuffersC(ctypes.Structure):
     _fields_ = [(k, ctypes.c_void_p) for k in (
         "rho", "volume", "actual_area", "vstar", "alpha", "source", "pressure", "pred_accel", "residual", "wall_rho",
         "wall_actual_area", "wall_alpha", "wall_source", "wall_pressure", "wall_residual", "wall_density_term",
-        "partials", "errors", "iters", "records")]
+        "partials", "errors", "iters", "records")] + [("list_capacity", ctypes.c_int32)]
 
 
 
@@ -98,6 +98,8 @@ class SimConfig:
     pair_headroom: float = 1.3
 
 
+DFSPH_LIST_MAX = 1020   # neighbors of the longest DFSPH list
+
 DIFFUSION = {"none": 0, "MOG": 1, "deltaSPH": 2}
 
 
@@ -106,8 +108,8 @@ class Simulation:
     wall_pos, ghost_pos, wall_area, vmin, vmax), e.g. from pytorchsph_gb300.workloads.
 
     pairs = "cells": the summations take each particle's pairs from its cell rows, tested once a
-    step into segment bit masks.  pairs = "csr": a CSR neighbor list is counted and filled every
-    step first.  Both visit the same pairs."""
+    step into segment bit masks (DFSPH: into neighbor lists).  pairs = "csr": a CSR neighbor list is
+    counted and filled every step first.  Both visit the same pairs."""
 
     def __init__(self, scene: dict, cfg: SimConfig, device=None, pairs: str = "cells"):
         if pairs not in ("cells", "csr"):
@@ -145,6 +147,9 @@ class Simulation:
         # walls, sorted once by their cell in the fluid grid
         self.nb = len(scene.get("wall_pos", ()))
         self._setup_walls(scene)
+        self.list_capacity = self._list_capacity(scene)
+        if cfg.solver == "dfsph" and self.list_capacity > DFSPH_LIST_MAX:
+            self.pairs = "csr"   # rows no list can hold
         self.pair_cap = 0
         self.offsets = self.cols = None
         self.stepped = False     # a right-hand side has run: every buffer has its size
@@ -153,6 +158,13 @@ class Simulation:
         self.graph = None
 
     # ------------------------------------------------------------------ set-up
+    def _list_capacity(self, scene):
+        """Neighbors that a DFSPH list has room for: a support's area over a particle's, 1.6 times as
+        dense (48 at the usual support of three spacings)."""
+        a = float(np.mean(np.asarray(scene["area"], np.float64))) if self.n else 0.0
+        rows = np.pi * self.h * self.h / a if a > 0 else 0.0
+        return max(48, 4 * int(np.ceil(0.4 * min(rows, 1e6))))
+
     def _grid_capacity(self):
         st = N.stream_ptr()
         scratch = self.ws.bytes("grid_scratch", self.lib.sph_grid_scratch_bytes(self.n))
@@ -318,9 +330,10 @@ class Simulation:
              "wall_alpha": g("walpha", nb), "wall_source": g("wsrc", nb), "wall_pressure": g("wp", nb),
              "wall_residual": g("wres", nb), "wall_density_term": self.wall_term,
              "partials": g("partials", int(self.lib.sph_dfsph_partials_count()), torch.float64),
-             "errors": g("errors", maxit), "iters": g("iters", 1, torch.int32), "records": g("records", self.lib.sph_dfsph_records_count(n, self.nb, int(self.pairs == "cells")))}
+             "errors": g("errors", maxit), "iters": g("iters", 1, torch.int32), "records": g("records", self.lib.sph_dfsph_records_count(
+                 n, self.nb, self.list_capacity if self.pairs == "cells" else 0))}
         self.dfsph_arrays = b
-        return DfsphBuffersC(*[N.ptr(b[k]) for k, _ in DfsphBuffersC._fields_])
+        return DfsphBuffersC(*[N.ptr(b[k]) for k, _ in DfsphBuffersC._fields_[:-1]], self.list_capacity)
 
     def _dfsph_rhs(self, acc, st):
         n = self.n
