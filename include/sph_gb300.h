@@ -428,8 +428,8 @@ sph_status_t sph_batch_nl_fill(const float* xy, const float* sorted_support, int
  * which must be every particle's support.
  * The force passes (pass1, diffusion) run over `groups` (a host array of ngroups entries
  * that tile [0, n) in order; a group holds whole scenes when its bounds are scene bounds):
- * `tpp` lanes per particle (each lane takes every 2nd or 4th segment; the lanes' sums are
- * added by warp shuffles, so the summation order, not the pair set, depends on it) and,
+ * `tpp` lanes per particle (each lane takes every 2nd or 4th candidate of a segment; the lanes'
+ * sums are added by warp shuffles, so the summation order, not the pair set, depends on it) and,
  * when all its scenes share one, the diffusion `scheme`, which selects a kernel compiled for
  * it.  ngroups = 0: one group, one lane, any schemes.
  * `phases` selects the launches (SPH_PHASE_ALL for a step; single phases, in order, let a

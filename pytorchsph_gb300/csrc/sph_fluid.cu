@@ -500,12 +500,18 @@ __global__ void __launch_bounds__(256) k_prep(FluidView F, SphParams P, Rec* __r
 }
 
 // Neighbor record and segment list of particle i by kRowLanes lanes, for launches too small to
-// hide one thread's chain of candidate tests: a lane takes a cell row each, at the place that the
-// rows before it leave (a row's segments by its length, empty ones among them, so no lane waits
-// for another's tests).  `live` false: a lane that only takes part.  Records and segments of
-// 8,192 particles 6.1 -> 4.7 us, 16,384: 6.9 -> 5.1, 36,864: 7.0 -> 7.1, 65,536: 7.3 -> 9.6.
+// hide one thread's chain of candidate tests: a lane tests a cell row each, then places its row's
+// non-empty segments behind those of the rows before it, the list that segments_body makes.  It
+// keeps the masks of two segments (rows of up to 64 candidates) and forms later ones again.
+// `live` false: a lane that only takes part.  Records and segments of 8,192 particles
+// 6.1 -> 4.9 us, 16,384: 6.9 -> 5.4, 32,400: 7.0 -> 5.9; 65,536 take 7.3 with one lane, 9.6 with four.
 constexpr int kRowLanes = 4;
 constexpr int kRowLanesMax = 32768;   // particles up to which it is faster
+
+__device__ __noinline__ uint32_t segment_mask_again(const float2* __restrict__ x, int c, int e, float xi, float yi,
+                                                    float thr) {
+  return segment_mask(x, c, e, xi, yi, thr);
+}
 
 __device__ __forceinline__ void prep_rows(int i, bool live, int sub, const FluidView& F, const sph_grid& g, int coff,
                                           const SphParams& P, Rec* __restrict__ rec, int32_t* __restrict__ nseg,
@@ -529,7 +535,15 @@ __device__ __forceinline__ void prep_rows(int i, bool live, int sub, const Fluid
       b = __ldg(row + x0);
       e = __ldg(row + x1 + 1);
     }
-    const int mine = (e - b + 31) >> 5;
+    uint32_t w0 = 0, w1 = 0;   // the row's first two segments
+    int mine = 0;
+    for (int c = b; c < e; c += 32) {
+      const uint32_t w = c + 32 <= F.n ? segment_mask_full(F.x, c, e, xi.x, xi.y, P.thr)
+                                       : segment_mask(F.x, c, e, xi.x, xi.y, P.thr);
+      if (c == b) w0 = w;
+      if (c == b + 32) w1 = w;
+      mine += w != 0;
+    }
     int k = mine, all = mine;
 #pragma unroll
     for (int o = 1; o < kRowLanes; o <<= 1) {
@@ -539,11 +553,15 @@ __device__ __forceinline__ void prep_rows(int i, bool live, int sub, const Fluid
     }
     k += first - mine;
     first += all;
-    for (int c = b; c < e && k < kMaxSegments; c += 32, ++k) {
+    const auto place = [&](int c, uint32_t w) {
+      if (w == 0 || k >= kMaxSegments) return;
       seg_start[k * n + i] = c;
-      seg_mask[k * n + i] = c + 32 <= F.n ? segment_mask_full(F.x, c, e, xi.x, xi.y, P.thr)
-                                          : segment_mask(F.x, c, e, xi.x, xi.y, P.thr);
-    }
+      seg_mask[k * n + i] = w;
+      ++k;
+    };
+    place(b, w0);
+    place(b + 32, w1);
+    for (int c = b + 64; c < e && k < kMaxSegments; c += 32) place(c, segment_mask_again(F.x, c, e, xi.x, xi.y, P.thr));
   }
   if (live && sub == 0) nseg[i] = first <= kMaxSegments ? first : -1;
 }
