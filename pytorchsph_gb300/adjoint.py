@@ -28,6 +28,9 @@ from .search import MAX_CELLS, GridSearch, _f2, grid_from_words
 from .sim import SphParamsC
 
 
+ROW_SLOTS = 1 << 26   # slots of one step's rows (256 MB) up to which a rollout without a record doubles them
+
+
 class DropRollout:
     def __init__(self, scene: dict, c0: float, dt: float, kinematic: float = 0.001, delta: float = 0.1,
                  rest_density: float = 1000.0, gravity=(0.0, 0.0), point_source: bool = True,
@@ -122,10 +125,13 @@ class DropRollout:
         """(final state, checkpoints, record of every step), the steps without host waits.
 
         The rows' slots are sized from the particles' areas with headroom; a step that overflows
-        one has the rollout run again with twice as many.  A float32 rollout's rows are in
-        increasing order, the order its sums are defined in.  A record holds the pairs and the
-        state of every step: the states take a tenth of the pairs' memory, and the backward
-        pass neither searches nor steps again."""
+        one has the rollout run again: with twice as many where half the rows need them (the slots
+        then take at most twice the memory of the reference's int64 lists, usually the same) or
+        one step's are a small buffer, else (particles gathered in places, whose rows would cost
+        every row of every step their length) over lists of exact length with a host wait per
+        step.  A float32 rollout's rows are in increasing order, the order its sums are defined
+        in.  A record holds the pairs and the state of every step: the states take a tenth of the
+        pairs' memory, and the backward pass neither searches nor steps again."""
         self.P.alpha = float(alpha)
         start = (self.x0.clone(), v0.to(self.dtype).reshape(self.n, 2).clone(memory_format=torch.contiguous_format),
                  self.rho0.clone())
@@ -164,14 +170,30 @@ class DropRollout:
             flags = int(status.item())
             if not flags & N.SPH_FLAG_PAIR_CAPACITY:
                 break
-            if cap >= n:
-                raise N.SPHError(f"neighbor search: {N.decode_flags(flags)}")
-            self._row_cap = min(2 * cap, n)
+            long_rows = float((counts == 0).sum(1).max()) / n   # (a row that fits holds its particle)
+            del counts, cols, second, mid, end, at
+            if long_rows < 0.5 and (record or 2 * cap * n > ROW_SLOTS):
+                return self._forward_lists(start, steps, checkpoints, record)
+            self._row_cap = 2 * cap
             status.zero_()
             x32.copy_(self.x0)
         if flags:
             raise N.SPHError(f"neighbor search: {N.decode_flags(flags)}")
         return end, ck, (start, mid, counts, cols, cap) if record else None
+
+    def _forward_lists(self, state, steps, checkpoints, record):
+        """_forward over (i, j)-ordered lists of the rows' exact lengths; the record is a list of
+        every step's (state, (offsets, int32 columns))."""
+        ck, rec = {}, []
+        for k in range(steps):
+            if checkpoints and k % self.every == 0:
+                ck[k] = state
+            off, cols = self.pairs(state[0])
+            pr = (off, cols.to(torch.int32))
+            if record:
+                rec.append((state, pr))
+            state = self._advance(state, pr)
+        return state, ck, rec if record else None
 
     def rollout(self, v0, alpha, steps, checkpoints=False, record_pairs=False):
         """Final positions after `steps` steps from (x0, v0, rho0) and the checkpoints (the states
@@ -236,10 +258,14 @@ class DropRollout:
         st, P, area, da = N.stream_ptr(), ctypes.byref(self.P), N.ptr(self.area), N.ptr(dalpha)
         a, b = [N.ptr(t) for t in cur], [N.ptr(t) for t in nxt]
         for k in reversed(range(steps)):
-            start, mid, counts, cols, cap = record
-            state = [t.data_ptr() + (k - 1) * t.stride(0) * t.element_size() for t in mid] if k else map(N.ptr, start)
-            N.call("sph_drop_adjoint_step", int(self.fp64), self.n, counts.data_ptr() + k * self.n * 4,
-                   cols.data_ptr() + k * self.n * cap * 4, cap, *state, area, P, self.dt, *a, *b, da, st)
+            if isinstance(record, list):
+                state, pr = record[k]
+                pairs, state = (*map(N.ptr, pr), 0), map(N.ptr, state)
+            else:
+                start, mid, counts, cols, cap = record
+                pairs = (counts.data_ptr() + k * self.n * 4, cols.data_ptr() + k * self.n * cap * 4, cap)
+                state = [t.data_ptr() + (k - 1) * t.stride(0) * t.element_size() for t in mid] if k else map(N.ptr, start)
+            N.call("sph_drop_adjoint_step", int(self.fp64), self.n, *pairs, *state, area, P, self.dt, *a, *b, da, st)
             a, b = b, a
             cur, nxt = nxt, cur
         return cur[1], dalpha.sum()
