@@ -720,8 +720,9 @@ class solidBoundaryModule(BoundaryModule):
 
         def find(positions, supports, radius):
             # row offsets come along unless the caller's search has a searchExisting of its own
-            if getattr(ns.searchExisting, '__func__', None) is neighborSearchModule.searchExisting:
-                return ns.searchExistingRows(positions, supports, simulationState, radius)
+            search = ns.searchExisting
+            if getattr(search, '__func__', None) is neighborSearchModule.searchExisting:
+                return search.__self__.searchExistingRows(positions, supports, simulationState, radius)
             return (*ns.searchExisting(positions, supports, simulationState, simulation, searchRadius=radius), None)
 
         *bf, bf_rows = find(self.boundaryPositions, self.boundarySupport, 1)
