@@ -270,11 +270,13 @@ class Simulation:
         n = self.n
         old, extra = self.arr, self.extra
         self.arr = {k: torch.empty_like(t) for k, t in old.items()}
-        order, skeys, cs = self._sort_keys(old["x"], n, "f_", tie=old["uid"],
-                                           rows=[(old[k], self.arr[k]) for k in old])
+        rows = [(old[k], self.arr[k]) for k in old]
+        order, skeys, cs = self._sort_keys(old["x"], n, "f_", tie=old["uid"], rows=rows[:8])
         if extra:
             self.extra = {k: torch.empty_like(t) for k, t in extra.items()}
-            N.permute_arrays(order, [(extra[k], self.extra[k]) for k in extra])
+            rows += [(extra[k], self.extra[k]) for k in extra]
+        for k in range(min(8, len(old)), len(rows), 8):   # the integrator's, and arrays a caller added
+            N.permute_arrays(order, rows[k:k + 8])
         self.skeys, self.cell_start = skeys, cs
         self.stepped = True
         if self.pairs == "cells":

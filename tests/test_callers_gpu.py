@@ -54,3 +54,31 @@ def test_searches_in_place_of_the_module(cuda, wrap):
     got, sim = wall_lists(cuda, wrap)
     assert len(want[0][0]) > 0 and all(torch.equal(a, b) for a, b in zip(want, got))
     assert wrap is Delegate or sim.neighborSearch.calls == 2
+
+
+@pytest.mark.parametrize("more", [1, 3, 4, 12])
+@pytest.mark.parametrize("integration", ["semiImplicitEuler", "RK4"])
+def test_arrays_added_to_a_simulation(cuda, more, integration):
+    """Per-particle arrays of a caller's in sim.arr move with the particles, however many, eagerly and in
+    a captured step."""
+    from pytorchsph_gb300 import workloads
+    from pytorchsph_gb300.sim import SimConfig, Simulation
+    sc = workloads.dam_break(20, 15, 0.01, (0.4, 0.3))
+    sc["vel"] = np.random.default_rng(1).uniform(-2, 2, sc["pos"].shape).astype(np.float32)
+    sim = Simulation(sc, SimConfig(dt=1e-3, c0=10.0, integration=integration, density_diffusion="MOG"), cuda)
+    added = {}
+    for k in range(more):
+        t = torch.arange(sim.n * (1, 2, 4)[k % 3], device=cuda).float().view(sim.n, -1)
+        added[f"tracer{k}"] = t
+        sim.arr[f"tracer{k}"] = t.clone()
+    for _ in range(3):
+        sim.step()
+    sim.capture()
+    for _ in range(3):
+        sim.step()
+    sim.check()
+    uid = sim.arr["uid"].long()
+    assert not torch.equal(uid, torch.arange(sim.n, device=cuda))
+    for k, t in added.items():
+        assert torch.equal(sim.arr[k], t[uid])
+    assert sim.steps == 6 and float(sim.time) == pytest.approx(6e-3)
