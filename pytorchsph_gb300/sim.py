@@ -442,8 +442,6 @@ class Simulation:
             self.extra = {}
         else:
             raise N.SPHError(f"integration scheme {c.integration!r} is not on the GB300 path")
-        if n == 0:
-            self.time += self.dt   # (the integrator's launch adds it)
         if not c.fixed_dt:
             self.last["dt_used"] = self.dt.clone()
             sc = self.ws.bytes("dt_scratch", self.lib.sph_dt_scratch_bytes())
