@@ -217,12 +217,17 @@ def ptr(t) -> int | None:
     return t.data_ptr()
 
 
+# torch's own short way to a stream, where it has one
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def stream_ptr() -> int:
     """The current device's current stream.  torch.cuda.current_stream() also reads the
     environment and builds a Stream object: 6 us of each call that launches 2 us of work."""
-    if not torch.cuda.is_initialized():
+    if _raw_stream is None or _device is None or not torch.cuda.is_initialized():
         return torch.cuda.current_stream().cuda_stream
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return _raw_stream(_device())
 
 
 _host = threading.local()   # each thread's pinned words for read_i32

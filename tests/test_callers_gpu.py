@@ -82,3 +82,15 @@ def test_arrays_added_to_a_simulation(cuda, more, integration):
     for k, t in added.items():
         assert torch.equal(sim.arr[k], t[uid])
     assert sim.steps == 6 and float(sim.time) == pytest.approx(6e-3)
+
+
+@pytest.mark.parametrize("missing", [None, "_raw_stream", "_device"])
+def test_stream_pointer(cuda, missing, monkeypatch):
+    """The current stream, also where torch lacks its private short way."""
+    from pytorchsph_gb300 import _native as N
+    if missing:
+        monkeypatch.setattr(N, missing, None)
+    side = torch.cuda.Stream(cuda)
+    assert N.stream_ptr() == torch.cuda.current_stream().cuda_stream
+    with torch.cuda.stream(side):
+        assert N.stream_ptr() == side.cuda_stream
