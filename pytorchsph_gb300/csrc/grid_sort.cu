@@ -343,7 +343,7 @@ __device__ __forceinline__ void fix_large_cell(int b, int e, const uint32_t* __r
 //     and the memset, at 2^20 20 against 15 + 2, at 3.1 M 82 against 50 + 2.
 // kFixInBlock is the line between them.  A block that has large cells ranks those of up to
 // kRankSortMax entries together and sorts longer ones one by one: 100,000 particles in cells of
-// 100 / 300 / 1,000 / 2,000 take 7 / 13 / 22 / 33 µs (one cell after the other and ranks up to 1,024
+// 100 / 300 / 1,000 / 2,000 take 7 / 12 / 22 / 35 µs (one cell after the other and ranks up to 1,024
 // 10 / 19 / 92 / 58; the launch of their own 10 / 14 / 34 / 36 with the small cells').
 // The sentinel cell (the key cell_capacity: particles outside every grid, or of no scene in
 // a pooled batch) keeps the scatter order: nothing reads its order.
@@ -351,7 +351,7 @@ constexpr int64_t kFixInBlock = 1 << 18;
 constexpr int kFixLarge = kFixThreads / (kSmallCell + 1) + 1;   // large cells that begin in one block
 
 template <bool kInBlock>
-__global__ void __launch_bounds__(kFixThreads) k_cell_fix(const uint32_t* __restrict__ keys, int64_t n,
+__global__ void __launch_bounds__(kFixThreads, kInBlock ? 4 : 8) k_cell_fix(const uint32_t* __restrict__ keys, int64_t n,
                                                           const int32_t* __restrict__ cell_start,
                                                           const uint32_t* __restrict__ tmp,
                                                           const uint32_t* __restrict__ tie,
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(kFixThreads) k_cell_fix(const uint32_t* __rest
 
 static_assert(kFixLarge * kRankSortMax <= kBlockSortMax, "the ranked cells of a block fit its shared words");
 
-__global__ void __launch_bounds__(512) k_cell_fix_large(const int32_t* __restrict__ cell_start,
+__global__ void __launch_bounds__(512, 2) k_cell_fix_large(const int32_t* __restrict__ cell_start,
                                                         const uint32_t* __restrict__ tmp,
                                                         const uint32_t* __restrict__ tie,
                                                         uint32_t* __restrict__ order,

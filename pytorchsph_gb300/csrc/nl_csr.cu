@@ -275,7 +275,7 @@ __device__ __forceinline__ int highest_bit(uint32_t w) {
 
 // Blocks of a fill, at least (or one per four rows): the dense rows of a small set would otherwise be
 // dealt to few warps, 32 rows each.  8,192 particles with rows of 1,024, all dense: 280 µs with the
-// 64 blocks of the rows alone, 22 with these; 8,192 lattice particles 4.4 and 5.1.
+// 64 blocks of the rows alone, 22 with these; 8,192 lattice particles 4.7 and 5.2.
 constexpr int kFillBlocks = 8 * kNumSMs;
 
 constexpr int kRowStage = 1280;   // 40 columns a row: the usual rows in one pass
@@ -296,10 +296,6 @@ __global__ void __launch_bounds__(128) k_nl_fill_segments(int64_t n, const uint3
   int32_t* const stage = stages[threadIdx.x >> 5];
   const sph_grid g = *gp;
   const int nd = __ldg(dense.count);
-  if (s0 >= n) {   // a block for dense rows alone
-    if (nd > 0) fill_dense_rows(dense, keys, g, offsets, pair_capacity, cols, status, nd);
-    return;
-  }
   // this lane's row: first column, end, segments (none for a row that is not written)
   const int lo = offsets[min(s, n)], hi = offsets[min(s + 1, n)];
   int ns = 0;

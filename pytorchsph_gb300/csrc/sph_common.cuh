@@ -199,7 +199,7 @@ __device__ __forceinline__ void copy_rows(const ArraySet& a, int64_t dst, int64_
 // One step of a bitonic sort of the p2 shared words s (a power of two) by `threads` threads, of which
 // this is number t: each pair (a, a ^ x), a = the p-th index without the bit `half`, is put in
 // increasing order.  x = 2 half - 1 (the step that begins a merge) or half.  A thread's
-// kPairs pairs are in flight together (kPairs threads >= p2 / 2).
+// kPairs pairs (p = t, t + threads, ..) are in flight together.
 template <int kPairs, typename W>
 __device__ __forceinline__ void compare_pairs(W* s, int p2, int half, int x, int t, int threads) {
   int a[kPairs];
@@ -220,17 +220,16 @@ __device__ __forceinline__ void compare_pairs(W* s, int p2, int half, int x, int
 }
 
 // The p2 words in increasing order, by a block (after a barrier; ends with one).
-constexpr int kBlockSortWords = 2048;   // of a block of at least 256 threads: 4 pairs each
+constexpr int kBlockSortWords = 2048;   // (more than two pairs of a thread in flight cost a block its registers)
 
 template <typename W>
 __device__ __forceinline__ void block_sort(W* s, int p2) {
   const auto step = [&](int half, int x) {
     if (p2 <= 2 * (int)blockDim.x)
       compare_pairs<1>(s, p2, half, x, threadIdx.x, blockDim.x);
-    else if (p2 <= 4 * (int)blockDim.x)
-      compare_pairs<2>(s, p2, half, x, threadIdx.x, blockDim.x);
     else
-      compare_pairs<4>(s, p2, half, x, threadIdx.x, blockDim.x);
+#pragma unroll 1
+      for (int t = threadIdx.x; t < p2 / 2; t += 2 * blockDim.x) compare_pairs<2>(s, p2, half, x, t, blockDim.x);
     __syncthreads();
   };
   for (int size = 2; size <= p2; size <<= 1) {
