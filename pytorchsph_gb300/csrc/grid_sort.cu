@@ -137,21 +137,42 @@ __device__ sph_grid make_grid(const Bounds& b, int has_min, float min_x, float m
 // Grids of many particle sets at once (one block per set): set s is the particles
 // [seg[s], seg[s+1]) of the concatenated arrays, with its own optional domain
 // min_coords[2s..2s+1] / max_coords[2s..2s+1].  Same arithmetic as sph_grid_build.
-// Bound by the latency of the largest set's loads: 100 sets of 2,048 to 131,072 particles
-// take 17 us with 1,024 threads per set, 25 with 512, 45 with 256; 1,000 sets 76, 92, 143.
-constexpr int kSegmentThreads = 1024;
+// Bound by the latency of the largest set's loads where sets are few, by the blocks' start and end where
+// they are many and small: kThreads threads with kLoads loads each.  us of 100 / 1,000 sets of 2,048
+// to 131,072 particles, 1,000 / 100,000 sets of 10:
+//   1,024 x 4:  16.5 / 76, 10.4 / 601;  512 x 8:  20.6 / 82, 8.2 / 317;  256 x 16:  31 / 105, 6.2 / 149
+template <int kThreads, int kLoads>
+__device__ __forceinline__ Bounds set_bounds(const float2* __restrict__ pos, const float* __restrict__ h,
+                                             int64_t first, int64_t end) {
+  Bounds b = no_bounds();
+  int64_t i = first + threadIdx.x;
+  for (; i + (kLoads - 1) * kThreads < end; i += kLoads * kThreads) {
+    float2 p[kLoads];
+    float hv[kLoads];
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q) {
+      p[q] = __ldg(pos + i + q * kThreads);
+      hv[q] = __ldg(h + i + q * kThreads);
+    }
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q)
+      merge(b, Bounds{hv[q], p[q].x, p[q].y, p[q].x, p[q].y, !isfinite(p[q].x) || !isfinite(p[q].y) || !isfinite(hv[q])});
+  }
+  merge(b, particle_bounds(pos, h, i, kThreads, end));
+  return b;
+}
 
-__global__ void __launch_bounds__(kSegmentThreads) k_grid_segments(const float2* __restrict__ pos,
-                                                               const float* __restrict__ h,
-                                                               const int64_t* __restrict__ seg, int nseg,
-                                                               const float* __restrict__ min_coords,
-                                                               const float* __restrict__ max_coords,
-                                                               int32_t cell_capacity, sph_grid* __restrict__ grids,
-                                                               int32_t* status) {
+template <int kThreads, int kLoads>
+__global__ void __launch_bounds__(kThreads) k_grid_segments(const float2* __restrict__ pos,
+                                                            const float* __restrict__ h,
+                                                            const int64_t* __restrict__ seg, int nseg,
+                                                            const float* __restrict__ min_coords,
+                                                            const float* __restrict__ max_coords,
+                                                            int32_t cell_capacity, sph_grid* __restrict__ grids,
+                                                            int32_t* status) {
   const int s = blockIdx.x;
   if (s >= nseg) return;
-  const Bounds b =
-      block_bounds<kSegmentThreads>(particle_bounds(pos, h, seg[s] + threadIdx.x, kSegmentThreads, seg[s + 1]));
+  const Bounds b = block_bounds<kThreads>(set_bounds<kThreads, kLoads>(pos, h, seg[s], seg[s + 1]));
   if (threadIdx.x != 0) return;
   grids[s] = make_grid(b, min_coords != nullptr, min_coords ? min_coords[2 * s] : 0.f,
                        min_coords ? min_coords[2 * s + 1] : 0.f, max_coords != nullptr,
@@ -676,9 +697,10 @@ sph_status_t sph_grid_build_segments(const float* pos, const float* support, con
                   cell_capacity < 0x7ffffffe,
               "grid_build_segments: bad arguments");
   if (nseg == 0) return SPH_OK;
-  k_grid_segments<<<nseg, kSegmentThreads, 0, as_stream(stream)>>>(reinterpret_cast<const float2*>(pos), support,
-                                                               seg_offsets, nseg, min_coords, max_coords,
-                                                               cell_capacity, grids, status);
+  const auto kernel = nseg <= 256 ? k_grid_segments<1024, 4> : nseg <= 4096 ? k_grid_segments<512, 8> : k_grid_segments<256, 16>;
+  kernel<<<nseg, nseg <= 256 ? 1024 : nseg <= 4096 ? 512 : 256, 0, as_stream(stream)>>>(
+      reinterpret_cast<const float2*>(pos), support, seg_offsets, nseg, min_coords, max_coords, cell_capacity, grids,
+      status);
   SPH_CHECK_LAUNCH("grid_build_segments");
   return SPH_OK;
 }

@@ -170,3 +170,36 @@ def test_constructed_pairs_of_long_rows_in_time(cuda):
                                    N.stream_ptr()))
     sorts = time_us(sorts_of((i, j)))
     assert torch.equal(a, i) and torch.equal(b, j) and taken < sorts, (taken, sorts)
+
+
+def test_grids_of_many_small_sets(cuda):
+    """256, 257, 4,096 and 4,097 sets of 1 to 9,000 particles, among them lengths around a block's loads,
+    against the grid of each set alone (the same words); and 100,000 sets of 10 in time: a
+    block of 256 threads each, 1.5 ns of the whole chip, take 150 us, 220 is held."""
+    from pytorchsph_gb300 import _native as N
+    rng = np.random.default_rng(0)
+    i32 = lambda m: torch.zeros(m, dtype=torch.int32, device=cuda)
+    for sets in (1, 256, 257, 4096, 4097):
+        sizes = rng.integers(1, 40, sets)
+        sizes[:7] = [1, 4096, 4097, 9000, 3841, 8191, 8193][:sets]
+        off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+        pos = torch.rand(int(off[-1]), 2, device=cuda) * 3
+        sup = torch.rand(int(off[-1]), device=cuda) * 0.1 + 0.05
+        grids, one, status = i32(8 * sets), i32(8), i32(1)
+        seg = torch.from_numpy(off).to(cuda)
+        N.call("sph_grid_build_segments", N.ptr(pos), N.ptr(sup), N.ptr(seg), sets, None, None, 1 << 28, N.ptr(grids),
+               N.ptr(status), N.stream_ptr())
+        for k in {0, 1, 2, 3, 4, 5, 6, sets // 2, sets - 1} & set(range(sets)):
+            a, b = int(off[k]), int(off[k + 1])
+            scr = torch.empty(N.load().sph_grid_scratch_bytes(b - a) // 8 + 1, dtype=torch.int64, device=cuda)
+            p, h = pos[a:b].clone(), sup[a:b].clone()
+            N.call("sph_grid_build", N.ptr(p), N.ptr(h), b - a, None, None, 1 << 28, N.ptr(one), N.ptr(status),
+                   N.ptr(scr), scr.numel() * 8, N.stream_ptr())
+            assert torch.equal(one, grids[8 * k:8 * k + 8]), (sets, k)
+        assert int(status.item()) == 0
+    sets = 100000
+    seg = torch.arange(0, 10 * sets + 1, 10, device=cuda)
+    pos, sup, grids = torch.rand(10 * sets, 2, device=cuda), torch.full((10 * sets,), 0.1, device=cuda), i32(8 * sets)
+    taken = time_us(graph_of(lambda: N.call("sph_grid_build_segments", N.ptr(pos), N.ptr(sup), N.ptr(seg), sets, None,
+                                            None, 1 << 28, N.ptr(grids), N.ptr(status), N.stream_ptr())))
+    assert taken < 220, taken
