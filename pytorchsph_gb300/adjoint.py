@@ -7,9 +7,9 @@ viscosity) integrated by semi-implicit Euler (src/simulationBase.py:647-652).  E
 searches neighbors on the GPU (the reference predicate) and advances the state in one launch
 (`sph_drop_search`, `sph_drop_step`); the adjoint (`sph_drop_adjoint_step`) runs the steps
 backwards, over recorded states or (`vjp`) recomputing each checkpoint segment's states
-forward first.  A rollout waits for the device before its first step (the grid) and after its last (the status).  Scalars are
-float64 (default) or float32; the search always sees float32 positions, as the reference's
-does.  `DropRollout.pairs` and `step` work on the reference's own (i, j)-ordered lists.
+forward first.  A rollout waits for the device before its first step (the grid) and after its last (the
+status).  Scalars are float64 (default) or float32; the search always sees float32 positions,
+as the reference's does.  `DropRollout.pairs` and `step` work on the reference's own (i, j)-ordered lists.
 
 Gradients are with respect to the initial velocity field and the artificial viscosity alpha.
 `DropRolloutFunction` puts the rollout behind torch.autograd: its forward records every
@@ -32,6 +32,10 @@ ROW_SLOTS = 1 << 26   # slots of one step's rows (256 MB) up to which a rollout 
 
 
 class DropRollout:
+    """A drop's rollouts and their gradients from one start.  `checkpoint_every` is the spacing of the states
+    that rollout(checkpoints=True) keeps and vjp starts its segments from; loss_and_grad and
+    DropRolloutFunction record every step's state instead."""
+
     def __init__(self, scene: dict, c0: float, dt: float, kinematic: float = 0.001, delta: float = 0.1,
                  rest_density: float = 1000.0, gravity=(0.0, 0.0), point_source: bool = True,
                  point_magnitude: float = 1.0, fp64: bool = True, checkpoint_every: int = 20, device=None,
