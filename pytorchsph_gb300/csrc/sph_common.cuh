@@ -300,26 +300,34 @@ static __device__ __noinline__ void warp_sort_row(const int32_t* __restrict__ in
 
 // Rows past kLongRow columns are sorted by a kernel of their own: counting the smaller columns of each
 // in a warp's registers, which the others do, is quadratic.  65,536 rows of 99 / 139 / 199 / 399
-// columns with their distances take 212 / 348 / 671 / 2,376 us that way and 218 / 239 / 261 / 612
-// sorted, 8,192 rows of 2,048 8.2 and 0.6 ms.  In the counting kernel itself the sort's shared words
-// cost short rows 7 to 10 %; the launch without a long row takes 2.9 us, at 260,017 rows 5.2
-// (5.8 with twice the blocks).
+// columns with their distances take 212 / 348 / 671 / 2,376 us that way and 218 / 244 / 271 / 641
+// sorted, 8,192 rows of 2,048 8.2 and 0.57 ms.  In the counting kernel itself the sort's shared words
+// cost short rows 7 to 10 %; the launch without a long row takes 2.0 us at 65,536 rows, 3.3 at 260,017
+// and 7.2 at 10^6 (2.9, 3.6 and 7.8 with twice the blocks).
 constexpr int kLongRow = 112;
 constexpr int kLongRowBlocks = 4 * kNumSMs;   // of 256 threads
 
-// use(row, length) by a whole warp for every long row of n; the rows are dealt one to a warp at a
-// time, so that neighboring long rows go to different warps.
+// use(row, length) by a whole warp for every long row of n, by blocks of 256 threads: a block looks its
+// share of the rows over, 256 at a time, and deals the long ones to its warps.
 template <typename Length, typename Use>
 __device__ __forceinline__ void for_long_rows(int64_t n, Length&& length, Use&& use) {
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  for (int64_t r0 = warp; r0 < n; r0 += 32 * warps) {
-    const int64_t mine = r0 + lane * warps;
-    const int len = mine < n ? length(mine) : 0;
-    for (unsigned w = __ballot_sync(0xffffffffu, len > kLongRow); w; w &= w - 1) {
-      const int l = __ffs(w) - 1;
-      use(r0 + l * warps, __shfl_sync(0xffffffffu, len, l));
+  __shared__ int at[256], lengths[256], count;
+  const int64_t share = (n + gridDim.x - 1) / gridDim.x;
+  const int64_t end = min((blockIdx.x + 1) * share, n);
+  for (int64_t base = blockIdx.x * share; base < end; base += 256) {   // the same in the whole block
+    const int64_t row = base + threadIdx.x;
+    const int len = row < end ? length(row) : 0;
+    if (!__syncthreads_or(len > kLongRow)) continue;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    if (len > kLongRow) {
+      const int q = atomicAdd(&count, 1);
+      at[q] = threadIdx.x;
+      lengths[q] = len;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x >> 5; q < count; q += 8) {
+      use(base + at[q], lengths[q]);
       __syncwarp();
     }
   }
